@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 
 #include "../../include/crs.h"
+#include "crs_fx_tab.cuh"
 #include "crs_internal.cuh"
 
 namespace crs {
@@ -58,6 +59,15 @@ cudaError_t launch_spec_sum(const unsigned char *img, const ImgLayout &L, const 
 cudaError_t launch_pack_bf16(const double *q, int64_t ldq, int64_t n, int R, int Kh,
                              const int *escale, void *A, int64_t lda, unsigned *outflag,
                              int sm_count, cudaStream_t s);
+// FP64 state tiles in fixed point (crs_fx.cu): scratch bytes of a launch (0:
+// none, < 0: the mechanism does not fit) and the launch.
+namespace fx {
+void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out);
+}
+long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
+                           const unsigned char *tab, const Batch &b, int sm_count,
+                           int smem_optin, double *scratch, cudaStream_t s);
 // Tables the fast kernels derive from the blob's tables at load time.
 bool build_fast_tables(const std::vector<unsigned char> &img,
                        const ImgLayout &L, std::vector<Derived> &extra);
@@ -94,6 +104,8 @@ struct crs_mech {
   int smem_optin = 0;
   crs::ImgLayout L{};
   unsigned char *d_img = nullptr;  // device table image
+  crs::fx::FxTab fx{};             // tables of the FP64 state-tile kernel
+  unsigned char *d_fx = nullptr;   // (fx.usable = 0: not for this mechanism)
   int32_t *d_status = nullptr;     // [0] flags, [1] non-finite count
   // dynamic-scheduling counter pairs of the one-state-per-thread kernels;
   // each launch draws the next slot, so launches in flight at the same time
@@ -637,6 +649,30 @@ int wdot_two_pass(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool fp64) {
   return rc != CRS_OK ? rc : rc2;
 }
 
+// CRS_MODE_FP64 by state tiles in fixed point, when the mechanism fits (and
+// no intermediates are asked for); *taken = false otherwise.  Net rates that
+// do not fit on chip go through the two-pass workspace.
+int wdot_fx(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool *taken) {
+  const long long scratch = crs::fx_scratch(m->fx, b.n, m->sm_count, m->smem_optin);
+  *taken = scratch >= 0 && !(b.conc || b.fwd || b.rev || b.pm);
+  if (!*taken) return CRS_OK;
+  cudaError_t e;
+  if (scratch == 0) {
+    e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin,
+                            nullptr, s);
+    return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
+  }
+  std::lock_guard<std::mutex> lk(m->ws_mu);
+  int rc = ensure_q(m, scratch / (8 * (int64_t)m->L.R), false);
+  if (rc == CRS_OK) rc = ws_begin(m, s);
+  if (rc != CRS_OK) return rc;
+  e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, m->d_q,
+                          s);
+  if (e != cudaSuccess) rc = cuda_fail(e, "crs_wdot launch");
+  const int rc2 = ws_end(m, s);
+  return rc != CRS_OK ? rc : rc2;
+}
+
 // CRS_MODE_GEMM: per chunk, the FP64 net rates (state tiles), their bf16
 // hi + lo rows scaled per state, the terms outside the bf16 window summed
 // in FP64 into wdot, and the contraction GEMM adding the rest.
@@ -689,9 +725,14 @@ int launch_mode(const crs_mech *m, crs::Batch &b, int mode, cudaStream_t s) {
     case CRS_MODE_FP64_STRICT:
       e = crs::launch_wdot_strict(m->d_img, m->L, b, m->sm_count, m->smem_optin, s);
       break;
-    case CRS_MODE_FP64:
-      // one state per thread when its columns fit on chip; else the
-      // two-pass state-tile path (per warp when intermediates are asked for)
+    case CRS_MODE_FP64: {
+      // state tiles in fixed point; for intermediates and mechanisms outside
+      // that scheme one state per thread when its columns fit on chip, else
+      // the two-pass state-tile path (per warp when intermediates are asked
+      // for)
+      bool taken;
+      const int rc = wdot_fx(const_cast<crs_mech *>(m), b, s, &taken);
+      if (taken) return rc;
       e = crs::launch_wdot_fp64_tps(m->d_img, m->L, b, m->sm_count, m->smem_optin, s);
       if (e == cudaErrorNotSupported) {
         if (!(b.conc || b.fwd || b.rev || b.pm) && tile_smem(m->L, true) <= (size_t)m->smem_optin)
@@ -699,6 +740,7 @@ int launch_mode(const crs_mech *m, crs::Batch &b, int mode, cudaStream_t s) {
         e = crs::launch_wdot_fp64(m->d_img, m->L, b, m->sm_count, m->smem_optin, s);
       }
       break;
+    }
     case CRS_MODE_FP64_TILE:
       if (b.conc || b.fwd || b.rev || b.pm)
         return fail(CRS_ERR_UNSUPPORTED, "CRS_MODE_FP64_TILE does not write intermediates");
@@ -771,6 +813,14 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
   if (e == cudaSuccess) e = cudaMalloc(&m->d_img, m->h_img.size());
   if (e == cudaSuccess)
     e = cudaMemcpy(m->d_img, m->h_img.data(), m->h_img.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    std::vector<unsigned char> fxb;
+    crs::fx::build(m->htab, m->fx, fxb);
+    if (m->fx.usable) {
+      e = cudaMalloc(&m->d_fx, fxb.size());
+      if (e == cudaSuccess) e = cudaMemcpy(m->d_fx, fxb.data(), fxb.size(), cudaMemcpyHostToDevice);
+    }
+  }
   if (e == cudaSuccess) e = cudaMalloc(&m->d_status, 4 * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMemset(m->d_status, 0, 4 * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc(&m->d_sched, 2 * SCHED_SLOTS * sizeof(unsigned long long));
@@ -856,6 +906,7 @@ int crs_mech_free(crs_mech *m) {
   if (!m) return CRS_OK;
   unbind(m);
   if (m->d_img) cudaFree(m->d_img);
+  if (m->d_fx) cudaFree(m->d_fx);
   if (m->d_status) cudaFree(m->d_status);
   if (m->d_sched) cudaFree(m->d_sched);
   if (m->d_nuB) cudaFree(m->d_nuB);

@@ -1,0 +1,291 @@
+// 64-bit fixed-point arithmetic of the FP64 state-tile kernel (crs_fx.cu).
+//
+// GB300 retires one FP64 warp instruction per SM sub-partition in ~70
+// clocks and a 32 x 32 -> 64 bit integer multiply-add in a few, so the smooth
+// parts of a rate -- exponents, exponentials, logarithms -- are evaluated as
+// 64-bit integers:
+//   * an exponent is the base-2 logarithm of its value in units of 2^-49
+//     (range +-16384).  A double of magnitude 100 resolves 2^-46, so the
+//     sums here are finer than the FP64 sums they replace;
+//   * bit 0 of every exponent is the sign of its value: adding exponents
+//     multiplies the values, signs included;
+//   * a 64-bit number is split into two signed 32-bit digits, v = hi 2^32 +
+//     lo, and a product keeps hi hi and the two mixed products (three
+//     multiply-adds); the dropped lo lo is at most a quarter of the unit.
+// Values return to FP64 from 57-bit mantissas with one rounding.  Plain
+// integer code: the same functions compile for the host, where the tests
+// compare them with 64-bit floating point.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#if defined(__CUDACC__)
+#include <cuda_runtime.h>
+#define FX_FN __host__ __device__ __forceinline__
+#else
+#define FX_FN inline
+#endif
+
+namespace crs {
+namespace fx {
+
+constexpr int YB = 49;                         // fraction bits of an exponent
+constexpr int64_t ZERO_EXP = -(3500LL << YB);  // exponent of a zero factor
+constexpr int LOGN = 512;                      // logarithm table: F = 1 + j / 512
+// The small tables, in 8-byte words: 2^(j/256) in units of 2^-56, then pairs
+// (1/F in units of 2^-62, log2 F in units of 2^-49).
+constexpr int EXP_ENTRIES = 256;
+constexpr int TAB_BYTES = EXP_ENTRIES * 8 + (LOGN + 1) * 16;
+
+// ---- the machine's integer operations -------------------------------------
+FX_FN int mulhi(int a, int b) {
+#if defined(__CUDA_ARCH__)
+  return __mulhi(a, b);
+#else
+  return (int)(((int64_t)a * b) >> 32);
+#endif
+}
+FX_FN int clz64(int64_t v) {
+#if defined(__CUDA_ARCH__)
+  return __clzll(v);
+#else
+  return v ? __builtin_clzll((unsigned long long)v) : 64;
+#endif
+}
+FX_FN uint64_t bits_of(double v) {
+#if defined(__CUDA_ARCH__)
+  return (uint64_t)__double_as_longlong(v);
+#else
+  uint64_t u;
+  memcpy(&u, &v, 8);
+  return u;
+#endif
+}
+FX_FN double of_bits(uint64_t u) {
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double((long long)u);
+#else
+  double v;
+  memcpy(&v, &u, 8);
+  return v;
+#endif
+}
+// floor(2^61 / d) to 24 bits, 2^30 <= d < 2^31
+FX_FN unsigned recip61(unsigned d) {
+#if defined(__CUDA_ARCH__)
+  return __float2uint_rz(__frcp_rn((float)d) * 2305843009213693952.0f);
+#else
+  return (unsigned)((1.0f / (float)d) * 2305843009213693952.0f);
+#endif
+}
+
+// ---- products ---------------------------------------------------------------
+struct Dg {
+  int hi, lo;
+};
+
+FX_FN Dg split(int64_t v) {
+  const int lo = (int)(unsigned)(uint64_t)v;
+  return Dg{(int)(v >> 32) + (int)((unsigned)lo >> 31), lo};
+}
+
+FX_FN int64_t mad(int a, int b, int64_t c) { return (int64_t)a * b + c; }
+
+// (a b) 2^(S - 64), rounded
+template <int S>
+FX_FN int64_t mul(Dg a, Dg b) {
+  const int64_t hh = mad(a.hi, b.hi, 0);
+  const int64_t mid = mad(a.lo, b.hi, mad(a.hi, b.lo, 1LL << (31 - S)));
+  return (int64_t)((uint64_t)hh << S) + (mid >> (32 - S));
+}
+
+// floor(v 2^lsb) towards zero for |v| < 2^(62 - lsb); infinities and NaN
+// give a meaningless number
+FX_FN int64_t d2fx(double v, int lsb) {
+  const uint64_t u = bits_of(v);
+  const int e = (int)(u >> 52) & 0x7ff;
+  const uint64_t m = (u & 0xfffffffffffffull) | 0x10000000000000ull;
+  int sh = 1023 + 62 - lsb - e;
+  sh = sh < 0 ? 0 : sh > 63 ? 63 : sh;
+  const int64_t r = (int64_t)((m << 10) >> sh);
+  return (int64_t)u < 0 ? -r : r;
+}
+
+// 2^y as M 2^(E - 56), M within 2^-9 of [2^56, 2^57): y split into an integer, an eight-
+// bit table index and |r| <= 2^-9, 2^r = 1 + r (d1 + r (d2 + r (d3 + r d4)))
+// with d_n = (ln 2)^n / n! (truncation below 2^-54).  The sign (bit 0 of y)
+// is dropped.
+FX_FN void exp2m(int64_t y, const int64_t *tab, uint64_t &M, int &E) {
+  const int64_t v = (y & ~1LL) + (1LL << (YB - 9));
+  const int vh = (int)(v >> 32);
+  const unsigned vl = (unsigned)(uint64_t)v;
+  E = vh >> (YB - 32);
+  const int64_t S = tab[(vh >> (YB - 40)) & 255];
+  // r in units of 2^-71: the low 41 bits, centred
+  const int64_t r64 =
+      (int64_t)(((uint64_t)(unsigned)(vh & 511) << 54) | ((uint64_t)vl << 22)) - (1LL << 62);
+  const int rh = (int)(r64 >> 32);  // 2^-39
+  constexpr int D4 = 5043;          // 2^-19
+  constexpr int D3 = 3724818;       // 2^-26
+  constexpr int D2 = 2063529982;    // 2^-33
+  constexpr int64_t D1 = 99893036290645748LL;  // 2^-57
+  const int t = mulhi(rh, D4) + D3;
+  const int g = mulhi(rh, t) + D2;
+  const int64_t h = D1 + (mad(rh, g, 0) >> 15);
+  const int64_t p = mul<0>(split(r64), split(h));  // 2^-64
+  M = (uint64_t)(S + mul<0>(split(S), split(p)));
+}
+
+// log2 of m 2^-63, m in [2^63, 2^64), in units of 2^-49: m = F (1 + u) with F
+// the nearest table point, |u| <= 2^-10, log2(1 + u) = u (c1 + u (c2 + ...))
+// to u^5 (truncation below 2^-62).
+FX_FN int64_t log2m(uint64_t m, const int64_t *ltab) {
+  const unsigned mh = (unsigned)(m >> 32) & 0x7fffffffu;
+  const int j = (int)((mh + (1u << 21)) >> 22);
+  const int64_t d = (int64_t)((m & 0x7fffffffffffffffull) - ((uint64_t)j << 54)) >> 10;  // 2^-53
+#if defined(__CUDA_ARCH__)
+  const longlong2 c = *reinterpret_cast<const longlong2 *>(ltab + 2 * j);
+  const int64_t inv = c.x, lf = c.y;
+#else
+  const int64_t inv = ltab[2 * j], lf = ltab[2 * j + 1];
+#endif
+  const int64_t u = mul<0>(split(d), split(inv));  // 2^-51
+  const int u32 = (int)((u + 512) >> 10);          // 2^-41
+  constexpr int C5 = 5;                            // 2^-4
+  constexpr int C4 = -2955;                        // 2^-13
+  constexpr int C3 = 2017034;                      // 2^-22
+  constexpr int C2 = -1549082005;                  // 2^-31
+  constexpr int64_t C1 = 6653256548922161246LL;    // 2^-62
+  int g = mulhi(u32, C5) + C4;
+  g = mulhi(u32, g) + C3;
+  g = mulhi(u32, g) + C2;
+  const int64_t h = C1 + (mad(u32, g, 0) >> 10);
+  return lf + mul<0>(split(u), split(h));
+}
+
+// An exponent with bit 0 cleared (to the nearest even number), ready for a
+// sign.
+FX_FN int64_t even(int64_t y) { return (y + 1) & ~1LL; }
+
+// log2 |v| of a normal double (bit 0 arbitrary)
+FX_FN int64_t log2d(double v, const int64_t *ltab) {
+  const uint64_t u = bits_of(v);
+  const int e = ((int)(u >> 52) & 0x7ff) - 1023;
+  return (int64_t)e * (1LL << YB) + log2m((u << 11) | 0x8000000000000000ull, ltab);
+}
+
+// log2 of a 2^-lsb, a > 0 (bit 0 arbitrary)
+FX_FN int64_t log2i(int64_t a, int lsb, const int64_t *ltab) {
+  const int lz = clz64(a);
+  return (int64_t)(63 - lz - lsb) * (1LL << YB) + log2m((uint64_t)a << lz, ltab);
+}
+
+// log2 of a normal positive double in units of 2^-58 (|log2| < 16): the
+// temperature's, which Kc polynomials multiply by tens.  hp: 1/F as in
+// ltab, log2 F in units of 2^-62 (pairs).
+FX_FN int64_t log2hp(double v, const int64_t *hp) {
+  const uint64_t u = bits_of(v);
+  const int e = ((int)(u >> 52) & 0x7ff) - 1023;
+  const uint64_t m = (u << 11) | 0x8000000000000000ull;
+  const unsigned mh = (unsigned)(m >> 32) & 0x7fffffffu;
+  const int j = (int)((mh + (1u << 21)) >> 22);
+  const int64_t d = (int64_t)((m & 0x7fffffffffffffffull) - ((uint64_t)j << 54));  // 2^-63
+  const Dg w = split(mul<1>(split(d * 2), split(hp[2 * j])));  // d 2^-64, 1/F 2^-62: 2^-63
+  // log2(1 + w) by its Taylor series to w^7 (truncation below 2^-66)
+  constexpr int64_t C[7] = {6653256548922161246LL, -3326628274461080623LL, 2217752182974053749LL,
+                            -1663314137230540311LL, 1330651309784432249LL, -1108876091487026874LL,
+                            950465221274594464LL};  // 2^-62
+  int64_t h = C[6];
+  for (int n = 5; n >= 0; --n) h = C[n] + mul<1>(w, split(h));
+  h = mul<1>(w, split(h)) + hp[2 * j + 1];  // 2^-62
+  return (int64_t)e * (1LL << 58) + (h >> 4);
+}
+
+// b^2 / (a^2 + b^2) in units of 2^-61 for |a|, |b| < 2^62; ok = false when
+// both are zero.  The quotient of the 64-bit squares from a 24-bit
+// reciprocal R0 of the denominator and two terms of its residual eps,
+// 1 / (1 - eps) = 1 + eps + eps^2 (next term below 2^-66).
+FX_FN int64_t ratio2(int64_t a, int64_t b, bool &ok) {
+  a = a < 0 ? -a : a;
+  b = b < 0 ? -b : b;
+  const int s = clz64((a > b ? a : b) | 1) - 2;
+  const Dg da = split(a << s), db = split(b << s);
+  int64_t B = mul<2>(db, db);
+  B = B < 0 ? 0 : B;
+  int64_t D = mul<2>(da, da) + B;
+  ok = D > 0;
+  const int s2 = clz64(D | 1) - 1;
+  D = (int64_t)((uint64_t)D << s2);
+  B = (int64_t)((uint64_t)B << s2);
+  const unsigned R0 = recip61((unsigned)(D >> 32));
+  const uint64_t one =
+      (D >> 32) * (uint64_t)R0 + (((uint64_t)(unsigned)(uint64_t)D * R0) >> 32);
+  const int eps = (int)((int64_t)((1ull << 61) - one) >> 8);  // 2^-53
+  const uint64_t q0 =
+      (B >> 32) * (uint64_t)R0 + (((uint64_t)(unsigned)(uint64_t)B * R0) >> 32);  // 2^-61
+  const int64_t t1 = mad((int)(q0 >> 31), eps, 0);
+  const int64_t t2 = mad((int)(t1 >> 32), eps, 0);
+  return (int64_t)q0 + (t1 >> 22) + (t2 >> 43);
+}
+
+// +-M 2^(E - 56) as a double, with overflow to infinity and gradual
+// underflow
+FX_FN double assemble(uint64_t M, int E, bool neg) {
+  const double m = (double)(int64_t)M;  // M < 2^57: rounds once
+  return ldexp(neg ? -m : m, E - 56);
+}
+
+// The value of one exponent, whatever its range.
+FX_FN double value_of(int64_t y, const int64_t *tab) {
+  uint64_t M;
+  int E;
+  exp2m(y, tab, M, E);
+  return assemble(M, E, y & 1);
+}
+
+// +-2^yf -+ 2^yr as a double (bit 0 of each exponent: its sign): the aligned
+// difference of the 57-bit mantissas, rounded once.  REV false: the first
+// term alone.  special: the result (or, with overflow, a term) lies outside
+// the normal range and net_special has to form it; the code has no branch.
+template <bool REV>
+FX_FN double net_of(int64_t yf, int64_t yr, const int64_t *tab, bool &special) {
+  uint64_t Mf;
+  int E;
+  exp2m(yf, tab, Mf, E);
+  unsigned neg = (unsigned)yf & 1u;
+  int64_t D = (int64_t)Mf;
+  if (REV) {
+    uint64_t Mr;
+    int Er;
+    exp2m(yr, tab, Mr, Er);
+    const int d = E - Er;
+    int sf = d < 0 ? -d : 0, sr = d > 0 ? d : 0;
+    sf = sf > 63 ? 63 : sf;
+    sr = sr > 63 ? 63 : sr;
+    const int64_t r = (int64_t)(Mr >> sr);
+    D = (int64_t)(Mf >> sf) + ((((unsigned)yr & 1u) != neg) ? r : -r);
+    E = d < 0 ? Er : E;
+    neg ^= D < 0;
+    D = D < 0 ? -D : D;
+  }
+  const int lz = clz64(D | 1);
+  const uint64_t m = (uint64_t)D << lz;
+  const int En = E + 7 - lz;  // value = m 2^(En - 63)
+  const bool zero = D == 0 || En < -1100;
+  special = E > 1023 || (!zero && En < -1022);
+  const uint64_t b = (m >> 11) + ((m >> 10) & 1u) + ((uint64_t)(unsigned)(En + 1022) << 52);
+  return of_bits(zero ? 0ull : b | ((uint64_t)neg << 63));
+}
+
+// net_of for any range: terms that overflow give infinities (and their
+// difference NaN), tiny results underflow gradually.
+template <bool REV>
+FX_FN double net_special(int64_t yf, int64_t yr, const int64_t *tab) {
+  const double f = value_of(yf, tab);
+  return REV ? f - value_of(yr, tab) : f;
+}
+
+}  // namespace fx
+}  // namespace crs
