@@ -331,6 +331,38 @@ __global__ void k_output(int64_t n, const float *Yh, int64_t ldy, int nsp, const
   }
 }
 
+// Rows i0 .. i0 + rows - 1 of the two members' outputs, read whole by the
+// warp (lane = column): returns max_k |y_k,a - y_k,b| of row i0 + lane and,
+// with mean, leaves the members' mean at mean[k * 33 + row].  NaN
+// differences count as zero, as fmaxf drops them.
+__device__ __forceinline__ float rows_of(const float *Ya, const float *Yb, int64_t ldy,
+                                         int64_t i0, int rows, int nsp, int lane, float *mean) {
+  float mine = 0.0f;
+  for (int j0 = 0; j0 < rows; j0 += 4) {
+    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int k = lane; k < nsp; k += 32) {
+      float a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {  // past the last row: that row again
+        const int64_t i = i0 + (j0 + u < rows ? j0 + u : rows - 1);
+        a[u] = __ldcs(Ya + i * ldy + k);
+        b[u] = __ldcs(Yb + i * ldy + k);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        d[u] = fmaxf(d[u], fabsf(a[u] - b[u]));
+        if (mean && j0 + u < rows) mean[k * 33 + j0 + u] = 0.5f * (a[u] + b[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // non-negative floats compare as their bits
+      const float r = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(d[u])));
+      if (lane == j0 + u) mine = r;
+    }
+  }
+  return mine;
+}
+
 // Two-member output with an error gate.  The served y_k is the mean of the
 // members' outputs; in y = sign(u) log1p|u| space a change dy moves w by
 // |dy| (|w| + s) to first order, so an error in y is the reported error
@@ -343,53 +375,71 @@ __global__ void k_output(int64_t n, const float *Yh, int64_t ldy, int nsp, const
 // D as an input, see k_disagreement).  A state
 // goes back to the exact kernel as in k_output, or when g > stol (NaN
 // included).  gate[i] (optional) receives g, for calibrating stol.
-__global__ void k_output2(int64_t n, const float *Ya, const float *Yb, int64_t ldy, int nsp,
-                          const float *sm, const int *se, const float *cons, int nelem,
-                          float tol, float dweight, const float *est, int64_t lde,
-                          float stol, const unsigned char *out_of_box, double *wdot,
-                          int64_t ld, unsigned char *fallback, float *gate) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float sum[MAX_ELEM], mag[MAX_ELEM];
+// Bound by memory: a warp reads its 32 states' rows whole (lane = column; 32
+// lanes reading 32 rows fetch each sector up to eight times) and keeps the
+// means in shared memory, column by state, for the sums over k that follow
+// with lane = state in the order of k.  2^20 states of 53 species
+// took 488 us with a row per thread.
+__global__ void __launch_bounds__(256)
+    k_output2(int64_t n, const float *Ya, const float *Yb, int64_t ldy, int nsp,
+              const float *sm, const int *se, const float *cons, int nelem, float tol,
+              float dweight, const float *est, int64_t lde, float stol,
+              const unsigned char *out_of_box, double *wdot, int64_t ld,
+              unsigned char *fallback, float *gate) {
+  extern __shared__ float mean[];
+  const int lane = threadIdx.x & 31;
+  float *col = mean + (size_t)(threadIdx.x >> 5) * nsp * 33;
+  const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; i0 < n;
+       i0 += nwarp * 32) {
+    const int rows = n - i0 < 32 ? (int)(n - i0) : 32;
+    const float d = rows_of(Ya, Yb, ldy, i0, rows, nsp, lane, col);
+    __syncwarp();
+    const int64_t i = i0 + lane;
+    if (i < n) {
+      float sum[MAX_ELEM], mag[MAX_ELEM];
 #pragma unroll
-    for (int e = 0; e < MAX_ELEM; ++e) sum[e] = mag[e] = 0.0f;
-    float d = 0.0f;
-    for (int k = 0; k < nsp; ++k) {
-      const float ya = Ya[i * ldy + k], yb = Yb[i * ldy + k];
-      d = fmaxf(d, fabsf(ya - yb));
-      const float y = 0.5f * (ya + yb);
-      const float u = copysignf(expm1f(fabsf(y)), y);
-      wdot[(int64_t)k * ld + i] = scale_to_double(u * sm[k], se[k]);
+      for (int e = 0; e < MAX_ELEM; ++e) sum[e] = mag[e] = 0.0f;
+      for (int k = 0; k < nsp; ++k) {
+        const float y = col[k * 33 + lane];
+        const float u = copysignf(expm1f(fabsf(y)), y);
+        wdot[(int64_t)k * ld + i] = scale_to_double(u * sm[k], se[k]);
 #pragma unroll
-      for (int e = 0; e < MAX_ELEM; ++e) {
-        if (e < nelem) {
-          const float c = cons[e * nsp + k];
-          sum[e] = fmaf(c, u, sum[e]);
-          mag[e] = fmaf(c, fabsf(u) + 1.0f, mag[e]);
+        for (int e = 0; e < MAX_ELEM; ++e) {
+          if (e < nelem) {
+            const float c = cons[e * nsp + k];
+            sum[e] = fmaf(c, u, sum[e]);
+            mag[e] = fmaf(c, fabsf(u) + 1.0f, mag[e]);
+          }
         }
       }
-    }
-    float worst = 0.0f;
+      float worst = 0.0f;
 #pragma unroll
-    for (int e = 0; e < MAX_ELEM; ++e)
-      if (e < nelem && mag[e] > 0.0f) worst = fmaxf(worst, fabsf(sum[e]) / mag[e]);
-    const float g = dweight * log10f(d + 1.0e-4f) + (est ? est[i * lde] : 0.0f);
-    const bool fb = !(worst <= tol) || !(g <= stol) || (out_of_box && out_of_box[i]);
-    fallback[i] = fb;
-    if (gate) gate[i] = g;
+      for (int e = 0; e < MAX_ELEM; ++e)
+        if (e < nelem && mag[e] > 0.0f) worst = fmaxf(worst, fabsf(sum[e]) / mag[e]);
+      const float g = dweight * log10f(d + 1.0e-4f) + (est ? est[i * lde] : 0.0f);
+      const bool fb = !(worst <= tol) || !(g <= stol) || (out_of_box && out_of_box[i]);
+      fallback[i] = fb;
+      if (gate) gate[i] = g;
+    }
+    __syncwarp();
   }
 }
 
 // The members' disagreement D = max_k |y_k,a - y_k,b| as an input of the
 // error network: X[i][col] = bf16((log10(D + 1e-4) - mu) / sd).
-__global__ void k_disagreement(int64_t n, const float *Ya, const float *Yb, int64_t ldy,
-                               int nsp, float mu, float sd, __nv_bfloat16 *X, int64_t ldx,
-                               int col) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float d = 0.0f;
-    for (int k = 0; k < nsp; ++k) d = fmaxf(d, fabsf(Ya[i * ldy + k] - Yb[i * ldy + k]));
-    X[i * ldx + col] = __float2bfloat16_rn((log10f(d + 1.0e-4f) - mu) / sd);
+// A warp takes 32 states (see rows_of).
+__global__ void __launch_bounds__(256)
+    k_disagreement(int64_t n, const float *Ya, const float *Yb, int64_t ldy, int nsp, float mu,
+                   float sd, __nv_bfloat16 *X, int64_t ldx, int col) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; i0 < n;
+       i0 += nwarp * 32) {
+    const int rows = n - i0 < 32 ? (int)(n - i0) : 32;
+    const float d = rows_of(Ya, Yb, ldy, i0, rows, nsp, lane, nullptr);
+    if (lane < rows)
+      X[(i0 + lane) * ldx + col] = __float2bfloat16_rn((log10f(d + 1.0e-4f) - mu) / sd);
   }
 }
 
@@ -594,7 +644,15 @@ int crs_surrogate_output2(int64_t n, const float *Ya, const float *Yb, int64_t l
       (est && lde < 1))
     return bad(__func__);
   if (n == 0) return CRS_OK;
-  mlp::k_output2<<<mlp::grid1(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  // as many warps per CTA (up to eight) as their columns of means allow
+  const size_t per_warp = (size_t)nsp * 33 * sizeof(float);
+  int nw = (int)(((size_t)200 << 10) / per_warp);
+  nw = nw > 8 ? 8 : nw;
+  if (nw < 1) return bad(__func__);
+  const cudaError_t e = set_smem_limit(mlp::k_output2, nw * per_warp);
+  if (e != cudaSuccess) return done(e, __func__);
+  mlp::k_output2<<<mlp::grid1(n, nw * 32), nw * 32, nw * per_warp,
+                   static_cast<cudaStream_t>(stream)>>>(
       n, Ya, Yb, ldy, nsp, scale_m, scale_e, cons, nelem, tol, dweight, est, lde, stol,
       out_of_box, wdot, ld, fallback, gate);
   return done(cudaGetLastError(), __func__);

@@ -6,18 +6,19 @@
 // here a CTA keeps its 128 x width activation tile on chip between layers,
 // so per state only the input features are read and the output written.
 //
-// One CTA = 128 states, 6 warps:
-//   warp 4 / lane 0  TMA producer: the tile's input features into the
+// One CTA = 128 states, 10 warps:
+//   warp 8 / lane 0  TMA producer: the tile's input features into the
 //                    activation buffer, then every layer's weights in
 //                    blocks of <= 128 rows x 64 columns through a two-slot
 //                    ring (the weights do not depend on the activations, so
 //                    the next layer's first blocks load during an epilogue);
-//   warp 5 / lane 0  MMA issuer: per layer, per 64-wide K block and per
+//   warp 9 / lane 0  MMA issuer: per layer, per 64-wide K block and per
 //                    128-column half of the layer's outputs, four
 //                    tcgen05.mma (K = 16) into the FP32 accumulator in TMEM
 //                    (columns 0..255), then tcgen05.commit;
-//   warps 0-3        epilogue: tcgen05.ld of their 32 accumulator lanes,
-//                    + bias, SiLU, bf16, written back into the activation
+//   warps 0-7        epilogue: tcgen05.ld of the 32 accumulator lanes of
+//                    their rank modulo 4, warps 0-3 the first half of the
+//                    columns and 4-7 the second, + bias, SiLU, bf16, written back into the activation
 //                    buffer in the 128-byte-swizzled K-major layout that the
 //                    next layer's MMAs read (the layout TMA writes), or, for
 //                    the last layer, + bias to the fp32 output in HBM.
@@ -45,7 +46,10 @@ constexpr int MAXL = 6;           // layers
 constexpr int MAXW = 256;         // widest layer input / output (padded)
 constexpr int BLK = 128 * 64 * 2;  // one 128-row x 64-column bf16 block: 16 KB
 constexpr int RING = 2;
-constexpr int NT = 192;
+// Epilogue warps: the epilogue (two MUFU operations per activation) bounds the
+// kernel; eight warps instead of four keep more of them in flight
+constexpr int EW = 8;
+constexpr int NT = (EW + 2) * 32;
 
 struct Maps {
   CUtensorMap x;
@@ -68,8 +72,15 @@ __device__ __forceinline__ uint32_t idesc_n(int n) {
          ((uint32_t)(128 >> 4) << 24);
 }
 
+// z / (1 + e^-z), the value of z * __fdividef(1, 1 + __expf(-z)) without the
+// scaling of subnormal operands around its two approximations: e^-z below
+// 2^-126 adds nothing to 1, and where 1 + e^-z exceeds 2^126 both forms give
+// zero.  Five instructions instead of twelve.
 __device__ __forceinline__ float silu(float z) {
-  return z * __fdividef(1.0f, 1.0f + __expf(-z));
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return z * r;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -133,7 +144,7 @@ __global__ void __launch_bounds__(NT, 2)
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&xfull)));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mdone)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(smem_u32(&aready)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(smem_u32(&aready)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     failed = 0;
     consumed = 0;
@@ -141,7 +152,7 @@ __global__ void __launch_bounds__(NT, 2)
   for (int l = 0; l < L; ++l)
     for (int i = threadIdx.x; i < net.pad[l + 1]; i += NT)
       sbias[l * MAXW + i] = i < net.dim[l + 1] ? net.bias[l][i] : 0.0f;
-  if (warp == 4) {
+  if (warp == EW) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&tmem_slot)),
                  "r"(256u)
@@ -154,7 +165,7 @@ __global__ void __launch_bounds__(NT, 2)
   const uint32_t tmem = tmem_slot;
   int issued = 0;
 
-  if (warp == 4 && lane == 0) {
+  if (warp == EW && lane == 0) {
     // ---- TMA producer ----
     const int kx = net.pad[0] / 64;
     gemm::expect_tx(&xfull, (uint32_t)(kx * BLK));
@@ -175,7 +186,7 @@ __global__ void __launch_bounds__(NT, 2)
           ++issued;
         }
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == EW + 1 && lane == 0) {
     // ---- MMA issuer ----
     int i = 0;
     if (!gemm::wait_bounded(&xfull, 0)) failed = 1;
@@ -207,9 +218,10 @@ __global__ void __launch_bounds__(NT, 2)
         }
       if (!failed) gemm::commit(&mdone);  // arrives when this layer's MMAs are done
     }
-  } else if (warp < 4) {
+  } else if (warp < EW) {
     // ---- epilogue ----
-    const int row = warp * 32 + lane;  // the TMEM lane quarter of warp 0..3
+    const int quarter = warp & 3;  // the TMEM lanes a warp of this rank may read
+    const int row = quarter * 32 + lane;
     for (int l = 0; l < L; ++l) {
       if (!gemm::wait_bounded(&mdone, (uint32_t)l & 1u)) {
         failed = 1;
@@ -262,19 +274,15 @@ __global__ void __launch_bounds__(NT, 2)
           }
         }
       };
-      // two 32-column buffers: the TMEM load of the next columns is in
-      // flight while the current ones are processed
-      const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
-      uint32_t va[32], vb[32];
-      ld32_nw(ta, va);
-      wait_ld(va);
-      for (int c = 0; c < nn; c += 64) {  // nn is a multiple of 64
-        ld32_nw(ta + (uint32_t)(c + 32), vb);
-        process(va, c);
-        wait_ld(vb);
-        if (c + 64 < nn) ld32_nw(ta + (uint32_t)(c + 64), va);
-        process(vb, c + 32);
-        wait_ld(va);
+      const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16);
+      // this warp's half of the columns: nn is a multiple of 64, so a whole
+      // number of 32-column groups.  One group in registers: the other warps
+      // work while its TMEM load is in flight
+      uint32_t v[32];
+      for (int c = warp < 4 ? 0 : nn / 2; c < (warp < 4 ? nn / 2 : nn); c += 32) {
+        ld32_nw(ta + (uint32_t)c, v);
+        wait_ld(v);
+        process(v, c);
       }
       if (!last) {
         // generic-proxy stores -> visible to the tensor core's async proxy
@@ -287,14 +295,14 @@ __global__ void __launch_bounds__(NT, 2)
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 4 && lane == 0) {
+  if (warp == EW && lane == 0) {
     // a failed CTA still waits for the weight blocks it had requested
     for (int j = consumed; j < issued; ++j)
       gemm::wait_bounded(&full[j % RING], (uint32_t)(j / RING) & 1u);
     if (consumed == 0) gemm::wait_bounded(&xfull, 0);
     if (failed && net.status) atomicOr(&net.status[0], STATUS_GEMM_TIMEOUT);
   }
-  if (warp == 4) {
+  if (warp == EW) {
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u)
