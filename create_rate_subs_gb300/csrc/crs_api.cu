@@ -663,7 +663,7 @@ int wdot_fx(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool *taken) {
     return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
   }
   std::lock_guard<std::mutex> lk(m->ws_mu);
-  int rc = ensure_q(m, scratch / (8 * (int64_t)m->L.R), false);
+  int rc = ensure_q(m, scratch / (8 * (int64_t)m->L.R) + 1, false);
   if (rc == CRS_OK) rc = ws_begin(m, s);
   if (rc != CRS_OK) return rc;
   e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, m->d_q,

@@ -3,37 +3,46 @@
 // What bounds it.  The FP64 pipe retires one warp instruction per SM sub-
 // partition in ~70 clocks, so 15,000 FP64 instructions per state (53
 // species / 325 reactions) held the one-state-per-thread kernel at 33.6 M
-// states/s, 95% of that pipe.  Of the arithmetic here only the sums keep
-// FP64: the mass-fraction sums in the reference's order and one
-// multiply-add per nonzero net stoichiometric coefficient.  Everything
-// multiplicative -- rate constants, equilibrium constants, concentrations,
-// third bodies, fall-off -- is an exponent in 64-bit fixed point
+// states/s, 95% of that pipe.  Of the arithmetic here FP64 keeps the sums:
+// the mass fractions in the reference's order, third bodies, forward minus
+// reverse, and one addition per net stoichiometric coefficient, ~2,000 in
+// all.  Everything multiplicative -- rate constants, equilibrium constants,
+// concentrations, fall-off -- is an exponent in 64-bit fixed point
 // (crs_fx.cuh): a product of factors is a sum of integers, a rate constant
 // a dot product of a reaction's coefficients with functions of T that are
 // formed once per state, and each rate one table exponential.
 //
-// A reaction's exponents.  On a temperature interval (bounded by the
-// mechanism's T_common values and the limits TLO, THI) with centre and
-// half width of log2 T, 1/T and T, the functions L, I, t, t^2, t^3, t^4 are
-// normalised to [-1, 1] and every exponent is c0 + cL L + cI I + c1 t + ...
-// + c4 t^4: three coefficients forward; the reverse rate's exponent, forward
-// minus ln Kc with the Gibbs polynomials of all its species, has seven.
-// Coefficients are rounded to 2^-52, the functions to 2^-61.
+// A reaction's exponents.  On a temperature interval (bounded by 200 K, the
+// mechanism's common T_common and 6000 K) with centre and half width of
+// log2 T, 1/T and T, the functions L, I, t, t^2, t^3, t^4 are normalised to
+// [-1, 1] and every exponent is c0 + cL L + cI I + c1 t + ... + c4 t^4: three
+// coefficients forward; the reverse rate's exponent, forward minus ln Kc
+// with the Gibbs polynomials of all its species, has seven.  Coefficients
+// are rounded to 2^-52, the functions to 2^-61.
 //
 // A tile: lane = state; the CTA's NW warps share the tile's exponents of
 // the concentrations ([N][32], 8 bytes each) and split first the species,
 // then the reactions (lists balanced at load by instruction counts), then
 // the species sums.  The net rates pass between the last two in shared
-// memory ([R][32]) or, when they do not fit, in global scratch of one tile
-// per CTA, which stays in L2.  Table reads are uniform across a warp up to
-// the temperature interval and go through L1.
+// memory or in scratch of one tile per CTA, which stays in L2: without them
+// on chip three CTAs share an SM, so that one's sums (FP64 pipe) overlap
+// another's rates (integer pipes).  A warp's reaction records stream through
+// its own ring of three slots in shared memory, two plain reversible
+// reactions at a time, so that their two chains interleave; the next tile's
+// mass-fraction sums, two chains of N dependent FP64 additions, run on
+// two warps beside the rates.
 //
-// States outside the scheme (T outside (TLO, THI], a non-positive or non-
-// finite density, |Y| >= 2, a subnormal Y) and reactions outside it (non-
+// Measured on GB300: 2^20 states of 53/325 in 7.2 ms (31.2 with the one-
+// state-per-thread kernel), FP64 pipe 53%, integer multiply pipe 43% busy.
+//
+// States outside the scheme (T outside (200, 6000] K, a density or mean
+// 1/W out of range, |Y| >= 2, a subnormal Y) and reactions outside it (non-
 // integer coefficients, PLOG, Chebyshev, coefficients beyond the bounds)
-// are evaluated lane by lane by the general FP64 arithmetic (slow_net).
+// are evaluated lane by lane by the general FP64 arithmetic (finish).
 #include <cuda_runtime.h>
 #include <math.h>
+
+#include <algorithm>
 
 #include "crs_fast.cuh"
 #include "crs_fx.cuh"
@@ -56,8 +65,9 @@ constexpr int64_t K014 = 645636042579834307LL;    // 0.14
 struct Basis {
   Dg L, I, t1, t2, t3, t4;
 };
-// rows of the per-tile block: the six functions, log2 rho, the mean 1/W,
-// y_N, rho, and the interval and the outside-the-scheme mark
+// Rows of a tile's block of per-state values: the six functions, log2 rho,
+// y_N, rho, sum Y / W, and two marks: the interval (-1: T outside the scheme)
+// and whether the state's sums or fractions are outside it.
 constexpr int ROWS = 11;
 
 __device__ __forceinline__ Dg dg(int2 v) { return Dg{v.x, v.y}; }
@@ -66,20 +76,23 @@ __device__ __forceinline__ int64_t word(int hi, int lo) {
 }
 __device__ __forceinline__ int64_t word(int2 v) { return word(v.x, v.y); }
 
+// c0 + sum of coefficient x function; c0 carries the 1 that rounds to even
 struct Dot {
   int64_t hh, mid;
   __device__ __forceinline__ explicit Dot(int64_t c0) : hh(c0), mid(1LL << 31) {}
   __device__ __forceinline__ void add(Dg c, Dg f) {
-    hh = mad(c.hi, f.hi, hh);
-    mid = mad(c.lo, f.hi, mad(c.hi, f.lo, mid));
+    // (long sums of products fuse from the C expression: 33 instructions for
+    // six functions against 48 with the instruction spelt out)
+    hh += (int64_t)c.hi * f.hi;
+    mid += (int64_t)c.hi * f.lo;
+    mid += (int64_t)c.lo * f.hi;
   }
-  __device__ __forceinline__ int64_t exponent() const { return even(hh + (mid >> 32)); }
+  __device__ __forceinline__ int64_t exponent() const { return (hh + (mid >> 32)) & ~1LL; }
 };
 
 // log2 of a fall-off factor from lth = log2 [M] (c: its record on the lane's
-// interval).  slow: outside the scheme (negative or tiny terms); the caller
-// evaluates the reaction in FP64.
-__device__ __noinline__ int64_t falloff(const int2 *__restrict__ c, int flags, int64_t lth,
+// interval).  slow: outside the scheme (negative or tiny terms).
+__device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags, int64_t lth,
                                         Dg L, Dg I, Dg t, const int64_t *et, const int64_t *lt,
                                         bool &slow) {
   Dot d(word(c[0]));
@@ -141,31 +154,9 @@ struct YConc {
   }
 };
 
-// The net rate of reaction r by the general FP64 arithmetic.
-__device__ __noinline__ double slow_net(const unsigned char *img, const ImgLayout &lay, int r,
-                                        double T, double P, const double *Y, int64_t ld,
-                                        double rho, double yN) {
-  const Tab t = make_tab(img, lay);
-  fast::State s;
-  s.T = T;
-  s.P = P;
-  s.invT = 1.0 / T;
-  s.logT = fast::log_t(T, t.logtab);
-  s.tab = t.exptab;
-  s.ltab = t.logtab;
-  KcPolyG kc;
-  kc.T = T;
-  kc.logT = s.logT;
-  kc.invT = s.invT;
-  double fwd, rev, pm;
-  return fast::rxn_net(t, r, s, P * s.invT * fast::INV_RU, YConc{Y, ld, rho, yN, t.inv_mw, t.N},
-                       kc, fwd, rev, pm);
-}
-
-template <bool REV>
-__device__ __noinline__ double net_far(int64_t yf, int64_t yr, const int64_t *tab) {
-  return net_special<REV>(yf, yr, tab);
-}
+// Stands in a rate's place until the general FP64 arithmetic has formed it:
+// the loops that form the others then hold no call.
+constexpr uint64_t LATER = 0x7ff8c5a1d3b70e29ull;
 
 // The normalised functions of T of one state into column `lane` of the
 // block; returns the temperature interval.  irr: T outside the scheme.
@@ -173,9 +164,7 @@ __device__ __forceinline__ int basis_of(const FxTab &f, const unsigned char *tab
                                         int64_t *blk, bool &irr) {
   irr = !(T > f.tb[0] && T <= f.tb[NI]);
   const double Tc = irr ? 1000.0 : T;
-  int iv = 0;
-#pragma unroll
-  for (int q = 1; q < NI; ++q) iv += Tc > f.tb[q];
+  const int iv = Tc > f.tb[1];
   const int64_t *w = reinterpret_cast<const int64_t *>(tab + f.basis) + BASIS * iv;
   const int64_t *hp = reinterpret_cast<const int64_t *>(tab + f.hp);
   const Dg L = split(mul<2>(split((log2hp(Tc, hp) - w[3]) << w[5]), split(w[4])));
@@ -198,284 +187,463 @@ __device__ __forceinline__ int basis_of(const FxTab &f, const unsigned char *tab
 }
 
 struct Args {
-  const unsigned char *img;  // table image (general FP64 arithmetic, sums)
   const unsigned char *tab;  // fixed-point tables
+  const unsigned char *img;  // table image (general FP64 arithmetic)
   double *q;                 // [gridDim.x][R][32] scratch when QS is false
 };
 
-// U plain reversible reactions at once: exponents, rates, net rates into q.
-template <int U>
-__device__ __forceinline__ void plain_block(const FxTab &f, const unsigned char *tab,
-                                            const int *list, const int64_t *yl, const Basis &B,
-                                            int iv, double T, const int64_t *et,
-                                            double *q) {
-  int64_t yf[U], yr[U];
-  int r[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    r[u] = list[u];
-    const int4 h0 = __ldg(reinterpret_cast<const int4 *>(tab + f.hdr) + 2 * r[u]);
-    const int4 h1 = __ldg(reinterpret_cast<const int4 *>(tab + f.hdr) + 2 * r[u] + 1);
-    int idx = iv;
-    if (!f.uniform) {
-      const int32_t *tp = reinterpret_cast<const int32_t *>(tab + f.thr_ptr);
-      idx = 0;
-      for (int e = tp[r[u]]; e < tp[r[u] + 1]; ++e)
-        idx += T > reinterpret_cast<const double *>(tab + f.thr)[e];
+// A reaction's record in shared memory: its head and the coefficients of
+// the lane's interval.
+struct Rec {
+  const unsigned char *p, *c;
+  __device__ __forceinline__ int4 word4(int o) const {
+    return *reinterpret_cast<const int4 *>(p + o);
+  }
+  __device__ __forceinline__ int4 coef(int u) const {
+    return reinterpret_cast<const int4 *>(c)[u];
+  }
+};
+
+// Copies of a warp's next records into its ring of D slots.
+template <int D>
+struct Ring {
+  const unsigned char *src;
+  unsigned base;
+  int stride, n, lane;
+  // record p (an empty group past the last one)
+  __device__ __forceinline__ void fill(int p) const {
+    if (p < n) {
+      const unsigned char *from = src + (int64_t)p * stride;
+      const unsigned to = base + (unsigned)((p % D) * stride);
+      for (int o = lane * 16; o < stride; o += 512)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + o), "l"(from + o)
+                     : "memory");
     }
-    const int4 *c = reinterpret_cast<const int4 *>(tab + f.coef) + 5 * (h0.z + idx);
-    const int4 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2), c3 = __ldg(c + 3),
-               c4 = __ldg(c + 4);
-    Dot a(word(c0.x, c0.y));
-    a.add(Dg{c0.z, c0.w}, B.L);
-    a.add(Dg{c1.x, c1.y}, B.I);
-    Dot b(word(c1.z, c1.w));
-    b.add(Dg{c2.x, c2.y}, B.L);
-    b.add(Dg{c2.z, c2.w}, B.I);
-    b.add(Dg{c3.x, c3.y}, B.t1);
-    b.add(Dg{c3.z, c3.w}, B.t2);
-    b.add(Dg{c4.x, c4.y}, B.t3);
-    b.add(Dg{c4.z, c4.w}, B.t4);
-    const int neg = (h0.y & RF_NEG) ? 1 : 0;
-    int64_t sf = yl[(h1.x & 0xffff) * 32] + yl[((unsigned)h1.x >> 16) * 32];
-    int64_t sr = yl[(h1.z & 0xffff) * 32] + yl[((unsigned)h1.z >> 16) * 32];
-    if (h0.y & RF_MORE_R) sf += yl[(h1.y & 0xffff) * 32] + yl[((unsigned)h1.y >> 16) * 32];
-    if (h0.y & RF_MORE_P) sr += yl[(h1.w & 0xffff) * 32] + yl[((unsigned)h1.w >> 16) * 32];
-    yf[u] = a.exponent() + neg + sf;
-    yr[u] = b.exponent() + neg + sr;
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  double v[U];
-  bool sp[U], any = false;
+  __device__ __forceinline__ void start() const {
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    v[u] = net_of<true>(yf[u], yr[u], et, sp[u]);
-    any |= sp[u];
+    for (int p = 0; p < D - 1; ++p) fill(p);
   }
-  if (any) {
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (sp[u]) v[u] = net_far<true>(yf[u], yr[u], et);
+  // Record p is on chip for the whole warp; the copy of record p + D - 1
+  // starts (its slot's reader, record p - 1, is done).
+  __device__ __forceinline__ void next(int p) const {
+    __syncwarp();
+    fill(p + D - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+    __syncwarp();
   }
-#pragma unroll
-  for (int u = 0; u < U; ++u) q[(int64_t)r[u] * 32] = v[u];
+};
+constexpr int DP = 3, DO = 3;  // slots for pairs of plain records and for other records
+
+__host__ __device__ inline int ring_bytes(const FxTab &f) {
+  return f.stride[0] * DP > f.stride[1] * DO ? f.stride[0] * DP : f.stride[1] * DO;
 }
 
-template <int LIST, bool QS, bool TS>
-__global__ void __launch_bounds__(warps_of(LIST) * 32, 16 / warps_of(LIST))
-    k_wdot_tile(const __grid_constant__ ImgLayout lay, const __grid_constant__ FxTab f, Args g,
-                Batch b) {
+// log2 v, bit 0 its sign; zero: ZERO_EXP
+__device__ __forceinline__ int64_t log2s(double v, const int64_t *lt) {
+  const int64_t l = even(log2d(v, lt)) | (int64_t)(bits_of(v) >> 63);
+  return v == 0.0 ? ZERO_EXP : l;
+}
+
+// Exponents of the forward and the reverse rate constant.
+__device__ __forceinline__ int64_t exponent3(const Rec &r, const Basis &B) {
+  const int4 c0 = r.coef(0);
+  const int2 c1 = reinterpret_cast<const int2 *>(r.c)[2];
+  Dot a(word(c0.x, c0.y));
+  a.add(Dg{c0.z, c0.w}, B.L);
+  a.add(dg(c1), B.I);
+  return a.exponent();
+}
+__device__ __forceinline__ int64_t exponent7(const Rec &r, const Basis &B) {
+  const int2 c0 = reinterpret_cast<const int2 *>(r.c)[3];
+  const int4 c1 = r.coef(2), c2 = r.coef(3), c3 = r.coef(4);
+  Dot d(word(c0));
+  d.add(Dg{c1.x, c1.y}, B.L);
+  d.add(Dg{c1.z, c1.w}, B.I);
+  d.add(Dg{c2.x, c2.y}, B.t1);
+  d.add(Dg{c2.z, c2.w}, B.t2);
+  d.add(Dg{c3.x, c3.y}, B.t3);
+  d.add(Dg{c3.z, c3.w}, B.t4);
+  return d.exponent();
+}
+
+// Loads of one tile's mass fractions (rows of this warp) straight into
+// shared memory; row N - 1 is y_N.
+template <int NW>
+__device__ __forceinline__ void load_y(const double *Y, int64_t ld, int N, int warp,
+                                       unsigned smem_rows) {
+  for (int k = warp; k < N - 1; k += NW)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_rows + k * 256),
+                 "l"(Y + (int64_t)k * ld)
+                 : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// y_N = 1 - sum y in the reference's order (rate_subs.py:1312-1320) on warp
+// 0, sum y / W and the density on warp 1: two dependent FP64 chains side by
+// side.  Rows 6.. of the block: log2 rho, y_N, rho, sum y / W.
+__device__ __forceinline__ void state_sums(const double *Y, int64_t ld, int N, int warp,
+                                           const double *inv_mw, double T, double P,
+                                           const int64_t *lt, double *row, int *irr) {
+  if (warp == 0) {
+    double ys = N > 1 ? Y[0] : 0.0;
+    int k = 1;
+    for (; k + 8 <= N - 1; k += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = Y[(int64_t)(k + u) * ld];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) ys += v[u];
+    }
+    for (; k < N - 1; ++k) ys += Y[(int64_t)k * ld];
+    row[7 * 32] = 1.0 - ys;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+  } else if (warp == 1) {
+    double mwi = 0.0;
+    int k = 0;
+    for (; k + 8 <= N - 1; k += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = Y[(int64_t)(k + u) * ld];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) mwi = fma(v[u], inv_mw[k + u], mwi);
+    }
+    for (; k < N - 1; ++k) mwi = fma(Y[(int64_t)k * ld], inv_mw[k], mwi);
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    mwi = fma(row[7 * 32], inv_mw[N - 1], mwi);
+    const double rho = P / mwi * ((1.0 / T) * fast::INV_RU);
+    // a positive density of moderate size, a mean 1/W below 2
+    const int e = (int)(bits_of(rho) >> 52), m = (int)(bits_of(mwi) >> 52);
+    *irr = e < 1023 - 400 || e > 1023 + 400 || m < 1023 - 40 || m > 1023;
+    reinterpret_cast<int64_t *>(row)[6 * 32] = even(log2d(rho, lt));
+    row[8 * 32] = rho;
+    row[9 * 32] = mwi;
+  }
+}
+
+// Functions of T, sums and marks of one tile's states into the block at o
+// (warps 0-2; i: the lane's state).  Called, not inlined: once per tile, and
+// its registers are not the rate loops'.
+__device__ __noinline__ void prepare(const FxTab &f, const Args &g, const double *inv_mw,
+                                     const Batch &b, int64_t i, int warp, int lane,
+                                     const int64_t *lt, unsigned char *o) {
+  int *marks = reinterpret_cast<int *>(o + 10 * 256 - lane * 8) + lane;
+  if (warp == 2) {
+    bool irr;
+    const int iv = basis_of(f, g.tab, b.T[i], reinterpret_cast<int64_t *>(o), irr);
+    marks[0] = irr ? -1 : iv;
+  } else if (warp < 2) {
+    state_sums(b.Y + i, b.ld, f.N, warp, inv_mw, b.T[i], b.P[i], lt,
+               reinterpret_cast<double *>(o), marks + 32);
+  }
+}
+
+// The warp's rates left to the general FP64 arithmetic (all: every one), for
+// the lane's state i.
+__device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const Batch &b,
+                                    int stride, Ring<DP> plain, Ring<DO> other, int64_t i,
+                                    bool all, double rho, double yN, unsigned char *q) {
+  const Tab t = make_tab(g.img, lay);
+  fast::State s;
+  s.T = b.T[i];
+  s.P = b.P[i];
+  s.invT = 1.0 / s.T;
+  s.logT = fast::log_t(s.T, t.logtab);
+  s.tab = t.exptab;
+  s.ltab = t.logtab;
+  KcPolyG kc;
+  kc.T = s.T;
+  kc.logT = s.logT;
+  kc.invT = s.invT;
+  const YConc C{b.Y + i, b.ld, rho, yN, t.inv_mw, t.N};
+  for (int p = 0; p < 2 * plain.n + other.n; ++p) {
+    const int o = p - 2 * plain.n;
+    const int4 h = __ldg(reinterpret_cast<const int4 *>(
+        o < 0 ? plain.src + (int64_t)p * stride : other.src + (int64_t)o * other.stride));
+    double *v = reinterpret_cast<double *>(q + h.x);
+    double fwd, rev, pm;
+    if (h.w >= 0 && (all || bits_of(*v) == LATER))
+      *v = fast::rxn_net(t, h.w, s, s.P * s.invT * fast::INV_RU, C, kc, fwd, rev, pm);
+  }
+}
+
+template <int LIST, int PER_SM, bool QS, bool TS>
+__global__ void __launch_bounds__(warps_of(LIST) * 32, PER_SM)
+    k_wdot_tile(const __grid_constant__ ImgLayout lay, const __grid_constant__ FxTab f,
+                const __grid_constant__ Args g, const __grid_constant__ Batch b) {
   constexpr int NW = warps_of(LIST);
   extern __shared__ __align__(128) unsigned char smem[];
   const int N = f.N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned char *tab = g.tab;
-  int64_t *yl = reinterpret_cast<int64_t *>(smem) + lane;         // [N + 1][32]
-  int64_t *blk = yl + (N + 1) * 32;                               // [ROWS][32]
-  double *s_yN = reinterpret_cast<double *>(blk + 8 * 32 - lane), *s_rho = s_yN + 32;
-  int *s_iv = reinterpret_cast<int *>(s_yN + 64), *s_irr = s_iv + 32;
-  int64_t *next = reinterpret_cast<int64_t *>(smem) + (N + 1 + ROWS) * 32;
+  // shared memory: [N + 1][32] y, then the exponents of C (row N: zeros);
+  // two blocks of per-state values; the small tables; each warp's ring of
+  // records; the net rates
+  unsigned char *yl = smem + lane * 8;
+  unsigned char *next = smem + (N + 1) * 256;
+  unsigned char *blk0 = next + lane * 8;
+  next += 2 * ROWS * 256;
   const int64_t *et = reinterpret_cast<const int64_t *>(tab + f.small);
   if (TS) {
-    for (int k = threadIdx.x; k < TAB_BYTES / 8; k += NW * 32) next[k] = et[k];
-    et = next;
-    next += TAB_BYTES / 8;
+    int64_t *st = reinterpret_cast<int64_t *>(next);
+    for (int k = threadIdx.x; k < TAB_BYTES / 8; k += NW * 32) st[k] = et[k];
+    et = st;
+    next += TAB_BYTES;
+    __syncthreads();
   }
-  const int64_t *lt = et + EXP_ENTRIES;
-  double *q = (QS ? reinterpret_cast<double *>(next)
-                  : g.q + (int64_t)blockIdx.x * f.R * 32) + lane;
-  if (warp == 0) yl[N * 32] = 0;
-  const Tab t = make_tab(g.img, lay);
-  const double *inv_mw = t.inv_mw;
-  const int64_t *lw = reinterpret_cast<const int64_t *>(tab + f.lw);
-  const int *list = reinterpret_cast<const int *>(tab + f.list[LIST]);
-  const int l0 = reinterpret_cast<const int *>(tab + f.list_ptr[LIST])[warp];
-  const int l1 = reinterpret_cast<const int *>(tab + f.list_ptr[LIST])[warp + 1];
-  const int lr = l0 + reinterpret_cast<const int *>(tab + f.list_rev[LIST])[warp];
-  const int *sum = reinterpret_cast<const int *>(tab + f.sum[LIST]);
-  const int s0 = reinterpret_cast<const int *>(tab + f.sum_ptr[LIST])[warp];
-  const int s1 = reinterpret_cast<const int *>(tab + f.sum_ptr[LIST])[warp + 1];
-  int bad = 0;
-  for (int64_t tile = blockIdx.x; tile * 32 < b.n; tile += gridDim.x) {
+  const int64_t *lt = et + EXP_WORDS;
+  const int rb = ring_bytes(f);
+  unsigned char *ring = next + warp * rb;
+  next += NW * rb;
+  unsigned char *q = (QS ? next : reinterpret_cast<unsigned char *>(g.q) +
+                                      (int64_t)blockIdx.x * (f.R + 1) * 256) + lane * 8;
+  auto Yl = [&](int off) -> int64_t & { return *reinterpret_cast<int64_t *>(yl + off); };
+  auto Q = [&](int off) -> double & { return *reinterpret_cast<double *>(q + off); };
+  if (warp == 0) {
+    Yl(N * 256) = 0;
+    Q(f.R * 256) = 0.0;
+  }
+  Ring<DP> plain_ring;
+  Ring<DO> other_ring;
+  {
+    const int *lp = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][0]) + warp;
+    const int *lo = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][1]) + warp;
+    plain_ring = Ring<DP>{tab + f.rec[LIST][0] + (int64_t)lp[0] * f.stride[0], smem_u32(ring),
+                          f.stride[0], lp[1] - lp[0], lane};
+    other_ring = Ring<DO>{tab + f.rec[LIST][1] + (int64_t)lo[0] * f.stride[1], smem_u32(ring),
+                          f.stride[1], lo[1] - lo[0], lane};
+  }
+  const int s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[warp];
+  const int s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[warp + 1];
+  const unsigned yrows = smem_u32(smem) + lane * 8;
+  const double *inv_mw = reinterpret_cast<const double *>(g.img + lay.inv_mw);
+  int bad = 0, bk = 0;
+  int64_t tile = blockIdx.x;
+  const int64_t ntiles = (b.n + 31) / 32;
+  if (tile < ntiles) {
+    const int64_t i = tile * 32 + lane < b.n ? tile * 32 + lane : tile * 32;
+    load_y<NW>(b.Y + i, b.ld, N, warp, yrows);
+    if (warp < 3) prepare(f, g, inv_mw, b, i, warp, lane, lt, blk0);
+  }
+  for (; tile < ntiles; tile += gridDim.x, bk ^= 1) {
     const int64_t i = tile * 32 + lane;
     const bool valid = i < b.n;
     const int64_t ic = valid ? i : tile * 32;  // idle lanes repeat a valid state
-    const double T = b.T[ic], P = b.P[ic];
-    // mass fractions on chip; the last warp also forms the functions of T
-#pragma unroll 4
-    for (int k = warp; k < N - 1; k += NW)
-      yl[k * 32] = __double_as_longlong(b.Y[(int64_t)k * b.ld + ic]);
-    if (warp == NW - 1) {
-      bool irr;
-      s_iv[lane] = basis_of(f, tab, T, blk, irr);
-      s_irr[lane] = irr;
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // y_N = 1 - sum y in the reference's order (rate_subs.py:1312-1320) on
-    // warp 0, the density on warp 1: two dependent FP64 chains side by side
-    if (warp == 0) {
-      double ys = N > 1 ? __longlong_as_double(yl[0]) : 0.0;
-      for (int k = 1; k < N - 1; ++k) ys += __longlong_as_double(yl[k * 32]);
-      s_yN[lane] = 1.0 - ys;
-      yl[(N - 1) * 32] = __double_as_longlong(1.0 - ys);
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-    } else if (warp == 1) {
-      double mwi = 0.0;
-      for (int k = 0; k < N - 1; ++k) mwi = fma(__longlong_as_double(yl[k * 32]), inv_mw[k], mwi);
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-      mwi = fma(s_yN[lane], inv_mw[N - 1], mwi);
-      const double rho = P / mwi * ((1.0 / T) * fast::INV_RU);
-      s_rho[lane] = rho;
-      // a positive density of moderate size, a mean 1/W below 2
-      const int e = (int)(bits_of(rho) >> 52), m = (int)(bits_of(mwi) >> 52);
-      if (e < 1023 - 400 || e > 1023 + 400 || m < 1023 - 40 || m > 1023) s_irr[lane] = 1;
-      blk[6 * 32] = even(log2d(rho, lt));
-      blk[7 * 32] = d2fx(mwi, 61 - f.eff_shift);
-    }
-    __syncthreads();
-    const int64_t lrho = blk[6 * 32];
-    // third-body concentrations: [M] = rho (1/mw + sum (eff - 1) Y / W), as
-    // exponents into the slots of their reactions' rates
-    if (f.NPM > 0) {
-      const int4 *pmh = reinterpret_cast<const int4 *>(tab + f.pmh);
-      const int *ep = reinterpret_cast<const int *>(tab + f.eff_ptr);
-      const int *es = reinterpret_cast<const int *>(tab + f.eff_sp);
-      const int2 *ek = reinterpret_cast<const int2 *>(tab + f.eff_k);
-      const int64_t m = blk[7 * 32];
+    unsigned char *o = blk0 + bk * ROWS * 256;
+    auto rowd = [&](int r) { return *reinterpret_cast<const double *>(o + r * 256); };
+    int *marks = reinterpret_cast<int *>(o + 10 * 256 - lane * 8) + lane;
+    const int64_t lrho = *reinterpret_cast<const int64_t *>(o + 6 * 256);
+    // a third-body concentration over rho: 1/mw + sum (eff - 1) Y / W
+    auto third_body = [&](int p) {
+      const int *ep = reinterpret_cast<const int *>(tab + f.eff_ptr) + p;
+      double s = rowd(9);
+      for (int e = ep[0]; e < ep[1]; ++e) {
+        const int4 w = __ldg(reinterpret_cast<const int4 *>(tab + f.eff) + e);
+        double y;
+        if (w.z == (N - 1) * 256) y = rowd(7);
+        else if (QS) y = __longlong_as_double(Yl(w.z));
+        else y = b.Y[(int64_t)(w.z >> 8) * b.ld + ic];
+        s = fma(__hiloint2double(w.y, w.x), y, s);
+      }
+      return s;
+    };
+    // (rates on chip) into the slots of their reactions' rates
+    if (QS && f.NPM > 0) {
       for (int p = warp; p < f.NPM; p += NW) {
-        const int4 h = __ldg(pmh + p);
-        if (!(h.x & PMF_SUM)) continue;
-        int64_t s = m;
-        for (int e = ep[p]; e < ep[p + 1]; ++e)
-          s += mul<4>(dg(__ldg(ek + e)), split(d2fx(__longlong_as_double(yl[es[e] * 32]), 60)));
-        const int64_t a = s < 0 ? -s : s;
-        int64_t l = even(log2i(a | (a == 0), 61 - f.eff_shift, lt) + lrho) | (s < 0);
-        if (a == 0) l = ZERO_EXP;
-        q[(int64_t)h.z * 32] = __longlong_as_double(l);
+        const int slot = __ldg(reinterpret_cast<const int2 *>(tab + f.pm) + p).x;
+        if (slot >= 0) Q(slot) = third_body(p);
       }
       __syncthreads();
     }
     // exponents of the concentrations in place of the mass fractions
+    bool odd = false;
     for (int k = warp; k < N; k += NW) {
-      const double y = __longlong_as_double(yl[k * 32]);
+      const double y = k == N - 1 ? rowd(7) : __longlong_as_double(Yl(k * 256));
       const uint64_t u = bits_of(y);
       const int e = (int)(u >> 52) & 0x7ff;
-      int64_t l = even(log2d(y, lt) + lw[k] + lrho) | (int64_t)(u >> 63);
-      if ((u << 1) == 0) l = ZERO_EXP;
-      else if (e == 0 || e > 1023) s_irr[lane] = 1;  // subnormal, |y| >= 2, NaN
-      yl[k * 32] = l;
+      int64_t l = even(log2d(y, lt) + reinterpret_cast<const int64_t *>(tab + f.lw)[k] + lrho) |
+                  (int64_t)(u >> 63);
+      const bool zero = (u << 1) == 0;
+      if (zero) l = ZERO_EXP;
+      odd |= !zero && (e == 0 || e > 1023);  // subnormal, |y| >= 2, NaN
+      Yl(k * 256) = l;
     }
+    if (odd) marks[32] = 1;
+    plain_ring.start();
     __syncthreads();
     // net rates
-    const bool irr = s_irr[lane] != 0;
     {
-      const int iv = s_iv[lane];
+      if (warp < 3 && tile + gridDim.x < ntiles) {
+        const int64_t j = (tile + gridDim.x) * 32;
+        prepare(f, g, inv_mw, b, j + lane < b.n ? j + lane : j, warp, lane, lt,
+                blk0 + (bk ^ 1) * ROWS * 256);
+      }
+      const int iv = marks[0] < 0 ? 0 : marks[0];
+      // states outside the scheme: every rate in FP64; later: single rates
+      bool later = false, all = marks[0] < 0 || marks[32];
       Basis B;
-      const int2 *o = reinterpret_cast<const int2 *>(blk);
-      B.L = dg(o[0]);
-      B.I = dg(o[32]);
-      B.t1 = dg(o[64]);
-      B.t2 = dg(o[96]);
-      B.t3 = dg(o[128]);
-      B.t4 = dg(o[160]);
-      int p = l0;
-      for (; p + 2 <= lr; p += 2) plain_block<2>(f, tab, list + p, yl, B, iv, T, et, q);
-      for (; p < lr; ++p) plain_block<1>(f, tab, list + p, yl, B, iv, T, et, q);
-      for (; p < l1; ++p) {
-        const int r = list[p];
-        const int4 h0 = __ldg(reinterpret_cast<const int4 *>(tab + f.hdr) + 2 * r);
-        const int4 h1 = __ldg(reinterpret_cast<const int4 *>(tab + f.hdr) + 2 * r + 1);
-        bool slow = (h0.y & RF_GEN) != 0;
-        double v = 0.0;
-        if (!(h0.y & RF_GEN)) {
-          int idx = iv;
-          if (!f.uniform) {
-            const int32_t *tp = reinterpret_cast<const int32_t *>(tab + f.thr_ptr);
-            idx = 0;
-            for (int e = tp[r]; e < tp[r + 1]; ++e)
-              idx += T > reinterpret_cast<const double *>(tab + f.thr)[e];
-          }
-          const int2 *c = reinterpret_cast<const int2 *>(tab + f.coef) + COEF * (h0.z + idx);
-          int64_t l = (h0.y & RF_NEG) ? 1 : 0;  // what both directions share
-          if (h0.w >= 0) {
-            const int4 ph = __ldg(reinterpret_cast<const int4 *>(tab + f.pmh) + h0.w);
-            int64_t lth = ph.y >= 0 ? yl[ph.y * 32]
-                                    : __double_as_longlong(q[(int64_t)r * 32]);
-            if (h0.y & RF_FALL)
-              lth = falloff(reinterpret_cast<const int2 *>(tab + f.pmc) + PMC * (NI * h0.w + iv),
-                            ph.x, lth, B.L, B.I, B.t1, et, lt, slow);
-            l += lth;
-          }
-          Dot a(word(c[0]));
-          a.add(dg(c[1]), B.L);
-          a.add(dg(c[2]), B.I);
-          int64_t yf = a.exponent() + l + yl[(h1.x & 0xffff) * 32] +
-                       yl[((unsigned)h1.x >> 16) * 32];
-          if (h0.y & RF_MORE_R)
-            yf += yl[(h1.y & 0xffff) * 32] + yl[((unsigned)h1.y >> 16) * 32];
-          bool sp;
-          if (h0.y & RF_REV) {
-            Dot d(word(c[3]));
-            d.add(dg(c[4]), B.L);
-            d.add(dg(c[5]), B.I);
-            d.add(dg(c[6]), B.t1);
-            d.add(dg(c[7]), B.t2);
-            d.add(dg(c[8]), B.t3);
-            d.add(dg(c[9]), B.t4);
-            int64_t yr = d.exponent() + l + yl[(h1.z & 0xffff) * 32] +
-                         yl[((unsigned)h1.z >> 16) * 32];
-            if (h0.y & RF_MORE_P)
-              yr += yl[(h1.w & 0xffff) * 32] + yl[((unsigned)h1.w >> 16) * 32];
-            v = net_of<true>(yf, yr, et, sp);
-            if (sp) v = net_far<true>(yf, yr, et);
-          } else {
-            v = net_of<false>(yf, 0, et, sp);
-            if (sp) v = net_far<false>(yf, 0, et);
+      B.L = dg(*reinterpret_cast<const int2 *>(o));
+      B.I = dg(*reinterpret_cast<const int2 *>(o + 256));
+      B.t1 = dg(*reinterpret_cast<const int2 *>(o + 512));
+      B.t2 = dg(*reinterpret_cast<const int2 *>(o + 768));
+      B.t3 = dg(*reinterpret_cast<const int2 *>(o + 1024));
+      B.t4 = dg(*reinterpret_cast<const int2 *>(o + 1280));
+      // the record at `at` whose coefficients begin `co` bytes on
+      auto record = [&](const unsigned char *at, int co) {
+        int idx = iv;
+        if (f.nthr) {
+          const double T = b.T[ic];
+          const double *thr = reinterpret_cast<const double *>(at + co + COEF * (f.nthr + 1));
+          idx = 0;
+          for (int e = 0; e < f.nthr; ++e) idx += T > thr[e];
+        }
+        return Rec{at, at + co + COEF * idx};
+      };
+      // two reactions at a time: independent chains side by side
+      const int one = f.stride[0] / 2;
+      unsigned char *at = ring;
+      for (int p = 0; p < plain_ring.n; ++p) {
+        plain_ring.next(p);
+        int64_t yf[2], yr[2];
+        int slot[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const Rec r = record(at + u * one, HEAD);
+          const int2 h = *reinterpret_cast<const int2 *>(r.p);  // slot, flags
+          const int4 x = r.word4(16);
+          slot[u] = h.x;
+          yf[u] = (exponent3(r, B) | (h.y & RF_NEG)) + Yl(x.x) + Yl(x.y);
+          yr[u] = (exponent7(r, B) | (h.y & RF_NEG)) + Yl(x.z) + Yl(x.w);
+          if (h.y & RF_MORE) {
+            const int4 m = r.word4(32);
+            yf[u] += Yl(m.x) + Yl(m.y);
+            yr[u] += Yl(m.z) + Yl(m.w);
           }
         }
-        if (slow)
-          v = slow_net(g.img, lay, r, T, P, b.Y + ic, b.ld, s_rho[lane], s_yN[lane]);
-        q[(int64_t)r * 32] = v;
+        bool far[2];
+        const double v0 = net_of<true>(yf[0], yr[0], et, far[0]);
+        const double v1 = net_of<true>(yf[1], yr[1], et, far[1]);
+        Q(slot[0]) = v0;
+        Q(slot[1]) = v1;
+        all |= far[0] | far[1];
+        at = at == ring + 2 * f.stride[0] ? ring : at + f.stride[0];
       }
-      if (irr)  // the state is outside the scheme: every rate in FP64
-        for (p = l0; p < l1; ++p)
-          q[(int64_t)list[p] * 32] =
-              slow_net(g.img, lay, list[p], T, P, b.Y + ic, b.ld, s_rho[lane], s_yN[lane]);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      other_ring.start();
+      for (int p = 0; p < other_ring.n; ++p) {
+        other_ring.next(p);
+        const Rec r = record(ring + (p % DO) * f.stride[1], HEAD + PMH + PMC * NI);
+        const int4 h = r.word4(0), x = r.word4(16), ph = r.word4(HEAD);
+        bool slow = h.y & RF_GEN;
+        int64_t l = h.y & RF_NEG;  // what both directions share
+        double thd = 1.0;
+        if (h.z >= 0) {
+          if (h.y & RF_FALL) {
+            const int64_t lth = ph.y >= 0
+                                    ? Yl(ph.y)
+                                    : log2s(QS ? Q(h.x) : third_body(h.z), lt) + lrho;
+            l += falloff(reinterpret_cast<const int2 *>(r.p + HEAD + PMH + PMC * iv), ph.x, lth,
+                         B.L, B.I, B.t1, et, lt, slow);
+          } else {
+            thd = rowd(8) * (QS ? Q(h.x) : third_body(h.z));
+          }
+        }
+        int64_t yf = exponent3(r, B) + l + Yl(x.x) + Yl(x.y);
+        const int4 m = r.word4(32);
+        yf += Yl(m.x) + Yl(m.y);
+        double v;
+        bool far;
+        if (h.y & RF_REV) {
+          const int64_t yr = exponent7(r, B) + l + Yl(x.z) + Yl(x.w) + Yl(m.z) + Yl(m.w);
+          v = net_of<true>(yf, yr, et, far);
+        } else {
+          v = net_of<false>(yf, 0, et, far);
+        }
+        slow |= far;
+        Q(h.x) = slow ? of_bits(LATER) : v * thd;
+        later |= slow;
+      }
+      if (later || all)
+        finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
     }
     __syncthreads();
-    // species sums
+    // the next tile's mass fractions replace exponents that every warp is
+    // done with, while the species sums run
+    if (tile + gridDim.x < ntiles) {
+      const int64_t j = (tile + gridDim.x) * 32;
+      load_y<NW>(b.Y + (j + lane < b.n ? j + lane : j), b.ld, N, warp, yrows);
+    }
     for (int a = s0; a < s1; ++a) {
-      const int k = sum[a];
-      const int e1 = t.spc_ptr[k + 1];
-      int e = t.spc_ptr[k];
+      const int4 sg = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a);
       double w = 0.0, w2 = 0.0;
-      for (; e + 4 <= e1; e += 4) {
-        double v[4], nu[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          v[u] = q[(int64_t)t.spc_r[e + u] * 32];
-          nu[u] = t.spc_nu[e + u];
+      if (!sg.w) {
+        const int4 *tm = reinterpret_cast<const int4 *>(tab + f.term) + sg.y;
+        int4 t = __ldg(tm);
+        for (int e = 0; e < sg.z; ++e) {
+          const int4 c = t;
+          t = __ldg(tm + e + 1);
+          auto signed_q = [&](int x) {
+            const double v = Q(x & 0x7fffffff);
+            return __hiloint2double(__double2hiint(v) ^ (x & 0x80000000), __double2loint(v));
+          };
+          const double v0 = signed_q(c.x), v1 = signed_q(c.y), v2 = signed_q(c.z),
+                       v3 = signed_q(c.w);
+          w += v0;
+          w2 += v1;
+          w += v2;
+          w2 += v3;
         }
-        w = fma(nu[0], v[0], w);
-        w2 = fma(nu[1], v[1], w2);
-        w = fma(nu[2], v[2], w);
-        w2 = fma(nu[3], v[3], w2);
+      } else {
+        for (int e = sg.y; e < sg.y + sg.z; ++e)
+          w = fma(__ldg(reinterpret_cast<const double *>(tab + f.wnu) + e),
+                  Q(__ldg(reinterpret_cast<const int *>(tab + f.wterm) + e)), w);
       }
-      for (; e < e1; ++e) w = fma(t.spc_nu[e], q[(int64_t)t.spc_r[e] * 32], w);
       w += w2;
       if (valid) {
         bad += ((__double2hiint(w) >> 20) & 0x7ff) == 0x7ff;  // inf or NaN, integer test
-        b.wdot[(int64_t)k * b.ld + i] = w;
+        b.wdot[(int64_t)sg.x * b.ld + i] = w;
       }
     }
-    // the next tile's mass fractions replace exponents that every warp is
-    // done with (the barrier before the sums); its third bodies replace
-    // rates only after two more barriers
+    // rates are replaced only after the barrier at the loop's head
   }
   if (bad && b.status) atomicAdd(&b.status[1], bad);
 }
 
-size_t smem_of(const FxTab &f, bool qs, bool ts) {
-  return (size_t)(f.N + 1 + ROWS) * 256 + (ts ? TAB_BYTES : 0) + (qs ? (size_t)f.R * 256 : 0);
+// Shared memory of a CTA of nw warps.
+size_t smem_of(const FxTab &f, int nw, bool qs, bool ts) {
+  return (size_t)(f.N + 1 + 2 * ROWS) * 256 + (ts ? TAB_BYTES : 0) + (size_t)nw * ring_bytes(f) +
+         (qs ? (size_t)(f.R + 1) * 256 : 0);
+}
+
+// How a launch over `tiles` tiles runs: warps per CTA (list), CTAs per SM,
+// rates and small tables on chip.
+struct Plan {
+  int list = 2, per_sm = 1;
+  bool qs = false, ts = false, ok = false;
+};
+
+Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
+  Plan p;
+  if (!f.usable) return p;
+  p.ok = true;
+  auto fits = [&](int nw, int per_sm, bool qs) {
+    return (smem_of(f, nw, qs, true) + 1024) * per_sm <= (size_t)smem_optin + 1024;
+  };
+  if (f.R < 100 && fits(4, 6, true)) {
+    p = Plan{0, 6, true, true, true};
+  } else if (tiles <= sm_count && fits(16, 1, true)) {
+    p = Plan{2, 1, true, true, true};
+  } else if (fits(8, 3, false)) {
+    p = Plan{1, 3, false, true, true};
+  } else {
+    p.ts = fits(16, 1, false);
+    p.ok = smem_of(f, 16, false, p.ts) <= (size_t)smem_optin;
+  }
+  return p;
 }
 
 }  // namespace fx
@@ -483,39 +651,31 @@ size_t smem_of(const FxTab &f, bool qs, bool ts) {
 // Scratch bytes of a launch over n states (0: the net rates fit on chip);
 // < 0: the mechanism does not fit this kernel.
 long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
-  if (!f.usable) return -1;
-  if (fx::smem_of(f, true, true) <= (size_t)smem_optin) return 0;
-  if (fx::smem_of(f, false, false) > (size_t)smem_optin) return -1;
   const int64_t tiles = (n + 31) / 32;
-  return (long long)(tiles < sm_count ? tiles : sm_count) * f.R * 256;
+  const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
+  if (!p.ok) return -1;
+  return p.qs ? 0 : (long long)std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm) *
+                        (f.R + 1) * 256;
 }
 
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                            const unsigned char *tab, const Batch &b, int sm_count,
                            int smem_optin, double *scratch, cudaStream_t s) {
   using fx::k_wdot_tile;
-  const fx::Args g{img, tab, scratch};
   const int64_t tiles = (b.n + 31) / 32;
-  const bool qs = !scratch;
-  const bool ts = fx::smem_of(f, qs, true) <= (size_t)smem_optin;
-  // sixteen warps per SM: in one CTA where tiles are few or large
-  int list = 2;
-  if (qs) {
-    const size_t need = fx::smem_of(f, true, true) + 2048;
-    if (4 * need <= (size_t)smem_optin && f.R < 100) list = 0;
-    else if (2 * need <= (size_t)smem_optin) list = 1;
-    if (list == 1 && tiles <= sm_count) list = 2;
-  }
-  const int per_sm = 16 / fx::warps_of(list);
-  const size_t bytes = fx::smem_of(f, qs, ts);
+  const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
+  if (!p.ok || p.qs != !scratch) return cudaErrorInvalidValue;
   void (*k)(const ImgLayout, const fx::FxTab, fx::Args, Batch);
-  if (qs) k = list == 0 ? k_wdot_tile<0, true, true> : list == 1 ? k_wdot_tile<1, true, true>
-                                                                 : k_wdot_tile<2, true, true>;
-  else k = ts ? k_wdot_tile<2, false, true> : k_wdot_tile<2, false, false>;
+  if (p.list == 0) k = k_wdot_tile<0, 6, true, true>;
+  else if (p.list == 1) k = k_wdot_tile<1, 3, false, true>;
+  else k = p.qs ? k_wdot_tile<2, 1, true, true>
+                : p.ts ? k_wdot_tile<2, 1, false, true> : k_wdot_tile<2, 1, false, false>;
+  const int nw = fx::warps_of(p.list);
+  const size_t bytes = fx::smem_of(f, nw, p.qs, p.ts);
   const cudaError_t e = set_smem_limit(k, bytes);
   if (e != cudaSuccess) return e;
-  const int64_t cap = (int64_t)sm_count * per_sm;
-  k<<<(unsigned)(tiles < cap ? tiles : cap), fx::warps_of(list) * 32, bytes, s>>>(L, f, g, b);
+  const int64_t grid = std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm);
+  k<<<(unsigned)grid, nw * 32, bytes, s>>>(L, f, fx::Args{tab, img, scratch}, b);
   return cudaGetLastError();
 }
 

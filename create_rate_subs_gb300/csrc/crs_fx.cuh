@@ -12,7 +12,7 @@
 //   * a 64-bit number is split into two signed 32-bit digits, v = hi 2^32 +
 //     lo, and a product keeps hi hi and the two mixed products (three
 //     multiply-adds); the dropped lo lo is at most a quarter of the unit.
-// Values return to FP64 from 57-bit mantissas with one rounding.  Plain
+// Values return to FP64 from 57-bit mantissas with one rounding each.  Plain
 // integer code: the same functions compile for the host, where the tests
 // compare them with 64-bit floating point.
 #pragma once
@@ -34,10 +34,12 @@ namespace fx {
 constexpr int YB = 49;                         // fraction bits of an exponent
 constexpr int64_t ZERO_EXP = -(3500LL << YB);  // exponent of a zero factor
 constexpr int LOGN = 512;                      // logarithm table: F = 1 + j / 512
-// The small tables, in 8-byte words: 2^(j/256) in units of 2^-56, then pairs
-// (1/F in units of 2^-62, log2 F in units of 2^-49).
-constexpr int EXP_ENTRIES = 256;
-constexpr int TAB_BYTES = EXP_ENTRIES * 8 + (LOGN + 1) * 16;
+// The small tables, in 8-byte words: 2^(j/256) in units of 2^-56 plus 8 units
+// (257 entries and one of padding), then pairs (1/F in units of 2^-62, log2 F
+// in units of 2^-49).
+constexpr int EXPN = 256;
+constexpr int EXP_WORDS = EXPN + 2;
+constexpr int TAB_BYTES = EXP_WORDS * 8 + (LOGN + 1) * 16;
 
 // ---- the machine's integer operations -------------------------------------
 FX_FN int mulhi(int a, int b) {
@@ -91,14 +93,25 @@ FX_FN Dg split(int64_t v) {
   return Dg{(int)(v >> 32) + (int)((unsigned)lo >> 31), lo};
 }
 
-FX_FN int64_t mad(int a, int b, int64_t c) { return (int64_t)a * b + c; }
+// a b + c as one instruction; of the C expression the compiler makes a
+// product and a 64-bit sum where the sums are short (8 instructions a mul
+// against 12)
+FX_FN int64_t mad(int a, int b, int64_t c) {
+#if defined(__CUDA_ARCH__)
+  int64_t d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+#else
+  return (int64_t)a * b + c;
+#endif
+}
 
 // (a b) 2^(S - 64), rounded
 template <int S>
 FX_FN int64_t mul(Dg a, Dg b) {
-  const int64_t hh = mad(a.hi, b.hi, 0);
   const int64_t mid = mad(a.lo, b.hi, mad(a.hi, b.lo, 1LL << (31 - S)));
-  return (int64_t)((uint64_t)hh << S) + (mid >> (32 - S));
+  if (S == 0) return mad(a.hi, b.hi, mid >> 32);
+  return (int64_t)((uint64_t)mad(a.hi, b.hi, 0) << S) + (mid >> (32 - S));
 }
 
 // floor(v 2^lsb) towards zero for |v| < 2^(62 - lsb); infinities and NaN
@@ -113,29 +126,31 @@ FX_FN int64_t d2fx(double v, int lsb) {
   return (int64_t)u < 0 ? -r : r;
 }
 
-// 2^y as M 2^(E - 56), M within 2^-9 of [2^56, 2^57): y split into an integer, an eight-
-// bit table index and |r| <= 2^-9, 2^r = 1 + r (d1 + r (d2 + r (d3 + r d4)))
-// with d_n = (ln 2)^n / n! (truncation below 2^-54).  The sign (bit 0 of y)
-// is dropped.
+// 2^y as M 2^(E - 56), M in [2^56, 2^57]: y split into an integer, the
+// nearest of 257 table points j / 256 and |r| <= 2^-9, 2^r = 1 + r (d1 + r
+// (d2 + r (d3 + r d4))) with d_n = (ln 2)^n / n! (truncation below 2^-54).
+// The table holds 2^(j/256) + 8 units: the rounding of M's four last bits.
+// The sign (bit 0 of y) is dropped.
 FX_FN void exp2m(int64_t y, const int64_t *tab, uint64_t &M, int &E) {
-  const int64_t v = (y & ~1LL) + (1LL << (YB - 9));
-  const int vh = (int)(v >> 32);
-  const unsigned vl = (unsigned)(uint64_t)v;
+  const int vh = (int)(y >> 32);
+  const unsigned vl = (unsigned)(uint64_t)y & ~1u;
   E = vh >> (YB - 32);
-  const int64_t S = tab[(vh >> (YB - 40)) & 255];
-  // r in units of 2^-71: the low 41 bits, centred
-  const int64_t r64 =
-      (int64_t)(((uint64_t)(unsigned)(vh & 511) << 54) | ((uint64_t)vl << 22)) - (1LL << 62);
-  const int rh = (int)(r64 >> 32);  // 2^-39
-  constexpr int D4 = 5043;          // 2^-19
-  constexpr int D3 = 3724818;       // 2^-26
-  constexpr int D2 = 2063529982;    // 2^-33
+  const int j = ((vh & ((1 << (YB - 32)) - 1)) + (1 << (YB - 41))) >> (YB - 40);
+  const int64_t S = tab[j];
+  // r in units of 2^-71: the fraction less j / 256, modulo 2^64
+  const int rh = (int)(((unsigned)vh << 22 | vl >> 10) ^ (unsigned)j << 31);  // 2^-39
+  const int rl = (int)(vl << 22);
+  constexpr int D4 = 5043;        // 2^-19
+  constexpr int D3 = 3724818;     // 2^-26
+  constexpr int D2 = 2063529982;  // 2^-33
   constexpr int64_t D1 = 99893036290645748LL;  // 2^-57
   const int t = mulhi(rh, D4) + D3;
   const int g = mulhi(rh, t) + D2;
   const int64_t h = D1 + (mad(rh, g, 0) >> 15);
-  const int64_t p = mul<0>(split(r64), split(h));  // 2^-64
-  M = (uint64_t)(S + mul<0>(split(S), split(p)));
+  const Dg r{rh + (int)((unsigned)rl >> 31), rl};
+  const Dg p = split(mul<0>(r, split(h))), s = split(S);  // 2^-64
+  const int64_t mid = mad(s.lo, p.hi, mad(s.hi, p.lo, 1LL << 31));
+  M = (uint64_t)mad(s.hi, p.hi, S + (mid >> 32));
 }
 
 // log2 of m 2^-63, m in [2^63, 2^64), in units of 2^-49: m = F (1 + u) with F
@@ -230,53 +245,42 @@ FX_FN int64_t ratio2(int64_t a, int64_t b, bool &ok) {
   return (int64_t)q0 + (t1 >> 22) + (t2 >> 43);
 }
 
-// +-M 2^(E - 56) as a double, with overflow to infinity and gradual
-// underflow
-FX_FN double assemble(uint64_t M, int E, bool neg) {
-  const double m = (double)(int64_t)M;  // M < 2^57: rounds once
-  return ldexp(neg ? -m : m, E - 56);
-}
-
-// The value of one exponent, whatever its range.
+// The value of one exponent (bit 0: its sign), with overflow to infinity and
+// gradual underflow.
 FX_FN double value_of(int64_t y, const int64_t *tab) {
   uint64_t M;
   int E;
   exp2m(y, tab, M, E);
-  return assemble(M, E, y & 1);
+  const double m = (double)(int64_t)M;  // M <= 2^57: rounds once
+  return ldexp((y & 1) ? -m : m, E - 56);
 }
 
-// +-2^yf -+ 2^yr as a double (bit 0 of each exponent: its sign): the aligned
-// difference of the 57-bit mantissas, rounded once.  REV false: the first
-// term alone.  special: the result (or, with overflow, a term) lies outside
-// the normal range and net_special has to form it; the code has no branch.
+// The value of one exponent as a normal double by integer operations; zero
+// far below the normal range.  far: overflow or gradual underflow, which
+// value_of has to form.
+FX_FN double normal_of(int64_t y, const int64_t *tab, bool &far) {
+  uint64_t M;
+  int E;
+  exp2m(y, tab, M, E);
+  const unsigned e = (unsigned)(E + 1022);
+  const bool in = e <= 2044u;
+  far = !in && E > -1081;
+  const unsigned lo = (unsigned)(M >> 4);
+  const unsigned hi = ((unsigned)(M >> 36) + (e << 20)) ^ ((unsigned)y << 31);
+  return of_bits((uint64_t)(in ? hi : 0u) << 32 | (in ? lo : 0u));
+}
+
+// +-2^yf -+ 2^yr (bit 0 of each exponent: its sign).  REV false: the first
+// term alone.  special: a term lies outside the normal range and net_special
+// has to form the result; the code has no branch.
 template <bool REV>
 FX_FN double net_of(int64_t yf, int64_t yr, const int64_t *tab, bool &special) {
-  uint64_t Mf;
-  int E;
-  exp2m(yf, tab, Mf, E);
-  unsigned neg = (unsigned)yf & 1u;
-  int64_t D = (int64_t)Mf;
-  if (REV) {
-    uint64_t Mr;
-    int Er;
-    exp2m(yr, tab, Mr, Er);
-    const int d = E - Er;
-    int sf = d < 0 ? -d : 0, sr = d > 0 ? d : 0;
-    sf = sf > 63 ? 63 : sf;
-    sr = sr > 63 ? 63 : sr;
-    const int64_t r = (int64_t)(Mr >> sr);
-    D = (int64_t)(Mf >> sf) + ((((unsigned)yr & 1u) != neg) ? r : -r);
-    E = d < 0 ? Er : E;
-    neg ^= D < 0;
-    D = D < 0 ? -D : D;
-  }
-  const int lz = clz64(D | 1);
-  const uint64_t m = (uint64_t)D << lz;
-  const int En = E + 7 - lz;  // value = m 2^(En - 63)
-  const bool zero = D == 0 || En < -1100;
-  special = E > 1023 || (!zero && En < -1022);
-  const uint64_t b = (m >> 11) + ((m >> 10) & 1u) + ((uint64_t)(unsigned)(En + 1022) << 52);
-  return of_bits(zero ? 0ull : b | ((uint64_t)neg << 63));
+  const double f = normal_of(yf, tab, special);
+  if (!REV) return f;
+  bool far;
+  const double r = normal_of(yr, tab, far);
+  special |= far;
+  return f - r;
 }
 
 // net_of for any range: terms that overflow give infinities (and their

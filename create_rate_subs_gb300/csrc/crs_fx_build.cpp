@@ -110,7 +110,8 @@ int64_t coefficient(ld v) {
   const Dg d = split(llroundl(std::ldexp(v, 52)));
   return (int64_t)(((uint64_t)(unsigned)d.lo << 32) | (unsigned)d.hi);
 }
-// a 64-bit number as an int2 {high, low}
+// a 64-bit number as an int2 {high, low}; the constant of a sum carries the
+// 1 that rounds its exponent to an even number
 int64_t number(int64_t v) {
   return (int64_t)(((uint64_t)v << 32) | ((uint64_t)v >> 32));
 }
@@ -153,7 +154,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   f.N = N;
   f.R = R;
   f.NPM = NPM;
-  if (R < 1 || N > 65534) return;
+  if (R < 1 || R >= (1 << 22)) return;  // slot offsets in 30 bits
   // interval bounds: the most common T_common in the middle
   double mid = 1000.0;
   {
@@ -169,10 +170,9 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       }
     }
   }
-  f.tb[0] = 120.0;
-  f.tb[1] = 200.0;
-  f.tb[2] = mid;
-  f.tb[3] = 6000.0;
+  f.tb[0] = 200.0;
+  f.tb[1] = mid;
+  f.tb[2] = 6000.0;
   std::vector<int64_t> basis;
   Norm nm[NI];
   for (int q = 0; q < NI; ++q) {
@@ -180,29 +180,17 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
     basis.insert(basis.end(), nm[q].word, nm[q].word + BASIS);
   }
   // pressure modification
-  std::vector<int32_t> pmh(4 * (size_t)std::max(NPM, 1), 0);
-  std::vector<int64_t> pmc((size_t)PMC * NI * std::max(NPM, 1), 0);
+  std::vector<int32_t> pmh(4 * (size_t)std::max(NPM, 1), 0), pm(2 * (size_t)std::max(NPM, 1), 0);
+  std::vector<int64_t> pmc((size_t)PMC / 8 * NI * std::max(NPM, 1), 0);
   std::vector<char> pm_ok(std::max(NPM, 1), 1);
   std::vector<int32_t> pm_rxn(std::max(NPM, 1), 0);
   for (int r = 0; r < R; ++r)
     if (t.pm_idx[r] >= 0) pm_rxn[t.pm_idx[r]] = r;
-  ld worst = 0;
-  for (int p = 0; p < NPM; ++p) {
-    ld s = 0;
-    for (int e = t.pm_eff_ptr[p]; e < t.pm_eff_ptr[p + 1]; ++e)
-      s += std::fabs((ld)t.pm_eff_val[e] * t.inv_mw[t.pm_eff_sp[e]]);
-    worst = std::max(worst, s);
-  }
-  // third-body sums: |sum| <= 2 and 1 / mw < 2 in units of 2^eff_shift
-  f.eff_shift = 1;
-  while (std::ldexp(worst, -f.eff_shift) > 1 && f.eff_shift < 60) ++f.eff_shift;
-  if (std::ldexp(worst, -f.eff_shift) > 1) return;
-  std::vector<int64_t> eff_k;
+  std::vector<double> eff;  // pairs: coefficient, row offset
   for (int p = 0; p < NPM; ++p) {
     int flags = 0;
     const bool thd = t.pm_kind[p] == PM_THD;
     const int sp = thd ? -1 : t.pm_sp[p];
-    if (sp < 0) flags |= PMF_SUM;
     bool ok = true;
     if (!thd) {
       const Row a = row_of(t, t.pm_k0[p]), b = row_of(t, t.pm_kinf[p]);
@@ -213,11 +201,11 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       if (form == FORM_TROE) flags |= PMF_TROE;
       if (form == FORM_SRI) flags |= PMF_SRI;
       for (int q = 0; q < NI && ok; ++q) {
-        int64_t *w = pmc.data() + (size_t)PMC * (NI * p + q);
+        int64_t *w = pmc.data() + (size_t)PMC / 8 * (NI * p + q);
         const Form z = form_of(nm[q], a.base - b.base, a.b - b.b, a.i - b.i, nullptr);
         ok = within(z);
         if (!ok) break;
-        w[0] = number(constant(z.c[0]));
+        w[0] = number(constant(z.c[0]) + 1);
         w[1] = coefficient(z.c[1]);
         w[2] = coefficient(z.c[2]);
         if (form == FORM_TROE) {
@@ -235,30 +223,52 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
             if (ok) {
               const Form y = form_of(nm[q], std::log2((ld)d[3]), d[4], 0, nullptr);
               ok = within(y);
-              w[9] = number(constant(y.c[0]));
+              w[9] = number(constant(y.c[0]) + 1);
               w[10] = coefficient(y.c[1]);
             }
           }
         }
       }
     }
-    for (int e = t.pm_eff_ptr[p]; e < t.pm_eff_ptr[p + 1]; ++e)
-      eff_k.push_back([&] {
-        const Dg d = split(llroundl(std::ldexp(
-            (ld)t.pm_eff_val[e] * t.inv_mw[t.pm_eff_sp[e]], 61 - f.eff_shift)));
-        return (int64_t)(((uint64_t)(unsigned)d.lo << 32) | (unsigned)d.hi);
-      }());
+    for (int e = t.pm_eff_ptr[p]; e < t.pm_eff_ptr[p + 1]; ++e) {
+      eff.push_back(t.pm_eff_val[e] * t.inv_mw[t.pm_eff_sp[e]]);
+      const int64_t off = (int64_t)t.pm_eff_sp[e] * 256;
+      double w;
+      memcpy(&w, &off, 8);
+      eff.push_back(w);
+    }
     pmh[4 * p] = flags;
-    pmh[4 * p + 1] = sp;
-    pmh[4 * p + 2] = pm_rxn[p];
+    pmh[4 * p + 1] = sp < 0 ? -1 : sp * 256;
+    pm[2 * p] = sp < 0 ? pm_rxn[p] * 256 : -1;
     pm_ok[p] = ok;
   }
-  // reactions
-  std::vector<int32_t> hdr(8 * (size_t)R, 0), thr_ptr(R + 1, 0);
-  std::vector<double> thr;
-  std::vector<int64_t> coef;
-  std::vector<int> weight(R);
-  f.uniform = 1;
+  // reactions: thresholds where their coefficients change (the interval
+  // bounds and their own T_common values), then the records
+  std::vector<std::vector<double>> thr(R);
+  size_t nthr = 1;
+  bool uniform = true;
+  for (int r = 0; r < R; ++r) {
+    std::vector<double> &th = thr[r];
+    th = {f.tb[1]};
+    const int j = t.rev_idx[r];
+    if (j >= 0)
+      for (int g = t.kc_ptr[j]; g < t.kc_ptr[j + 1]; ++g) {
+        const double x = t.kc_tmid[g];
+        if (x > f.tb[0] && x < f.tb[NI] && std::find(th.begin(), th.end(), x) == th.end()) {
+          th.push_back(x);
+          uniform = false;
+        }
+      }
+    std::sort(th.begin(), th.end());
+    nthr = std::max(nthr, th.size());
+  }
+  f.nthr = uniform ? 0 : (int)nthr;
+  const int nco = (int)nthr + 1;
+  const int one = HEAD + COEF * nco + (uniform ? 0 : ((int)nthr + 1) / 2 * 16);
+  f.stride[0] = 2 * one;
+  f.stride[1] = one + PMH + PMC * NI;
+  std::vector<std::vector<unsigned char>> rec(R);
+  std::vector<int> weight(R), kind(R);
   int generic = 0;
   for (int r = 0; r < R; ++r) {
     const int j = t.rev_idx[r], p = t.pm_idx[r];
@@ -269,7 +279,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
     for (int side = 0; side < 2; ++side) {
       const int32_t *ptr = side ? t.px_ptr : t.rx_ptr, *sp = side ? t.px_sp : t.rx_sp;
       const int32_t *nint = side ? t.px_nint : t.rx_nint;
-      for (int q = 0; q < 4; ++q) fac[side][q] = N;
+      for (int q = 0; q < 4; ++q) fac[side][q] = N;  // the row of zeros
       if (side && j < 0) break;
       for (int e = ptr[r]; e < ptr[r + 1]; ++e) {
         if (nint[e] < 0) ok = false;
@@ -278,23 +288,13 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       }
       ok &= cnt[side] <= 4;
     }
-    // thresholds: the interval bounds and the reaction's own T_common values
-    std::vector<double> th = {f.tb[1], f.tb[2]};
-    if (j >= 0)
-      for (int g = t.kc_ptr[j]; g < t.kc_ptr[j + 1]; ++g) {
-        const double x = t.kc_tmid[g];
-        if (x > f.tb[0] && x < f.tb[3] && std::find(th.begin(), th.end(), x) == th.end()) {
-          th.push_back(x);
-          f.uniform = 0;
-        }
-      }
-    std::sort(th.begin(), th.end());
-    const int base = (int)(coef.size() / COEF);
+    std::vector<unsigned char> co((size_t)COEF * nco, 0);
+    const std::vector<double> &th = thr[r];
     for (size_t q = 0; q <= th.size(); ++q) {
-      const double hi = q < th.size() ? th[q] : f.tb[3];
+      const double hi = q < th.size() ? th[q] : f.tb[NI];
       int iv = 0;
       while (hi > f.tb[iv + 1]) ++iv;
-      int64_t w[COEF] = {0};
+      int64_t w[COEF / 8] = {0};
       const Form y = form_of(nm[iv], a.base, a.b, a.i, nullptr);
       ok &= within(y);
       Form z = y;
@@ -311,36 +311,45 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
         ok &= within(z);
       }
       if (ok) {
-        w[0] = number(constant(y.c[0]));
+        w[0] = number(constant(y.c[0]) + 1);
         w[1] = coefficient(y.c[1]);
         w[2] = coefficient(y.c[2]);
-        w[3] = number(constant(z.c[0]));
+        w[3] = number(constant(z.c[0]) + 1);
         for (int k = 1; k < 7; ++k) w[3 + k] = coefficient(z.c[k]);
       }
-      coef.insert(coef.end(), w, w + COEF);
+      memcpy(co.data() + COEF * q, w, COEF);
     }
-    thr.insert(thr.end(), th.begin(), th.end());
-    thr_ptr[r + 1] = (int32_t)thr.size();
     if (j >= 0) flags |= RF_REV;
     if (p >= 0) flags |= t.pm_kind[p] == PM_THD ? RF_THD : RF_FALL;
-    if (cnt[0] > 2) flags |= RF_MORE_R;
-    if (cnt[1] > 2) flags |= RF_MORE_P;
+    if (cnt[0] > 2 || cnt[1] > 2) flags |= RF_MORE;
     if (a.neg) flags |= RF_NEG;
     // instruction counts, in units of ten
     weight[r] = (j >= 0 ? 26 : 15) + (p < 0 ? 0 : flags & RF_THD ? 4 : 45);
+    kind[r] = p >= 0 ? 2 : j >= 0 ? 0 : 1;
     if (!ok) {
       flags |= RF_GEN;
       weight[r] = 900;
+      kind[r] = 3;
       ++generic;
     }
-    int32_t *h = hdr.data() + 8 * (size_t)r;
-    h[0] = r;
-    h[1] = flags;
-    h[2] = base;
-    h[3] = p;
-    for (int side = 0; side < 2; ++side) {
-      h[4 + 2 * side] = fac[side][0] | (fac[side][1] << 16);
-      h[5 + 2 * side] = fac[side][2] | (fac[side][3] << 16);
+    const int32_t h[12] = {r * 256, flags, p, r,
+                           fac[0][0] * 256, fac[0][1] * 256, fac[1][0] * 256, fac[1][1] * 256,
+                           fac[0][2] * 256, fac[0][3] * 256, fac[1][2] * 256, fac[1][3] * 256};
+    std::vector<unsigned char> &at = rec[r];
+    auto add = [&](const void *v, size_t n) {
+      at.insert(at.end(), (const unsigned char *)v, (const unsigned char *)v + n);
+    };
+    add(h, HEAD);
+    if (kind[r] != 0) {
+      static const unsigned char none[PMH + PMC * NI] = {0};
+      add(p >= 0 ? (const void *)(pmh.data() + 4 * p) : none, PMH);
+      add(p >= 0 ? (const void *)(pmc.data() + (size_t)PMC / 8 * NI * p) : none, PMC * NI);
+    }
+    add(co.data(), co.size());
+    if (!uniform) {
+      std::vector<double> v((nthr + 1) / 2 * 2, INFINITY);
+      std::copy(th.begin(), th.end(), v.begin());
+      add(v.data(), v.size() * sizeof(double));
     }
   }
   // a reaction in FP64 costs this kernel about four times what it costs the
@@ -348,13 +357,13 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   // reactions those are faster
   f.usable = generic * 5 <= R;
   Buf b;
-  std::vector<int64_t> small(EXP_ENTRIES + 2 * (LOGN + 1)), hp(2 * (LOGN + 1)), lw(N);
-  for (int k = 0; k < EXP_ENTRIES; ++k)
-    small[k] = llroundl(std::ldexp(std::exp2((ld)k / EXP_ENTRIES), 56));
+  std::vector<int64_t> small(EXP_WORDS + 2 * (LOGN + 1)), hp(2 * (LOGN + 1)), lw(N);
+  for (int k = 0; k <= EXPN; ++k)
+    small[k] = llroundl(std::ldexp(std::exp2((ld)k / EXPN), 56)) + 8;
   for (int k = 0; k <= LOGN; ++k) {
     const ld F = 1 + (ld)k / LOGN;
-    small[EXP_ENTRIES + 2 * k] = hp[2 * k] = llroundl(std::ldexp((ld)1, 62) / F);
-    small[EXP_ENTRIES + 2 * k + 1] = llroundl(std::ldexp(std::log2(F), YB));
+    small[EXP_WORDS + 2 * k] = hp[2 * k] = llroundl(std::ldexp((ld)1, 62) / F);
+    small[EXP_WORDS + 2 * k + 1] = llroundl(std::ldexp(std::log2(F), YB));
     hp[2 * k + 1] = llroundl(std::ldexp(std::log2(F), 62));
   }
   for (int k = 0; k < N; ++k) lw[k] = llroundl(std::ldexp(std::log2((ld)t.inv_mw[k]), YB));
@@ -362,24 +371,63 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   f.hp = b.put(hp);
   f.basis = b.put(basis);
   f.lw = b.put(lw);
-  f.hdr = b.put(hdr);
-  f.coef = b.put(coef);
-  f.thr_ptr = b.put(thr_ptr);
-  f.thr = b.put(thr);
-  f.pmh = b.put(pmh);
-  f.pmc = b.put(pmc);
+  f.pm = b.put(pm);
   f.eff_ptr = b.put(std::vector<int32_t>(t.pm_eff_ptr, t.pm_eff_ptr + NPM + 1));
-  f.eff_sp = b.put(std::vector<int32_t>(t.pm_eff_sp, t.pm_eff_sp + t.pm_eff_ptr[NPM]));
-  f.eff_k = b.put(eff_k);
+  f.eff = b.put(eff);
+  // species' terms: coefficients +-1 (small integers repeated) or weighted
+  std::vector<int32_t> term, wterm, where(4 * (size_t)N, 0);
+  std::vector<double> wnu;
+  for (int k = 0; k < N; ++k) {
+    bool small_int = true;
+    for (int e = t.spc_ptr[k]; e < t.spc_ptr[k + 1]; ++e)
+      small_int &= std::fabs(t.spc_nu[e]) <= 3 && t.spc_nu[e] == std::rint(t.spc_nu[e]);
+    int32_t *w = where.data() + 4 * (size_t)k;
+    w[0] = k;
+    w[3] = !small_int;
+    if (small_int) {
+      w[1] = (int32_t)(term.size() / 4);
+      for (int e = t.spc_ptr[k]; e < t.spc_ptr[k + 1]; ++e)
+        for (int q = 0; q < std::abs((int)t.spc_nu[e]); ++q)
+          term.push_back((int32_t)((unsigned)t.spc_r[e] * 256u |
+                                   (t.spc_nu[e] < 0 ? 0x80000000u : 0u)));
+      while (term.size() % 4) term.push_back(R * 256);
+      w[2] = (int32_t)(term.size() / 4) - w[1];
+    } else {
+      w[1] = (int32_t)wterm.size();
+      for (int e = t.spc_ptr[k]; e < t.spc_ptr[k + 1]; ++e) {
+        wterm.push_back(t.spc_r[e] * 256);
+        wnu.push_back(t.spc_nu[e]);
+      }
+      w[2] = t.spc_ptr[k + 1] - t.spc_ptr[k];
+    }
+  }
+  for (int q = 0; q < 4; ++q) term.push_back(R * 256);  // read ahead
+  f.term = b.put(term);
+  f.wterm = b.put(wterm);
+  f.wnu = b.put(wnu);
+  std::vector<int> sw(N);
+  for (int k = 0; k < N; ++k) sw[k] = 2 + t.spc_ptr[k + 1] - t.spc_ptr[k];
+  // the reaction that completes a pair: both rates zero, into the slot of
+  // zeros
+  std::vector<unsigned char> nothing(one, 0);
+  {
+    const int32_t h[12] = {R * 256, RF_REV, -1, -1, N * 256, N * 256, N * 256, N * 256,
+                           N * 256, N * 256, N * 256, N * 256};
+    memcpy(nothing.data(), h, HEAD);
+    const int64_t z = number(ZERO_EXP);
+    for (int q = 0; q < nco; ++q) {
+      memcpy(nothing.data() + HEAD + COEF * q, &z, 8);
+      memcpy(nothing.data() + HEAD + COEF * q + 24, &z, 8);
+    }
+  }
   // work lists: longest first onto the least loaded warp
   for (int l = 0; l < NLIST; ++l) {
     const int nw = warps_of(l);
-    auto deal = [&](const std::vector<int> &w) {
+    auto deal = [&](const std::vector<int> &w, std::vector<long long> load) {
       std::vector<int> order(w.size());
       for (size_t i = 0; i < w.size(); ++i) order[i] = (int)i;
       std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return w[a] > w[c]; });
       std::vector<std::vector<int>> bins(nw);
-      std::vector<long long> load(nw, 0);
       for (int i : order) {
         const int best = (int)(std::min_element(load.begin(), load.end()) - load.begin());
         bins[best].push_back(i);
@@ -387,32 +435,42 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       }
       return bins;
     };
-    std::vector<std::vector<int>> bins = deal(weight);
-    std::vector<int32_t> ptr(1, 0), rev, list;
-    for (auto &v : bins) {
-      auto plain = [&](int r) { return hdr[8 * (size_t)r + 1] == (RF_REV | (hdr[8 * (size_t)r + 1] & (RF_MORE_R | RF_MORE_P | RF_NEG))); };
-      std::sort(v.begin(), v.end(), [&](int a, int c) {
-        const bool pa = plain(a), pc = plain(c);
-        return pa != pc ? pa : a < c;
-      });
-      rev.push_back((int32_t)std::count_if(v.begin(), v.end(), plain));
-      list.insert(list.end(), v.begin(), v.end());
-      ptr.push_back((int32_t)list.size());
+    // warps 0 and 1 also form the next tile's sums (chains of N dependent
+    // FP64 additions), warp 2 its functions of T
+    std::vector<long long> load(nw, 0);
+    load[0] = load[1] = 2 * N;
+    load[2] = 60;
+    std::vector<std::vector<int>> bins = deal(weight, load);
+    for (int c = 0; c < 2; ++c) {
+      std::vector<int32_t> ptr(1, 0);
+      std::vector<unsigned char> lr;
+      for (auto &v : bins) {
+        std::sort(v.begin(), v.end(), [&](int x, int y) {
+          return kind[x] != kind[y] ? kind[x] < kind[y] : x < y;
+        });
+        int n = 0;
+        for (int r : v)
+          if ((kind[r] != 0) == (c == 1)) {
+            lr.insert(lr.end(), rec[r].begin(), rec[r].end());
+            ++n;
+          }
+        if (c == 0) {
+          if (n & 1) lr.insert(lr.end(), nothing.begin(), nothing.end());
+          n = (n + 1) / 2;
+        }
+        ptr.push_back(ptr.back() + n);
+      }
+      f.list_ptr[l][c] = b.put(ptr);
+      f.rec[l][c] = b.put(lr);
     }
-    f.list_ptr[l] = b.put(ptr);
-    f.list_rev[l] = b.put(rev);
-    f.list[l] = b.put(list);
-    std::vector<int> sw(N);
-    for (int k = 0; k < N; ++k) sw[k] = 2 + t.spc_ptr[k + 1] - t.spc_ptr[k];
-    bins = deal(sw);
-    ptr.assign(1, 0);
-    list.clear();
+    bins = deal(sw, std::vector<long long>(nw, 0));
+    std::vector<int32_t> ptr(1, 0), seg;
     for (auto &v : bins) {
-      list.insert(list.end(), v.begin(), v.end());
-      ptr.push_back((int32_t)list.size());
+      for (int k : v) seg.insert(seg.end(), where.begin() + 4 * k, where.begin() + 4 * k + 4);
+      ptr.push_back((int32_t)(seg.size() / 4));
     }
-    f.sum_ptr[l] = b.put(ptr);
-    f.sum[l] = b.put(list);
+    f.seg_ptr[l] = b.put(ptr);
+    f.seg[l] = b.put(seg);
   }
   f.bytes = (int)b.b.size();
   out.swap(b.b);

@@ -7,38 +7,47 @@
 namespace crs {
 namespace fx {
 
-// Temperature intervals (TB[q], TB[q + 1]] on which the functions of T are
-// normalised; the middle bound is the mechanism's most common T_common.
-constexpr int NI = 3;
-constexpr int NLIST = 3;               // work lists for 4, 8 and 16 warps per CTA
-constexpr int COEF = 10;               // 8-byte words per coefficient record
-constexpr int PMC = 12;                // and per pressure-modification record
-constexpr int BASIS = 9;               // and per interval's normalisation
+// Temperature intervals (tb[q], tb[q + 1]] on which the functions of T are
+// normalised; the second bound is the mechanism's most common T_common.
+constexpr int NI = 2;
+constexpr int NLIST = 3;  // work lists for 4, 8 and 16 warps per CTA
+// A reaction's record: its head, int4 {slot offset, flags, fall-off entry,
+// reaction}, int4 {two reactants, two products}, int4 {the third and fourth
+// of each}, as offsets of tile rows; for reactions with pressure
+// modification int4 {flags, species row or -1, 0, 0} and a record per
+// interval; its coefficients per interval; its T thresholds if any.
+constexpr int HEAD = 48;
+constexpr int PMH = 16, PMC = 96;
+constexpr int COEF = 80;
+constexpr int BASIS = 9;  // words of an interval's normalisation
 
-// reaction flags
-enum { RF_REV = 1, RF_THD = 2, RF_FALL = 4, RF_GEN = 8, RF_MORE_R = 16, RF_MORE_P = 32,
-       RF_NEG = 64 };
+// reaction flags (RF_NEG is bit 0: the sign bit of an exponent)
+enum { RF_NEG = 1, RF_REV = 2, RF_THD = 4, RF_FALL = 8, RF_GEN = 16, RF_MORE = 32 };
 // pressure-modification flags; T1, T2, T3: exponential terms present
 enum { PMF_LOW = 1, PMF_TROE = 2, PMF_SRI = 4, PMF_DE = 8, PMF_T1 = 16, PMF_T2 = 32,
-       PMF_T3 = 64, PMF_SUM = 128 };
+       PMF_T3 = 64 };
 
 // Passed by value; offsets in bytes into the buffer.
 struct FxTab {
   int N, R, NPM;
-  int usable;       // the kernel takes this mechanism
-  int uniform;      // every reaction changes coefficients at the interval bounds only
-  int eff_shift;    // third-body sums are formed in units of 2^eff_shift
+  int usable;            // the kernel takes this mechanism
+  int nthr;              // T thresholds per reaction record; 0: the interval bounds
+  int stride[2];         // bytes of a pair of plain reversible reactions' records and of
+                         // another reaction's
   double tb[NI + 1];
-  int small, hp, basis;        // exponential and logarithm tables; log2 T; normalisation
-  int lw;                      // [N] log2(1 / W_k)
-  int hdr, coef;               // [R] 2 x int4; coefficient records
-  int thr_ptr, thr;            // [R + 1], T thresholds of each reaction (uniform = 0)
-  int pmh, pmc;                // [NPM] int4 {flags, species, reaction, 0}; [NPM][NI] records
-  int eff_ptr, eff_sp, eff_k;  // third-body lists
-  // per warp: its reactions, plain reversible ones first (their number in
-  // list_rev), and its species
-  int list_ptr[NLIST], list_rev[NLIST], list[NLIST];
-  int sum_ptr[NLIST], sum[NLIST];
+  int small, hp, basis;  // exponential and logarithm tables; log2 T; normalisation
+  int lw;                // [N] log2(1 / W_k)
+  int pm;                // [NPM] int2 {slot offset or -1: no third-body sum, 0}
+  int eff_ptr, eff;      // third-body lists: {double (eff - 1) / W, int row offset, int 0}
+  // per warp: its plain reversible reactions' records in pairs (an odd
+  // number is completed with one that puts zero into the slot of zeros), its
+  // other reactions' records, and its species' terms
+  int list_ptr[NLIST][2], rec[NLIST][2];
+  // int4 {species, first, number, weighted}: groups of four terms {slot
+  // offset, bit 31: subtract}, completed with the slot of zeros (row R); or,
+  // weighted, single terms with a coefficient
+  int seg_ptr[NLIST], seg[NLIST];
+  int term, wterm, wnu;
   int bytes;
 };
 

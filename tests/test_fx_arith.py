@@ -21,9 +21,8 @@ SOURCE = r"""
 using namespace crs::fx;
 typedef long double ld;
 int main() {
-  std::vector<int64_t> et(EXP_ENTRIES), lt(2 * (LOGN + 1)), hp(2 * (LOGN + 1));
-  for (int j = 0; j < EXP_ENTRIES; ++j)
-    et[j] = llroundl(ldexpl(exp2l((ld)j / EXP_ENTRIES), 56));
+  std::vector<int64_t> et(EXP_WORDS), lt(2 * (LOGN + 1)), hp(2 * (LOGN + 1));
+  for (int j = 0; j <= EXPN; ++j) et[j] = llroundl(ldexpl(exp2l((ld)j / EXPN), 56)) + 8;
   for (int j = 0; j <= LOGN; ++j) {
     const ld F = 1 + (ld)j / LOGN;
     lt[2 * j] = hp[2 * j] = llroundl(ldexpl(1, 62) / F);
