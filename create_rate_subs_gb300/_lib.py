@@ -82,6 +82,8 @@ def _sig(lib):
                               _i64, _vp, _i64, _vp, _vp],
         "crs_adam_step": [_vp, _vp, _vp, _vp, _i64, _i64, ctypes.c_float, ctypes.c_float,
                           ctypes.c_float, ctypes.c_float, _i32, _vp, _i64, _vp, _i64, _vp],
+        "crs_adam_steps": [_i32, _vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_float, ctypes.c_float,
+                           ctypes.c_float, ctypes.c_float, _i32, _vp, _vp, _vp, _vp, _vp],
         "crs_surrogate_features": [_i64, _vp, _vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _vp,
                                    _i64, _vp, _i64, _i32, _vp, _vp, _vp],
         "crs_surrogate_output": [_i64, _vp, _i64, _i32, _vp, _vp, _vp, _i32, ctypes.c_float,

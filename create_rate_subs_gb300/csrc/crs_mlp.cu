@@ -152,75 +152,134 @@ struct EpiPartial {
   }
 };
 
-__global__ void k_reduce_partials(const float *P, int splits, int64_t rows_pad,
-                                  int64_t cols_pad, int64_t rows, int64_t cols, float *dW) {
-  const int64_t n = rows * cols;
+// Sums in slice order, eight slices of loads in flight.
+__global__ void __launch_bounds__(256)
+    k_reduce_partials(const float *P, int splits, int64_t rows_pad, int64_t cols_pad,
+                      int64_t rows, int64_t cols, float *dW) {
+  const int64_t n = rows * cols, slice = rows_pad * cols_pad;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
        idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx / cols, c = idx % cols;
+    const float *p = P + idx / cols * cols_pad + idx % cols;
     float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += P[((int64_t)z * rows_pad + r) * cols_pad + c];
+#pragma unroll 8
+    for (int z = 0; z < splits; ++z) s += p[z * slice];
     dW[idx] = s;
   }
 }
 
-// Row sums of a [rows][ld] bf16 matrix over its first m columns (one warp
-// per row, fixed order).
-__global__ void k_row_sums(const __nv_bfloat16 *X, int64_t ld, int64_t rows, int64_t m,
-                           float *out) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
+// Row sums of a [rows][ld] bf16 matrix over its first m columns: a CTA per
+// row, eight columns per load where the rows' addresses allow it (one warp
+// per row and a column per load took 30 us for 256 rows of 16,384), a fixed
+// order of summation.
+__global__ void __launch_bounds__(256)
+    k_row_sums(const __nv_bfloat16 *X, int64_t ld, int64_t m, float *out) {
+  __shared__ float part[8];
+  const __nv_bfloat16 *x = X + (int64_t)blockIdx.x * ld;
   float s = 0.0f;
-  for (int64_t i = lane; i < m; i += 32) s += __bfloat162float(X[row * ld + i]);
+  int64_t done = 0;
+  if (!(reinterpret_cast<uintptr_t>(x) & 15)) {
+    done = m / 8 * 8;
+    for (int64_t i = (int64_t)threadIdx.x * 8; i < done; i += 256 * 8) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(x + i);
+      const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 f = __bfloat1622float2(h[u]);
+        s += f.x;
+        s += f.y;
+      }
+    }
+  }
+  for (int64_t i = done + threadIdx.x; i < m; i += 256) s += __bfloat162float(x[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[row] = s;
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w];
+    out[blockIdx.x] = t;
+  }
 }
 
 // loss = sum (y - t)^2 * scale, dY = 2 scale (y - t) (bf16, row-major and
-// transposed); columns >= n are zero in dY.
-__global__ void k_loss_grad(const float *Yh, int64_t ldy, const float *Tg, int64_t ldt,
-                            int64_t m, int64_t n, int64_t n_pad, float scale,
-                            __nv_bfloat16 *dY, int64_t ld, __nv_bfloat16 *dYT, int64_t ldtt,
-                            float *loss) {
+// transposed); columns >= n are zero in dY.  A CTA takes 64 x 64 values
+// through shared memory, so that the rows of both outputs are written
+// whole (element by element the transposed stores took 53 us for 16,384 x
+// 64).
+__global__ void __launch_bounds__(256)
+    k_loss_grad(const float *Yh, int64_t ldy, const float *Tg, int64_t ldt, int64_t m, int64_t n,
+                int64_t n_pad, float scale, __nv_bfloat16 *dY, int64_t ld, __nv_bfloat16 *dYT,
+                int64_t ldtt, float *loss) {
+  __shared__ __nv_bfloat16 tile[64][66];
+  __shared__ float part[8];
+  const int64_t r0 = (int64_t)blockIdx.x * 64, c0 = (int64_t)blockIdx.y * 64;
+  const int x = threadIdx.x & 63, y = threadIdx.x >> 6;
   float acc = 0.0f;
-  const int64_t total = m * n_pad;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx / n_pad, c = idx % n_pad;
+#pragma unroll 4
+  for (int j = y; j < 64; j += 4) {
+    const int64_t r = r0 + j, c = c0 + x;
     float g = 0.0f;
-    if (c < n) {
+    if (r < m && c < n) {
       const float d = Yh[r * ldy + c] - Tg[r * ldt + c];
       acc += d * d;
       g = 2.0f * scale * d;
     }
     const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    dY[r * ld + c] = gb;
-    dYT[c * ldtt + r] = gb;
+    tile[j][x] = gb;
+    if (r < m && c < n_pad) dY[r * ld + c] = gb;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, acc * scale);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+  __syncthreads();
+#pragma unroll 4
+  for (int j = y; j < 64; j += 4)
+    if (r0 + x < m && c0 + j < n_pad) dYT[(c0 + j) * ldtt + r0 + x] = tile[x][j];
+  if (threadIdx.x == 0 && loss) {
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w];
+    atomicAdd(loss, t * scale);
+  }
 }
 
-__global__ void k_adam(float *p, const float *g, float *mo, float *ve, int64_t rows,
-                       int64_t cols, float lr, float b1, float b2, float eps, float c1,
-                       float c2, __nv_bfloat16 *W, int64_t ldw, __nv_bfloat16 *WT,
-                       int64_t ldwt) {
-  const int64_t n = rows * cols;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const float gi = g[idx];
-    const float m = b1 * mo[idx] + (1.0f - b1) * gi;
-    const float v = b2 * ve[idx] + (1.0f - b2) * gi * gi;
-    mo[idx] = m;
-    ve[idx] = v;
-    const float w = p[idx] - lr * (m * c1) / (sqrtf(v * c2) + eps);
-    p[idx] = w;
-    const int64_t r = idx / cols, c = idx % cols;
-    if (W) W[r * ldw + c] = __float2bfloat16_rn(w);
-    if (WT) WT[c * ldwt + r] = __float2bfloat16_rn(w);
+// One tensor of an Adam step.
+struct AdamTensor {
+  float *p;
+  const float *g;
+  float *m, *v;
+  __nv_bfloat16 *W, *WT;
+  int64_t rows, cols, ldw, ldwt;
+};
+constexpr int ADAM_MAX = 16;
+struct AdamSet {
+  AdamTensor t[ADAM_MAX];
+  int first[ADAM_MAX + 1];  // first CTA of each tensor
+};
+
+// All tensors of a step in one launch: a CTA belongs to one tensor.
+__global__ void __launch_bounds__(256)
+    k_adam(const __grid_constant__ AdamSet set, int count, float lr, float b1, float b2,
+           float eps, float c1, float c2) {
+  int q = 0;
+  while (q + 1 < count && (int)blockIdx.x >= set.first[q + 1]) ++q;
+  const AdamTensor &a = set.t[q];
+  const int64_t n = a.rows * a.cols;
+  const int64_t step = (int64_t)(set.first[q + 1] - set.first[q]) * blockDim.x;
+  for (int64_t idx = (int64_t)(blockIdx.x - set.first[q]) * blockDim.x + threadIdx.x; idx < n;
+       idx += step) {
+    const float gi = a.g[idx];
+    const float m = b1 * a.m[idx] + (1.0f - b1) * gi;
+    const float v = b2 * a.v[idx] + (1.0f - b2) * gi * gi;
+    a.m[idx] = m;
+    a.v[idx] = v;
+    const float w = a.p[idx] - lr * (m * c1) / (sqrtf(v * c2) + eps);
+    a.p[idx] = w;
+    const int64_t r = idx / a.cols, c = idx % a.cols;
+    if (a.W) a.W[r * a.ldw + c] = __float2bfloat16_rn(w);
+    if (a.WT) a.WT[c * a.ldwt + r] = __float2bfloat16_rn(w);
   }
 }
 
@@ -500,8 +559,18 @@ cudaError_t gemm_bn(const CUtensorMap &ta, const CUtensorMap &tb, int64_t M_pad,
   }
 }
 
-inline int pick_bn(int64_t n_pad) {
-  return n_pad % 256 == 0 ? 256 : n_pad % 128 == 0 ? 128 : n_pad % 64 == 0 ? 64 : 0;
+// Columns per CTA: the narrowest tile whose CTAs (m_tiles rows of 128 each)
+// still run as one wave, two per SM, so that one's epilogue overlaps
+// another's loads; re-reading A from L2 for more column tiles costs less
+// than an idle SM, a second wave does not.
+inline int pick_bn(int64_t n_pad, int64_t m_tiles) {
+  int bn = n_pad % 256 == 0 ? 256 : n_pad % 128 == 0 ? 128 : n_pad % 64 == 0 ? 64 : 0;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return bn;
+  while (bn > 64 && m_tiles * (n_pad / bn) * 2 <= 2 * (int64_t)sms) bn /= 2;
+  return bn;
 }
 
 inline int bad(const char *fn) {
@@ -530,7 +599,7 @@ int crs_mlp_forward(const void *X, const void *W, const float *b, int64_t M_pad,
                     int64_t K, int64_t M, int64_t N, int act, float *Z, int64_t ldz, void *A,
                     int64_t lda, void *AT, int64_t ldat, float *Y32, int64_t ldy,
                     void *stream) {
-  const int bn = mlp::pick_bn(N_pad);
+  const int bn = mlp::pick_bn(N_pad, M_pad / 128);
   if (!X || !W || M_pad % 128 || K % 64 || !bn || M > M_pad || N > N_pad) return bad(__func__);
   CUtensorMap ta, tb;
   if (!make_tmap_bf16(&ta, X, M_pad, K, 128) || !make_tmap_bf16(&tb, W, N_pad, K, bn))
@@ -545,7 +614,7 @@ int crs_mlp_backward_data(const void *dZ, const void *WT, int64_t M_pad, int64_t
                           int64_t Kout, int64_t M, int64_t Nin, const float *Zprev,
                           int64_t ldz, void *dZprev, int64_t ld, void *dZprevT, int64_t ldt,
                           void *stream) {
-  const int bn = mlp::pick_bn(Nin_pad);
+  const int bn = mlp::pick_bn(Nin_pad, M_pad / 128);
   if (!dZ || !WT || !Zprev || !dZprev || M_pad % 128 || Kout % 64 || !bn) return bad(__func__);
   CUtensorMap ta, tb;
   if (!make_tmap_bf16(&ta, dZ, M_pad, Kout, 128) || !make_tmap_bf16(&tb, WT, Nin_pad, Kout, bn))
@@ -559,7 +628,7 @@ int crs_mlp_backward_data(const void *dZ, const void *WT, int64_t M_pad, int64_t
 int crs_mlp_backward_weight(const void *dZT, const void *AT, int64_t Nout_pad, int64_t Nin_pad,
                             int64_t M_pad, int64_t Nout, int64_t Nin, int splits,
                             float *partial, float *dW, void *stream) {
-  const int bn = mlp::pick_bn(Nin_pad);
+  const int bn = mlp::pick_bn(Nin_pad, Nout_pad / 128 * (splits > 0 ? splits : 1));
   if (!dZT || !AT || !partial || !dW || Nout_pad % 128 || M_pad % 64 || !bn || splits < 1 ||
       (M_pad / 64) % splits)
     return bad(__func__);
@@ -579,8 +648,8 @@ int crs_mlp_row_sums(const void *X, int64_t ld, int64_t rows, int64_t m, float *
                      void *stream) {
   if (!X || !out || rows < 0 || m < 0 || ld < m) return bad(__func__);
   if (rows == 0) return CRS_OK;
-  mlp::k_row_sums<<<(unsigned)((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16 *>(X), ld, rows, m, out);
+  mlp::k_row_sums<<<(unsigned)rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16 *>(X), ld, m, out);
   return done(cudaGetLastError(), __func__);
 }
 
@@ -588,9 +657,37 @@ int crs_mlp_loss_grad(const float *Yh, int64_t ldy, const float *Tg, int64_t ldt
                       int64_t n, int64_t n_pad, float scale, void *dY, int64_t ld, void *dYT,
                       int64_t ldtt, float *loss, void *stream) {
   if (!Yh || !Tg || !dY || !dYT || m < 0 || n > n_pad) return bad(__func__);
-  mlp::k_loss_grad<<<mlp::grid1(m * n_pad), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  if (m == 0 || n_pad == 0) return CRS_OK;
+  const dim3 grid((unsigned)((m + 63) / 64), (unsigned)((n_pad + 63) / 64));
+  mlp::k_loss_grad<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       Yh, ldy, Tg, ldt, m, n, n_pad, scale, static_cast<__nv_bfloat16 *>(dY), ld,
       static_cast<__nv_bfloat16 *>(dYT), ldtt, loss);
+  return done(cudaGetLastError(), __func__);
+}
+
+int crs_adam_steps(int count, float *const *p, const float *const *g, float *const *m,
+                   float *const *v, const int64_t *rows, const int64_t *cols, float lr, float b1,
+                   float b2, float eps, int step, void *const *W, const int64_t *ldw,
+                   void *const *WT, const int64_t *ldwt, void *stream) {
+  if (count < 0 || count > mlp::ADAM_MAX || !p || !g || !m || !v || !rows || !cols || !W ||
+      !ldw || !WT || !ldwt || step < 1)
+    return bad(__func__);
+  mlp::AdamSet set{};
+  int ctas = 0;
+  for (int q = 0; q < count; ++q) {
+    if (!p[q] || !g[q] || !m[q] || !v[q] || rows[q] < 0 || cols[q] < 0) return bad(__func__);
+    set.t[q] = mlp::AdamTensor{p[q], g[q], m[q], v[q], static_cast<__nv_bfloat16 *>(W[q]),
+                               static_cast<__nv_bfloat16 *>(WT[q]), rows[q], cols[q], ldw[q],
+                               ldwt[q]};
+    set.first[q] = ctas;
+    ctas += mlp::grid1(rows[q] * cols[q]);
+  }
+  for (int q = count; q <= mlp::ADAM_MAX; ++q) set.first[q] = ctas;
+  if (ctas == 0) return CRS_OK;
+  const float c1 = 1.0f / (1.0f - powf(b1, (float)step));
+  const float c2 = 1.0f / (1.0f - powf(b2, (float)step));
+  mlp::k_adam<<<(unsigned)ctas, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      set, count, lr, b1, b2, eps, c1, c2);
   return done(cudaGetLastError(), __func__);
 }
 
@@ -598,12 +695,8 @@ int crs_adam_step(float *p, const float *g, float *m, float *v, int64_t rows, in
                   float lr, float b1, float b2, float eps, int step, void *W, int64_t ldw,
                   void *WT, int64_t ldwt, void *stream) {
   if (!p || !g || !m || !v || rows < 0 || cols < 0 || step < 1) return bad(__func__);
-  const float c1 = 1.0f / (1.0f - powf(b1, (float)step));
-  const float c2 = 1.0f / (1.0f - powf(b2, (float)step));
-  mlp::k_adam<<<mlp::grid1(rows * cols), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      p, g, m, v, rows, cols, lr, b1, b2, eps, c1, c2, static_cast<__nv_bfloat16 *>(W), ldw,
-      static_cast<__nv_bfloat16 *>(WT), ldwt);
-  return done(cudaGetLastError(), __func__);
+  return crs_adam_steps(1, &p, &g, &m, &v, &rows, &cols, lr, b1, b2, eps, step, &W, &ldw, &WT,
+                        &ldwt, stream);
 }
 
 int crs_surrogate_features(int64_t n, const double *T, const double *P, const double *Y,

@@ -269,19 +269,25 @@ class MLP(object):
                     _p(b["Z"][l - 1]), d[l], _p(b["dZ"][l - 1]), p[l],
                     _p(b["dZT"][l - 1]), M, s))
         self.step += 1
-        for l in range(L):
-            _lib.check(lib.crs_adam_step(
-                _p(self.W32[l]), _p(self.gW[l]), _p(self.mW[l]), _p(self.vW[l]),
-                d[l + 1], d[l], lr, b1, b2, eps, self.step,
-                _p(self.W[l]), p[l], _p(self.WT[l]), p[l + 1], s))
-            _lib.check(lib.crs_adam_step(
-                _p(self.b32[l]), _p(self.gb[l]), _p(self.mb[l]), _p(self.vb[l]),
-                1, d[l + 1], lr, b1, b2, eps, self.step, None, 0, None, 0, s))
+        # every tensor's update in one launch (16 tensors at most per call)
+        ts = [(self.W32[l], self.gW[l], self.mW[l], self.vW[l], d[l + 1], d[l], self.W[l], p[l],
+               self.WT[l], p[l + 1]) for l in range(L)]
+        ts += [(self.b32[l], self.gb[l], self.mb[l], self.vb[l], 1, d[l + 1], None, 0, None, 0)
+               for l in range(L)]
+        for o in range(0, len(ts), 16):
+            cols = list(zip(*ts[o:o + 16]))
+            k = len(cols[0])
+            ptr = [(ctypes.c_void_p * k)(*[None if t is None else t.data_ptr() for t in cols[j]])
+                   for j in (0, 1, 2, 3, 6, 8)]
+            num = [(ctypes.c_int64 * k)(*cols[j]) for j in (4, 5, 7, 9)]
+            _lib.check(lib.crs_adam_steps(k, ptr[0], ptr[1], ptr[2], ptr[3], num[0], num[1], lr,
+                                          b1, b2, eps, self.step, ptr[4], num[2], ptr[5], num[3],
+                                          s))
         return b
 
     def launches_per_step(self):
         """Kernels one train_step launches."""
-        return self.L + 1 + 2 * self.L + self.L + (self.L - 1) + 2 * self.L
+        return self.L + 1 + 2 * self.L + self.L + (self.L - 1) + (2 * self.L + 15) // 16
 
 
 def surrogate_error(w, w_exact, scale):

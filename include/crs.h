@@ -283,6 +283,13 @@ int crs_adam_step(float *p, const float *g, float *m, float *v, int64_t rows,
                   int64_t cols, float lr, float b1, float b2, float eps,
                   int step, void *W, int64_t ldw, void *WT, int64_t ldwt,
                   void *stream);
+/* The same for `count` (at most 16) tensors in one launch: arrays of their
+ * pointers, sizes and strides. */
+int crs_adam_steps(int count, float *const *p, const float *const *g,
+                   float *const *m, float *const *v, const int64_t *rows,
+                   const int64_t *cols, float lr, float b1, float b2, float eps,
+                   int step, void *const *W, const int64_t *ldw,
+                   void *const *WT, const int64_t *ldwt, void *stream);
 /* Network input of n states (SoA as crs_wdot): features T, ln P and
  * ln(Y_k + 1e-12) for all nsp species (Y_N = 1 - sum), standardised by
  * mu/sd, as bf16 X [n][ldx] (zero to nfeat_pad; nfeat_pad and ldx
