@@ -189,7 +189,8 @@ __device__ __forceinline__ int basis_of(const FxTab &f, const unsigned char *tab
 struct Args {
   const unsigned char *tab;  // fixed-point tables
   const unsigned char *img;  // table image (general FP64 arithmetic)
-  double *q;                 // [gridDim.x][R][32] scratch when QS is false
+  double *q;                 // [gridDim.x / CL][R + 1][32] scratch when QS is false
+  int list;                  // the work list for NW CL warps
 };
 
 // A reaction's record in shared memory: its head and the coefficients of
@@ -368,11 +369,26 @@ __device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const B
   }
 }
 
-template <int LIST, int PER_SM, bool QS, bool TS>
-__global__ void __launch_bounds__(warps_of(LIST) * 32, PER_SM)
+// Barrier of the CTAs that share a tile.
+template <int CL>
+__device__ __forceinline__ void tile_barrier() {
+  if (CL == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+// NW warps per CTA, CL CTAs (a cluster) per tile: each forms the tile's
+// exponents for itself, evaluates its share of the reactions and, the rates
+// exchanged through global memory, of the species.
+template <int NW, int PER_SM, int CL, bool QS, bool TS>
+__global__ void __launch_bounds__(NW * 32, PER_SM)
     k_wdot_tile(const __grid_constant__ ImgLayout lay, const __grid_constant__ FxTab f,
                 const __grid_constant__ Args g, const __grid_constant__ Batch b) {
-  constexpr int NW = warps_of(LIST);
+  static_assert(CL == 1 || !QS, "a cluster's rates are in global memory");
+  const int LIST = g.list;
   extern __shared__ __align__(128) unsigned char smem[];
   const int N = f.N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -397,7 +413,7 @@ __global__ void __launch_bounds__(warps_of(LIST) * 32, PER_SM)
   unsigned char *ring = next + warp * rb;
   next += NW * rb;
   unsigned char *q = (QS ? next : reinterpret_cast<unsigned char *>(g.q) +
-                                      (int64_t)blockIdx.x * (f.R + 1) * 256) + lane * 8;
+                                      (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256) + lane * 8;
   auto Yl = [&](int off) -> int64_t & { return *reinterpret_cast<int64_t *>(yl + off); };
   auto Q = [&](int off) -> double & { return *reinterpret_cast<double *>(q + off); };
   if (warp == 0) {
@@ -406,32 +422,36 @@ __global__ void __launch_bounds__(warps_of(LIST) * 32, PER_SM)
   }
   Ring<DP> plain_ring;
   Ring<DO> other_ring;
+  const int gw = CL == 1 ? warp : (int)(blockIdx.x % CL) * NW + warp;  // the tile's warp
   {
-    const int *lp = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][0]) + warp;
-    const int *lo = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][1]) + warp;
+    const int *lp = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][0]) + gw;
+    const int *lo = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][1]) + gw;
     plain_ring = Ring<DP>{tab + f.rec[LIST][0] + (int64_t)lp[0] * f.stride[0], smem_u32(ring),
                           f.stride[0], lp[1] - lp[0], lane};
     other_ring = Ring<DO>{tab + f.rec[LIST][1] + (int64_t)lo[0] * f.stride[1], smem_u32(ring),
                           f.stride[1], lo[1] - lo[0], lane};
   }
-  const int s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[warp];
-  const int s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[warp + 1];
+  const int s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw];
+  const int s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw + 1];
+  const int4 *terms = reinterpret_cast<const int4 *>(tab + f.term[LIST]) +
+                      reinterpret_cast<const int *>(tab + f.term_ptr[LIST])[gw];
   const unsigned yrows = smem_u32(smem) + lane * 8;
   const double *inv_mw = reinterpret_cast<const double *>(g.img + lay.inv_mw);
   int bad = 0, bk = 0;
-  int64_t tile = blockIdx.x;
+  int64_t tile = blockIdx.x / CL;
+  const int64_t step = gridDim.x / CL;
   const int64_t ntiles = (b.n + 31) / 32;
   if (tile < ntiles) {
     const int64_t i = tile * 32 + lane < b.n ? tile * 32 + lane : tile * 32;
     load_y<NW>(b.Y + i, b.ld, N, warp, yrows);
     if (warp < 3) prepare(f, g, inv_mw, b, i, warp, lane, lt, blk0);
   }
-  for (; tile < ntiles; tile += gridDim.x, bk ^= 1) {
+  for (; tile < ntiles; tile += step, bk ^= 1) {
     const int64_t i = tile * 32 + lane;
     const bool valid = i < b.n;
     const int64_t ic = valid ? i : tile * 32;  // idle lanes repeat a valid state
     asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
+    tile_barrier<CL>();
     unsigned char *o = blk0 + bk * ROWS * 256;
     auto rowd = [&](int r) { return *reinterpret_cast<const double *>(o + r * 256); };
     int *marks = reinterpret_cast<int *>(o + 10 * 256 - lane * 8) + lane;
@@ -476,8 +496,8 @@ __global__ void __launch_bounds__(warps_of(LIST) * 32, PER_SM)
     __syncthreads();
     // net rates
     {
-      if (warp < 3 && tile + gridDim.x < ntiles) {
-        const int64_t j = (tile + gridDim.x) * 32;
+      if (warp < 3 && tile + step < ntiles) {
+        const int64_t j = (tile + step) * 32;
         prepare(f, g, inv_mw, b, j + lane < b.n ? j + lane : j, warp, lane, lt,
                 blk0 + (bk ^ 1) * ROWS * 256);
       }
@@ -570,42 +590,51 @@ __global__ void __launch_bounds__(warps_of(LIST) * 32, PER_SM)
       if (later || all)
         finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
     }
-    __syncthreads();
+    tile_barrier<CL>();
     // the next tile's mass fractions replace exponents that every warp is
     // done with, while the species sums run
-    if (tile + gridDim.x < ntiles) {
-      const int64_t j = (tile + gridDim.x) * 32;
+    if (tile + step < ntiles) {
+      const int64_t j = (tile + step) * 32;
       load_y<NW>(b.Y + (j + lane < b.n ? j + lane : j), b.ld, N, warp, yrows);
     }
-    for (int a = s0; a < s1; ++a) {
-      const int4 sg = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a);
-      double w = 0.0, w2 = 0.0;
-      if (!sg.w) {
-        const int4 *tm = reinterpret_cast<const int4 *>(tab + f.term) + sg.y;
-        int4 t = __ldg(tm);
-        for (int e = 0; e < sg.z; ++e) {
-          const int4 c = t;
-          t = __ldg(tm + e + 1);
-          auto signed_q = [&](int x) {
-            const double v = Q(x & 0x7fffffff);
-            return __hiloint2double(__double2hiint(v) ^ (x & 0x80000000), __double2loint(v));
-          };
-          const double v0 = signed_q(c.x), v1 = signed_q(c.y), v2 = signed_q(c.z),
-                       v3 = signed_q(c.w);
-          w += v0;
-          w2 += v1;
-          w += v2;
-          w2 += v3;
+    {
+      // the groups of the warp's species are one stream: the rates of the
+      // next group are on their way while a group is added
+      auto rates = [&](int4 t, double (&v)[4]) {
+        const int x[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double d = Q(x[u] & 0x7fffffff);
+          v[u] = __hiloint2double(__double2hiint(d) ^ (x[u] & 0x80000000), __double2loint(d));
         }
-      } else {
-        for (int e = sg.y; e < sg.y + sg.z; ++e)
+      };
+      const int4 *tm = terms;
+      double v[4];
+      rates(__ldg(tm), v);
+      int4 t = __ldg(tm + 1);
+      for (int a = s0; a < s1; ++a) {
+        const int4 sg = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a);
+        double w = 0.0, w2 = 0.0;
+        for (int e = 0; e < sg.y; ++e) {
+          double u[4];
+          rates(t, u);
+          t = __ldg(tm + 2);
+          ++tm;
+          w += v[0];
+          w2 += v[1];
+          w += v[2];
+          w2 += v[3];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[c] = u[c];
+        }
+        for (int e = sg.z; e < sg.z + sg.w; ++e)
           w = fma(__ldg(reinterpret_cast<const double *>(tab + f.wnu) + e),
                   Q(__ldg(reinterpret_cast<const int *>(tab + f.wterm) + e)), w);
-      }
-      w += w2;
-      if (valid) {
-        bad += ((__double2hiint(w) >> 20) & 0x7ff) == 0x7ff;  // inf or NaN, integer test
-        b.wdot[(int64_t)sg.x * b.ld + i] = w;
+        w += w2;
+        if (valid) {
+          bad += ((__double2hiint(w) >> 20) & 0x7ff) == 0x7ff;  // inf or NaN, integer test
+          b.wdot[(int64_t)sg.x * b.ld + i] = w;
+        }
       }
     }
     // rates are replaced only after the barrier at the loop's head
@@ -619,31 +648,43 @@ size_t smem_of(const FxTab &f, int nw, bool qs, bool ts) {
          (qs ? (size_t)(f.R + 1) * 256 : 0);
 }
 
-// How a launch over `tiles` tiles runs: warps per CTA (list), CTAs per SM,
-// rates and small tables on chip.
+// How a launch over `tiles` tiles runs: warps per CTA, CTAs per SM and per
+// tile, rates and small tables on chip.
 struct Plan {
-  int list = 2, per_sm = 1;
+  int nw = 24, per_sm = 1, cl = 1;
   bool qs = false, ts = false, ok = false;
 };
 
 Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
-  Plan p;
-  if (!f.usable) return p;
-  p.ok = true;
+  if (!f.usable) return Plan{};
   auto fits = [&](int nw, int per_sm, bool qs) {
     return (smem_of(f, nw, qs, true) + 1024) * per_sm <= (size_t)smem_optin + 1024;
   };
-  if (f.R < 100 && fits(4, 6, true)) {
-    p = Plan{0, 6, true, true, true};
-  } else if (tiles <= sm_count && fits(16, 1, true)) {
-    p = Plan{2, 1, true, true, true};
-  } else if (fits(8, 3, false)) {
-    p = Plan{1, 3, false, true, true};
-  } else {
-    p.ts = fits(16, 1, false);
-    p.ok = smem_of(f, 16, false, p.ts) <= (size_t)smem_optin;
-  }
+  // few tiles: a cluster of CTAs shares each, as long as its warps get two
+  // reactions or more (97 states of 53/325: 47 us with one CTA per tile)
+  for (int cl = 8; cl > 1; cl /= 2)
+    if (tiles * cl <= sm_count && f.R >= 32 * cl && fits(16, 1, false))
+      return Plan{16, 1, cl, false, true, true};
+  if (f.R < 100 && fits(4, 6, true)) return Plan{4, 6, 1, true, true, true};
+  if (tiles <= sm_count && fits(16, 1, true)) return Plan{16, 1, 1, true, true, true};
+  if (fits(8, 3, false)) return Plan{8, 3, 1, false, true, true};
+  if (fits(24, 1, false)) return Plan{24, 1, 1, false, true, true};
+  Plan p{24, 1, 1, false, false, false};
+  p.ok = smem_of(f, 24, false, false) <= (size_t)smem_optin;
   return p;
+}
+
+using Kernel = void (*)(const ImgLayout, const FxTab, const Args, const Batch);
+Kernel kernel_of(const Plan &p) {
+  switch (p.cl) {
+    case 8: return k_wdot_tile<16, 1, 8, false, true>;
+    case 4: return k_wdot_tile<16, 1, 4, false, true>;
+    case 2: return k_wdot_tile<16, 1, 2, false, true>;
+  }
+  if (p.nw == 4) return k_wdot_tile<4, 6, 1, true, true>;
+  if (p.nw == 16) return k_wdot_tile<16, 1, 1, true, true>;
+  if (p.nw == 8) return k_wdot_tile<8, 3, 1, false, true>;
+  return p.ts ? k_wdot_tile<24, 1, 1, false, true> : k_wdot_tile<24, 1, 1, false, false>;
 }
 
 }  // namespace fx
@@ -661,22 +702,28 @@ long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                            const unsigned char *tab, const Batch &b, int sm_count,
                            int smem_optin, double *scratch, cudaStream_t s) {
-  using fx::k_wdot_tile;
   const int64_t tiles = (b.n + 31) / 32;
   const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
   if (!p.ok || p.qs != !scratch) return cudaErrorInvalidValue;
-  void (*k)(const ImgLayout, const fx::FxTab, fx::Args, Batch);
-  if (p.list == 0) k = k_wdot_tile<0, 6, true, true>;
-  else if (p.list == 1) k = k_wdot_tile<1, 3, false, true>;
-  else k = p.qs ? k_wdot_tile<2, 1, true, true>
-                : p.ts ? k_wdot_tile<2, 1, false, true> : k_wdot_tile<2, 1, false, false>;
-  const int nw = fx::warps_of(p.list);
-  const size_t bytes = fx::smem_of(f, nw, p.qs, p.ts);
+  int list = 0;
+  while (list < fx::NLIST - 1 && fx::list_warps[list] != p.nw * p.cl) ++list;
+  const fx::Kernel k = fx::kernel_of(p);
+  const size_t bytes = fx::smem_of(f, p.nw, p.qs, p.ts);
   const cudaError_t e = set_smem_limit(k, bytes);
   if (e != cudaSuccess) return e;
-  const int64_t grid = std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm);
-  k<<<(unsigned)grid, nw * 32, bytes, s>>>(L, f, fx::Args{tab, img, scratch}, b);
-  return cudaGetLastError();
+  const int64_t grid = std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm) * p.cl;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)p.nw * 32);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)p.cl;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = p.cl > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, L, f, fx::Args{tab, img, scratch, list}, b);
 }
 
 }  // namespace crs

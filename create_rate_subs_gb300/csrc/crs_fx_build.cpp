@@ -375,7 +375,8 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   f.eff_ptr = b.put(std::vector<int32_t>(t.pm_eff_ptr, t.pm_eff_ptr + NPM + 1));
   f.eff = b.put(eff);
   // species' terms: coefficients +-1 (small integers repeated) or weighted
-  std::vector<int32_t> term, wterm, where(4 * (size_t)N, 0);
+  std::vector<std::vector<int32_t>> terms(N);
+  std::vector<int32_t> wterm, where(4 * (size_t)N, 0);
   std::vector<double> wnu;
   for (int k = 0; k < N; ++k) {
     bool small_int = true;
@@ -383,26 +384,21 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       small_int &= std::fabs(t.spc_nu[e]) <= 3 && t.spc_nu[e] == std::rint(t.spc_nu[e]);
     int32_t *w = where.data() + 4 * (size_t)k;
     w[0] = k;
-    w[3] = !small_int;
-    if (small_int) {
-      w[1] = (int32_t)(term.size() / 4);
-      for (int e = t.spc_ptr[k]; e < t.spc_ptr[k + 1]; ++e)
+    w[2] = (int32_t)wterm.size();
+    for (int e = t.spc_ptr[k]; e < t.spc_ptr[k + 1]; ++e) {
+      if (small_int) {
         for (int q = 0; q < std::abs((int)t.spc_nu[e]); ++q)
-          term.push_back((int32_t)((unsigned)t.spc_r[e] * 256u |
-                                   (t.spc_nu[e] < 0 ? 0x80000000u : 0u)));
-      while (term.size() % 4) term.push_back(R * 256);
-      w[2] = (int32_t)(term.size() / 4) - w[1];
-    } else {
-      w[1] = (int32_t)wterm.size();
-      for (int e = t.spc_ptr[k]; e < t.spc_ptr[k + 1]; ++e) {
+          terms[k].push_back((int32_t)((unsigned)t.spc_r[e] * 256u |
+                                       (t.spc_nu[e] < 0 ? 0x80000000u : 0u)));
+      } else {
         wterm.push_back(t.spc_r[e] * 256);
         wnu.push_back(t.spc_nu[e]);
       }
-      w[2] = t.spc_ptr[k + 1] - t.spc_ptr[k];
     }
+    while (terms[k].size() % 4) terms[k].push_back(R * 256);
+    w[1] = (int32_t)(terms[k].size() / 4);
+    w[3] = (int32_t)wterm.size() - w[2];
   }
-  for (int q = 0; q < 4; ++q) term.push_back(R * 256);  // read ahead
-  f.term = b.put(term);
   f.wterm = b.put(wterm);
   f.wnu = b.put(wnu);
   std::vector<int> sw(N);
@@ -422,7 +418,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   }
   // work lists: longest first onto the least loaded warp
   for (int l = 0; l < NLIST; ++l) {
-    const int nw = warps_of(l);
+    const int nw = list_warps[l];
     auto deal = [&](const std::vector<int> &w, std::vector<long long> load) {
       std::vector<int> order(w.size());
       for (size_t i = 0; i < w.size(); ++i) order[i] = (int)i;
@@ -464,13 +460,23 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       f.rec[l][c] = b.put(lr);
     }
     bins = deal(sw, std::vector<long long>(nw, 0));
-    std::vector<int32_t> ptr(1, 0), seg;
+    std::vector<int32_t> ptr(1, 0), tptr(1, 0), seg, term;
     for (auto &v : bins) {
-      for (int k : v) seg.insert(seg.end(), where.begin() + 4 * k, where.begin() + 4 * k + 4);
+      std::stable_sort(v.begin(), v.end(), [&](int x, int y) {
+        return (where[4 * x + 3] > 0) < (where[4 * y + 3] > 0);
+      });
+      for (int k : v) {
+        seg.insert(seg.end(), where.begin() + 4 * k, where.begin() + 4 * k + 4);
+        term.insert(term.end(), terms[k].begin(), terms[k].end());
+      }
       ptr.push_back((int32_t)(seg.size() / 4));
+      tptr.push_back((int32_t)(term.size() / 4));
     }
+    for (int q = 0; q < 8; ++q) term.push_back(R * 256);  // read ahead
     f.seg_ptr[l] = b.put(ptr);
     f.seg[l] = b.put(seg);
+    f.term_ptr[l] = b.put(tptr);
+    f.term[l] = b.put(term);
   }
   f.bytes = (int)b.b.size();
   out.swap(b.b);

@@ -10,7 +10,9 @@ namespace fx {
 // Temperature intervals (tb[q], tb[q + 1]] on which the functions of T are
 // normalised; the second bound is the mechanism's most common T_common.
 constexpr int NI = 2;
-constexpr int NLIST = 3;  // work lists for 4, 8 and 16 warps per CTA
+// Work lists for so many warps per tile (a CTA's, or a cluster's).
+constexpr int NLIST = 7;
+constexpr int list_warps[NLIST] = {4, 8, 16, 24, 32, 64, 128};
 // A reaction's record: its head, int4 {slot offset, flags, fall-off entry,
 // reaction}, int4 {two reactants, two products}, int4 {the third and fourth
 // of each}, as offsets of tile rows; for reactions with pressure
@@ -43,15 +45,14 @@ struct FxTab {
   // number is completed with one that puts zero into the slot of zeros), its
   // other reactions' records, and its species' terms
   int list_ptr[NLIST][2], rec[NLIST][2];
-  // int4 {species, first, number, weighted}: groups of four terms {slot
-  // offset, bit 31: subtract}, completed with the slot of zeros (row R); or,
-  // weighted, single terms with a coefficient
-  int seg_ptr[NLIST], seg[NLIST];
-  int term, wterm, wnu;
+  // its species, int4 {species, groups of terms, first weighted term, their
+  // number}, those with weighted terms last; its groups of four terms {slot
+  // offset, bit 31: subtract}, one after another, completed with the slot of
+  // zeros (row R)
+  int seg_ptr[NLIST], seg[NLIST], term_ptr[NLIST], term[NLIST];
+  int wterm, wnu;
   int bytes;
 };
-
-constexpr int warps_of(int list) { return 4 << list; }
 
 }  // namespace fx
 }  // namespace crs
