@@ -689,22 +689,42 @@ Kernel kernel_of(const Plan &p) {
 
 }  // namespace fx
 
+// A launch over n states is one or two kernels: whole waves of tiles, and
+// what is left over, whose few tiles are shared by clusters (626 tiles of a
+// large mechanism on 152 SMs: the fifth wave held 18).  Tiles of the first:
+static int64_t first_tiles(const fx::FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
+  const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
+  const int64_t wave = (int64_t)sm_count * p.per_sm;
+  const int64_t rest = tiles % wave;
+  // worth a launch when two or more CTAs may share each tile
+  return p.cl > 1 || tiles < wave || rest == 0 || 2 * rest > sm_count || f.R < 64
+             ? tiles
+             : tiles - rest;
+}
+
 // Scratch bytes of a launch over n states (0: the net rates fit on chip);
 // < 0: the mechanism does not fit this kernel.
 long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
-  const int64_t tiles = (n + 31) / 32;
-  const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
-  if (!p.ok) return -1;
-  return p.qs ? 0 : (long long)std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm) *
-                        (f.R + 1) * 256;
+  const int64_t tiles = (n + 31) / 32, first = first_tiles(f, tiles, sm_count, smem_optin);
+  long long most = 0;
+  for (int64_t part : {first, tiles - first}) {
+    if (part == 0) continue;
+    const fx::Plan p = fx::plan_of(f, part, sm_count, smem_optin);
+    if (!p.ok) return -1;
+    if (p.qs) continue;
+    const long long need = (long long)std::min<int64_t>(part, (int64_t)sm_count * p.per_sm) *
+                           (f.R + 1) * 256;
+    most = std::max(most, need);
+  }
+  return most;
 }
 
-cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
-                           const unsigned char *tab, const Batch &b, int sm_count,
-                           int smem_optin, double *scratch, cudaStream_t s) {
+static cudaError_t launch_tiles(const unsigned char *img, const ImgLayout &L,
+                                const fx::FxTab &f, const unsigned char *tab, const Batch &b,
+                                int sm_count, int smem_optin, double *scratch, cudaStream_t s) {
   const int64_t tiles = (b.n + 31) / 32;
   const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
-  if (!p.ok || p.qs != !scratch) return cudaErrorInvalidValue;
+  if (!p.ok || (!p.qs && !scratch)) return cudaErrorInvalidValue;
   int list = 0;
   while (list < fx::NLIST - 1 && fx::list_warps[list] != p.nw * p.cl) ++list;
   const fx::Kernel k = fx::kernel_of(p);
@@ -724,6 +744,23 @@ cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const f
   cfg.attrs = at;
   cfg.numAttrs = p.cl > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, k, L, f, fx::Args{tab, img, scratch, list}, b);
+}
+
+cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
+                           const unsigned char *tab, const Batch &b, int sm_count,
+                           int smem_optin, double *scratch, cudaStream_t s) {
+  const int64_t tiles = (b.n + 31) / 32, first = first_tiles(f, tiles, sm_count, smem_optin);
+  Batch part = b;
+  part.n = std::min<int64_t>(b.n, first * 32);
+  cudaError_t e = launch_tiles(img, L, f, tab, part, sm_count, smem_optin, scratch, s);
+  if (e != cudaSuccess || first == tiles) return e;
+  const int64_t o = part.n;
+  part.n = b.n - o;
+  part.T += o;
+  part.P += o;
+  part.Y += o;
+  part.wdot += o;
+  return launch_tiles(img, L, f, tab, part, sm_count, smem_optin, scratch, s);
 }
 
 }  // namespace crs
