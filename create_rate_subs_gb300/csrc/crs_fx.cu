@@ -112,7 +112,7 @@ __device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags
   const int64_t zP = z > ZMIN ? z : ZMIN;
   // Fcent (Troe) or the base of the SRI power, in units of 2^-59
   int64_t S = 0;
-#pragma unroll
+#pragma unroll 1
   for (int q = 0; q < 3; ++q) {
     if (flags & (PMF_T1 << q)) {
       const int64_t y = word(c[3 + 2 * q]);
@@ -216,6 +216,7 @@ struct Ring {
     if (p < n) {
       const unsigned char *from = src + (int64_t)p * stride;
       const unsigned to = base + (unsigned)((p % D) * stride);
+#pragma unroll 1
       for (int o = lane * 16; o < stride; o += 512)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + o), "l"(from + o)
                      : "memory");
@@ -274,6 +275,7 @@ __device__ __forceinline__ int64_t exponent7(const Rec &r, const Basis &B) {
 template <int NW>
 __device__ __forceinline__ void load_y(const double *Y, int64_t ld, int N, int warp,
                                        unsigned smem_rows) {
+#pragma unroll 4
   for (int k = warp; k < N - 1; k += NW)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_rows + k * 256),
                  "l"(Y + (int64_t)k * ld)
@@ -358,6 +360,7 @@ __device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const B
   kc.logT = s.logT;
   kc.invT = s.invT;
   const YConc C{b.Y + i, b.ld, rho, yN, t.inv_mw, t.N};
+#pragma unroll 1
   for (int p = 0; p < 2 * plain.n + other.n; ++p) {
     const int o = p - 2 * plain.n;
     const int4 h = __ldg(reinterpret_cast<const int4 *>(
@@ -460,6 +463,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     auto third_body = [&](int p) {
       const int *ep = reinterpret_cast<const int *>(tab + f.eff_ptr) + p;
       double s = rowd(9);
+#pragma unroll 1
       for (int e = ep[0]; e < ep[1]; ++e) {
         const int4 w = __ldg(reinterpret_cast<const int4 *>(tab + f.eff) + e);
         double y;
@@ -472,6 +476,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     };
     // (rates on chip) into the slots of their reactions' rates
     if (QS && f.NPM > 0) {
+#pragma unroll 1
       for (int p = warp; p < f.NPM; p += NW) {
         const int slot = __ldg(reinterpret_cast<const int2 *>(tab + f.pm) + p).x;
         if (slot >= 0) Q(slot) = third_body(p);
@@ -480,6 +485,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     }
     // exponents of the concentrations in place of the mass fractions
     bool odd = false;
+#pragma unroll 1
     for (int k = warp; k < N; k += NW) {
       const double y = k == N - 1 ? rowd(7) : __longlong_as_double(Yl(k * 256));
       const uint64_t u = bits_of(y);
@@ -518,6 +524,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
           const double T = b.T[ic];
           const double *thr = reinterpret_cast<const double *>(at + co + COEF * (f.nthr + 1));
           idx = 0;
+  #pragma unroll 1
           for (int e = 0; e < f.nthr; ++e) idx += T > thr[e];
         }
         return Rec{at, at + co + COEF * idx};
@@ -525,6 +532,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       // two reactions at a time: independent chains side by side
       const int one = f.stride[0] / 2;
       unsigned char *at = ring;
+#pragma unroll 1
       for (int p = 0; p < plain_ring.n; ++p) {
         plain_ring.next(p);
         int64_t yf[2], yr[2];
@@ -554,6 +562,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncwarp();
       other_ring.start();
+#pragma unroll 1
       for (int p = 0; p < other_ring.n; ++p) {
         other_ring.next(p);
         const Rec r = record(ring + (p % DO) * f.stride[1], HEAD + PMH + PMC * NI);
@@ -612,9 +621,11 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       double v[4];
       rates(__ldg(tm), v);
       int4 t = __ldg(tm + 1);
+#pragma unroll 1
       for (int a = s0; a < s1; ++a) {
         const int4 sg = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a);
         double w = 0.0, w2 = 0.0;
+#pragma unroll 1
         for (int e = 0; e < sg.y; ++e) {
           double u[4];
           rates(t, u);
@@ -627,6 +638,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
 #pragma unroll
           for (int c = 0; c < 4; ++c) v[c] = u[c];
         }
+#pragma unroll 1
         for (int e = sg.z; e < sg.z + sg.w; ++e)
           w = fma(__ldg(reinterpret_cast<const double *>(tab + f.wnu) + e),
                   Q(__ldg(reinterpret_cast<const int *>(tab + f.wterm) + e)), w);

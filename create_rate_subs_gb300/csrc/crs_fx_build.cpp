@@ -324,7 +324,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
     if (cnt[0] > 2 || cnt[1] > 2) flags |= RF_MORE;
     if (a.neg) flags |= RF_NEG;
     // instruction counts, in units of ten
-    weight[r] = (j >= 0 ? 26 : 15) + (p < 0 ? 0 : flags & RF_THD ? 4 : 45);
+    weight[r] = (j >= 0 ? 24 : 20) + (p < 0 ? 0 : flags & RF_THD ? 21 : 84);
     kind[r] = p >= 0 ? 2 : j >= 0 ? 0 : 1;
     if (!ok) {
       flags |= RF_GEN;
