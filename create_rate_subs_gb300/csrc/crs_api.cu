@@ -64,6 +64,7 @@ cudaError_t launch_pack_bf16(const double *q, int64_t ldq, int64_t n, int R, int
 namespace fx {
 void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out);
 }
+cudaError_t fx_init(int smem_optin);
 long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                            const unsigned char *tab, const Batch &b, int sm_count,
@@ -834,6 +835,14 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
   // kernels' static __shared__ part (the staging mbarrier, which the
   // 128-byte alignment of the dynamic part pads to 128 bytes) and slack
   m->smem_optin -= 256;
+  if (m->fx.usable) {
+    e = crs::fx_init(m->smem_optin);
+    if (e != cudaSuccess) {
+      int r = cuda_fail(e, "crs_mech_load");
+      crs_mech_free(m);
+      return r;
+    }
+  }
   *out = m;
   return CRS_OK;
 }

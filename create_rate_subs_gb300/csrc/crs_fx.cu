@@ -112,7 +112,7 @@ __device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags
   const int64_t zP = z > ZMIN ? z : ZMIN;
   // Fcent (Troe) or the base of the SRI power, in units of 2^-59
   int64_t S = 0;
-#pragma unroll 1
+#pragma unroll
   for (int q = 0; q < 3; ++q) {
     if (flags & (PMF_T1 << q)) {
       const int64_t y = word(c[3 + 2 * q]);
@@ -385,12 +385,12 @@ __device__ __forceinline__ void tile_barrier() {
 
 // NW warps per CTA, CL CTAs (a cluster) per tile: each forms the tile's
 // exponents for itself, evaluates its share of the reactions and, the rates
-// exchanged through global memory, of the species.
+// exchanged through the first CTA's shared memory (QS) or scratch, of the
+// species.
 template <int NW, int PER_SM, int CL, bool QS, bool TS>
 __global__ void __launch_bounds__(NW * 32, PER_SM)
     k_wdot_tile(const __grid_constant__ ImgLayout lay, const __grid_constant__ FxTab f,
                 const __grid_constant__ Args g, const __grid_constant__ Batch b) {
-  static_assert(CL == 1 || !QS, "a cluster's rates are in global memory");
   const int LIST = g.list;
   extern __shared__ __align__(128) unsigned char smem[];
   const int N = f.N;
@@ -415,13 +415,15 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   const int rb = ring_bytes(f);
   unsigned char *ring = next + warp * rb;
   next += NW * rb;
-  unsigned char *q = (QS ? next : reinterpret_cast<unsigned char *>(g.q) +
+  unsigned char *q = (QS && CL > 1 ? static_cast<unsigned char *>(__cluster_map_shared_rank(next, 0))
+                      : QS ? next : reinterpret_cast<unsigned char *>(g.q) +
                                       (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256) + lane * 8;
   auto Yl = [&](int off) -> int64_t & { return *reinterpret_cast<int64_t *>(yl + off); };
   auto Q = [&](int off) -> double & { return *reinterpret_cast<double *>(q + off); };
   if (warp == 0) {
     Yl(N * 256) = 0;
-    Q(f.R * 256) = 0.0;
+    if (!QS || CL == 1) Q(f.R * 256) = 0.0;
+    else reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
   }
   Ring<DP> plain_ring;
   Ring<DO> other_ring;
@@ -468,14 +470,14 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         const int4 w = __ldg(reinterpret_cast<const int4 *>(tab + f.eff) + e);
         double y;
         if (w.z == (N - 1) * 256) y = rowd(7);
-        else if (QS) y = __longlong_as_double(Yl(w.z));
+        else if (QS && CL == 1) y = __longlong_as_double(Yl(w.z));
         else y = b.Y[(int64_t)(w.z >> 8) * b.ld + ic];
         s = fma(__hiloint2double(w.y, w.x), y, s);
       }
       return s;
     };
     // (rates on chip) into the slots of their reactions' rates
-    if (QS && f.NPM > 0) {
+    if (QS && CL == 1 && f.NPM > 0) {
 #pragma unroll 1
       for (int p = warp; p < f.NPM; p += NW) {
         const int slot = __ldg(reinterpret_cast<const int2 *>(tab + f.pm) + p).x;
@@ -574,11 +576,11 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
           if (h.y & RF_FALL) {
             const int64_t lth = ph.y >= 0
                                     ? Yl(ph.y)
-                                    : log2s(QS ? Q(h.x) : third_body(h.z), lt) + lrho;
+                                    : log2s(QS && CL == 1 ? Q(h.x) : third_body(h.z), lt) + lrho;
             l += falloff(reinterpret_cast<const int2 *>(r.p + HEAD + PMH + PMC * iv), ph.x, lth,
                          B.L, B.I, B.t1, et, lt, slow);
           } else {
-            thd = rowd(8) * (QS ? Q(h.x) : third_body(h.z));
+            thd = rowd(8) * (QS && CL == 1 ? Q(h.x) : third_body(h.z));
           }
         }
         int64_t yf = exponent3(r, B) + l + Yl(x.x) + Yl(x.y);
@@ -599,6 +601,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       if (later || all)
         finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
     }
+    // the first terms are on their way before the barrier
+    const int4 t0 = __ldg(terms), t1 = __ldg(terms + 1);
+    const int4 sg0 = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + s0);
     tile_barrier<CL>();
     // the next tile's mass fractions replace exponents that every warp is
     // done with, while the species sums run
@@ -619,11 +624,12 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       };
       const int4 *tm = terms;
       double v[4];
-      rates(__ldg(tm), v);
-      int4 t = __ldg(tm + 1);
+      rates(t0, v);
+      int4 t = t1, sgn = sg0;
 #pragma unroll 1
       for (int a = s0; a < s1; ++a) {
-        const int4 sg = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a);
+        const int4 sg = sgn;
+        sgn = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a + 1);
         double w = 0.0, w2 = 0.0;
 #pragma unroll 1
         for (int e = 0; e < sg.y; ++e) {
@@ -651,6 +657,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     }
     // rates are replaced only after the barrier at the loop's head
   }
+  if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here
   if (bad && b.status) atomicAdd(&b.status[1], bad);
 }
 
@@ -675,10 +682,12 @@ Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
   // few tiles: a cluster of CTAs shares each, as long as its warps get two
   // reactions or more (97 states of 53/325: 47 us with one CTA per tile)
   for (int cl = 8; cl > 1; cl /= 2)
-    if (tiles * cl <= sm_count && f.R >= 32 * cl && fits(16, 1, false))
-      return Plan{16, 1, cl, false, true, true};
-  if (f.R < 100 && fits(4, 6, true)) return Plan{4, 6, 1, true, true, true};
+    if (tiles * cl <= sm_count && f.R >= 32 * cl) {
+      if (fits(16, 1, true)) return Plan{16, 1, cl, true, true, true};
+      if (fits(16, 1, false)) return Plan{16, 1, cl, false, true, true};
+    }
   if (tiles <= sm_count && fits(16, 1, true)) return Plan{16, 1, 1, true, true, true};
+  if (f.R < 100 && fits(4, 6, true)) return Plan{4, 6, 1, true, true, true};
   if (fits(8, 3, false)) return Plan{8, 3, 1, false, true, true};
   if (fits(24, 1, false)) return Plan{24, 1, 1, false, true, true};
   Plan p{24, 1, 1, false, false, false};
@@ -689,9 +698,9 @@ Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
 using Kernel = void (*)(const ImgLayout, const FxTab, const Args, const Batch);
 Kernel kernel_of(const Plan &p) {
   switch (p.cl) {
-    case 8: return k_wdot_tile<16, 1, 8, false, true>;
-    case 4: return k_wdot_tile<16, 1, 4, false, true>;
-    case 2: return k_wdot_tile<16, 1, 2, false, true>;
+    case 8: return p.qs ? k_wdot_tile<16, 1, 8, true, true> : k_wdot_tile<16, 1, 8, false, true>;
+    case 4: return p.qs ? k_wdot_tile<16, 1, 4, true, true> : k_wdot_tile<16, 1, 4, false, true>;
+    case 2: return p.qs ? k_wdot_tile<16, 1, 2, true, true> : k_wdot_tile<16, 1, 2, false, true>;
   }
   if (p.nw == 4) return k_wdot_tile<4, 6, 1, true, true>;
   if (p.nw == 16) return k_wdot_tile<16, 1, 1, true, true>;
@@ -700,6 +709,22 @@ Kernel kernel_of(const Plan &p) {
 }
 
 }  // namespace fx
+
+// Raises the kernels' shared-memory limit to the device's, once per load of a
+// mechanism (a microsecond or two per launch otherwise).
+cudaError_t fx_init(int smem_optin) {
+  cudaError_t e = cudaSuccess;
+  for (int q = 0; q < 7 && e == cudaSuccess; ++q) {
+    fx::Plan p;
+    p.cl = q < 3 ? 2 << q : 1;
+    p.nw = q == 3 ? 4 : q == 4 ? 16 : q == 5 ? 8 : 24;
+    p.ts = p.qs = true;
+    e = set_smem_limit(fx::kernel_of(p), (size_t)smem_optin);
+    p.ts = p.qs = false;
+    if (e == cudaSuccess) e = set_smem_limit(fx::kernel_of(p), (size_t)smem_optin);
+  }
+  return e;
+}
 
 // A launch over n states is one or two kernels: whole waves of tiles, and
 // what is left over, whose few tiles are shared by clusters (626 tiles of a
@@ -741,8 +766,6 @@ static cudaError_t launch_tiles(const unsigned char *img, const ImgLayout &L,
   while (list < fx::NLIST - 1 && fx::list_warps[list] != p.nw * p.cl) ++list;
   const fx::Kernel k = fx::kernel_of(p);
   const size_t bytes = fx::smem_of(f, p.nw, p.qs, p.ts);
-  const cudaError_t e = set_smem_limit(k, bytes);
-  if (e != cudaSuccess) return e;
   const int64_t grid = std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm) * p.cl;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);

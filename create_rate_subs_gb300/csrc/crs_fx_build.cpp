@@ -473,6 +473,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       tptr.push_back((int32_t)(term.size() / 4));
     }
     for (int q = 0; q < 8; ++q) term.push_back(R * 256);  // read ahead
+    seg.insert(seg.end(), {0, 0, 0, 0});  // read ahead
     f.seg_ptr[l] = b.put(ptr);
     f.seg[l] = b.put(seg);
     f.term_ptr[l] = b.put(tptr);

@@ -41,7 +41,7 @@ def _torch():
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 class RateSubs(object):
@@ -57,6 +57,7 @@ class RateSubs(object):
         self.device = torch.device("cuda", torch.cuda.current_device()
                                    if device is None else device)
         h = ctypes.c_void_p()
+        self._dev = self.device.index
         with torch.cuda.device(self.device):
             _lib.check(self.lib.crs_mech_load(blob, len(blob), ctypes.byref(h)))
         self.h = h
@@ -81,12 +82,17 @@ class RateSubs(object):
 
     # -- helpers ---------------------------------------------------------
     def _stream(self):
-        return ctypes.c_void_p(_torch().cuda.current_stream(self.device).cuda_stream)
+        # the raw handle of current_stream(self.device), without the Stream
+        # object around it (a microsecond or two per call)
+        raw = getattr(_torch()._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None:
+            return raw(self._dev)
+        return _torch().cuda.current_stream(self.device).cuda_stream
 
     def _check_states(self, T, P, Y=None, rows=None):
-        torch = _torch()
+        f64 = _torch().float64
         for name, a in (("T", T), ("P", P)):
-            if a.dtype != torch.float64 or a.dim() != 1 or not a.is_cuda:
+            if a.dtype != f64 or a.dim() != 1 or not a.is_cuda:
                 raise ValueError("%s must be a 1-D float64 CUDA tensor" % name)
             if a.stride(0) != 1:
                 raise ValueError("%s must be contiguous" % name)
@@ -95,13 +101,14 @@ class RateSubs(object):
             raise ValueError("T and P differ in length")
         ld = n
         if Y is not None:
-            if Y.dtype != torch.float64 or Y.dim() != 2 or not Y.is_cuda:
+            if Y.dtype != f64 or Y.dim() != 2 or not Y.is_cuda:
                 raise ValueError("Y must be a 2-D float64 CUDA tensor (species, n)")
-            if Y.shape[1] != n or Y.stride(1) != 1:
+            have, cols = Y.shape
+            ld, unit = Y.stride()
+            if cols != n or unit != 1:
                 raise ValueError("Y must be (species, n) with unit state stride")
-            if Y.shape[0] < (rows if rows is not None else self.n_species - 1):
+            if have < (rows if rows is not None else self.n_species - 1):
                 raise ValueError("Y has too few species rows")
-            ld = Y.stride(0)
         return n, ld
 
     def _out(self, rows, n):
