@@ -107,6 +107,7 @@ struct crs_mech {
   unsigned char *d_img = nullptr;  // device table image
   crs::fx::FxTab fx{};             // tables of the FP64 state-tile kernel
   unsigned char *d_fx = nullptr;   // (fx.usable = 0: not for this mechanism)
+  cudaMemPool_t fx_pool = nullptr; // its kernels' scratch (freed with the mechanism)
   int32_t *d_status = nullptr;     // [0] flags, [1] non-finite count
   // dynamic-scheduling counter pairs of the one-state-per-thread kernels;
   // each launch draws the next slot, so launches in flight at the same time
@@ -650,9 +651,23 @@ int wdot_two_pass(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool fp64) {
   return rc != CRS_OK ? rc : rc2;
 }
 
+// A pool for stream-ordered scratch; what is free stays with it between
+// synchronisations up to 256 MiB (the scratch of 53/325: 38 MB, of 561/2539:
+// 99 MB; mapped anew on each call it cost more than the kernel).
+cudaError_t make_pool(int device, cudaMemPool_t *pool) {
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaError_t e = cudaMemPoolCreate(pool, &props);
+  uint64_t keep = (uint64_t)256 << 20;
+  if (e == cudaSuccess) e = cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  return e;
+}
+
 // CRS_MODE_FP64 by state tiles in fixed point, when the mechanism fits (and
 // no intermediates are asked for); *taken = false otherwise.  Net rates that
-// do not fit on chip go through the two-pass workspace.
+// do not fit on chip (at most one tile's per resident CTA) get scratch.
 int wdot_fx(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool *taken) {
   const long long scratch = crs::fx_scratch(m->fx, b.n, m->sm_count, m->smem_optin);
   *taken = scratch >= 0 && !(b.conc || b.fwd || b.rev || b.pm);
@@ -663,15 +678,20 @@ int wdot_fx(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool *taken) {
                             nullptr, s);
     return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
   }
-  std::lock_guard<std::mutex> lk(m->ws_mu);
-  int rc = ensure_q(m, scratch / (8 * (int64_t)m->L.R) + 1, false);
-  if (rc == CRS_OK) rc = ws_begin(m, s);
-  if (rc != CRS_OK) return rc;
-  e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, m->d_q,
-                          s);
-  if (e != cudaSuccess) rc = cuda_fail(e, "crs_wdot launch");
-  const int rc2 = ws_end(m, s);
-  return rc != CRS_OK ? rc : rc2;
+  // in stream order, from the mechanism's pool: calls on several streams do
+  // not share it, and under capture it becomes a node of the graph
+  double *q = nullptr;
+  e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&q), (size_t)scratch, m->fx_pool, s);
+  if (e == cudaErrorMemoryAllocation) {  // the kernels that need none
+    cudaGetLastError();
+    *taken = false;
+    return CRS_OK;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "crs_wdot scratch");
+  e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, q, s);
+  const cudaError_t e2 = cudaFreeAsync(q, s);
+  if (e == cudaSuccess) e = e2;
+  return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
 }
 
 // CRS_MODE_GEMM: per chunk, the FP64 net rates (state tiles), their bf16
@@ -837,6 +857,7 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
   m->smem_optin -= 256;
   if (m->fx.usable) {
     e = crs::fx_init(m->smem_optin);
+    if (e == cudaSuccess) e = make_pool(m->device, &m->fx_pool);
     if (e != cudaSuccess) {
       int r = cuda_fail(e, "crs_mech_load");
       crs_mech_free(m);
@@ -916,6 +937,7 @@ int crs_mech_free(crs_mech *m) {
   unbind(m);
   if (m->d_img) cudaFree(m->d_img);
   if (m->d_fx) cudaFree(m->d_fx);
+  if (m->fx_pool) cudaMemPoolDestroy(m->fx_pool);
   if (m->d_status) cudaFree(m->d_status);
   if (m->d_sched) cudaFree(m->d_sched);
   if (m->d_nuB) cudaFree(m->d_nuB);

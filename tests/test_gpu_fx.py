@@ -72,3 +72,34 @@ def test_tiles_and_states_outside_the_scheme(name, n, golden, synth_mech):
     judge = np.where(cold, _wdot(mech, T, P, Y, "fp64_warp")[0], ref["wdot"])
     assert wdot_errors(w[:, fin], judge[:, fin], G[:, fin])["scaled"] <= TOL
     assert status == (0, int(np.sum(~np.isfinite(w))))
+
+
+@pytest.mark.parametrize("name,n", [("gri53", 153 * 32), ("large561", 33)])
+def test_scratch_under_capture_and_on_two_streams(name, n, synth_mech):
+    """Launches whose net rates live in scratch: a handle's first call may be
+    captured, a replay and calls on two streams at once give the eager bits."""
+    from create_rate_subs_gb300.rates import RateSubs
+    mech = synth_mech(name)
+    N = mech.n_species
+    sets = [[torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (T, P, Y[: N - 1])]
+            for T, P, Y in (synth.make_states(N, n, seed=s) for s in (1, 2))]
+    rs = RateSubs(mech)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = rs.wdot(*sets[0])
+    eager = [rs.wdot(*d) for d in sets]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, eager[0])
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = []
+    for _ in range(8):
+        for d, st in zip(sets, streams):
+            with torch.cuda.stream(st):
+                outs.append(rs.wdot(*d))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, eager[0])
+    for k, o in enumerate(outs):
+        assert torch.equal(o, eager[k % 2])
