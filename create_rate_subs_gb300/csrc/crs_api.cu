@@ -69,6 +69,12 @@ long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                            const unsigned char *tab, const Batch &b, int sm_count,
                            int smem_optin, double *scratch, cudaStream_t s);
+// Mixed precision by state tiles (crs_mixed_tile.cu), likewise.
+cudaError_t mixed_tile_init(int smem_optin);
+long long mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
+                              const unsigned char *tab, const Batch &b, int sm_count,
+                              int smem_optin, double *scratch, cudaStream_t s);
 // Tables the fast kernels derive from the blob's tables at load time.
 bool build_fast_tables(const std::vector<unsigned char> &img,
                        const ImgLayout &L, std::vector<Derived> &extra);
@@ -665,31 +671,30 @@ cudaError_t make_pool(int device, cudaMemPool_t *pool) {
   return e;
 }
 
-// CRS_MODE_FP64 by state tiles in fixed point, when the mechanism fits (and
-// no intermediates are asked for); *taken = false otherwise.  Net rates that
-// do not fit on chip (at most one tile's per resident CTA) get scratch.
-int wdot_fx(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool *taken) {
-  const long long scratch = crs::fx_scratch(m->fx, b.n, m->sm_count, m->smem_optin);
+// CRS_MODE_FP64 and CRS_MODE_MIXED by state tiles, when the mechanism fits
+// (and no intermediates are asked for); *taken = false otherwise.  Net rates
+// that do not fit on chip (at most one tile's per resident CTA) get scratch.
+int wdot_tiles(crs_mech *m, const crs::Batch &b, bool mixed, cudaStream_t s, bool *taken) {
+  const long long scratch =
+      mixed ? crs::mixed_tile_scratch(m->fx, b.n, m->sm_count, m->smem_optin)
+            : crs::fx_scratch(m->fx, b.n, m->sm_count, m->smem_optin);
   *taken = scratch >= 0 && !(b.conc || b.fwd || b.rev || b.pm);
   if (!*taken) return CRS_OK;
-  cudaError_t e;
-  if (scratch == 0) {
-    e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin,
-                            nullptr, s);
-    return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
-  }
   // in stream order, from the mechanism's pool: calls on several streams do
   // not share it, and under capture it becomes a node of the graph
   double *q = nullptr;
-  e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&q), (size_t)scratch, m->fx_pool, s);
+  cudaError_t e = cudaSuccess;
+  if (scratch)
+    e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&q), (size_t)scratch, m->fx_pool, s);
   if (e == cudaErrorMemoryAllocation) {  // the kernels that need none
     cudaGetLastError();
     *taken = false;
     return CRS_OK;
   }
   if (e != cudaSuccess) return cuda_fail(e, "crs_wdot scratch");
-  e = crs::launch_wdot_fx(m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, q, s);
-  const cudaError_t e2 = cudaFreeAsync(q, s);
+  e = (mixed ? crs::launch_mixed_tile : crs::launch_wdot_fx)(
+      m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, q, s);
+  const cudaError_t e2 = q ? cudaFreeAsync(q, s) : cudaSuccess;
   if (e == cudaSuccess) e = e2;
   return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
 }
@@ -752,7 +757,7 @@ int launch_mode(const crs_mech *m, crs::Batch &b, int mode, cudaStream_t s) {
       // the two-pass state-tile path (per warp when intermediates are asked
       // for)
       bool taken;
-      const int rc = wdot_fx(const_cast<crs_mech *>(m), b, s, &taken);
+      const int rc = wdot_tiles(const_cast<crs_mech *>(m), b, false, s, &taken);
       if (taken) return rc;
       e = crs::launch_wdot_fp64_tps(m->d_img, m->L, b, m->sm_count, m->smem_optin, s);
       if (e == cudaErrorNotSupported) {
@@ -766,9 +771,13 @@ int launch_mode(const crs_mech *m, crs::Batch &b, int mode, cudaStream_t s) {
       if (b.conc || b.fwd || b.rev || b.pm)
         return fail(CRS_ERR_UNSUPPORTED, "CRS_MODE_FP64_TILE does not write intermediates");
       return wdot_two_pass(const_cast<crs_mech *>(m), b, s, true);
-    case CRS_MODE_MIXED:
-      // one state per thread when its columns fit on chip; else the
+    case CRS_MODE_MIXED: {
+      // state tiles; for intermediates and reactions with several T_common
+      // values one state per thread when its columns fit on chip, else the
       // two-pass state-tile path (per warp when intermediates are asked for)
+      bool taken;
+      const int rc = wdot_tiles(const_cast<crs_mech *>(m), b, true, s, &taken);
+      if (taken) return rc;
       e = crs::launch_wdot_mixed_tps(m->d_img, m->L, b, m->sm_count, m->smem_optin, s);
       if (e == cudaErrorNotSupported) {
         if (!(b.conc || b.fwd || b.rev || b.pm) && tile_smem(m->L, false) <= (size_t)m->smem_optin)
@@ -776,6 +785,7 @@ int launch_mode(const crs_mech *m, crs::Batch &b, int mode, cudaStream_t s) {
         e = crs::launch_wdot_mixed(m->d_img, m->L, b, m->sm_count, m->smem_optin, s);
       }
       break;
+    }
     case CRS_MODE_MIXED_TILE:
       if (b.conc || b.fwd || b.rev || b.pm)
         return fail(CRS_ERR_UNSUPPORTED, "CRS_MODE_MIXED_TILE does not write intermediates");
@@ -837,7 +847,7 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
   if (e == cudaSuccess) {
     std::vector<unsigned char> fxb;
     crs::fx::build(m->htab, m->fx, fxb);
-    if (m->fx.usable) {
+    if (m->fx.usable || m->fx.mixed) {
       e = cudaMalloc(&m->d_fx, fxb.size());
       if (e == cudaSuccess) e = cudaMemcpy(m->d_fx, fxb.data(), fxb.size(), cudaMemcpyHostToDevice);
     }
@@ -855,8 +865,9 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
   // kernels' static __shared__ part (the staging mbarrier, which the
   // 128-byte alignment of the dynamic part pads to 128 bytes) and slack
   m->smem_optin -= 256;
-  if (m->fx.usable) {
+  if (m->fx.usable || m->fx.mixed) {
     e = crs::fx_init(m->smem_optin);
+    if (e == cudaSuccess) e = crs::mixed_tile_init(m->smem_optin);
     if (e == cudaSuccess) e = make_pool(m->device, &m->fx_pool);
     if (e != cudaSuccess) {
       int r = cuda_fail(e, "crs_mech_load");

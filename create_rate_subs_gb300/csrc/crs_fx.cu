@@ -47,6 +47,7 @@
 #include "crs_fast.cuh"
 #include "crs_fx.cuh"
 #include "crs_fx_tab.cuh"
+#include "crs_fx_tile.cuh"
 #include "crs_internal.cuh"
 #include "crs_tile.cuh"
 
@@ -205,37 +206,6 @@ struct Rec {
   }
 };
 
-// Copies of a warp's next records into its ring of D slots.
-template <int D>
-struct Ring {
-  const unsigned char *src;
-  unsigned base;
-  int stride, n, lane;
-  // record p (an empty group past the last one)
-  __device__ __forceinline__ void fill(int p) const {
-    if (p < n) {
-      const unsigned char *from = src + (int64_t)p * stride;
-      const unsigned to = base + (unsigned)((p % D) * stride);
-#pragma unroll 1
-      for (int o = lane * 16; o < stride; o += 512)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + o), "l"(from + o)
-                     : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  __device__ __forceinline__ void start() const {
-#pragma unroll
-    for (int p = 0; p < D - 1; ++p) fill(p);
-  }
-  // Record p is on chip for the whole warp; the copy of record p + D - 1
-  // starts (its slot's reader, record p - 1, is done).
-  __device__ __forceinline__ void next(int p) const {
-    __syncwarp();
-    fill(p + D - 1);
-    asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
-    __syncwarp();
-  }
-};
 constexpr int DP = 3, DO = 3;  // slots for pairs of plain records and for other records
 
 __host__ __device__ inline int ring_bytes(const FxTab &f) {
@@ -372,17 +342,6 @@ __device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const B
   }
 }
 
-// Barrier of the CTAs that share a tile.
-template <int CL>
-__device__ __forceinline__ void tile_barrier() {
-  if (CL == 1) {
-    __syncthreads();
-  } else {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  }
-}
-
 // NW warps per CTA, CL CTAs (a cluster) per tile: each forms the tile's
 // exponents for itself, evaluates its share of the reactions and, the rates
 // exchanged through the first CTA's shared memory (QS) or scratch, of the
@@ -436,10 +395,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     other_ring = Ring<DO>{tab + f.rec[LIST][1] + (int64_t)lo[0] * f.stride[1], smem_u32(ring),
                           f.stride[1], lo[1] - lo[0], lane};
   }
-  const int s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw];
-  const int s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw + 1];
-  const int4 *terms = reinterpret_cast<const int4 *>(tab + f.term[LIST]) +
-                      reinterpret_cast<const int *>(tab + f.term_ptr[LIST])[gw];
+  Sums sums(f, tab, LIST, gw);
   const unsigned yrows = smem_u32(smem) + lane * 8;
   const double *inv_mw = reinterpret_cast<const double *>(g.img + lay.inv_mw);
   int bad = 0, bk = 0;
@@ -601,9 +557,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       if (later || all)
         finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
     }
-    // the first terms are on their way before the barrier
-    const int4 t0 = __ldg(terms), t1 = __ldg(terms + 1);
-    const int4 sg0 = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + s0);
+    sums.ahead();
     tile_barrier<CL>();
     // the next tile's mass fractions replace exponents that every warp is
     // done with, while the species sums run
@@ -611,50 +565,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       const int64_t j = (tile + step) * 32;
       load_y<NW>(b.Y + (j + lane < b.n ? j + lane : j), b.ld, N, warp, yrows);
     }
-    {
-      // the groups of the warp's species are one stream: the rates of the
-      // next group are on their way while a group is added
-      auto rates = [&](int4 t, double (&v)[4]) {
-        const int x[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const double d = Q(x[u] & 0x7fffffff);
-          v[u] = __hiloint2double(__double2hiint(d) ^ (x[u] & 0x80000000), __double2loint(d));
-        }
-      };
-      const int4 *tm = terms;
-      double v[4];
-      rates(t0, v);
-      int4 t = t1, sgn = sg0;
-#pragma unroll 1
-      for (int a = s0; a < s1; ++a) {
-        const int4 sg = sgn;
-        sgn = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a + 1);
-        double w = 0.0, w2 = 0.0;
-#pragma unroll 1
-        for (int e = 0; e < sg.y; ++e) {
-          double u[4];
-          rates(t, u);
-          t = __ldg(tm + 2);
-          ++tm;
-          w += v[0];
-          w2 += v[1];
-          w += v[2];
-          w2 += v[3];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) v[c] = u[c];
-        }
-#pragma unroll 1
-        for (int e = sg.z; e < sg.z + sg.w; ++e)
-          w = fma(__ldg(reinterpret_cast<const double *>(tab + f.wnu) + e),
-                  Q(__ldg(reinterpret_cast<const int *>(tab + f.wterm) + e)), w);
-        w += w2;
-        if (valid) {
-          bad += ((__double2hiint(w) >> 20) & 0x7ff) == 0x7ff;  // inf or NaN, integer test
-          b.wdot[(int64_t)sg.x * b.ld + i] = w;
-        }
-      }
-    }
+    sums.run(f, tab, q, b.wdot, b.ld, i, valid, bad);
     // rates are replaced only after the barrier at the loop's head
   }
   if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here

@@ -10,6 +10,7 @@
 #include "../../include/crs_tables.h"
 #include "crs_fx.cuh"
 #include "crs_fx_tab.cuh"
+#include "crs_shapes.cuh"
 
 namespace crs {
 namespace fx {
@@ -143,6 +144,160 @@ bool term(const Norm &n, ld a, ld x, bool inv, int64_t *w, int *flags, int bit) 
   w[0] = number((constant(c0) & ~1LL) | (a < 0));
   w[1] = coefficient(c1);
   return true;
+}
+
+// Lists of items for as many warps as `load` has entries (what they carry
+// already): longest first onto the least loaded.
+std::vector<std::vector<int>> deal(const std::vector<int> &w, std::vector<long long> load) {
+  std::vector<int> order(w.size());
+  for (size_t i = 0; i < w.size(); ++i) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return w[a] > w[c]; });
+  std::vector<std::vector<int>> bins(load.size());
+  for (int i : order) {
+    const int best = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    bins[best].push_back(i);
+    load[best] += w[i];
+  }
+  return bins;
+}
+
+// a double as the float-float pair that the mixed kernels use
+void pair_of(double v, float *w) {
+  w[0] = (float)v;
+  w[1] = (float)(v - (double)w[0]);
+}
+
+// The mixed-precision kernel's records and lists.
+void build_mixed(const Tab &t, FxTab &f, Buf &b) {
+  const int N = t.N, R = t.R;
+  f.mixed = N + 2 < 65536;
+  for (int j = 0; j < t.NREV; ++j) f.mixed &= t.kc_ptr[j + 1] - t.kc_ptr[j] <= 1;
+  if (!f.mixed) return;
+  // rows of the tile: the concentrations, ones, zeros
+  struct Rec {
+    int32_t slot;
+    uint16_t fac[6];
+    float rate[8], kc[32];
+  };
+  struct Eff {
+    float w;
+    int32_t row;
+  };
+  struct Other {
+    Rec r;
+    int32_t neff, ext, flags, sp;
+    float fall[8], broad[8];
+    Eff eff[MEFF];
+  };
+  static_assert(sizeof(Rec) == MREC && sizeof(Other) == MPAIR, "");
+  std::vector<char> shape(R, 0);
+  for (int p = t.seg[0]; p < t.seg[NSHAPE]; ++p) shape[t.perm[p]] = 1;
+  std::vector<Other> rec(R);
+  // kind: of shape groups, 2 x irreversible + third factors; third body,
+  // fall-off, neither, general
+  std::vector<int> weight(R), kind(R);
+  for (int r = 0; r < R; ++r) {
+    const int j = t.rev_idx[r], p = t.pm_idx[r];
+    Other &o = rec[r];
+    o = Other();
+    o.r.slot = r * 256;
+    bool ok = t.rate_kind[r] < RATE_PLOG;
+    int most = 0;
+    for (int side = 0; side < 2; ++side) {
+      const int32_t *ptr = side ? t.px_ptr : t.rx_ptr, *sp = side ? t.px_sp : t.rx_sp;
+      const int32_t *nint = side ? t.px_nint : t.rx_nint;
+      int n = 0;
+      for (int q = 0; q < 3; ++q) o.r.fac[3 * side + q] = (uint16_t)N;
+      if (side && j < 0) break;
+      for (int e = ptr[r]; e < ptr[r + 1]; ++e) {
+        ok &= nint[e] >= 0;
+        for (int q = 0; q < nint[e]; ++q, ++n)
+          if (n < 3) o.r.fac[3 * side + n] = (uint16_t)sp[e];
+      }
+      ok &= n <= 3;
+      most = std::max(most, n);
+    }
+    memcpy(o.r.rate, t.rate_ff + 8 * r, sizeof o.r.rate);
+    if (j >= 0) memcpy(o.r.kc, t.kc_mix + 32 * j, sizeof o.r.kc);
+    int flags = j >= 0 ? MF_REV : 0;
+    o.sp = -1;
+    if (p >= 0) {
+      const bool thd = t.pm_kind[p] == PM_THD;
+      flags |= thd ? MF_THD : MF_FALL;
+      if (!thd) {
+        o.sp = t.pm_sp[p];
+        const float *a = t.rate_ff + 8 * t.pm_k0[p], *c = t.rate_ff + 8 * t.pm_kinf[p];
+        for (int q = 0; q < 6; q += 2)
+          pair_of(((double)a[q] - c[q]) + ((double)a[q + 1] - c[q + 1]), o.fall + q);
+        o.fall[6] = a[6] * c[6];
+        const int form = t.pm_form[p];
+        if (t.pm_kind[p] == PM_FALL_LOW) o.flags |= PMF_LOW;
+        if (form == FORM_TROE) o.flags |= PMF_TROE | (t.pm_troe_t2[p] ? PMF_T2 : 0);
+        if (form == FORM_SRI) o.flags |= PMF_SRI | (t.pm_sri_de[p] ? PMF_DE : 0);
+        if (form != FORM_LINDEMANN)
+          memcpy(o.broad, (form == FORM_TROE ? t.troe_ff : t.sri_ff) + 8 * p, sizeof o.broad);
+      }
+      if (o.sp < 0) {
+        // an even number of terms
+        std::vector<Eff> more;
+        for (int e = t.pm_eff_ptr[p]; e < t.pm_eff_ptr[p + 1]; ++e)
+          more.push_back(Eff{t.eff_f[e], t.pm_eff_sp[e]});
+        if (more.size() & 1) more.push_back(Eff{0.0f, N});
+        o.neff = (int)more.size();
+        const size_t in = std::min<size_t>(more.size(), MEFF);
+        std::copy(more.begin(), more.begin() + in, o.eff);
+        more.erase(more.begin(), more.begin() + in);
+        if (!more.empty()) o.ext = b.put(more);
+      }
+    }
+    // instruction counts, in units of ten
+    if (shape[r]) {
+      kind[r] = (j >= 0 ? 0 : 2) + (most > 2);
+      weight[r] = j >= 0 ? 24 : 11;
+      flags = 0;
+    } else if (ok) {
+      kind[r] = p < 0 ? 6 : flags & MF_THD ? 4 : 5;
+      weight[r] = 28 + (p < 0 ? 0 : flags & MF_THD ? 2 + o.neff / 2 : 45);
+    } else {
+      flags = MF_GEN;
+      kind[r] = 7;
+      weight[r] = 250;
+    }
+    o.r.slot |= flags;
+  }
+  Rec none = Rec();  // completes a pair: both rates zero, into the slot of zeros
+  none.slot = R * 256;
+  for (int q = 0; q < 6; ++q) none.fac[q] = (uint16_t)(N + 1);
+  for (int l = 0; l < NLIST; ++l) {
+    const int nw = list_warps[l];
+    std::vector<long long> load(nw, 0);
+    load[0] = load[1] = 2 * N;  // the next tile's sums and functions of T
+    load[2] = 20;
+    std::vector<int32_t> ptr(1, 0), pairs;
+    std::vector<unsigned char> lr;
+    auto add = [&](const void *v, size_t n) {
+      lr.insert(lr.end(), (const unsigned char *)v, (const unsigned char *)v + n);
+    };
+    for (const auto &v : deal(weight, load)) {
+      for (int c = 0; c < 4; ++c) {
+        std::vector<Rec> two;
+        for (int r : v)
+          if (kind[r] == c) two.push_back(rec[r].r);
+        if (two.size() & 1) two.push_back(none);
+        for (size_t q = 0; q < two.size(); q += 2)
+          two[q].slot |= (c & 1 ? MF_MORE : 0) | (c < 2 ? MF_REV : 0);
+        if (!two.empty()) add(two.data(), two.size() * MREC);
+      }
+      pairs.push_back((int32_t)(lr.size() / MPAIR) - ptr.back());
+      for (int c = 4; c < 8; ++c)
+        for (int r : v)
+          if (kind[r] == c) add(&rec[r], MPAIR);
+      ptr.push_back((int32_t)(lr.size() / MPAIR));
+    }
+    f.mlist_ptr[l] = b.put(ptr);
+    f.mpairs[l] = b.put(pairs);
+    f.mrec[l] = b.put(lr);
+  }
 }
 
 }  // namespace
@@ -416,21 +571,9 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
       memcpy(nothing.data() + HEAD + COEF * q + 24, &z, 8);
     }
   }
-  // work lists: longest first onto the least loaded warp
+  // work lists
   for (int l = 0; l < NLIST; ++l) {
     const int nw = list_warps[l];
-    auto deal = [&](const std::vector<int> &w, std::vector<long long> load) {
-      std::vector<int> order(w.size());
-      for (size_t i = 0; i < w.size(); ++i) order[i] = (int)i;
-      std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return w[a] > w[c]; });
-      std::vector<std::vector<int>> bins(nw);
-      for (int i : order) {
-        const int best = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        bins[best].push_back(i);
-        load[best] += w[i];
-      }
-      return bins;
-    };
     // warps 0 and 1 also form the next tile's sums (chains of N dependent
     // FP64 additions), warp 2 its functions of T
     std::vector<long long> load(nw, 0);
@@ -479,6 +622,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
     f.term_ptr[l] = b.put(tptr);
     f.term[l] = b.put(term);
   }
+  build_mixed(t, f, b);
   f.bytes = (int)b.b.size();
   out.swap(b.b);
 }

@@ -51,8 +51,24 @@ struct FxTab {
   // zeros (row R)
   int seg_ptr[NLIST], seg[NLIST], term_ptr[NLIST], term[NLIST];
   int wterm, wnu;
+  // mixed precision (crs_mixed_tile.cu), in the same lists: per warp, its
+  // records (lists of MPAIR bytes each), those of pairs of shape-group
+  // reactions first
+  int mixed;  // the kernel takes this mechanism
+  int mlist_ptr[NLIST], mpairs[NLIST], mrec[NLIST];
   int bytes;
 };
+// A mixed record: int {slot offset | MF flags}, uint16 {three reactants, three
+// products} as rows of the tile, the rate row, the Kc polynomials.  Two of
+// them are a pair; a reaction outside the shape groups has one, then int4
+// {third-body terms, the first beyond the record, PMF flags, species row},
+// the fall-off's ln (k0 / kinf) row, its broadening's coefficients and MEFF
+// third-body terms {float, int row}.
+constexpr int MREC = 16 + 32 + 128, MPAIR = 2 * MREC;
+constexpr int MPM = MREC, MFALL = MPM + 16, MBROAD = MFALL + 32, MEFFS = MBROAD + 32;
+constexpr int MEFF = (MPAIR - MEFFS) / 8;
+// (of a pair's first record: some factor is a third one; reversible)
+enum { MF_MORE = 1, MF_REV = 2, MF_THD = 4, MF_FALL = 8, MF_GEN = 16 };
 
 }  // namespace fx
 }  // namespace crs

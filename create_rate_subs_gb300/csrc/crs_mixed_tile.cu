@@ -1,0 +1,525 @@
+// CRS_MODE_MIXED by tiles of 32 states: the arithmetic of crs_mixed.cuh in the
+// layout of crs_fx.cu.
+//
+// What bounds it.  The one-state-per-thread kernel holds 11 warps per SM
+// (12 bytes of shared memory per species and thread, 168 registers) and
+// waits: 42% of its issue slots, 35% of the FP64 pipe.  Here lane = state and
+// the warps of a CTA share the tile's concentrations and split its
+// reactions, then its species sums, so that 24 warps of 80 registers fit
+// whatever the mechanism's size; few tiles are shared by clusters.  Records
+// stream through each warp's ring in shared memory, two reactions of one
+// shape group at a time.  Three-body and fall-off reactions have records
+// too: read through the general tables, with their calls, the 60 of them
+// among 53/325 took more than the other 265.
+//
+// Every FP32 operation of a rate is that of the one-state-per-thread kernel
+// (a factor of one in place of an absent one is exact), so the FP32 roundings
+// are the same; FP64 keeps forward minus reverse, concentrations and sums.
+//
+// Measured on GB300 (before: one state per thread, large mechanisms in two
+// passes): 2^22 states of 53/325 35.6 -> 23.7 ms, 65,536 of 561/2539 5.32 ->
+// 3.60 ms.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "crs_exp.cuh"
+#include "crs_fx_tab.cuh"
+#include "crs_fx_tile.cuh"
+#include "crs_internal.cuh"
+#include "crs_mixed.cuh"
+
+namespace crs {
+namespace mixt {
+
+using namespace mixed;
+using namespace fx;
+
+struct Args {
+  const unsigned char *tab;  // fixed-point tables (lists, records)
+  const unsigned char *img;  // table image
+  double *q;                 // [gridDim.x / CL][R + 1][32] scratch when QS is false
+  int list;                  // the work list for NW CL warps
+};
+
+constexpr int D = 3;  // slots of a warp's ring of pairs of records
+
+// Per-state values of a tile, one block of 32 states: rho, y_N, and the
+// float-float T, ln T and 1/T, and P / (R T).
+constexpr int BLOCK = 256 + 256 + 7 * 128;
+
+// Sums, density and functions of T of one tile's states into the block at o,
+// on warps 0-2, in the operations and the order of the one-state-per-thread
+// kernel.  Called, not inlined: once per tile, and its registers are not the
+// rate loops'.
+__device__ __noinline__ void prepare(const Tab &t, const Batch &b, int64_t i, int warp, int lane,
+                                     unsigned char *o) {
+  double *rho = reinterpret_cast<double *>(o) + lane, *yN = rho + 32;
+  const int N = t.N;
+  const double *Y = b.Y + i;
+  const int64_t ld = b.ld;
+  if (warp == 0) {
+    double ys = 0.0;
+    int k = 0;
+    for (; k + 8 <= N - 1; k += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = Y[(int64_t)(k + u) * ld];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) ys += v[u];
+    }
+    for (; k < N - 1; ++k) ys += Y[(int64_t)k * ld];
+    *yN = 1.0 - ys;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+  } else if (warp == 1) {
+    double mwi = 0.0;
+    int k = 0;
+    for (; k + 8 <= N - 1; k += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = Y[(int64_t)(k + u) * ld];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) mwi = fma(v[u], t.inv_mw[k + u], mwi);
+    }
+    for (; k < N - 1; ++k) mwi = fma(Y[(int64_t)k * ld], t.inv_mw[k], mwi);
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    mwi = fma(*yN, t.inv_mw[N - 1], mwi);
+    *rho = b.P[i] / mwi * ((1.0 / b.T[i]) * INV_RU);
+  } else {
+    const double T = b.T[i];
+    const ff a = ff_from_double_int(T), l = ff_from_double_int(texp::log_t(T, t.logtab));
+    const ff v = ff_from_double_int(1.0 / T);
+    float *w = reinterpret_cast<float *>(o + 512) + lane;
+    w[0] = a.h;
+    w[32] = a.l;
+    w[64] = l.h;
+    w[96] = l.l;
+    w[128] = v.h;
+    w[160] = v.l;
+    w[192] = d2f_rn(b.P[i] * (1.0 / T) * INV_RU);
+  }
+}
+
+// Net rate of a reaction outside the shape groups.
+__device__ __noinline__ double other_rate(const unsigned char *img, const ImgLayout &lay, int r,
+                                          const Batch &b, int64_t i, const float *C,
+                                          const unsigned char *o, int lane) {
+  const Tab t = make_tab(img, lay);
+  const float *w = reinterpret_cast<const float *>(o + 512) + lane;
+  State s;
+  s.T = b.T[i];
+  s.P = b.P[i];
+  s.invT = 1.0 / s.T;
+  s.logT = 0.0;
+  s.Tf = (float)s.T;
+  s.Tff = ff{w[0], w[32]};
+  s.lTff = ff{w[64], w[96]};
+  s.iTff = ff{w[128], w[160]};
+  KcMix kc;
+  kc.Tbits = __double_as_longlong(s.T);
+  kc.T = s.Tff;
+  kc.logT = s.lTff;
+  kc.invT = s.iTff;
+  const float mix = d2f_rn(s.P * s.invT * INV_RU);
+  const FCol col{const_cast<float *>(C), 32};
+  double fwd, rev;
+  float pm;
+  if (t.rate_kind[r] >= RATE_PLOG) {
+    s.logT = texp::log_t(s.T, t.logtab);
+    return rxn_net<true>(t, r, s, mix, col, kc, fwd, rev, pm);
+  }
+  return rxn_net<false>(t, r, s, mix, col, kc, fwd, rev, pm);
+}
+
+// p * 2^k, rounded once, for a normal p and a result that may be subnormal or
+// zero; |k| <= 250
+__device__ __forceinline__ float scale2(float p, int k) {
+  const int a = k >> 1;
+  return p * __int_as_float((a + 127) << 23) * __int_as_float((k - a + 127) << 23);
+}
+
+// ff_expf, without calls
+__device__ __forceinline__ float expf_of(ff x) {
+  int k;
+  const float p = ff_exp(x, k);
+  const float v = scale2(p, min(max(k, -250), 250));
+  return x.h > 88.0f ? INFINITY : x.h < -103.0f ? 0.0f : v;
+}
+
+// The fall-off factor of the record at r for a third-body concentration thd:
+// mixed::pres_mod's operations, the exponent of k0 / kinf from one row.
+__device__ __forceinline__ float falloff(const unsigned char *r, int flags, float thd, ff T,
+                                         ff lT, ff iT) {
+  const float4 a = *reinterpret_cast<const float4 *>(r + MFALL);
+  const float4 c = *reinterpret_cast<const float4 *>(r + MFALL + 16);
+  ff z = ff_add(ff{a.x, a.y}, ff_mul(ff{a.z, a.w}, lT));
+  z = ff_add(z, ff_mul(ff{c.x, c.y}, iT));
+  int E, et, e2;
+  float m = ff_exp(z, E);
+  m = fsplit(m * fsplit(thd * c.z, et), e2);
+  E += et + e2;
+  // Pr/(1+Pr) and 1/(1+Pr) from whichever of Pr and 1/Pr is at most 1
+  const bool less = E < 0;
+  const float s = scale2(less ? m : __frcp_rn(m), max(less ? E : -E, -250));
+  const float d = __frcp_rn(1.0f + s), u = s * d;
+  float frac = less ? u : d, inv1p = less ? d : u;
+  if (m <= 0.0f) {
+    frac = 0.0f;
+    inv1p = 1.0f;
+  }
+  const float side = (flags & PMF_LOW) ? frac : inv1p;
+  if (!(flags & (PMF_TROE | PMF_SRI))) return side;
+  ff lnPr = ff{-1.0e30f, 0.0f};
+  if (m > 0.0f) {
+    const float Ef = (float)E;
+    lnPr = ff_add(ff{Ef * LN2_H12_F, 0.0f}, ff{fmaf(Ef, LN2_L12_F, logf(m)), 0.0f});
+  }
+  ff lP = ff_mul(lnPr, ff{INV_LN10_F, INV_LN10_LO_F});
+  if (lP.h < -300.0f) lP = ff{-300.0f, 0.0f};
+  const float4 g = *reinterpret_cast<const float4 *>(r + MBROAD);
+  const float4 h = *reinterpret_cast<const float4 *>(r + MBROAD + 16);
+  // F = exp(ln base * w)
+  float ln, F;
+  ff w;
+  if (flags & PMF_TROE) {
+    float f = g.x * expf_of(ff_mul(T, ff{g.y, g.z})) + g.w * expf_of(ff_mul(T, ff{h.x, h.y}));
+    if (flags & PMF_T2) f += expf_of(ff_mul(iT, ff{h.z, h.w}));
+    ln = logf(fmaxf(f, 1.0e-37f));
+    const ff lF = ff_mul(ff{ln, 0.0f}, ff{INV_LN10_F, INV_LN10_LO_F});
+    const ff A =
+        ff_add(ff_add(lP, ff_neg(ff_mul(ff{0.6700000166893005f, -1.668930060816365e-08f}, lF))),
+               ff{-0.4000000059604645f, 5.9604645663569045e-09f});
+    const ff B =
+        ff_add(ff_add(ff{0.8059999942779541f, 5.7220459481754915e-09f},
+                      ff_neg(ff_mul(ff{1.176200032234192f, -3.2234190427971043e-08f}, lF))),
+               ff_neg(ff_mul(ff{0.14000000059604645f, -5.9604643443123e-10f}, lP)));
+    const ff B2 = ff_mul(B, B);
+    w = ff_div(B2, ff_add(ff_mul(A, A), B2));
+    F = expf_of(ff_mul(ff{ln, 0.0f}, w));
+  } else {
+    w = ff_div(ff{1.0f, 0.0f}, ff_add(ff{1.0f, 0.0f}, ff_mul(lP, lP)));
+    ln = logf(g.x * expf_of(ff_mul(iT, ff{g.y, g.z})) + expf_of(ff_mul(T, ff{g.w, h.x})));
+    F = expf_of(ff_mul(w, ff{ln, 0.0f}));
+    if (flags & PMF_DE) F *= h.y * expf_of(ff_mul(ff{h.z, 0.0f}, lT));
+  }
+  return F * side;
+}
+
+// NW warps per CTA, CL CTAs (a cluster) per tile.
+template <int NW, int PER_SM, int CL, bool QS>
+__global__ void __launch_bounds__(NW * 32, PER_SM)
+    k_wdot_tile(const __grid_constant__ ImgLayout lay, const __grid_constant__ FxTab f,
+                const __grid_constant__ Args g, const __grid_constant__ Batch b) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int N = f.N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned char *tab = g.tab;
+  // shared memory: the concentrations [N][32], a row of ones, a row of zeros;
+  // two blocks of per-state values; each warp's ring of records; the rates
+  unsigned char *cl = smem + lane * 4;
+  unsigned char *next = smem + (N + 2) * 128;
+  unsigned char *blk = next;
+  next += 2 * BLOCK;
+  unsigned char *ring = next + warp * (D * MPAIR);
+  next += NW * (D * MPAIR);
+  unsigned char *q =
+      (QS && CL > 1 ? static_cast<unsigned char *>(__cluster_map_shared_rank(next, 0))
+       : QS ? next
+            : reinterpret_cast<unsigned char *>(g.q) +
+                  (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256) +
+      lane * 8;
+  auto C = [&](int row) -> float & { return *reinterpret_cast<float *>(cl + row * 128); };
+  auto Q = [&](int off) -> double & { return *reinterpret_cast<double *>(q + off); };
+  if (warp == 0) {
+    C(N) = 1.0f;
+    C(N + 1) = 0.0f;
+    if (!QS || CL == 1) Q(f.R * 256) = 0.0;
+    else reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
+  }
+  const int gw = CL == 1 ? warp : (int)(blockIdx.x % CL) * NW + warp;  // the tile's warp
+  const int *lp = reinterpret_cast<const int *>(tab + f.mlist_ptr[g.list]) + gw;
+  const Ring<D> recs{tab + f.mrec[g.list] + (int64_t)lp[0] * MPAIR, smem_u32(ring), MPAIR,
+                     lp[1] - lp[0], lane};
+  const int npairs = reinterpret_cast<const int *>(tab + f.mpairs[g.list])[gw];
+  Sums sums(f, tab, g.list, gw);
+  int bad = 0, bk = 0;
+  int64_t tile = blockIdx.x / CL;
+  const int64_t step = gridDim.x / CL;
+  const int64_t ntiles = (b.n + 31) / 32;
+  const Tab t = make_tab(g.img, lay);
+  if (tile < ntiles && warp < 3)
+    prepare(t, b, tile * 32 + lane < b.n ? tile * 32 + lane : tile * 32, warp, lane, blk);
+  for (; tile < ntiles; tile += step, bk ^= 1) {
+    const int64_t i = tile * 32 + lane;
+    const bool valid = i < b.n;
+    const int64_t ic = valid ? i : tile * 32;  // idle lanes repeat a valid state
+    tile_barrier<CL>();
+    recs.start();
+    const unsigned char *o = blk + bk * BLOCK;
+    const double rho = reinterpret_cast<const double *>(o)[lane];
+#pragma unroll 4
+    for (int k = warp; k < N; k += NW) {
+      const double y = k == N - 1 ? reinterpret_cast<const double *>(o + 256)[lane]
+                                  : b.Y[(int64_t)k * b.ld + ic];
+      C(k) = d2f_rn(y * (rho * __ldg(t.inv_mw + k)));
+    }
+    __syncthreads();
+    // net rates
+    if (warp < 3 && tile + step < ntiles) {
+      const int64_t j = (tile + step) * 32;
+      prepare(t, b, j + lane < b.n ? j + lane : j, warp, lane, blk + (bk ^ 1) * BLOCK);
+    }
+    {
+      const float *w = reinterpret_cast<const float *>(o + 512) + lane;
+      const ff T{w[0], w[32]}, lT{w[64], w[96]}, iT{w[128], w[160]};
+      const long long Tbits = __double_as_longlong(b.T[ic]);
+      // mantissa times the factors' (rounding errors kept), their exponents
+      auto factor = [&](int row, float &m, float &err, int &E) {
+        const unsigned u = __float_as_uint(C(row));
+        const int fe = (int)((u >> 23) & 0xffu);
+        // (a zero's exponent does not matter: the product is zero)
+        const float x = fe == 0 ? 0.0f : __uint_as_float((u & 0x807fffffu) | 0x3f800000u);
+        const float mm = m * x;
+        err = fmaf(err, x, fmaf(m, x, -mm));
+        m = mm;
+        E += fe - 127;
+      };
+      auto exponent = [&](const unsigned char *r) {
+        const float4 a = *reinterpret_cast<const float4 *>(r + 16);
+        const float2 c = *reinterpret_cast<const float2 *>(r + 32);
+        const ff x = ff_add(ff{a.x, a.y}, ff_mul(ff{a.z, a.w}, lT));
+        return ff_add(x, ff_mul(ff{c.x, c.y}, iT));
+      };
+      auto kc_of = [&](const unsigned char *r) {
+        const longlong2 *lo3 = reinterpret_cast<const longlong2 *>(r + 96);
+        const float4 *c = reinterpret_cast<const float4 *>(r + 48 + (Tbits <= lo3->y ? 0 : 64));
+        const float4 a = c[0], d = c[1], e = c[2], h = c[3];
+        ff v = ff{e.z, e.w};
+        v = ff_fma(v, T, ff{e.x, e.y});
+        v = ff_fma(v, T, ff{d.z, d.w});
+        v = ff_fma(v, T, ff{d.x, d.y});
+        v = ff_fma(v, T, ff{a.x, a.y});
+        v = ff_fma(ff{a.z, a.w}, lT, v);
+        return ff_fma(ff{h.x, h.y}, iT, v);
+      };
+      const unsigned char *at = ring;
+#pragma unroll 1
+      for (int p = 0; p < npairs; ++p) {
+        recs.next(p);
+        const int4 h[2] = {*reinterpret_cast<const int4 *>(at),
+                           *reinterpret_cast<const int4 *>(at + MREC)};
+        const bool more = h[0].x & MF_MORE, reversible = h[0].x & MF_REV;
+        ff x[2];
+        float m[2], err[2];
+        int E[2];
+        double v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          x[u] = exponent(at + u * MREC);
+          m[u] = ff_exp(x[u], E[u]);
+          err[u] = 0.0f;
+          factor(h[u].y & 0xffff, m[u], err[u], E[u]);
+          factor((unsigned)h[u].y >> 16, m[u], err[u], E[u]);
+        }
+        if (more) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) factor(h[u].z & 0xffff, m[u], err[u], E[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) v[u] = assemble(m[u] + err[u], E[u]);
+        if (reversible) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            m[u] = ff_exp(ff_add(x[u], ff_neg(kc_of(at + u * MREC))), E[u]);
+            err[u] = 0.0f;
+            factor((unsigned)h[u].z >> 16, m[u], err[u], E[u]);
+            factor(h[u].w & 0xffff, m[u], err[u], E[u]);
+          }
+          if (more) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) factor((unsigned)h[u].w >> 16, m[u], err[u], E[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) v[u] -= assemble(m[u] + err[u], E[u]);  // FP64
+        }
+        Q(h[0].x & ~255) = v[0];
+        Q(h[1].x) = v[1];
+        at = at == ring + (D - 1) * MPAIR ? ring : at + MPAIR;
+      }
+#pragma unroll 1
+      for (int p = npairs; p < recs.n; ++p) {
+        recs.next(p);
+        const int4 h = *reinterpret_cast<const int4 *>(at);
+        if (h.x & MF_GEN) {
+          Q(h.x & ~255) = other_rate(g.img, lay, h.x >> 8, b, ic, &C(0), o, lane);
+        } else {
+          float pm = 0.0f;
+          if (h.x & (MF_THD | MF_FALL)) {
+            const int4 ph = *reinterpret_cast<const int4 *>(at + MPM);
+            if (ph.w >= 0) {
+              pm = C(ph.w);
+            } else {
+              pm = reinterpret_cast<const float *>(o + 512 + 768)[lane];
+              const float4 *e = reinterpret_cast<const float4 *>(at + MEFFS);
+#pragma unroll 1
+              for (int c = 0; c < ph.x; c += 2) {
+                if (c == MEFF) e = reinterpret_cast<const float4 *>(tab + ph.y) - MEFF / 2;
+                const float4 v = e[c / 2];
+                pm = fmaf(v.x, C(__float_as_int(v.y)), pm);
+                pm = fmaf(v.z, C(__float_as_int(v.w)), pm);
+              }
+            }
+            if (h.x & MF_FALL) pm = falloff(at, ph.z, pm, T, lT, iT);
+          }
+          const ff xf = exponent(at), xr = ff_add(xf, ff_neg(kc_of(at)));
+          const float sg = *reinterpret_cast<const float *>(at + 40);
+          int Ef, Er;
+          float mf = ff_exp(xf, Ef), mr = ff_exp(xr, Er), ef = 0.0f, er = 0.0f;
+          factor(h.y & 0xffff, mf, ef, Ef);
+          factor((unsigned)h.z >> 16, mr, er, Er);
+          factor((unsigned)h.y >> 16, mf, ef, Ef);
+          factor(h.w & 0xffff, mr, er, Er);
+          factor(h.z & 0xffff, mf, ef, Ef);
+          factor((unsigned)h.w >> 16, mr, er, Er);
+          double v = assemble(sg * (mf + ef), Ef);
+          if (h.x & MF_REV) v -= assemble(sg * (mr + er), Er);  // FP64
+          if (h.x & (MF_THD | MF_FALL)) v *= f2d_exact(pm);
+          Q(h.x & ~255) = v;
+        }
+        at = at == ring + (D - 1) * MPAIR ? ring : at + MPAIR;
+      }
+    }
+    sums.ahead();
+    tile_barrier<CL>();
+    sums.run(f, tab, q, b.wdot, b.ld, i, valid, bad);
+    // rates are replaced only after the barrier at the loop's head
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here
+  if (bad && b.status) atomicAdd(&b.status[1], bad);
+}
+
+size_t smem_of(const FxTab &f, int nw, bool qs) {
+  return (size_t)(f.N + 2) * 128 + 2 * BLOCK + (size_t)nw * D * MPAIR +
+         (qs ? (size_t)(f.R + 1) * 256 : 0);
+}
+
+struct Plan {
+  int nw = 24, per_sm = 1, cl = 1;
+  bool qs = false, ok = false;
+};
+
+Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
+  if (!f.mixed) return Plan{};
+  auto fits = [&](int nw, int per_sm, bool qs) {
+    return (smem_of(f, nw, qs) + 1024) * per_sm <= (size_t)smem_optin + 1024;
+  };
+  for (int cl = 8; cl > 1; cl /= 2)
+    if (tiles * cl <= sm_count && f.R >= 32 * cl) {
+      if (fits(16, 1, true)) return Plan{16, 1, cl, true, true};
+      if (fits(16, 1, false)) return Plan{16, 1, cl, false, true};
+    }
+  if (tiles <= sm_count && fits(16, 1, true)) return Plan{16, 1, 1, true, true};
+  if (f.R < 100 && fits(4, 6, true)) return Plan{4, 6, 1, true, true};
+  if (fits(8, 3, false)) return Plan{8, 3, 1, false, true};
+  Plan p{24, 1, 1, false, false};
+  p.ok = fits(24, 1, false);
+  return p;
+}
+
+using Kernel = void (*)(const ImgLayout, const FxTab, const Args, const Batch);
+Kernel kernel_of(const Plan &p) {
+  switch (p.cl) {
+    case 8: return p.qs ? k_wdot_tile<16, 1, 8, true> : k_wdot_tile<16, 1, 8, false>;
+    case 4: return p.qs ? k_wdot_tile<16, 1, 4, true> : k_wdot_tile<16, 1, 4, false>;
+    case 2: return p.qs ? k_wdot_tile<16, 1, 2, true> : k_wdot_tile<16, 1, 2, false>;
+  }
+  if (p.nw == 4) return k_wdot_tile<4, 6, 1, true>;
+  if (p.nw == 16) return k_wdot_tile<16, 1, 1, true>;
+  if (p.nw == 8) return k_wdot_tile<8, 3, 1, false>;
+  return k_wdot_tile<24, 1, 1, false>;
+}
+
+}  // namespace mixt
+
+cudaError_t mixed_tile_init(int smem_optin) {
+  cudaError_t e = cudaSuccess;
+  for (int q = 0; q < 7 && e == cudaSuccess; ++q) {
+    mixt::Plan p;
+    p.cl = q < 3 ? 2 << q : 1;
+    p.nw = q == 3 ? 4 : q == 4 ? 16 : q == 5 ? 8 : 24;
+    p.qs = true;
+    e = set_smem_limit(mixt::kernel_of(p), (size_t)smem_optin);
+    p.qs = false;
+    if (e == cudaSuccess) e = set_smem_limit(mixt::kernel_of(p), (size_t)smem_optin);
+  }
+  return e;
+}
+
+static int64_t mixed_first(const fx::FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
+  const mixt::Plan p = mixt::plan_of(f, tiles, sm_count, smem_optin);
+  const int64_t wave = (int64_t)sm_count * p.per_sm;
+  const int64_t rest = tiles % wave;
+  return p.cl > 1 || tiles < wave || rest == 0 || 2 * rest > sm_count || f.R < 64 ? tiles
+                                                                                  : tiles - rest;
+}
+
+long long mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
+  const int64_t tiles = (n + 31) / 32, first = mixed_first(f, tiles, sm_count, smem_optin);
+  long long most = 0;
+  for (int64_t part : {first, tiles - first}) {
+    if (part == 0) continue;
+    const mixt::Plan p = mixt::plan_of(f, part, sm_count, smem_optin);
+    if (!p.ok) return -1;
+    if (p.qs) continue;
+    const long long need = (long long)std::min<int64_t>(part, (int64_t)sm_count * p.per_sm) *
+                           (f.R + 1) * 256;
+    most = std::max(most, need);
+  }
+  return most;
+}
+
+static cudaError_t launch_mixed_part(const unsigned char *img, const ImgLayout &L,
+                                     const fx::FxTab &f, const unsigned char *tab, const Batch &b,
+                                     int sm_count, int smem_optin, double *scratch,
+                                     cudaStream_t s) {
+  const int64_t tiles = (b.n + 31) / 32;
+  const mixt::Plan p = mixt::plan_of(f, tiles, sm_count, smem_optin);
+  if (!p.ok || (!p.qs && !scratch)) return cudaErrorInvalidValue;
+  int list = 0;
+  while (list < fx::NLIST - 1 && fx::list_warps[list] != p.nw * p.cl) ++list;
+  const mixt::Kernel k = mixt::kernel_of(p);
+  const size_t bytes = mixt::smem_of(f, p.nw, p.qs);
+  const int64_t grid = std::min<int64_t>(tiles, (int64_t)sm_count * p.per_sm) * p.cl;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)p.nw * 32);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)p.cl;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = p.cl > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, L, f, mixt::Args{tab, img, scratch, list}, b);
+}
+
+cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
+                              const unsigned char *tab, const Batch &b, int sm_count,
+                              int smem_optin, double *scratch, cudaStream_t s) {
+  const int64_t tiles = (b.n + 31) / 32, first = mixed_first(f, tiles, sm_count, smem_optin);
+  Batch part = b;
+  part.n = std::min<int64_t>(b.n, first * 32);
+  cudaError_t e = launch_mixed_part(img, L, f, tab, part, sm_count, smem_optin, scratch, s);
+  if (e != cudaSuccess || first == tiles) return e;
+  const int64_t o = part.n;
+  part.n = b.n - o;
+  part.T += o;
+  part.P += o;
+  part.Y += o;
+  part.wdot += o;
+  return launch_mixed_part(img, L, f, tab, part, sm_count, smem_optin, scratch, s);
+}
+
+}  // namespace crs

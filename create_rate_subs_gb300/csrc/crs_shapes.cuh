@@ -12,6 +12,8 @@
 // Only the order in which reactions add into wdot changes.
 #pragma once
 
+#include "../../include/crs_tables.h"
+
 namespace crs {
 
 struct Shape {
@@ -21,7 +23,7 @@ struct Shape {
 // The shapes with specialised code paths (2->2 reversible first: it is by
 // far the most common elementary form).
 constexpr int NSHAPE = 11;
-__host__ __device__ constexpr Shape shape_of(int s) {
+CRS_HD constexpr Shape shape_of(int s) {
   return s == 0 ? Shape{2, 2, 4, 1}
        : s == 1 ? Shape{2, 3, 5, 1}
        : s == 2 ? Shape{2, 2, 4, 0}
