@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       if (later || all)
         finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
     }
-    sums.ahead();
+    sums.ahead(f, tab);
     tile_barrier<CL>();
     // the next tile's mass fractions replace exponents that every warp is
     // done with, while the species sums run
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       const int64_t j = (tile + step) * 32;
       load_y<NW>(b.Y + (j + lane < b.n ? j + lane : j), b.ld, N, warp, yrows);
     }
-    sums.run(f, tab, q, b.wdot, b.ld, i, valid, bad);
+    sums.run(f, tab, q, 0u, b.wdot, b.ld, i, valid, bad);
     // rates are replaced only after the barrier at the loop's head
   }
   if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here

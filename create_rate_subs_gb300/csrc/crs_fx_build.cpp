@@ -173,7 +173,7 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
   f.mixed = N + 2 < 65536;
   for (int j = 0; j < t.NREV; ++j) f.mixed &= t.kc_ptr[j + 1] - t.kc_ptr[j] <= 1;
   if (!f.mixed) return;
-  // rows of the tile: the concentrations, ones, zeros
+  // rows of the tile: the concentrations, one, zero
   struct Rec {
     int32_t slot;
     uint16_t fac[6];
@@ -218,7 +218,20 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
       most = std::max(most, n);
     }
     memcpy(o.r.rate, t.rate_ff + 8 * r, sizeof o.r.rate);
-    if (j >= 0) memcpy(o.r.kc, t.kc_mix + 32 * j, sizeof o.r.kc);
+    if (j >= 0) {
+      // the reverse exponent: forward minus the equilibrium constant's, each
+      // block c0, c1 (ln T), c2 .. c5 (powers of T), 1/T and, of the first,
+      // T_common
+      memcpy(o.r.kc, t.kc_mix + 32 * j, sizeof o.r.kc);
+      for (int blk = 0; blk < 32; blk += 16)
+        for (int q = 0; q < 14; q += 2) {
+          float *c = o.r.kc + blk + q;
+          const int w = q == 0 ? 0 : q == 2 ? 2 : q == 12 ? 4 : -1;  // the rate row's term
+          double v = -((double)c[0] + c[1]);
+          if (w >= 0) v += (double)o.r.rate[w] + o.r.rate[w + 1];
+          pair_of(v, c);
+        }
+    }
     int flags = j >= 0 ? MF_REV : 0;
     o.sp = -1;
     if (p >= 0) {
