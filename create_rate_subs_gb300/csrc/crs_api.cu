@@ -75,6 +75,12 @@ long long mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int sm
 cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                               const unsigned char *tab, const Batch &b, int sm_count,
                               int smem_optin, double *scratch, cudaStream_t s);
+// The contraction's operand by the same tiles.
+long long mixed_pack_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+cudaError_t launch_mixed_pack(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
+                              const unsigned char *tab, const Batch &b, int sm_count,
+                              int smem_optin, double *scratch, void *A, int Kh, int *escale,
+                              cudaStream_t s);
 // Tables the fast kernels derive from the blob's tables at load time.
 bool build_fast_tables(const std::vector<unsigned char> &img,
                        const ImgLayout &L, std::vector<Derived> &extra);
@@ -561,10 +567,10 @@ int64_t q_chunk(const crs::ImgLayout &L, int64_t n) {
 }
 
 // Workspace of the two-pass paths for chunks of `rows` states (caller
-// holds ws_mu); with_ws: also the contraction's bf16 rows and exponents.
-int ensure_q(crs_mech *m, int64_t rows, bool with_ws) {
+// holds ws_mu); with_q: the rates; with_ws: the contraction's bf16 rows and exponents.
+int ensure_q(crs_mech *m, int64_t rows, bool with_q, bool with_ws) {
   cudaError_t e = cudaSuccess;
-  if (m->q_rows < rows) {
+  if (with_q && m->q_rows < rows) {
     if (m->d_q) cudaFree(m->d_q);
     m->d_q = nullptr;
     m->q_rows = 0;
@@ -632,7 +638,7 @@ int wdot_two_pass(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool fp64) {
     return fail(CRS_ERR_UNSUPPORTED, "mechanism too large for the rates tile");
   std::lock_guard<std::mutex> lk(m->ws_mu);
   const int64_t rows = q_chunk(m->L, b.n);
-  int rc = ensure_q(m, rows, false);
+  int rc = ensure_q(m, rows, true, false);
   if (rc == CRS_OK) rc = ws_begin(m, s);
   if (rc != CRS_OK) return rc;
   for (int64_t c0 = 0; c0 < b.n && rc == CRS_OK; c0 += rows) {
@@ -710,9 +716,21 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
   if (rc != CRS_OK) return rc;
   const int64_t K = 2 * (int64_t)m->Kh;
   const int64_t rows = q_chunk(m->L, b.n);
-  rc = ensure_q(m, rows, true);
+  // rates and packing in one kernel when the mechanism fits its tiles
+  const long long scratch = crs::mixed_pack_scratch(m->fx, rows, m->sm_count, m->smem_optin);
+  double *q = nullptr;
+  if (scratch > 0) {
+    const cudaError_t e =
+        cudaMallocFromPoolAsync(reinterpret_cast<void **>(&q), (size_t)scratch, m->fx_pool, s);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    else if (e != cudaSuccess) return cuda_fail(e, "gemm scratch");
+  }
+  rc = ensure_q(m, rows, !q, true);
   if (rc == CRS_OK) rc = ws_begin(m, s);
-  if (rc != CRS_OK) return rc;
+  if (rc != CRS_OK) {
+    if (q) cudaFreeAsync(q, s);
+    return rc;
+  }
   for (int64_t c0 = 0; c0 < b.n && rc == CRS_OK; c0 += rows) {
     const int64_t cnt = std::min<int64_t>(rows, b.n - c0);
     crs::Batch bc = b;
@@ -721,14 +739,20 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
     bc.P = b.P + c0;
     bc.Y = b.Y + c0;
     bc.wdot = b.wdot + c0;
-    cudaError_t e = crs::launch_rates_tile(m->d_img, m->L, bc, m->sm_count, m->smem_optin, s,
-                                           m->d_q, rows, m->d_escale);
-    if (e == cudaSuccess)
-      e = crs::launch_pack_bf16(m->d_q, rows, cnt, m->L.R, m->Kh, m->d_escale, m->d_ws, K,
-                                m->d_outflag, m->sm_count, s);
-    if (e == cudaSuccess)
-      e = crs::launch_spec_sum(m->d_img, m->L, m->d_q, rows, cnt, m->d_escale, m->d_outflag,
-                               bc.wdot, b.ld, m->d_status, m->sm_count, s);
+    cudaError_t e;
+    if (q) {
+      e = crs::launch_mixed_pack(m->d_img, m->L, m->fx, m->d_fx, bc, m->sm_count, m->smem_optin,
+                                 q, m->d_ws, m->Kh, m->d_escale, s);
+    } else {
+      e = crs::launch_rates_tile(m->d_img, m->L, bc, m->sm_count, m->smem_optin, s, m->d_q, rows,
+                                 m->d_escale);
+      if (e == cudaSuccess)
+        e = crs::launch_pack_bf16(m->d_q, rows, cnt, m->L.R, m->Kh, m->d_escale, m->d_ws, K,
+                                  m->d_outflag, m->sm_count, s);
+      if (e == cudaSuccess)
+        e = crs::launch_spec_sum(m->d_img, m->L, m->d_q, rows, cnt, m->d_escale, m->d_outflag,
+                                 bc.wdot, b.ld, m->d_status, m->sm_count, s);
+    }
     const int64_t M_pad = (cnt + 127) / 128 * 128;
     if (e == cudaSuccess)
       e = crs::launch_gemm_wdot(m->d_ws, m->d_nuB, M_pad, m->N_pad, K, m->block_n, bc.wdot,
@@ -736,6 +760,7 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
     if (e == cudaErrorNotSupported) rc = fail(CRS_ERR_UNSUPPORTED, "rates tile not available");
     else if (e != cudaSuccess) rc = cuda_fail(e, "gemm launch");
   }
+  if (q) cudaFreeAsync(q, s);
   const int rc2 = ws_end(m, s);
   return rc != CRS_OK ? rc : rc2;
 }

@@ -186,7 +186,7 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
   struct Other {
     Rec r;
     int32_t neff, ext, flags, sp;
-    float fall[8], broad[8];
+    float fall[16], broad[8];
     Eff eff[MEFF];
   };
   static_assert(sizeof(Rec) == MREC && sizeof(Other) == MPAIR, "");
@@ -239,10 +239,9 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
       flags |= thd ? MF_THD : MF_FALL;
       if (!thd) {
         o.sp = t.pm_sp[p];
-        const float *a = t.rate_ff + 8 * t.pm_k0[p], *c = t.rate_ff + 8 * t.pm_kinf[p];
-        for (int q = 0; q < 6; q += 2)
-          pair_of(((double)a[q] - c[q]) + ((double)a[q + 1] - c[q + 1]), o.fall + q);
-        o.fall[6] = a[6] * c[6];
+        memcpy(o.fall, t.rate_ff + 8 * t.pm_k0[p], 32);
+        memcpy(o.fall + 8, t.rate_ff + 8 * t.pm_kinf[p], 32);
+        o.fall[6] *= o.fall[14];  // the signs
         const int form = t.pm_form[p];
         if (t.pm_kind[p] == PM_FALL_LOW) o.flags |= PMF_LOW;
         if (form == FORM_TROE) o.flags |= PMF_TROE | (t.pm_troe_t2[p] ? PMF_T2 : 0);

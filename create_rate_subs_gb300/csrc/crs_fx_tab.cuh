@@ -62,10 +62,10 @@ struct FxTab {
 // products} as rows of the tile, the rate row, the Kc polynomials.  Two of
 // them are a pair; a reaction outside the shape groups has one, then int4
 // {third-body terms, the first beyond the record, PMF flags, species row},
-// the fall-off's ln (k0 / kinf) row, its broadening's coefficients and MEFF
+// the fall-off's two rate rows, its broadening's coefficients and MEFF
 // third-body terms {float, int row}.
 constexpr int MREC = 16 + 32 + 128, MPAIR = 2 * MREC;
-constexpr int MPM = MREC, MFALL = MPM + 16, MBROAD = MFALL + 32, MEFFS = MBROAD + 32;
+constexpr int MPM = MREC, MFALL = MPM + 16, MBROAD = MFALL + 64, MEFFS = MBROAD + 32;
 constexpr int MEFF = (MPAIR - MEFFS) / 8;
 // (of a pair's first record: some factor is a third one; reversible)
 enum { MF_MORE = 1, MF_REV = 2, MF_THD = 4, MF_FALL = 8, MF_GEN = 16 };

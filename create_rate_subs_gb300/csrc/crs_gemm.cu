@@ -81,10 +81,10 @@ cudaError_t launch_gemm_wdot(const void *A, const void *B, int64_t M_pad, int64_
     return cudaErrorInvalidValue;
   gemm::EpiWdot epi{out, ld, m_valid, n_valid, escale};
   switch (block_n) {
-    case 64: return launch_gemm<64>(ta, tb, M_pad, N_pad, K, epi, status, s);
-    case 128: return launch_gemm<128>(ta, tb, M_pad, N_pad, K, epi, status, s);
-    case 192: return launch_gemm<192>(ta, tb, M_pad, N_pad, K, epi, status, s);
-    case 256: return launch_gemm<256>(ta, tb, M_pad, N_pad, K, epi, status, s);
+    case 64: return launch_gemm<64, gemm::EpiWdot, 2, 256, true>(ta, tb, M_pad, N_pad, K, epi, status, s);
+    case 128: return launch_gemm<128, gemm::EpiWdot, 2, 256, true>(ta, tb, M_pad, N_pad, K, epi, status, s);
+    case 192: return launch_gemm<192, gemm::EpiWdot, 2, 256, true>(ta, tb, M_pad, N_pad, K, epi, status, s);
+    case 256: return launch_gemm<256, gemm::EpiWdot, 2, 256, true>(ta, tb, M_pad, N_pad, K, epi, status, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -102,7 +102,9 @@ constexpr size_t smem_bytes() {
 // rank allows) and, with NT = 256, half of the columns.  ST = 2 and NT = 256
 // let two CTAs share an SM (registers capped for two), so one tile's
 // epilogue overlaps the next tile's loads and MMAs.
-template <int BN, class Epi, int ST = STAGES, int NT = 128>
+// NF: the CTAs of one row block follow each other (blockIdx.x is the column
+// block), so that its rows of A are read from HBM once.
+template <int BN, class Epi, int ST = STAGES, int NT = 128, bool NF = false>
 __global__ void __launch_bounds__(NT, ST <= 2 ? 2 : 1)
     k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
            int kblocks, Epi epi, int32_t *status) {
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(NT, ST <= 2 ? 2 : 1)
   unsigned char *sA = base;
   unsigned char *sB = base + ST * A_BYTES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  const int m0 = (NF ? blockIdx.y : blockIdx.x) * BM, n0 = (NF ? blockIdx.x : blockIdx.y) * BN;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < ST; ++s) {
@@ -231,21 +233,39 @@ struct EpiStoreF32 {
 
 // wdot[col * ld + row] += acc * 2^escale[row]: the contraction's epilogue
 // (column-major FP64 output: consecutive lanes write consecutive states).
+// With one CTA per SM the loop of a tile and this epilogue took turns, and
+// with the row blocks side by side A was read once per column block: 65,536
+// states of 561/2539 (K = 5120, three column blocks) 1.33 ms; two CTAs per
+// SM, eight warps each, column blocks side by side: 0.53 ms.
 struct EpiWdot {
   double *out;
   int64_t ld;
   int m_valid, n_valid;
   const int *escale;
+  // x * 2^E in FP64 (E within +-1100, x zero or normal)
+  __device__ __forceinline__ static double scaled(uint32_t x, int E) {
+    const unsigned e = (x >> 23) & 0xffu;
+    const int d = (int)e + 896 + E;
+    if (e == 0 || e == 0xffu || d <= 0 || d >= 2047)  // exact all the same, or inf, NaN
+      return (double)__uint_as_float(x) * __hiloint2double((E + 1023) << 20, 0);
+    return __hiloint2double((int)((x & 0x80000000u) | ((unsigned)d << 20) | ((x & 0x7fffffu) >> 3)),
+                            (int)(x << 29));
+  }
   __device__ void operator()(int row, int col0, const uint32_t (&v)[32]) const {
     if (row >= m_valid) return;
-    const double sc = __hiloint2double((escale[row] + 1023) << 20, 0);
+    const int E = escale[row];
+    double *o = out + (int64_t)col0 * ld + row;
+    // the loads of a group ahead of its stores; the scaled term is formed by
+    // integer operations, exactly, so that FP64 only adds
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int col = col0 + j;
-      if (col < n_valid) {
-        double *o = out + (int64_t)col * ld + row;
-        *o = fma((double)__uint_as_float(v[j]), sc, *o);
-      }
+    for (int j = 0; j < 32; j += 8) {
+      double w[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        w[u] = col0 + j + u < n_valid ? o[(int64_t)(j + u) * ld] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (col0 + j + u < n_valid) o[(int64_t)(j + u) * ld] = w[u] + scaled(v[j + u], E);
     }
   }
 };
@@ -257,7 +277,7 @@ struct EpiWdot {
 bool make_tmap_bf16(CUtensorMap *map, const void *ptr, int64_t rows, int64_t cols,
                     int box_rows);
 
-template <int BN, class Epi, int ST = gemm::STAGES, int NT = 128>
+template <int BN, class Epi, int ST = gemm::STAGES, int NT = 128, bool NF = false>
 cudaError_t launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, int64_t M_pad,
                         int64_t N_pad, int64_t K, const Epi &epi, int32_t *status,
                         cudaStream_t s, int splits = 1) {
@@ -265,11 +285,12 @@ cudaError_t launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, int64_t M_
   if (M_pad % gemm::BM || N_pad % BN || K % gemm::BK || K <= 0 || splits < 1 ||
       (K / gemm::BK) % splits)
     return cudaErrorInvalidValue;
-  auto k = gemm::k_gemm<BN, Epi, ST, NT>;
+  auto k = gemm::k_gemm<BN, Epi, ST, NT, NF>;
   const size_t smem = gemm::smem_bytes<BN, ST>();
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  dim3 grid((unsigned)(M_pad / gemm::BM), (unsigned)(N_pad / BN), (unsigned)splits);
+  const unsigned gm = (unsigned)(M_pad / gemm::BM), gn = (unsigned)(N_pad / BN);
+  dim3 grid(NF ? gn : gm, NF ? gm : gn, (unsigned)splits);
   k<<<grid, NT, smem, s>>>(ta, tb, (int)(K / gemm::BK / splits), epi, status);
   return cudaGetLastError();
 }

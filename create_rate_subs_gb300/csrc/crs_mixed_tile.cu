@@ -25,6 +25,7 @@
 // Measured on GB300 (before: one state per thread, large mechanisms in two
 // passes): 2^22 states of 53/325 35.6 -> 21.0 ms, 65,536 of 561/2539 5.32 ->
 // 3.17 ms.
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,6 +35,7 @@
 #include "crs_fx_tile.cuh"
 #include "crs_internal.cuh"
 #include "crs_mixed.cuh"
+#include "crs_tile.cuh"
 
 namespace crs {
 namespace mixt {
@@ -46,7 +48,38 @@ struct Args {
   const unsigned char *img;  // table image
   double *q;                 // [gridDim.x / CL][R + 1][32] scratch when QS is false
   int list;                  // the work list for NW CL warps
+  // contraction (PACK): bf16 rows [i][2 Kh] and the states' scale exponents
+  __nv_bfloat16 *A;
+  int Kh;
+  int *escale;
 };
+
+constexpr int WINDOW = 100;  // binary orders around the scale carried by bf16 hi + lo
+
+__device__ __forceinline__ bool in_window(double v, int c) {
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  const int e = (hi >> 20) & 0x7ff;
+  const bool zero = ((hi & 0x7fffffff) | lo) == 0;
+  return zero || (e != 0 && e != 0x7ff && abs(e - 1023 - c) <= WINDOW);
+}
+
+// Sum and count of the binary exponents of the rates that a lane has formed.
+struct Scale {
+  int sum = 0, count = 0;
+  __device__ __forceinline__ void add(double v) {
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+    const bool c = e != 0x7ff && ((hi & 0x7fffffff) | __double2loint(v)) != 0;
+    sum += c ? e - 1023 : 0;
+    count += c;
+  }
+};
+
+// 32 bytes to a 32-byte aligned address: a whole sector per lane
+__device__ __forceinline__ void store32(void *p, const unsigned (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]),
+               "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 
 constexpr int D = 3;  // slots of a warp's ring of pairs of records
 
@@ -154,7 +187,7 @@ constexpr long long LATER = 0x7ff8c5a1d3b70e29ll;
 __device__ __noinline__ void finish(const unsigned char *img, const ImgLayout &lay,
                                     const unsigned char *src, int npairs, int n, const Batch &b,
                                     int64_t i, Conc C, const unsigned char *o, int lane,
-                                    unsigned char *q) {
+                                    unsigned char *q, Scale *scale) {
   const Tab t = make_tab(img, lay);
   const float *w = reinterpret_cast<const float *>(o + 512) + lane;
   State s;
@@ -189,6 +222,7 @@ __device__ __noinline__ void finish(const unsigned char *img, const ImgLayout &l
       *v = __longlong_as_double(0x7ff8000000000000ll);
     else
       *v = rxn_net<false>(t, r, s, w[192], C, kc, fwd, rev, pm);
+    if (scale) scale->add(*v);
   }
 }
 
@@ -215,10 +249,13 @@ struct Rate {
     m = fmaf(p, r, 1.0f);
     err = 0.0f;
   }
+  // FUSE: the last product may fuse with the addition of the errors, as in
+  // the shape groups' code; else it is rounded by itself, as in product()
+  template <bool FUSE>
   __device__ __forceinline__ void times(const Conc &C, unsigned off) {
     const int2 c = C.at(off);
     const float f = __int_as_float(c.x);
-    const float mm = m * f;
+    const float mm = FUSE ? m * f : __fmul_rn(m, f);
     err = fmaf(err, f, fmaf(m, f, -mm));
     m = mm;
     E += c.y;
@@ -252,17 +289,21 @@ __device__ __forceinline__ float expf_of(ff x) {
 }
 
 // The fall-off factor of the record at r for a third-body concentration thd:
-// mixed::pres_mod's operations, the exponent of k0 / kinf from one row.
+// mixed::pres_mod's operations without its calls and branches.
 __device__ __forceinline__ float falloff(const unsigned char *r, int flags, float thd, ff T,
                                          ff lT, ff iT) {
-  const float4 a = *reinterpret_cast<const float4 *>(r + MFALL);
-  const float4 c = *reinterpret_cast<const float4 *>(r + MFALL + 16);
-  ff z = ff_fma(ff{a.z, a.w}, lT, ff{a.x, a.y});
-  z = ff_fma(ff{c.x, c.y}, iT, z);
-  z = ff_norm(z.h, z.l);
+  // ln k0 - ln kinf; every rounding as in the general code
+  auto row = [&](int o, float &sign) {
+    const float4 a = *reinterpret_cast<const float4 *>(r + o);
+    const float4 c = *reinterpret_cast<const float4 *>(r + o + 16);
+    sign = c.z;
+    return ff_add(ff_add(ff{a.x, a.y}, ff_mul(ff{a.z, a.w}, lT)), ff_mul(ff{c.x, c.y}, iT));
+  };
+  float sign, none;
+  const ff x0 = row(MFALL, sign), z = ff_add(x0, ff_neg(row(MFALL + 32, none)));
   int E, et, e2;
   float m = ff_exp(z, E);
-  m = fsplit(m * fsplit(thd * c.z, et), e2);
+  m = fsplit(m * fsplit(thd * sign, et), e2);
   E += et + e2;
   // Pr/(1+Pr) and 1/(1+Pr) from whichever of Pr and 1/Pr is at most 1
   const bool less = E < 0;
@@ -288,7 +329,9 @@ __device__ __forceinline__ float falloff(const unsigned char *r, int flags, floa
   float ln, F;
   ff w;
   if (flags & PMF_TROE) {
-    float f = g.x * expf_of(ff_mul(T, ff{g.y, g.z})) + g.w * expf_of(ff_mul(T, ff{h.x, h.y}));
+    // (the fused product is the one that the general code's compilation fuses)
+    float f = fmaf(g.w, expf_of(ff_mul(T, ff{h.x, h.y})),
+                   __fmul_rn(g.x, expf_of(ff_mul(T, ff{g.y, g.z}))));
     if (flags & PMF_T2) f += expf_of(ff_mul(iT, ff{h.z, h.w}));
     ln = logf(fmaxf(f, 1.0e-37f));
     const ff lF = ff_mul(ff{ln, 0.0f}, ff{INV_LN10_F, INV_LN10_LO_F});
@@ -311,8 +354,13 @@ __device__ __forceinline__ float falloff(const unsigned char *r, int flags, floa
   return F * side;
 }
 
-// NW warps per CTA, CL CTAs (a cluster) per tile.
-template <int NW, int PER_SM, int CL, bool QS>
+// NW warps per CTA, CL CTAs (a cluster) per tile.  PACK: in place of the
+// species sums, the contraction's operand -- each rate, scaled by the state's
+// mean binary exponent, as bf16 hi and lo parts -- and the sums of the terms
+// outside its window.  The operand is formed from the tile's rates while they
+// are in L2.  Per 65,536 states of 561/2539: 3.04 ms; as kernels of their own
+// with the rates through HBM, rates 3.92, operand 0.54, sums 0.83 ms.
+template <int NW, int PER_SM, int CL, bool QS, bool PACK = false>
 __global__ void __launch_bounds__(NW * 32, PER_SM)
     k_wdot_tile(const __grid_constant__ ImgLayout lay, const __grid_constant__ FxTab f,
                 const __grid_constant__ Args g, const __grid_constant__ Batch b) {
@@ -328,6 +376,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   next += 2 * BLOCK;
   unsigned char *ring = next + warp * (D * MPAIR);
   next += NW * (D * MPAIR);
+  // (PACK) the warps' exponent sums, a bit per reaction with terms outside
+  Scale *scales = reinterpret_cast<Scale *>(next) + threadIdx.x;
+  unsigned *outside = reinterpret_cast<unsigned *>(next + NW * 32 * sizeof(Scale));
   unsigned char *qt = QS && CL > 1 ? static_cast<unsigned char *>(__cluster_map_shared_rank(next, 0))
                       : QS ? next : reinterpret_cast<unsigned char *>(g.q) +
                                       (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256;
@@ -360,6 +411,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     tile_barrier<CL>();
 #pragma unroll
     for (int p = 0; p < D - 1; ++p) recs.fill(p, p);
+    if (PACK)
+      for (int k = threadIdx.x; k <= f.R / 32; k += NW * 32) outside[k] = 0;
     const unsigned char *o = blk + bk * BLOCK;
     const double rho = reinterpret_cast<const double *>(o)[lane];
 #pragma unroll 4
@@ -403,6 +456,11 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       };
       int slot = 0;
       bool later = false;
+      Scale scale;
+      auto put = [&](int off, double v) {
+        Q(off) = v;
+        if (PACK) scale.add(v);
+      };
 #pragma unroll 1
       for (int p = 0; p < npairs; ++p) {
         recs.next(p, slot);
@@ -412,25 +470,25 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         const int4 h1 = *reinterpret_cast<const int4 *>(at + MREC);
         const bool more = h0.x & MF_MORE;
         Rate f0(forward(at)), f1(forward(at + MREC));
-        f0.times(C, row_lo(h0.y));
-        f1.times(C, row_lo(h1.y));
-        f0.times(C, row_hi(h0.y));
-        f1.times(C, row_hi(h1.y));
+        f0.times<true>(C, row_lo(h0.y));
+        f1.times<true>(C, row_lo(h1.y));
+        f0.times<true>(C, row_hi(h0.y));
+        f1.times<true>(C, row_hi(h1.y));
         if (more) {
-          f0.times(C, row_lo(h0.z));
-          f1.times(C, row_lo(h1.z));
+          f0.times<true>(C, row_lo(h0.z));
+          f1.times<true>(C, row_lo(h1.z));
         }
         bool far = f0.far() || f1.far();
         double v0 = f0.value(), v1 = f1.value();
         if (h0.x & MF_REV) {
           Rate r0(reverse(at)), r1(reverse(at + MREC));
-          r0.times(C, row_hi(h0.z));
-          r1.times(C, row_hi(h1.z));
-          r0.times(C, row_lo(h0.w));
-          r1.times(C, row_lo(h1.w));
+          r0.times<true>(C, row_hi(h0.z));
+          r1.times<true>(C, row_hi(h1.z));
+          r0.times<true>(C, row_lo(h0.w));
+          r1.times<true>(C, row_lo(h1.w));
           if (more) {
-            r0.times(C, row_hi(h0.w));
-            r1.times(C, row_hi(h1.w));
+            r0.times<true>(C, row_hi(h0.w));
+            r1.times<true>(C, row_hi(h1.w));
           }
           far |= r0.far() || r1.far();
           v0 -= r0.value();  // FP64
@@ -438,8 +496,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         }
         if (far) v0 = v1 = __longlong_as_double(LATER);
         later |= far;
-        Q(h0.x & ~255) = v0;
-        Q(h1.x) = v1;
+        put(h0.x & ~255, v0);
+        put(h1.x, v1);
       }
 #pragma unroll 1
       for (int p = npairs; p < recs.n; ++p) {
@@ -470,12 +528,12 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
           }
           const float sg = *reinterpret_cast<const float *>(at + 40);
           Rate f(forward(at)), r(reverse(at));
-          f.times(C, row_lo(h.y));
-          r.times(C, row_hi(h.z));
-          f.times(C, row_hi(h.y));
-          r.times(C, row_lo(h.w));
-          f.times(C, row_lo(h.z));
-          r.times(C, row_hi(h.w));
+          f.times<false>(C, row_lo(h.y));
+          r.times<false>(C, row_hi(h.z));
+          f.times<false>(C, row_hi(h.y));
+          r.times<false>(C, row_lo(h.w));
+          f.times<false>(C, row_lo(h.z));
+          r.times<false>(C, row_hi(h.w));
           v = f.value(sg);
           far = f.far();
           if (h.x & MF_REV) {
@@ -486,9 +544,76 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         }
         if (far) v = __longlong_as_double(LATER);
         later |= far;
-        Q(h.x & ~255) = v;
+        put(h.x & ~255, v);
       }
-      if (later) finish(g.img, lay, recs.src, npairs, recs.n, b, ic, C, o, lane, q);
+      if (PACK) *scales = scale;
+      if (later)
+        finish(g.img, lay, recs.src, npairs, recs.n, b, ic, C, o, lane, q,
+               PACK ? scales : nullptr);
+    }
+    if constexpr (PACK) {
+      __syncthreads();
+      int es = 0, ec = 0;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const Scale a = scales[(w - warp) * 32];
+        es += a.sum;
+        ec += a.count;
+      }
+      const int c = tile::scale_exponent(es, ec);
+      if (warp == 0 && valid) g.escale[i] = c;
+      __nv_bfloat16 *row = g.A + i * (2 * (int64_t)g.Kh);
+#pragma unroll 1
+      for (int r0 = warp * 16; r0 < g.Kh; r0 += NW * 16) {
+        unsigned hi[8], lo[8];
+#pragma unroll
+        for (int u = 0; u < 16; u += 2) {
+          float x[2];
+#pragma unroll
+          for (int w = 0; w < 2; ++w) {
+            const int r = r0 + u + w;
+            const double v = r < f.R ? Q(r * 256) : 0.0;
+            const bool in = in_window(v, c);
+            if (__any_sync(0xffffffffu, valid && !in) && lane == 0)
+              atomicOr(&outside[r >> 5], 1u << (r & 31));
+            // v * 2^-c exactly through the exponent field (the result stays a
+            // normal number within 2^+-WINDOW), then rounded to fp32
+            x[w] = in && v != 0.0 ? d2f_rn(__hiloint2double(__double2hiint(v) - c * (1 << 20),
+                                                            __double2loint(v)))
+                                  : 0.0f;
+          }
+          const __nv_bfloat162 h = __floats2bfloat162_rn(x[0], x[1]);
+          const __nv_bfloat162 l = __floats2bfloat162_rn(x[0] - __low2float(h),
+                                                         x[1] - __high2float(h));
+          hi[u / 2] = *reinterpret_cast<const unsigned *>(&h);
+          lo[u / 2] = *reinterpret_cast<const unsigned *>(&l);
+        }
+        if (valid) {
+          store32(row + r0, hi);
+          store32(row + g.Kh + r0, lo);
+        }
+      }
+      __syncthreads();
+      // terms outside the window in FP64, in reaction order per species; 32
+      // terms are looked up at a time
+#pragma unroll 1
+      for (int k = warp; k < N; k += NW) {
+        double w = 0.0;
+        const int e1 = __ldg(t.spc_ptr + k + 1);
+#pragma unroll 1
+        for (int e = __ldg(t.spc_ptr + k); e < e1; e += 32) {
+          const int r = e + lane < e1 ? __ldg(t.spc_r + e + lane) : -1;
+          unsigned some =
+              __ballot_sync(0xffffffffu, r >= 0 && (outside[r >> 5] >> (r & 31) & 1u));
+          for (; some; some &= some - 1) {
+            const int j = __ffs(some) - 1;
+            const double v = Q(__shfl_sync(0xffffffffu, r, j) * 256);
+            if (!in_window(v, c)) w = fma(__ldg(t.spc_nu + e + j), v, w);
+          }
+        }
+        if (valid) b.wdot[(int64_t)k * b.ld + i] = w;
+      }
+      continue;  // rates and bits are replaced after the barrier at the loop's head
     }
     sums.ahead(f, tab);
     tile_barrier<CL>();
@@ -500,8 +625,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   if (bad && b.status) atomicAdd(&b.status[1], bad);
 }
 
-size_t smem_of(const FxTab &f, int nw, bool qs) {
-  return (size_t)(f.N + 2) * 256 + 2 * BLOCK + (size_t)nw * D * MPAIR +
+size_t smem_of(const FxTab &f, int nw, bool qs, bool pack = false) {
+  return (pack ? (size_t)nw * 32 * sizeof(Scale) + (f.R / 32 + 1) * 4 : 0) +
+         (size_t)(f.N + 2) * 256 + 2 * BLOCK + (size_t)nw * D * MPAIR +
          (qs ? (size_t)(f.R + 1) * 256 : 0);
 }
 
@@ -541,10 +667,15 @@ Kernel kernel_of(const Plan &p) {
   return k_wdot_tile<24, 1, 1, false>;
 }
 
+// the contraction's producer: one CTA of 24 warps per SM
+constexpr int PACK_NW = 24;
+constexpr Kernel k_pack = k_wdot_tile<PACK_NW, 1, 1, false, true>;
+
 }  // namespace mixt
 
 cudaError_t mixed_tile_init(int smem_optin) {
   cudaError_t e = cudaSuccess;
+  e = set_smem_limit(mixt::k_pack, (size_t)smem_optin);
   for (int q = 0; q < 7 && e == cudaSuccess; ++q) {
     mixt::Plan p;
     p.cl = q < 3 ? 2 << q : 1;
@@ -603,7 +734,7 @@ static cudaError_t launch_mixed_part(const unsigned char *img, const ImgLayout &
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = p.cl > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k, L, f, mixt::Args{tab, img, scratch, list}, b);
+  return cudaLaunchKernelEx(&cfg, k, L, f, mixt::Args{tab, img, scratch, list, nullptr, 0, nullptr}, b);
 }
 
 cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
@@ -621,6 +752,28 @@ cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, cons
   part.Y += o;
   part.wdot += o;
   return launch_mixed_part(img, L, f, tab, part, sm_count, smem_optin, scratch, s);
+}
+
+// Scratch bytes of the contraction's producer over n states; < 0: the
+// mechanism does not fit.
+long long mixed_pack_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
+  if (!f.mixed || mixt::smem_of(f, mixt::PACK_NW, false, true) > (size_t)smem_optin) return -1;
+  return (long long)std::min<int64_t>((n + 31) / 32, sm_count) * (f.R + 1) * 256;
+}
+
+// A: rows of 2 Kh (a multiple of 64), 32-byte aligned.
+cudaError_t launch_mixed_pack(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
+                              const unsigned char *tab, const Batch &b, int sm_count,
+                              int smem_optin, double *scratch, void *A, int Kh, int *escale,
+                              cudaStream_t s) {
+  if (mixed_pack_scratch(f, b.n, sm_count, smem_optin) < 0 || Kh % 64 || Kh < f.R)
+    return cudaErrorInvalidValue;
+  int list = 0;
+  while (list < fx::NLIST - 1 && fx::list_warps[list] != mixt::PACK_NW) ++list;
+  mixt::k_pack<<<(unsigned)std::min<int64_t>((b.n + 31) / 32, sm_count), mixt::PACK_NW * 32,
+                 mixt::smem_of(f, mixt::PACK_NW, false, true), s>>>(
+      L, f, mixt::Args{tab, img, scratch, list, static_cast<__nv_bfloat16 *>(A), Kh, escale}, b);
+  return cudaGetLastError();
 }
 
 }  // namespace crs
