@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "crs_exp.cuh"
 #include "crs_internal.cuh"
 
 namespace crs {
@@ -142,19 +143,55 @@ __global__ void k_conc(const unsigned char *__restrict__ img, ImgLayout L,
 // chip idle below ~10^5 states, and the FP64 pipe waiting on its one chain.
 // 20,000 states of 53/325, all four functions: 3.4 ms without the split.
 
+// Exponentials and divisions by T of the two kernels of reactions, whose
+// bound they are: the table exponential (error below 1 ulp, 9 FP64
+// instructions), and a / T from T's correctly rounded reciprocal by two
+// fused multiply-adds (Markstein, IBM J. Res. Dev. 34 (1990): the correctly
+// rounded quotient), three instead of a division's ten.  Outside the range
+// where the latter holds the division stands.
+struct FastMath {
+  const double *tab;
+  double y;  // 1 / T
+  bool in;
+  __device__ __forceinline__ FastMath(const double *tab, double T)
+      : tab(tab), y(1.0 / T), in(T >= 1.0 && T <= 0x1p100) {}
+  __device__ __forceinline__ double exp_of(double x) const { return texp::exp_t(x, tab); }
+  // 10^x = e^(x ln 10), the product's rounding error carried
+  __device__ __forceinline__ double pow10(double x) const {
+    constexpr double LN10 = 0x1.26bb1bbb55516p+1, LN10_LO = -0x1.f48ad494ea3e9p-53;
+    const double t = x * LN10, e = fma(x, LN10_LO, fma(x, LN10, -t));
+    if (!(fabs(t) < 600.0)) return pow(10.0, x);
+    const double v = texp::exp_core(t, tab);
+    return fma(v, e, v);
+  }
+  __device__ __forceinline__ double over_T(double a, double T) const {
+    const double q = a * y;
+    return in ? fma(fma(-T, q, a), y, q) : a / T;
+  }
+};
+
+// The exponential's table in shared memory (all threads).
+__device__ __forceinline__ void stage_exp(double *s, const Tab &t) {
+  for (int k = threadIdx.x; k < 256; k += blockDim.x) s[k] = t.exptab[k];
+  __syncthreads();
+}
+
 // b.conc holds C (input).
 __global__ void __launch_bounds__(128)
     k_rxn_rates(const unsigned char *__restrict__ img, ImgLayout L, Batch b, int per) {
+  __shared__ double tab[256];
   const Tab t = make_tab(img, L);
+  stage_exp(tab, t);
   const int r0 = blockIdx.y * per, r1 = min(t.R, r0 + per);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b.n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double T = b.T[i], P = b.P[i];
     Col C{b.conc + i, b.ld};
     const double logT = log(T);
+    const FastMath m(tab, T);
     for (int r = r0; r < r1; ++r) {
       double fwd, rev;
-      rxn_rates(t, r, T, logT, P, C, fwd, rev);
+      rxn_rates(t, r, T, logT, P, C, fwd, rev, m);
       b.fwd[(int64_t)r * b.ld + i] = fwd;
       const int j = t.rev_idx[r];
       if (j >= 0 && b.rev) b.rev[(int64_t)j * b.ld + i] = rev;
@@ -164,7 +201,9 @@ __global__ void __launch_bounds__(128)
 
 __global__ void __launch_bounds__(128)
     k_pres_mod(const unsigned char *__restrict__ img, ImgLayout L, Batch b, int per) {
+  __shared__ double tab[256];
   const Tab t = make_tab(img, L);
+  stage_exp(tab, t);
   const int p0 = blockIdx.y * per, p1 = min(t.NPM, p0 + per);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b.n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -172,8 +211,9 @@ __global__ void __launch_bounds__(128)
     Col C{b.conc + i, b.ld};
     const double logT = log(T);
     const double mix = P / (8.31446210e+03 * T);
+    const FastMath m(tab, T);
     for (int p = p0; p < p1; ++p)
-      b.pm[(int64_t)p * b.ld + i] = pres_mod(t, p, T, logT, mix, C);
+      b.pm[(int64_t)p * b.ld + i] = pres_mod(t, p, T, logT, mix, C, m);
   }
 }
 

@@ -40,18 +40,27 @@ struct Strided {
   CRS_HD V &operator[](int k) const { return p[(int64_t)k * stride]; }
 };
 
+// The exponentials and divisions of the functions below: as emitted.  (A
+// kernel may pass its own of the same accuracy.)
+struct Math {
+  CRS_HD double exp_of(double x) const { return exp(x); }
+  CRS_HD double pow10(double x) const { return pow(10.0, x); }
+  CRS_HD double over_T(double a, double T) const { return a / T; }
+};
+
 // rxn_rate_const (rate_subs.py:60-135): A > 0 as exp(logA + b ln T - Ta/T),
 // A < 0 as A exp(b ln T - Ta/T), integer b with zero Ta as repeated
 // multiplication, a constant.
-CRS_HD inline double rate_const(const Tab &t, int row, double T, double logT) {
+template <class M = Math>
+CRS_HD inline double rate_const(const Tab &t, int row, double T, double logT, const M &m = M()) {
   const double *p = t.rate_par + 4 * row;  // A, logA, b, Ta
   switch (t.rate_kind[row]) {
     case RATE_CONST:
       return p[0];
     case RATE_EXP:
-      return exp(p[1] + p[2] * logT - (p[3] / T));
+      return m.exp_of(p[1] + p[2] * logT - m.over_T(p[3], T));
     case RATE_NEGEXP:
-      return p[0] * exp(p[2] * logT - (p[3] / T));
+      return p[0] * m.exp_of(p[2] * logT - m.over_T(p[3], T));
     default: {
       double k = p[0];
       for (int j = 0; j < t.rate_npow[row]; ++j) k = k * T;
@@ -143,13 +152,15 @@ CRS_HD inline double conc_product(const int32_t *sp, const int32_t *nint, const 
 
 // Exponent of the equilibrium constant of reversible reaction j, summed
 // over its T_common groups (rate_subs.py:592-655).
-CRS_HD inline double kc_exponent(const Tab &t, int j, double T, double logT) {
+template <class M = Math>
+CRS_HD inline double kc_exponent(const Tab &t, int j, double T, double logT, const M &m = M()) {
   double kc = 0.0;
   const int g0 = t.kc_ptr[j], g1 = t.kc_ptr[j + 1];
   for (int g = g0; g < g1; ++g) {
     const double *c = (T <= t.kc_tmid[g]) ? t.kc_lo + 7 * g : t.kc_hi + 7 * g;
     const double v =
-        (c[0] + c[1] * logT + T * (c[2] + T * (c[3] + T * (c[4] + c[5] * T))) - c[6] / T);
+        (c[0] + c[1] * logT + T * (c[2] + T * (c[3] + T * (c[4] + c[5] * T))) -
+         m.over_T(c[6], T));
     kc = (g == g0) ? v : kc + v;
   }
   return kc;
@@ -158,23 +169,23 @@ CRS_HD inline double kc_exponent(const Tab &t, int j, double T, double logT) {
 // fwd (and rev when reversible) of reaction r (rate_subs.py:433-693).
 // PLOG / Chebyshev rows print kf first and use it like a reversible
 // reaction's kf (rate_subs.py:437-448, 503-505).
-template <class CS>
+template <class CS, class M = Math>
 CRS_HD inline void rxn_rates(const Tab &t, int r, double T, double logT, double pres,
-                             const CS &C, double &fwd, double &rev) {
+                             const CS &C, double &fwd, double &rev, const M &m = M()) {
   bool have;
   const double p =
       conc_product(t.rx_sp, t.rx_nint, t.rx_nu, t.rx_ptr[r], t.rx_ptr[r + 1], C, have);
   const int j = t.rev_idx[r];
   const bool pdep = t.rate_kind[r] >= RATE_PLOG;
   if (j >= 0 || pdep) {
-    const double kf = pdep ? pdep_kf(t, r, T, logT, pres) : rate_const(t, r, T, logT);
+    const double kf = pdep ? pdep_kf(t, r, T, logT, pres) : rate_const(t, r, T, logT, m);
     fwd = have ? p * kf : kf;
     if (j < 0) {
       rev = 0.0;
       return;
     }
-    double Kc = kc_exponent(t, j, T, logT);
-    Kc = t.kc_pref[j] * exp(Kc);
+    double Kc = kc_exponent(t, j, T, logT, m);
+    Kc = t.kc_pref[j] * m.exp_of(Kc);
     bool hq;
     const double q =
         conc_product(t.px_sp, t.px_nint, t.px_nu, t.px_ptr[r], t.px_ptr[r + 1], C, hq);
@@ -182,7 +193,7 @@ CRS_HD inline void rxn_rates(const Tab &t, int r, double T, double logT, double 
   } else {
     rev = 0.0;
     if (!have) {
-      fwd = rate_const(t, r, T, logT);
+      fwd = rate_const(t, r, T, logT, m);
       return;
     }
     // irreversible: the rate expression is printed inline after the
@@ -190,8 +201,8 @@ CRS_HD inline void rxn_rates(const Tab &t, int r, double T, double logT, double 
     const double *a = t.rate_par + 4 * r;
     switch (t.rate_kind[r]) {
       case RATE_CONST: fwd = p * a[0]; break;
-      case RATE_EXP: fwd = p * exp(a[1] + a[2] * logT - (a[3] / T)); break;
-      case RATE_NEGEXP: fwd = p * a[0] * exp(a[2] * logT - (a[3] / T)); break;
+      case RATE_EXP: fwd = p * m.exp_of(a[1] + a[2] * logT - m.over_T(a[3], T)); break;
+      case RATE_NEGEXP: fwd = p * a[0] * m.exp_of(a[2] * logT - m.over_T(a[3], T)); break;
       default: {
         double v = p * a[0];
         for (int q = 0; q < t.rate_npow[r]; ++q) v = v * T;
@@ -213,31 +224,31 @@ CRS_HD inline double third_body(const Tab &t, int p, double mix, const CS &C) {
 
 // pres_mod entry p (rate_subs.py:881-1064): third body, or the Lindemann /
 // Troe / SRI fall-off factor with LOW or HIGH.
-template <class CS>
+template <class CS, class M = Math>
 CRS_HD inline double pres_mod(const Tab &t, int p, double T, double logT, double mix,
-                              const CS &C) {
+                              const CS &C, const M &m = M()) {
   if (t.pm_kind[p] == PM_THD) return third_body(t, p, mix, C);
   const int sp = t.pm_sp[p];
   const double thd = (sp < 0) ? third_body(t, p, mix, C) : 0.0;
-  const double k0 = rate_const(t, t.pm_k0[p], T, logT);
-  const double kinf = rate_const(t, t.pm_kinf[p], T, logT);
+  const double k0 = rate_const(t, t.pm_k0[p], T, logT, m);
+  const double kinf = rate_const(t, t.pm_kinf[p], T, logT, m);
   const double Pr = (sp >= 0) ? k0 * C[sp] / kinf : k0 * thd / kinf;
   const bool low = t.pm_kind[p] == PM_FALL_LOW;
   const int form = t.pm_form[p];
   if (form == FORM_TROE) {
     const double *c = t.pm_troe + 5 * p;
-    double s = c[0] * exp(-T / c[1]) + c[2] * exp(-T / c[3]);
-    if (t.pm_troe_t2[p]) s = s + exp(-c[4] / T);
+    double s = c[0] * m.exp_of(-T / c[1]) + c[2] * m.exp_of(-T / c[3]);
+    if (t.pm_troe_t2[p]) s = s + m.exp_of(m.over_T(-c[4], T));
     const double logFcent = log10(fmax(s, 1.0e-300));
     const double A = log10(fmax(Pr, 1.0e-300)) - 0.67 * logFcent - 0.4;
     const double B = 0.806 - 1.1762 * logFcent - 0.14 * log10(fmax(Pr, 1.0e-300));
-    const double F = pow(10.0, logFcent / (1.0 + A * A / (B * B)));
+    const double F = m.pow10(logFcent / (1.0 + A * A / (B * B)));
     return low ? F * Pr / (1.0 + Pr) : F / (1.0 + Pr);
   }
   if (form == FORM_SRI) {
     const double *c = t.pm_sri + 5 * p;
     const double X = 1.0 / (1.0 + log10(fmax(Pr, 1.0e-300)) * log10(fmax(Pr, 1.0e-300)));
-    double F = pow(c[0] * exp(-c[1] / T) + exp(-T / c[2]), X);
+    double F = pow(c[0] * m.exp_of(m.over_T(-c[1], T)) + m.exp_of(-T / c[2]), X);
     if (t.pm_sri_de[p]) F = F * c[3] * pow(T, c[4]);
     return low ? F * Pr / (1.0 + Pr) : F / (1.0 + Pr);
   }
