@@ -47,7 +47,6 @@
 #include "crs_fast.cuh"
 #include "crs_fx.cuh"
 #include "crs_fx_tab.cuh"
-#include "crs_fx_tile.cuh"
 #include "crs_internal.cuh"
 #include "crs_tile.cuh"
 
@@ -206,6 +205,37 @@ struct Rec {
   }
 };
 
+// Copies of a warp's next records into its ring of D slots.
+template <int D>
+struct Ring {
+  const unsigned char *src;
+  unsigned base;
+  int stride, n, lane;
+  // record p (an empty group past the last one)
+  __device__ __forceinline__ void fill(int p) const {
+    if (p < n) {
+      const unsigned char *from = src + (int64_t)p * stride;
+      const unsigned to = base + (unsigned)((p % D) * stride);
+#pragma unroll 1
+      for (int o = lane * 16; o < stride; o += 512)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + o), "l"(from + o)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  __device__ __forceinline__ void start() const {
+#pragma unroll
+    for (int p = 0; p < D - 1; ++p) fill(p);
+  }
+  // Record p is on chip for the whole warp; the copy of record p + D - 1
+  // starts (its slot's reader, record p - 1, is done).
+  __device__ __forceinline__ void next(int p) const {
+    __syncwarp();
+    fill(p + D - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+    __syncwarp();
+  }
+};
 constexpr int DP = 3, DO = 3;  // slots for pairs of plain records and for other records
 
 __host__ __device__ inline int ring_bytes(const FxTab &f) {
@@ -342,6 +372,17 @@ __device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const B
   }
 }
 
+// Barrier of the CTAs that share a tile.
+template <int CL>
+__device__ __forceinline__ void tile_barrier() {
+  if (CL == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
 // NW warps per CTA, CL CTAs (a cluster) per tile: each forms the tile's
 // exponents for itself, evaluates its share of the reactions and, the rates
 // exchanged through the first CTA's shared memory (QS) or scratch, of the
@@ -395,7 +436,10 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     other_ring = Ring<DO>{tab + f.rec[LIST][1] + (int64_t)lo[0] * f.stride[1], smem_u32(ring),
                           f.stride[1], lo[1] - lo[0], lane};
   }
-  Sums sums(f, tab, LIST, gw);
+  const int s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw];
+  const int s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw + 1];
+  const int4 *terms = reinterpret_cast<const int4 *>(tab + f.term[LIST]) +
+                      reinterpret_cast<const int *>(tab + f.term_ptr[LIST])[gw];
   const unsigned yrows = smem_u32(smem) + lane * 8;
   const double *inv_mw = reinterpret_cast<const double *>(g.img + lay.inv_mw);
   int bad = 0, bk = 0;
@@ -421,14 +465,34 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     auto third_body = [&](int p) {
       const int *ep = reinterpret_cast<const int *>(tab + f.eff_ptr) + p;
       double s = rowd(9);
-#pragma unroll 1
-      for (int e = ep[0]; e < ep[1]; ++e) {
+      auto term = [&](int e, double &c) {
         const int4 w = __ldg(reinterpret_cast<const int4 *>(tab + f.eff) + e);
-        double y;
-        if (w.z == (N - 1) * 256) y = rowd(7);
-        else if (QS && CL == 1) y = __longlong_as_double(Yl(w.z));
-        else y = b.Y[(int64_t)(w.z >> 8) * b.ld + ic];
-        s = fma(__hiloint2double(w.y, w.x), y, s);
+        c = __hiloint2double(w.y, w.x);
+        return w.z == (N - 1) * 256 ? rowd(7)
+               : QS && CL == 1      ? __longlong_as_double(Yl(w.z))
+                                    : b.Y[(int64_t)(w.z >> 8) * b.ld + ic];
+      };
+      // the loads of a group of terms ahead of its chain of additions, where
+      // one CTA's latency shows (97 states of 53/325: 22.5 -> 21.6 us, 65,536
+      // of 561/2539: 4.45 -> 4.41 ms); with more CTAs per SM the registers
+      // count (2^20 states of 53/325: 6.41 -> 6.50 ms)
+      int e = __ldg(ep);
+      const int e1 = __ldg(ep + 1);
+      if constexpr (PER_SM == 1) {
+#pragma unroll 1
+        for (; e + 4 <= e1; e += 4) {
+          double c[4], y[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) y[u] = term(e + u, c[u]);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) s = fma(c[u], y[u], s);
+        }
+      }
+#pragma unroll 1
+      for (; e < e1; ++e) {
+        double c;
+        const double y = term(e, c);
+        s = fma(c, y, s);
       }
       return s;
     };
@@ -557,7 +621,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       if (later || all)
         finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
     }
-    sums.ahead(f, tab);
+    // the first terms are on their way before the barrier
+    const int4 t0 = __ldg(terms), t1 = __ldg(terms + 1);
+    const int4 sg0 = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + s0);
     tile_barrier<CL>();
     // the next tile's mass fractions replace exponents that every warp is
     // done with, while the species sums run
@@ -565,7 +631,50 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       const int64_t j = (tile + step) * 32;
       load_y<NW>(b.Y + (j + lane < b.n ? j + lane : j), b.ld, N, warp, yrows);
     }
-    sums.run(f, tab, q, 0u, b.wdot, b.ld, i, valid, bad);
+    {
+      // the groups of the warp's species are one stream: the rates of the
+      // next group are on their way while a group is added
+      auto rates = [&](int4 t, double (&v)[4]) {
+        const int x[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double d = Q(x[u] & 0x7fffffff);
+          v[u] = __hiloint2double(__double2hiint(d) ^ (x[u] & 0x80000000), __double2loint(d));
+        }
+      };
+      const int4 *tm = terms;
+      double v[4];
+      rates(t0, v);
+      int4 t = t1, sgn = sg0;
+#pragma unroll 1
+      for (int a = s0; a < s1; ++a) {
+        const int4 sg = sgn;
+        sgn = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + a + 1);
+        double w = 0.0, w2 = 0.0;
+#pragma unroll 1
+        for (int e = 0; e < sg.y; ++e) {
+          double u[4];
+          rates(t, u);
+          t = __ldg(tm + 2);
+          ++tm;
+          w += v[0];
+          w2 += v[1];
+          w += v[2];
+          w2 += v[3];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[c] = u[c];
+        }
+#pragma unroll 1
+        for (int e = sg.z; e < sg.z + sg.w; ++e)
+          w = fma(__ldg(reinterpret_cast<const double *>(tab + f.wnu) + e),
+                  Q(__ldg(reinterpret_cast<const int *>(tab + f.wterm) + e)), w);
+        w += w2;
+        if (valid) {
+          bad += ((__double2hiint(w) >> 20) & 0x7ff) == 0x7ff;  // inf or NaN, integer test
+          b.wdot[(int64_t)sg.x * b.ld + i] = w;
+        }
+      }
+    }
     // rates are replaced only after the barrier at the loop's head
   }
   if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here

@@ -32,7 +32,6 @@
 
 #include "crs_exp.cuh"
 #include "crs_fx_tab.cuh"
-#include "crs_fx_tile.cuh"
 #include "crs_internal.cuh"
 #include "crs_mixed.cuh"
 #include "crs_tile.cuh"
@@ -83,28 +82,127 @@ __device__ __forceinline__ void store32(void *p, const unsigned (&w)[8]) {
 
 constexpr int D = 3;  // slots of a warp's ring of pairs of records
 
-// Copies of a warp's next records into its ring of D slots (fx::Ring for
-// records of one known size).
-struct Records {
+// (The ring, the barrier and the sums are crs_fx.cu's in other words: there,
+// as functions shared by both kernels, they cost 6.41 -> 6.50 ms for 2^20
+// states of 53/325, the registers falling otherwise.)
+
+// Copies of a warp's next records into its ring of D slots.
+template <int D>
+struct Ring {
   const unsigned char *src;
   unsigned base;
-  int n, lane;
+  int stride, n, lane;
   // record p into slot s (an empty group past the last one)
   __device__ __forceinline__ void fill(int p, int s) const {
-    static_assert(MPAIR % 16 == 0 && MPAIR <= 512, "one 16-byte copy per lane");
-    if (p < n && lane < MPAIR / 16)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + s * MPAIR + lane * 16),
-                   "l"(src + p * MPAIR + lane * 16)
-                   : "memory");
+    if (p < n) {
+      const unsigned char *from = src + (unsigned)(p * stride + lane * 16);
+      const unsigned to = base + (unsigned)(s * stride + lane * 16);
+      if (lane * 16 < stride)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+      if (stride > 512) {
+#pragma unroll 1
+        for (int o = 512; o < stride - lane * 16; o += 512)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + o), "l"(from + o)
+                       : "memory");
+      }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  __device__ __forceinline__ void start() const {
+#pragma unroll
+    for (int p = 0; p < D - 1; ++p) fill(p, p);
+  }
   // Record p, in slot s, is on chip for the whole warp; the copy of record
-  // p + D - 1 starts (its slot's reader, record p - 1, is done).
-  __device__ __forceinline__ void next(int p, int s) const {
+  // p + D - 1 starts (its slot's reader, record p - 1, is done).  Returns the
+  // next record's slot.
+  __device__ __forceinline__ int next(int p, int s) const {
     __syncwarp();
     fill(p + D - 1, s == 0 ? D - 1 : s - 1);
     asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
     __syncwarp();
+    return s == D - 1 ? 0 : s + 1;
+  }
+};
+
+// Barrier of the CTAs that share a tile.
+template <int CL>
+__device__ __forceinline__ void tile_barrier() {
+  if (CL == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+// The species sums of one warp (gw of list `list`) of a tile: each species'
+// terms in FP64, four at a time in two chains.  The groups of the warp's
+// species are one stream: the rates of the next group are on their way while
+// a group is added.
+struct Sums {
+  const int4 *tm;
+  int4 t0, t1, sg0;
+  int s0, s1, list;
+  __device__ __forceinline__ Sums(const FxTab &f, const unsigned char *tab, int list_, int gw)
+      : list(list_) {
+    s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[list])[gw];
+    s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[list])[gw + 1];
+    tm = reinterpret_cast<const int4 *>(tab + f.term[list]) +
+         reinterpret_cast<const int *>(tab + f.term_ptr[list])[gw];
+  }
+  // the first terms, on their way before the barrier
+  __device__ __forceinline__ void ahead(const FxTab &f, const unsigned char *tab) {
+    t0 = __ldg(tm);
+    t1 = __ldg(tm + 1);
+    sg0 = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[list]) + s0);
+  }
+  // q + col: the lane's column of the rates (a q that is the same for the
+  // whole warp spares the scratch's 64-bit additions: 21.8 -> 20.9 ms, 2^22
+  // states of 53/325); the state's sums to wdot if valid
+  __device__ __forceinline__ void run(const FxTab &f, const unsigned char *tab,
+                                      const unsigned char *q, unsigned col, double *wdot, int64_t ld,
+                                      int64_t i, bool valid, int &bad) const {
+    auto Q = [&](unsigned off) { return *reinterpret_cast<const double *>(q + off); };
+    auto rates = [&](int4 t, double (&v)[4]) {
+      const int x[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double d = Q(((unsigned)x[u] & 0x7fffff00u) | col);
+        v[u] = __hiloint2double(__double2hiint(d) ^ (x[u] & 0x80000000), __double2loint(d));
+      }
+    };
+    const int4 *tp = tm;
+    double v[4];
+    rates(t0, v);
+    int4 t = t1, sgn = sg0;
+#pragma unroll 1
+    for (int a = s0; a < s1; ++a) {
+      const int4 s = sgn;
+      sgn = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[list]) + a + 1);
+      double w = 0.0, w2 = 0.0;
+#pragma unroll 1
+      for (int e = 0; e < s.y; ++e) {
+        double u[4];
+        rates(t, u);
+        t = __ldg(tp + 2);
+        ++tp;
+        w += v[0];
+        w2 += v[1];
+        w += v[2];
+        w2 += v[3];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = u[c];
+      }
+#pragma unroll 1
+      for (int e = s.z; e < s.z + s.w; ++e)
+        w = fma(__ldg(reinterpret_cast<const double *>(tab + f.wnu) + e),
+                Q((unsigned)__ldg(reinterpret_cast<const int *>(tab + f.wterm) + e) | col), w);
+      w += w2;
+      if (valid) {
+        bad += ((__double2hiint(w) >> 20) & 0x7ff) == 0x7ff;  // inf or NaN, integer test
+        wdot[(int64_t)s.x * ld + i] = w;
+      }
+    }
   }
 };
 
@@ -393,8 +491,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   }
   const int gw = CL == 1 ? warp : (int)(blockIdx.x % CL) * NW + warp;  // the tile's warp
   const int *lp = reinterpret_cast<const int *>(tab + f.mlist_ptr[g.list]) + gw;
-  const Records recs{tab + f.mrec[g.list] + (int64_t)lp[0] * MPAIR, smem_u32(ring), lp[1] - lp[0],
-                     lane};
+  const Ring<D> recs{tab + f.mrec[g.list] + (int64_t)lp[0] * MPAIR, smem_u32(ring), MPAIR,
+                     lp[1] - lp[0], lane};
   const int npairs = reinterpret_cast<const int *>(tab + f.mpairs[g.list])[gw];
   Sums sums(f, tab, g.list, gw);
   int bad = 0, bk = 0;
@@ -409,8 +507,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     const bool valid = i < b.n;
     const int64_t ic = valid ? i : tile * 32;  // idle lanes repeat a valid state
     tile_barrier<CL>();
-#pragma unroll
-    for (int p = 0; p < D - 1; ++p) recs.fill(p, p);
+    recs.start();
     if (PACK)
       for (int k = threadIdx.x; k <= f.R / 32; k += NW * 32) outside[k] = 0;
     const unsigned char *o = blk + bk * BLOCK;
@@ -463,9 +560,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       };
 #pragma unroll 1
       for (int p = 0; p < npairs; ++p) {
-        recs.next(p, slot);
         const unsigned char *at = ring + slot * MPAIR;
-        slot = slot == D - 1 ? 0 : slot + 1;
+        slot = recs.next(p, slot);
         const int4 h0 = *reinterpret_cast<const int4 *>(at);
         const int4 h1 = *reinterpret_cast<const int4 *>(at + MREC);
         const bool more = h0.x & MF_MORE;
@@ -501,9 +597,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       }
 #pragma unroll 1
       for (int p = npairs; p < recs.n; ++p) {
-        recs.next(p, slot);
         const unsigned char *at = ring + slot * MPAIR;
-        slot = slot == D - 1 ? 0 : slot + 1;
+        slot = recs.next(p, slot);
         const int4 h = *reinterpret_cast<const int4 *>(at);
         bool far = h.x & MF_GEN;
         double v = 0.0;
