@@ -522,7 +522,7 @@ def run_ours(args):
 
     flags, bad = rs.status()
     traffic = _traffic_from_profiles("fp64")
-    roof = _roofline(mech.tables, "fp64", value / world, peaks, N)
+    roof = _roofline(mech.tables, "fixed", value / world, peaks, N)
     roof["traffic"] = traffic * n if traffic is not None else None
     roof["traffic_note"] = ("DRAM bytes per launch: the per-state figure of the ncu capture "
                             "in profiles/ (2^18 states) scaled to this launch's states")
@@ -746,7 +746,7 @@ def _bench_large(args, stream, dist, world, peaks, rank):
     sub = 4096
     steps = max(5, args.steps // 2)
     got = {}
-    precision = {"fp64": "fp64", "mixed": "mixed_tile", "gemm": "rates"}
+    precision = {"fp64": "fixed", "mixed": "mixed", "gemm": "operand"}
     for mode in ("fp64", "mixed", "gemm"):
         ms = _time_steps(lambda: rs.wdot(dT, dP, dY, mode, out=out), steps, 3, stream, dist)
         got[mode] = rs.wdot(dT[:sub], dP[:sub], dY[:, :sub], mode).cpu().numpy()

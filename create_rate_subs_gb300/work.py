@@ -104,8 +104,13 @@ def fp64_slots(tables, precision, exp_slots):
         ``exp_slots``, the measured FP64-pipe cost of the cheapest FP64
         exponential of this library (the table exp: FP64 FMA rate / its
         rate, ~9); logs and powers cost more, so this undercounts.
-    precision "mixed": only what the mixed one-state-per-thread kernel
-        keeps in FP64: one subtraction (forward - reverse) per reversible
+    precision "fixed": what the state tiles of CRS_MODE_FP64 keep in FP64
+        beside 64-bit fixed point: the two sums of the mass fractions, one
+        FMA per third-body efficiency, two multiplies per three-body
+        reaction and one addition per nonzero net stoichiometric
+        coefficient.
+    precision "mixed": only what the mixed state tiles (and the mixed
+        one-state-per-thread kernel) keep in FP64: one subtraction (forward - reverse) per reversible
         reaction, one multiply per reaction with a pres_mod term, one FMA
         per nonzero net stoichiometric coefficient (the wdot accumulation).
         Its equilibrium-constant exponents run as float-float on the FP32
@@ -114,6 +119,8 @@ def fp64_slots(tables, precision, exp_slots):
     precision "mixed_tile": the mixed split of the large-mechanism state
         tile, which keeps the Kc exponents in FP64 (6 FMAs per T_common
         group) beside the same subtraction, multiplies and accumulation.
+    precision "operand": mixed without the accumulation (the rates producer
+        of the tensor-core contraction by state tiles).
     precision "rates": mixed_tile without the accumulation (the rates
         producer of the tensor-core contraction, whose products and sums
         run on the tensor cores).
@@ -129,15 +136,20 @@ def fp64_slots(tables, precision, exp_slots):
         w = work(t)
         parts = {"algebraic": w["flops"] / 2.0,
                  "transcendental": w["transcendentals"] * float(exp_slots)}
-    elif precision in ("mixed", "mixed_tile", "rates"):
+    elif precision == "fixed":
+        thd = sum(1 for k in t["pm_kind"][: int(t["dims"][3])] if int(k) == 0)
+        parts = {"mass_fraction_sums": 2.0 * int(t["dims"][0]),
+                 "third_body": float(len(t["pm_eff_val"])) + 2.0 * thd,
+                 "accumulation": float(nnz)}
+    elif precision in ("mixed", "operand", "mixed_tile", "rates"):
         single = all(int(t["kc_ptr"][j + 1]) - int(t["kc_ptr"][j]) <= 1 for j in range(NREV))
         parts = {"net_rate": float(NREV), "pres_mod_product": float(n_pm)}
-        if precision != "mixed" or not single:
+        if precision in ("mixed_tile", "rates") or not single:
             parts["kc_exponent"] = 6.0 * groups
-        if precision != "rates":
+        if precision not in ("rates", "operand"):
             parts["accumulation"] = float(nnz)
     else:
-        raise ValueError("precision must be fp64, mixed, mixed_tile or rates")
+        raise ValueError("precision must be fp64, fixed, mixed, operand, mixed_tile or rates")
     return {"slots": float(sum(parts.values())), "parts": parts}
 
 

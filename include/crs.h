@@ -48,16 +48,23 @@ typedef struct crs_mech crs_mech;
 #define CRS_ERR_NOMECH 6      /* per-state call without a bound mechanism */
 
 /* Evaluation modes of crs_wdot. */
-#define CRS_MODE_FP64 0        /* FP64 throughout; <=1e-12 of the reference */
+#define CRS_MODE_FP64 0        /* 64-bit fixed-point exponents, FP64 sums; <=1e-12 of the reference */
 #define CRS_MODE_FP64_STRICT 1 /* FP64 in the reference's operation order */
-#define CRS_MODE_MIXED 2       /* FP32 bulk, float-float Kc exponent, FP64 net rate/sum */
-/* The arithmetic of CRS_MODE_FP64 / CRS_MODE_MIXED with a fixed thread
- * layout: one state per thread (TPS) or one state per warp (WARP).  The
- * default modes pick the faster layout that fits the mechanism.
+#define CRS_MODE_MIXED 2       /* FP32 bulk, float-float exponents, FP64 net rate/sum */
+/* CRS_MODE_FP64 and CRS_MODE_MIXED evaluate tiles of 32 states (the warps of
+ * a CTA, or of a cluster when tiles are few, split the reactions).  Net rates
+ * that do not fit on chip take scratch in stream order from a pool of the
+ * handle (one tile's per resident CTA: 38 MB at 53/325, 99 MB at 561/2539; it
+ * keeps at most 256 MiB between synchronisations); the calls may be captured
+ * into a graph and run on several streams at once.  Calls for intermediates
+ * and mechanisms outside the tiles' scheme take the layouts below.
+ *
+ * FP64 throughout, and the operations of CRS_MODE_MIXED, with a fixed thread
+ * layout: one state per thread (TPS) or one state per warp (WARP).
  * CRS_MODE_MIXED_TPS also needs every stoichiometric coefficient to be
  * exact in 5 significant bits (integers up to 31, halves, ...); else, like a
  * mechanism whose per-thread columns do not fit, it returns
- * CRS_ERR_UNSUPPORTED and CRS_MODE_MIXED runs the warp layout. */
+ * CRS_ERR_UNSUPPORTED (CRS_MODE_MIXED itself needs neither). */
 #define CRS_MODE_FP64_TPS 3
 #define CRS_MODE_MIXED_TPS 4
 #define CRS_MODE_FP64_WARP 5
@@ -69,18 +76,14 @@ typedef struct crs_mech crs_mech;
 #define CRS_MODE_GEMM 7
 /* The arithmetic of CRS_MODE_MIXED in two passes: net rates of tiles of 32
  * states (all warps of a CTA on one tile) to HBM in FP64, then the species
- * sums.  CRS_MODE_MIXED takes this path when a mechanism's per-thread
- * columns do not fit on chip and no intermediates are asked for.  No
- * intermediates.
+ * sums.  No intermediates.
  * CRS_MODE_GEMM and the two-pass paths use a workspace owned by the handle,
  * allocated on first use (FP64 rates of up to 2^17 states, <= ~2 GiB, plus
  * 4 bytes per reaction and state for the contraction): calls on one handle
  * take turns on the GPU, whatever their streams. */
 #define CRS_MODE_MIXED_TILE 8
-/* The arithmetic of CRS_MODE_FP64 in the same two passes (FP64
- * concentrations of the tile in shared memory); CRS_MODE_FP64 takes this
- * path when the per-thread columns do not fit and no intermediates are
- * asked for. */
+/* FP64 throughout in the same two passes (FP64 concentrations of the tile in
+ * shared memory). */
 #define CRS_MODE_FP64_TILE 9
 
 /* ---- mechanism tables ------------------------------------------------ */
