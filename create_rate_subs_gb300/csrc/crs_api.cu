@@ -119,7 +119,7 @@ struct crs_mech {
   unsigned char *d_img = nullptr;  // device table image
   crs::fx::FxTab fx{};             // tables of the FP64 state-tile kernel
   unsigned char *d_fx = nullptr;   // (fx.usable = 0: not for this mechanism)
-  cudaMemPool_t fx_pool = nullptr; // its kernels' scratch (freed with the mechanism)
+  cudaMemPool_t fx_pool = nullptr; // stream-ordered scratch (freed with the mechanism)
   int32_t *d_status = nullptr;     // [0] flags, [1] non-finite count
   // dynamic-scheduling counter pairs of the one-state-per-thread kernels;
   // each launch draws the next slot, so launches in flight at the same time
@@ -145,6 +145,9 @@ struct crs_mech {
   // producer): FP64 net rates of one chunk of states [R][q_rows]
   double *d_q = nullptr;
   int64_t q_rows = 0;
+  // state tiles: net rates of one tile per resident CTA
+  double *d_tile = nullptr;
+  size_t tile_bytes = 0;
   // recorded after the last kernel that used the workspaces, waited on by
   // the next call's stream: calls on several streams take turns on the GPU
   cudaEvent_t ws_done = nullptr;
@@ -664,8 +667,7 @@ int wdot_two_pass(crs_mech *m, const crs::Batch &b, cudaStream_t s, bool fp64) {
 }
 
 // A pool for stream-ordered scratch; what is free stays with it between
-// synchronisations up to 256 MiB (the scratch of 53/325: 38 MB, of 561/2539:
-// 99 MB; mapped anew on each call it cost more than the kernel).
+// synchronisations up to 256 MiB.
 cudaError_t make_pool(int device, cudaMemPool_t *pool) {
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
@@ -677,32 +679,78 @@ cudaError_t make_pool(int device, cudaMemPool_t *pool) {
   return e;
 }
 
+// Scratch of the state tiles for the launches that follow on stream s (caller
+// holds ws_mu and ends with tile_scratch_end): the handle's buffer, whose users
+// take turns, of the most that any launch needs, so that it stays where it is
+// and in L2 (blocks of a pool, a new one for each call: 20,011 states of
+// 561/2539 1.28 -> 1.65 ms); while the stream is captured, a block of the pool
+// that becomes a node of the graph.  *q = NULL when there is no memory.
+int tile_scratch_begin(crs_mech *m, size_t bytes, cudaStream_t s, double **q, bool *node) {
+  *q = nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &cs);
+  if (e != cudaSuccess) return cuda_fail(e, "scratch");
+  *node = cs != cudaStreamCaptureStatusNone;
+  if (*node) {
+    e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(q), bytes, m->fx_pool, s);
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return cuda_fail(e, "scratch");
+    if (e != cudaSuccess) cudaGetLastError();
+    return CRS_OK;
+  }
+  if (m->tile_bytes < bytes) {
+    if (m->d_tile) cudaFree(m->d_tile);
+    m->d_tile = nullptr;
+    m->tile_bytes = 0;
+    e = cudaMalloc(&m->d_tile, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return CRS_OK;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "scratch");
+    m->tile_bytes = bytes;
+  }
+  const int rc = ensure_q(m, 0, false, false);  // the event
+  if (rc != CRS_OK) return rc;
+  *q = m->d_tile;
+  return ws_begin(m, s);
+}
+
+int tile_scratch_end(crs_mech *m, double *q, bool node, cudaStream_t s) {
+  if (!node) return ws_end(m, s);
+  const cudaError_t e = cudaFreeAsync(q, s);
+  return e == cudaSuccess ? CRS_OK : cuda_fail(e, "scratch");
+}
+
 // CRS_MODE_FP64 and CRS_MODE_MIXED by state tiles, when the mechanism fits
 // (and no intermediates are asked for); *taken = false otherwise.  Net rates
 // that do not fit on chip (at most one tile's per resident CTA) get scratch.
 int wdot_tiles(crs_mech *m, const crs::Batch &b, bool mixed, cudaStream_t s, bool *taken) {
-  const long long scratch =
-      mixed ? crs::mixed_tile_scratch(m->fx, b.n, m->sm_count, m->smem_optin)
-            : crs::fx_scratch(m->fx, b.n, m->sm_count, m->smem_optin);
+  auto scratch_of = [&](int64_t n) {
+    return mixed ? crs::mixed_tile_scratch(m->fx, n, m->sm_count, m->smem_optin)
+                 : crs::fx_scratch(m->fx, n, m->sm_count, m->smem_optin);
+  };
+  auto launch = [&](double *q) {
+    const cudaError_t e = (mixed ? crs::launch_mixed_tile : crs::launch_wdot_fx)(
+        m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, q, s);
+    return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
+  };
+  const long long scratch = scratch_of(b.n);
   *taken = scratch >= 0 && !(b.conc || b.fwd || b.rev || b.pm);
   if (!*taken) return CRS_OK;
-  // in stream order, from the mechanism's pool: calls on several streams do
-  // not share it, and under capture it becomes a node of the graph
-  double *q = nullptr;
-  cudaError_t e = cudaSuccess;
-  if (scratch)
-    e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&q), (size_t)scratch, m->fx_pool, s);
-  if (e == cudaErrorMemoryAllocation) {  // the kernels that need none
-    cudaGetLastError();
+  if (scratch == 0) return launch(nullptr);
+  std::lock_guard<std::mutex> lk(m->ws_mu);
+  double *q;
+  bool node;
+  const size_t most = (size_t)std::max(scratch, scratch_of((int64_t)1 << 40));
+  int rc = tile_scratch_begin(m, most, s, &q, &node);
+  if (rc != CRS_OK) return rc;
+  if (!q) {  // the kernels that need none
     *taken = false;
     return CRS_OK;
   }
-  if (e != cudaSuccess) return cuda_fail(e, "crs_wdot scratch");
-  e = (mixed ? crs::launch_mixed_tile : crs::launch_wdot_fx)(
-      m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, q, s);
-  const cudaError_t e2 = q ? cudaFreeAsync(q, s) : cudaSuccess;
-  if (e == cudaSuccess) e = e2;
-  return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
+  rc = launch(q);
+  const int rc2 = tile_scratch_end(m, q, node, s);
+  return rc != CRS_OK ? rc : rc2;
 }
 
 // CRS_MODE_GEMM: per chunk, the FP64 net rates (state tiles), their bf16
@@ -719,16 +767,13 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
   // rates and packing in one kernel when the mechanism fits its tiles
   const long long scratch = crs::mixed_pack_scratch(m->fx, rows, m->sm_count, m->smem_optin);
   double *q = nullptr;
-  if (scratch > 0) {
-    const cudaError_t e =
-        cudaMallocFromPoolAsync(reinterpret_cast<void **>(&q), (size_t)scratch, m->fx_pool, s);
-    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
-    else if (e != cudaSuccess) return cuda_fail(e, "gemm scratch");
-  }
+  bool node = false;
+  if (scratch > 0) rc = tile_scratch_begin(m, (size_t)scratch, s, &q, &node);
+  if (rc != CRS_OK) return rc;
   rc = ensure_q(m, rows, !q, true);
   if (rc == CRS_OK) rc = ws_begin(m, s);
   if (rc != CRS_OK) {
-    if (q) cudaFreeAsync(q, s);
+    if (q) tile_scratch_end(m, q, node, s);
     return rc;
   }
   for (int64_t c0 = 0; c0 < b.n && rc == CRS_OK; c0 += rows) {
@@ -760,7 +805,7 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
     if (e == cudaErrorNotSupported) rc = fail(CRS_ERR_UNSUPPORTED, "rates tile not available");
     else if (e != cudaSuccess) rc = cuda_fail(e, "gemm launch");
   }
-  if (q) cudaFreeAsync(q, s);
+  if (q && node) cudaFreeAsync(q, s);
   const int rc2 = ws_end(m, s);
   return rc != CRS_OK ? rc : rc2;
 }
@@ -981,6 +1026,7 @@ int crs_mech_free(crs_mech *m) {
   if (m->d_escale) cudaFree(m->d_escale);
   if (m->d_outflag) cudaFree(m->d_outflag);
   if (m->d_q) cudaFree(m->d_q);
+  if (m->d_tile) cudaFree(m->d_tile);
   if (m->ws_done) cudaEventDestroy(m->ws_done);
   if (m->d_host) cudaFree(m->d_host);
   for (cudaStream_t st : m->hs)
@@ -1135,7 +1181,9 @@ int crs_dydt(const crs_mech *m, int64_t n, const double *p_or_rho, const double 
   // pressure row
   double *ws = nullptr;
   const size_t bytes = ((size_t)N * ld + (conv ? (size_t)ld : 0)) * sizeof(double);
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&ws), bytes, s);
+  cudaError_t e = m->fx_pool ? cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), bytes,
+                                                       m->fx_pool, s)
+                             : cudaMallocAsync(reinterpret_cast<void **>(&ws), bytes, s);
   if (e != cudaSuccess) return cuda_fail(e, "crs_dydt scratch");
   double *W = ws, *Pw = ws + (size_t)N * ld;
   if (conv)
@@ -1188,10 +1236,21 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
   cudaError_t e = cudaSuccess;
   if (!mm->hs[0]) e = cudaStreamCreateWithFlags(&mm->hs[0], cudaStreamNonBlocking);
   if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host streams");
-  if (!staged_only) {
-    // arrays the device addresses in place: one launch reads the states
-    // from host memory and writes wdot back over the host link (NVLink-C2C
-    // on Grace), without staging copies or per-chunk launches
+  const int64_t per = 2 + (N - 1) + N;  // doubles per state: T, P, Y, wdot
+  // The state tiles read mass fractions three times: from 2^17 states on
+  // chunked copies, each over the link once, are faster than reading in place
+  // (CRS_MODE_FP64, 53/325: 131,072 states 1.04 against 1.19 ms, 200,003 1.50
+  // against 2.22, 2^20 7.2 against 9.5; 561/2539, 131,072: 11.4 against 15.3;
+  // below, the copies' latency counts: 4,000 states of 53/325 0.10 against
+  // 0.07), but not the short rows of small mechanisms (10/27, 2^20: 1.09
+  // against 0.85)
+  const bool copies = n >= ((int64_t)1 << 17) && m->L.R >= 100 &&
+                      ((mode == CRS_MODE_FP64 && m->fx.usable) ||
+                       (mode == CRS_MODE_MIXED && m->fx.mixed));
+  // arrays the device addresses in place: one launch reads the states
+  // from host memory and writes wdot back over the host link (NVLink-C2C
+  // on Grace), without staging copies or per-chunk launches
+  auto in_place = [&](int &result) {
     void *vT = mapped_view(T), *vP = mapped_view(P), *vY = mapped_view(Y),
          *vW = mapped_view(wdot);
     if (vT && vP && vY && vW) {
@@ -1200,25 +1259,36 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
       b.P = static_cast<const double *>(vP);
       b.Y = static_cast<const double *>(vY);
       b.wdot = static_cast<double *>(vW);
-      int result = launch_mode(m, b, mode, mm->hs[0]);
+      result = launch_mode(m, b, mode, mm->hs[0]);
       const cudaError_t es = cudaStreamSynchronize(mm->hs[0]);
       if (es != cudaSuccess && result == CRS_OK) result = cuda_fail(es, "crs_wdot_host");
-      return result;
+      return true;
     }
-  }
-  const int64_t per = 2 + (N - 1) + N;  // doubles per state: T, P, Y, wdot
-  // chunks of up to 2^17 states, at most 256 MB per buffer
-  int64_t chunk = ((int64_t)256 << 20) / (per * 8);
-  if (chunk > ((int64_t)1 << 17)) chunk = (int64_t)1 << 17;
-  if (chunk < 128) chunk = 128;
-  if (mm->host_chunk < chunk) {
+    return false;
+  };
+  int done = CRS_OK;
+  if (!staged_only && !copies && in_place(done)) return done;
+  // buffers of up to 2^17 states, at most 256 MB each
+  int64_t most = ((int64_t)256 << 20) / (per * 8);
+  if (most > ((int64_t)1 << 17)) most = (int64_t)1 << 17;
+  if (most < 128) most = 128;
+  if (mm->host_chunk < most) {
     if (mm->d_host) cudaFree(mm->d_host);
     mm->d_host = nullptr;
     mm->host_chunk = 0;
-    e = cudaMalloc(&mm->d_host, (size_t)2 * chunk * per * sizeof(double));
+    e = cudaMalloc(&mm->d_host, (size_t)2 * most * per * sizeof(double));
+    if (e == cudaErrorMemoryAllocation && !staged_only) {
+      cudaGetLastError();
+      if (in_place(done)) return done;
+    }
     if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host buffers");
-    mm->host_chunk = chunk;
+    mm->host_chunk = most;
   }
+  // the first copy in and the last copy out stand alone (200,003 states:
+  // chunks of 32,768 1.43 ms, of 65,536 1.52, of 16,384 2.16; 2^20: of 65,536
+  // 7.16 ms, of 32,768 7.22, of 131,072 7.42)
+  int64_t chunk = std::max<int64_t>((n / 16 + 127) / 128 * 128, 32768);
+  if (chunk > most) chunk = most;
   for (int j = 0; j < 2 && e == cudaSuccess; ++j)
     if (!mm->hs[j]) e = cudaStreamCreateWithFlags(&mm->hs[j], cudaStreamNonBlocking);
   if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host streams");

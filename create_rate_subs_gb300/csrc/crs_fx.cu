@@ -32,8 +32,10 @@
 // mass-fraction sums, two chains of N dependent FP64 additions, run on
 // two warps beside the rates.
 //
-// Measured on GB300: 2^20 states of 53/325 in 7.2 ms (31.2 with the one-
-// state-per-thread kernel), FP64 pipe 53%, integer multiply pipe 43% busy.
+// Measured on GB300 (before: one state per thread, 561/2539 in two passes):
+// 2^20 states of 53/325 31.2 -> 6.41 ms, 97 states 716 -> 21.6 us, 20,011
+// states of 561/2539 4.87 -> 1.64 ms; FP64 pipe 53%, integer multiply pipe
+// 43% busy.
 //
 // States outside the scheme (T outside (200, 6000] K, a density or mean
 // 1/W out of range, |Y| >= 2, a subnormal Y) and reactions outside it (non-
@@ -700,14 +702,22 @@ Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
     return (smem_of(f, nw, qs, true) + 1024) * per_sm <= (size_t)smem_optin + 1024;
   };
   // few tiles: a cluster of CTAs shares each, as long as its warps get two
-  // reactions or more (97 states of 53/325: 47 us with one CTA per tile)
+  // reactions or more (97 states of 53/325: 47 us with one CTA per tile, 21.6
+  // with eight)
   for (int cl = 8; cl > 1; cl /= 2)
     if (tiles * cl <= sm_count && f.R >= 32 * cl) {
       if (fits(16, 1, true)) return Plan{16, 1, cl, true, true, true};
       if (fits(16, 1, false)) return Plan{16, 1, cl, false, true, true};
     }
+  // one tile per SM: its rates on chip, more warps (4,000 states of 53/325:
+  // 57 us with three CTAs of eight warps, 45 so)
   if (tiles <= sm_count && fits(16, 1, true)) return Plan{16, 1, 1, true, true, true};
+  // small mechanisms: a tile's work does not fill more warps (131,072 states
+  // of 10/27: 115 us with three CTAs of eight, 101 so)
   if (f.R < 100 && fits(4, 6, true)) return Plan{4, 6, 1, true, true, true};
+  // rates in L2, so that three CTAs share an SM and their phases overlap (2^20
+  // states of 53/325: 6.41 ms; rates on chip, one CTA of 16 warps: 8.5; six
+  // CTAs of four: 6.89)
   if (fits(8, 3, false)) return Plan{8, 3, 1, false, true, true};
   if (fits(24, 1, false)) return Plan{24, 1, 1, false, true, true};
   Plan p{24, 1, 1, false, false, false};

@@ -733,6 +733,9 @@ struct Plan {
 
 Plan plan_of(const FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
   if (!f.mixed) return Plan{};
+  // the lines of crs_fx.cu, whose shapes these are: 1,024 states of 53/325
+  // (clusters) 28.7 us, 5,000 (three CTAs per SM) 72 us; one state per thread
+  // took 455 us for either
   auto fits = [&](int nw, int per_sm, bool qs) {
     return (smem_of(f, nw, qs) + 1024) * per_sm <= (size_t)smem_optin + 1024;
   };

@@ -53,11 +53,12 @@ typedef struct crs_mech crs_mech;
 #define CRS_MODE_MIXED 2       /* FP32 bulk, float-float exponents, FP64 net rate/sum */
 /* CRS_MODE_FP64 and CRS_MODE_MIXED evaluate tiles of 32 states (the warps of
  * a CTA, or of a cluster when tiles are few, split the reactions).  Net rates
- * that do not fit on chip take scratch in stream order from a pool of the
- * handle (one tile's per resident CTA: 38 MB at 53/325, 99 MB at 561/2539; it
- * keeps at most 256 MiB between synchronisations); the calls may be captured
- * into a graph and run on several streams at once.  Calls for intermediates
- * and mechanisms outside the tiles' scheme take the layouts below.
+ * that do not fit on chip take scratch (one tile's per resident CTA: 38 MB at
+ * 53/325, 99 MB at 561/2539), owned by the handle and allocated on first use:
+ * calls that need it take turns on the GPU, whatever their streams.  A call
+ * captured into a graph, be it the first, has its own as a node of the graph.
+ * Calls for intermediates and mechanisms outside the tiles' scheme take the
+ * layouts below.
  *
  * FP64 throughout, and the operations of CRS_MODE_MIXED, with a fixed thread
  * layout: one state per thread (TPS) or one state per warp (WARP).
