@@ -253,7 +253,8 @@ class RateSubs(object):
         """wdot (N, n) from host arrays, through crs_wdot_host.  T, P: (n,),
         Y: (>= N-1, n) float64 numpy arrays or CPU torch tensors; out: same
         kinds, (N, n).  Pinned CPU tensors (all four) are read and written
-        in place by one launch over the host link; other arrays, or
+        in place by one launch over the host link (large batches by
+        chunked copies, where those are faster); other arrays, or
         staged=True, pass through the GPU in chunks on two streams, copies
         overlapping kernels.  Returns out (a numpy array when allocated
         here)."""

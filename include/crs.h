@@ -181,8 +181,9 @@ int crs_dydt(const crs_mech *mech, int64_t n, const double *p_or_rho,
  * arrays are page-locked host memory that the current device can address
  * (cudaHostAlloc, torch's pin_memory, cudaHostRegister), one launch reads
  * the states and writes wdot in place over the host link (NVLink-C2C on
- * Grace).  Otherwise, or with CRS_HOST_STAGED or'ed into `mode`, states go
- * through device buffers in chunks on two streams owned by the handle, so
+ * Grace).  Otherwise, with CRS_HOST_STAGED or'ed into `mode`, or where it is
+ * faster (CRS_MODE_FP64 and CRS_MODE_MIXED, 2^17 states and 100 reactions or
+ * more), states go through device buffers in chunks on two streams owned by the handle, so
  * that the copies of one chunk overlap the kernel of the other (pinned
  * memory is needed for that overlap; the buffers, <= 2 x 256 MB, are
  * allocated on first use and kept by the handle).  Returns when wdot is on
