@@ -168,38 +168,40 @@ __global__ void __launch_bounds__(256)
 }
 
 // Row sums of a [rows][ld] bf16 matrix over its first m columns: a CTA per
-// row, eight columns per load where the rows' addresses allow it (one warp
-// per row and a column per load took 30 us for 256 rows of 16,384), a fixed
-// order of summation.
+// row.  The order of summation is a warp's with a column per lane, whose 2-byte
+// loads took 30 us for 256 rows of 16,384: here seven warps bring the next
+// 4,096 columns on chip, eight per load where the row's address allows it,
+// while the first adds the present ones.
+constexpr int ROW_CHUNK = 4096;
 __global__ void __launch_bounds__(256)
     k_row_sums(const __nv_bfloat16 *X, int64_t ld, int64_t m, float *out) {
-  __shared__ float part[8];
+  __shared__ __align__(16) __nv_bfloat16 buf[2][ROW_CHUNK];
   const __nv_bfloat16 *x = X + (int64_t)blockIdx.x * ld;
+  const bool quads = !(reinterpret_cast<uintptr_t>(x) & 15);
+  const int lane = threadIdx.x & 31;
+  auto fetch = [&](int64_t c0, __nv_bfloat16 *to) {
+    const int cnt = m - c0 < ROW_CHUNK ? (int)(m - c0) : ROW_CHUNK;
+    const int done = quads ? cnt / 8 * 8 : 0;
+    for (int i = ((int)threadIdx.x - 32) * 8; i < done; i += 224 * 8)
+      *reinterpret_cast<uint4 *>(to + i) = *reinterpret_cast<const uint4 *>(x + c0 + i);
+    for (int i = done + (int)threadIdx.x - 32; i < cnt; i += 224) to[i] = x[c0 + i];
+  };
+  if (threadIdx.x >= 32) fetch(0, buf[0]);
   float s = 0.0f;
-  int64_t done = 0;
-  if (!(reinterpret_cast<uintptr_t>(x) & 15)) {
-    done = m / 8 * 8;
-    for (int64_t i = (int64_t)threadIdx.x * 8; i < done; i += 256 * 8) {
-      const uint4 v = *reinterpret_cast<const uint4 *>(x + i);
-      const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float2 f = __bfloat1622float2(h[u]);
-        s += f.x;
-        s += f.y;
-      }
+  for (int64_t c0 = 0, k = 0; c0 < m; c0 += ROW_CHUNK, ++k) {
+    __syncthreads();
+    if (threadIdx.x >= 32) {
+      if (c0 + ROW_CHUNK < m) fetch(c0 + ROW_CHUNK, buf[(k + 1) & 1]);
+    } else {
+      const int cnt = m - c0 < ROW_CHUNK ? (int)(m - c0) : ROW_CHUNK;
+#pragma unroll 16
+      for (int i = lane; i < cnt; i += 32) s += __bfloat162float(buf[k & 1][i]);
     }
   }
-  for (int64_t i = done + threadIdx.x; i < m; i += 256) s += __bfloat162float(x[i]);
+  if (threadIdx.x < 32) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) t += part[w];
-    out[blockIdx.x] = t;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[blockIdx.x] = s;
   }
 }
 
