@@ -541,8 +541,8 @@ def run_ours(args):
         "e2e": {"value": n * world / (ms_e2e * 1e-3), "unit": "states/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": ms_e2e, "matches_device_result": e2e_ok,
-                "path": "crs_wdot_host via ctypes on pinned host arrays: one launch reads "
-                        "T, P, Y from host memory and writes wdot to it over NVLink-C2C; "
+                "path": "crs_wdot_host via ctypes on pinned host arrays: at this size chunked "
+                        "copies over NVLink-C2C on two streams beside the kernels; "
                         "host clock around each call",
                 "staged": {"value": n * world / (ms_staged * 1e-3), "unit": "states/s",
                            "ms_per_step": ms_staged, "matches_device_result": staged_ok,

@@ -1,4 +1,6 @@
-// Mixed precision for mechanisms whose per-state columns do not fit on chip
+// CRS_MODE_MIXED_TILE, and CRS_MODE_MIXED and _GEMM where the state tiles of
+// crs_mixed_tile.cu do not take a mechanism:
+// mixed precision for mechanisms whose per-state columns do not fit on chip
 // (hundreds of species, thousands of reactions): the rates and the species
 // sums as separate passes over HBM.
 //

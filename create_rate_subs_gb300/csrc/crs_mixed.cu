@@ -1,4 +1,7 @@
-// CRS_MODE_MIXED: FP32 bulk arithmetic, FP64 where stability needs it.
+// CRS_MODE_MIXED: FP32 bulk arithmetic, FP64 where stability needs it.  The
+// kernels here serve CRS_MODE_MIXED_TPS and _WARP, and CRS_MODE_MIXED for
+// intermediates and reactions with several T_common values; its state tiles
+// (crs_mixed_tile.cu) take the same arithmetic.
 //
 // FP64 instructions are kept for
 //   * the net rate fwd - rev (cancels near equilibrium);
