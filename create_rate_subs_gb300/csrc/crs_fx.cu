@@ -56,12 +56,6 @@ namespace crs {
 namespace fx {
 
 constexpr int64_t ZMIN = -561023779885736503LL;   // log2 1e-300
-constexpr int64_t LOG2_10 = 1870079266285788LL;   // log2 10
-constexpr int64_t C04 = 748031706514315LL;        // 0.4 log2 10
-constexpr int64_t C0806 = 1507283888626345LL;     // 0.806 log2 10
-constexpr int64_t K067 = 3089829632346349896LL;   // 0.67, 2^-62
-constexpr int64_t K11762 = 5424265094874293653LL; // 1.1762
-constexpr int64_t K014 = 645636042579834307LL;    // 0.14
 
 // The lane's functions of T.
 struct Basis {
@@ -93,7 +87,8 @@ struct Dot {
 };
 
 // log2 of a fall-off factor from lth = log2 [M] (c: its record on the lane's
-// interval).  slow: outside the scheme (negative or tiny terms).
+// interval).  slow: outside the scheme (a negative collider or centre, see
+// Sum::outside).
 __device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags, int64_t lth,
                                         Dg L, Dg I, Dg t, const int64_t *et, const int64_t *lt,
                                         bool &slow) {
@@ -112,30 +107,21 @@ __device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags
   int64_t f = ((flags & PMF_LOW) ? (z < 0 ? z : 0) : (z > 0 ? -z : 0)) - lv;
   if (!(flags & (PMF_TROE | PMF_SRI))) return even(f);
   const int64_t zP = z > ZMIN ? z : ZMIN;
-  // Fcent (Troe) or the base of the SRI power, in units of 2^-59
-  int64_t S = 0;
+  // Fcent (Troe) or the base of the SRI power
+  Sum S;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     if (flags & (PMF_T1 << q)) {
       const int64_t y = word(c[3 + 2 * q]);
       exp2m(y + mul<0>(dg(c[4 + 2 * q]), q == 2 ? I : t), et, M, E);
-      slow |= E > 1;
-      const int64_t v = (int64_t)((M << 6) >> min(max(3 - E, 2), 63));
-      S += (y & 1) ? -v : v;
+      S.add(M, E, y & 1);
     }
   }
-  slow |= S < (1LL << 39);
-  const int64_t zF = log2i(S > 1 ? S : 1, 59, lt);
-  int64_t A = zP, B = LOG2_10;
-  if (flags & PMF_TROE) {
-    const Dg kF = split(zF);
-    A = zP - mul<2>(kF, split(K067)) - C04;
-    B = C0806 - mul<2>(kF, split(K11762)) - mul<2>(split(zP), split(K014));
-  }
+  slow |= S.outside();
+  const int64_t zF = S.log2(lt);
   bool ok;
-  const int64_t rho = ratio2(A, B, ok);
+  f += broadening(zF, zP, flags & PMF_TROE, ok);
   slow |= !ok;
-  f += mul<3>(split(zF), split(rho));
   if (flags & PMF_DE) {
     Dot e(word(c[9]));
     e.add(dg(c[10]), L);

@@ -218,6 +218,29 @@ FX_FN int64_t log2hp(double v, const int64_t *hp) {
   return (int64_t)e * (1LL << 58) + (h >> 4);
 }
 
+// The sum of up to three signed numbers M 2^(E - 56), M in [2^56, 2^57], in
+// units of 2^(e - 60) with e the largest term's exponent: a fall-off centre
+// may be any power of two, and an absolute unit would leave a small one
+// without its last bits (in units of 2^-59, centres near 2^-20: up to 5e-12 of
+// the factor).
+struct Sum {
+  int64_t v = 0;
+  int e = -4000;
+  FX_FN void add(uint64_t M, int E, bool neg) {
+    const int64_t m = (int64_t)(M << 4);
+    const int d = E - e, n = d > 63 ? 63 : d < -63 ? 63 : d < 0 ? -d : d;
+    const int64_t t = neg ? -m : m;
+    v = d > 0 ? (v >> n) + t : v + (t >> n);
+    e = d > 0 ? E : e;
+  }
+  // Not a positive number that the general arithmetic would leave as it is:
+  // below its limit of 1e-300, above two (E <= 1), or less than 1/16 of the
+  // largest term, whose exponent's rounding the difference would magnify.
+  FX_FN bool outside() const { return e > 1 || e < -990 || v < (1LL << 56); }
+  // log2 of the sum (bit 0 arbitrary)
+  FX_FN int64_t log2(const int64_t *ltab) const;
+};
+
 // b^2 / (a^2 + b^2) in units of 2^-61 for |a|, |b| < 2^62; ok = false when
 // both are zero.  The quotient of the 64-bit squares from a 24-bit
 // reciprocal R0 of the denominator and two terms of its residual eps,
@@ -244,6 +267,27 @@ FX_FN int64_t ratio2(int64_t a, int64_t b, bool &ok) {
   const int64_t t2 = mad((int)(t1 >> 32), eps, 0);
   return (int64_t)q0 + (t1 >> 22) + (t2 >> 43);
 }
+
+// log2 of the broadening factor, log2 of the centre over 1 + (A / B)^2 (Troe)
+// or of the SRI base over 1 + log10(Pr)^2; zF: log2 of the centre or base, zP:
+// log2 Pr.  ok = false: 0 / 0.
+constexpr int64_t LOG2_10 = 1870079266285788LL;   // log2 10
+constexpr int64_t C04 = 748031706514315LL;        // 0.4 log2 10
+constexpr int64_t C0806 = 1507283888626345LL;     // 0.806 log2 10
+constexpr int64_t K067 = 3089829632346349896LL;   // 0.67, 2^-62
+constexpr int64_t K11762 = 5424265094874293653LL; // 1.1762
+constexpr int64_t K014 = 645636042579834307LL;    // 0.14
+FX_FN int64_t broadening(int64_t zF, int64_t zP, bool troe, bool &ok) {
+  int64_t A = zP, B = LOG2_10;
+  const Dg kF = split(zF);
+  if (troe) {
+    A = zP - mul<2>(kF, split(K067)) - C04;
+    B = C0806 - mul<2>(kF, split(K11762)) - mul<2>(split(zP), split(K014));
+  }
+  return mul<3>(kF, split(ratio2(A, B, ok)));
+}
+
+FX_FN int64_t Sum::log2(const int64_t *ltab) const { return log2i(v > 1 ? v : 1, 60 - e, ltab); }
 
 // The value of one exponent (bit 0: its sign), with overflow to infinity and
 // gradual underflow.
