@@ -61,9 +61,6 @@ cudaError_t launch_pack_bf16(const double *q, int64_t ldq, int64_t n, int R, int
                              int sm_count, cudaStream_t s);
 // FP64 state tiles in fixed point (crs_fx.cu): scratch bytes of a launch (0:
 // none, < 0: the mechanism does not fit) and the launch.
-namespace fx {
-void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out);
-}
 cudaError_t fx_init(int smem_optin);
 long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,

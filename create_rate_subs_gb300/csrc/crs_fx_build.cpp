@@ -312,9 +312,28 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
   }
 }
 
+// An upper bound of the tables' size (one: bytes of a plain reaction's
+// record).
+int64_t bytes_bound(const Tab &t, int64_t one) {
+  const int64_t N = t.N, R = t.R, NPM = t.NPM, nnz = t.nu_ptr[R];
+  const int64_t neff = t.pm_eff_ptr[NPM];
+  const int64_t records = R * (one + PMH + PMC * NI + MPAIR);
+  const int64_t terms = 16 * N + 4 * 3 * nnz;
+  // the small tables and the sections' alignment (a section per pressure-
+  // modified reaction with many colliders), then the lists, whose pairs are
+  // completed once per warp that has reactions (and kind of pair)
+  int64_t all = (1 << 15) + 8 * N + (20 + 144) * NPM + 24 * neff + 12 * nnz;
+  for (int l = 0; l < NLIST; ++l) {
+    const int64_t nw = list_warps[l];
+    all += records + terms + 16 * N + std::min(nw, R) * one + std::min(4 * nw, R) * MREC +
+           6 * 4 * (nw + 1);
+  }
+  return all;
+}
+
 }  // namespace
 
-void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
+void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limit) {
   f = FxTab();
   out.clear();
   const int N = t.N, R = t.R, NPM = t.NPM;
@@ -322,6 +341,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   f.R = R;
   f.NPM = NPM;
   if (R < 1 || R >= (1 << 22)) return;  // slot offsets in 30 bits
+  limit = std::min<int64_t>(limit, INT32_MAX);  // the tables' offsets are ints
   // interval bounds: the most common T_common in the middle
   double mid = 1000.0;
   {
@@ -434,6 +454,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out) {
   const int one = HEAD + COEF * nco + (uniform ? 0 : ((int)nthr + 1) / 2 * 16);
   f.stride[0] = 2 * one;
   f.stride[1] = one + PMH + PMC * NI;
+  if (bytes_bound(t, one) > limit) return;
   std::vector<std::vector<unsigned char>> rec(R);
   std::vector<int> weight(R), kind(R);
   int generic = 0;

@@ -3,6 +3,9 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
+
+#include "../../include/crs_tables.h"
 
 namespace crs {
 namespace fx {
@@ -69,6 +72,11 @@ constexpr int MPM = MREC, MFALL = MPM + 16, MBROAD = MFALL + 64, MEFFS = MBROAD 
 constexpr int MEFF = (MPAIR - MEFFS) / 8;
 // (of a pair's first record: some factor is a third one; reversible)
 enum { MF_MORE = 1, MF_REV = 2, MF_THD = 4, MF_FALL = 8, MF_GEN = 16 };
+
+// The tables of a mechanism; none (f.usable = f.mixed = 0) when they might
+// take more than `limit` bytes or more than 32-bit offsets reach, from some
+// 390,000 reactions on.
+void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limit = INT32_MAX);
 
 }  // namespace fx
 }  // namespace crs
