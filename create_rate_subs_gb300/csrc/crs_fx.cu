@@ -37,7 +37,7 @@
 // states of 561/2539 4.87 -> 1.64 ms; FP64 pipe 53%, integer multiply pipe
 // 43% busy.
 //
-// States outside the scheme (T outside (200, 6000] K, a density or mean
+// States outside the scheme (T outside (200, 6000] K, a density beyond 2^+-60, a mean
 // 1/W out of range, |Y| >= 2, a subnormal Y) and reactions outside it (non-
 // integer coefficients, PLOG, Chebyshev, coefficients beyond the bounds)
 // are evaluated lane by lane by the general FP64 arithmetic (finish).
@@ -105,28 +105,32 @@ __device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags
   if (w >> 62) w = (1LL << 62) - 1;
   const int64_t lv = log2m((uint64_t)((1LL << 62) + w) << 1, lt);
   int64_t f = ((flags & PMF_LOW) ? (z < 0 ? z : 0) : (z > 0 ? -z : 0)) - lv;
-  if (!(flags & (PMF_TROE | PMF_SRI))) return even(f);
-  const int64_t zP = z > ZMIN ? z : ZMIN;
-  // Fcent (Troe) or the base of the SRI power
-  Sum S;
+  if (flags & (PMF_TROE | PMF_SRI)) {
+    const int64_t zP = z > ZMIN ? z : ZMIN;
+    // Fcent (Troe) or the base of the SRI power
+    Sum S;
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    if (flags & (PMF_T1 << q)) {
-      const int64_t y = word(c[3 + 2 * q]);
-      exp2m(y + mul<0>(dg(c[4 + 2 * q]), q == 2 ? I : t), et, M, E);
-      S.add(M, E, y & 1);
+    for (int q = 0; q < 3; ++q) {
+      if (flags & (PMF_T1 << q)) {
+        const int64_t y = word(c[3 + 2 * q]);
+        exp2m(y + mul<0>(dg(c[4 + 2 * q]), q == 2 ? I : t), et, M, E);
+        S.add(M, E, y & 1);
+      }
+    }
+    slow |= S.outside();
+    const int64_t zF = S.log2(lt);
+    bool ok;
+    f += broadening(zF, zP, flags & PMF_TROE, ok);
+    slow |= !ok;
+    if (flags & PMF_DE) {
+      Dot e(word(c[9]));
+      e.add(dg(c[10]), L);
+      f += e.exponent();
     }
   }
-  slow |= S.outside();
-  const int64_t zF = S.log2(lt);
-  bool ok;
-  f += broadening(zF, zP, flags & PMF_TROE, ok);
-  slow |= !ok;
-  if (flags & PMF_DE) {
-    Dot e(word(c[9]));
-    e.add(dg(c[10]), L);
-    f += e.exponent();
-  }
+  // (without its collider a rate in the low-pressure limit is zero)
+  if ((flags & PMF_LOW) && lth == ZERO_EXP) f = FALL_MIN_EXP;
+  slow |= f < FALL_MIN_EXP;
   return even(f);
 }
 
@@ -304,9 +308,9 @@ __device__ __forceinline__ void state_sums(const double *Y, int64_t ld, int N, i
     asm volatile("bar.sync 1, 64;" ::: "memory");
     mwi = fma(row[7 * 32], inv_mw[N - 1], mwi);
     const double rho = P / mwi * ((1.0 / T) * fast::INV_RU);
-    // a positive density of moderate size, a mean 1/W below 2
+    // a positive density of moderate size (RHO_MAX), a mean 1/W below 2
     const int e = (int)(bits_of(rho) >> 52), m = (int)(bits_of(mwi) >> 52);
-    *irr = e < 1023 - 400 || e > 1023 + 400 || m < 1023 - 40 || m > 1023;
+    *irr = e < 1023 - RHO_MAX || e >= 1023 + RHO_MAX || m < 1023 - 40 || m > 1023;
     reinterpret_cast<int64_t *>(row)[6 * 32] = even(log2d(rho, lt));
     row[8 * 32] = rho;
     row[9 * 32] = mwi;

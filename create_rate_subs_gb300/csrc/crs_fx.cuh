@@ -5,8 +5,9 @@
 // parts of a rate -- exponents, exponentials, logarithms -- are evaluated as
 // 64-bit integers:
 //   * an exponent is the base-2 logarithm of its value in units of 2^-49
-//     (range +-16384).  A double of magnitude 100 resolves 2^-46, so the
-//     sums here are finer than the FP64 sums they replace;
+//     (range +-16384): a fixed step of 1.2e-15 of the value, where a double
+//     resolves an exponent of 16 binary orders as finely, smaller ones more
+//     finely and larger ones less;
 //   * bit 0 of every exponent is the sign of its value: adding exponents
 //     multiplies the values, signs included;
 //   * a 64-bit number is split into two signed 32-bit digits, v = hi 2^32 +
@@ -32,7 +33,28 @@ namespace crs {
 namespace fx {
 
 constexpr int YB = 49;                         // fraction bits of an exponent
-constexpr int64_t ZERO_EXP = -(3500LL << YB);  // exponent of a zero factor
+// The ranges (in binary orders) that keep the sum of a rate's exponents inside
+// 64 bits and a zero factor zero; what lies outside is left to the general
+// arithmetic.  A rate has a constant, at most four concentrations and a fall-
+// off factor.
+constexpr int CONST_MAX = 800, TERMS_MAX = 500;  // an exponent: c0, its functions of T
+constexpr int RATE_MAX = CONST_MAX + TERMS_MAX;
+constexpr int RHO_MAX = 60;                      // density: 2^-60 to 2^60
+constexpr int W_MAX = 20;                        // 1 / W: 2^-20 to 2^20
+constexpr int CONC_MAX = 1 + W_MAX + RHO_MAX;    // mass fractions below 2
+constexpr int DE_MAX = 100;                      // the factor d T^e of an SRI form
+constexpr int FALL_MIN = -2750, FALL_MAX = DE_MAX + 4;
+constexpr int ZERO = -3050;                      // a zero factor
+constexpr int NORMAL_MIN = -1081;                // results below it are zero (normal_of)
+static_assert(4 * ZERO - RATE_MAX + FALL_MIN > -(1 << (63 - YB)) &&
+                  4 * CONC_MAX + RATE_MAX + FALL_MAX < 1 << (63 - YB),
+              "the exponent of a rate stays within 64 bits");
+static_assert(ZERO + 3 * CONC_MAX + RATE_MAX + FALL_MAX < NORMAL_MIN &&
+                  FALL_MIN + 4 * CONC_MAX + RATE_MAX < NORMAL_MIN,
+              "a rate with a zero factor is zero");
+static_assert(-1022 - W_MAX - RHO_MAX > ZERO, "no concentration is below a zero one");
+constexpr int64_t ZERO_EXP = -((int64_t)-ZERO << YB);  // exponent of a zero factor
+constexpr int64_t FALL_MIN_EXP = -((int64_t)-FALL_MIN << YB);
 constexpr int LOGN = 512;                      // logarithm table: F = 1 + j / 512
 // The small tables, in 8-byte words: 2^(j/256) in units of 2^-56 plus 8 units
 // (257 entries and one of padding), then pairs (1/F in units of 2^-62, log2 F
@@ -308,7 +330,7 @@ FX_FN double normal_of(int64_t y, const int64_t *tab, bool &far) {
   exp2m(y, tab, M, E);
   const unsigned e = (unsigned)(E + 1022);
   const bool in = e <= 2044u;
-  far = !in && E > -1081;
+  far = !in && E > NORMAL_MIN;
   const unsigned lo = (unsigned)(M >> 4);
   const unsigned hi = ((unsigned)(M >> 36) + (e << 20)) ^ ((unsigned)y << 31);
   return of_bits((uint64_t)(in ? hi : 0u) << 32 | (in ? lo : 0u));

@@ -95,13 +95,12 @@ Form form_of(const Norm &n, ld base, ld b, ld i, const ld *p) {
 
 // The bounds that keep every sum of the kernel inside 64 bits: with
 // coefficients of at most 500 in all, six products of the low digits (2^31
-// by 2^29) and of the high ones (500 2^20 by 2^31) stay below 2^63; with
-// constants of at most 4000, an exponent plus four concentrations stays
-// within 2^14.
-bool within(const Form &f) {
+// by 2^29) and of the high ones (500 2^20 by 2^31) stay below 2^63; for the
+// constants see CONST_MAX.
+bool within(const Form &f, ld most = CONST_MAX, ld terms = TERMS_MAX) {
   ld s = 0;
   for (int k = 1; k < 7; ++k) s += std::fabs(f.c[k]);
-  return std::isfinite((double)f.c[0]) && std::fabs(f.c[0]) <= 4000 && s <= 500;
+  return std::isfinite((double)f.c[0]) && std::fabs(f.c[0]) <= most && s <= terms;
 }
 
 int64_t constant(ld v) { return llroundl(std::ldexp(v, YB)); }
@@ -137,7 +136,7 @@ bool term(const Norm &n, ld a, ld x, bool inv, int64_t *w, int *flags, int bit) 
   ld c0 = std::log2(std::fabs(a)) + x * m, c1 = x * h;
   *flags |= bit;
   if (c0 + std::fabs(c1) < -1200) {
-    c0 = -3500;
+    c0 = ZERO;
     c1 = 0;
   }
   if (std::fabs(c0) > 4000 || std::fabs(c1) > 450) return false;
@@ -409,7 +408,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
             ok = d[3] > 0.0;
             if (ok) {
               const Form y = form_of(nm[q], std::log2((ld)d[3]), d[4], 0, nullptr);
-              ok = within(y);
+              ok = within(y, DE_MAX / 2, DE_MAX / 2);
               w[9] = number(constant(y.c[0]) + 1);
               w[10] = coefficient(y.c[1]);
             }
@@ -544,6 +543,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
   // kernels that evaluate every reaction so; beyond a fifth of such
   // reactions those are faster
   f.usable = generic * 5 <= R;
+  for (int k = 0; k < N; ++k) f.usable &= std::fabs(std::log2(t.inv_mw[k])) <= W_MAX;
   Buf b;
   std::vector<int64_t> small(EXP_WORDS + 2 * (LOGN + 1)), hp(2 * (LOGN + 1)), lw(N);
   for (int k = 0; k <= EXPN; ++k)

@@ -77,3 +77,29 @@ def test_no_table_beyond_the_limit(name, tool, golden, synth_mech):
     assert size_above == size and on_above == (usable or mixed)
     if not name.startswith("features"):
         assert usable and mixed
+
+
+@pytest.mark.parametrize("change,usable", [
+    (lambda a, b, e: (a, b, e), True),
+    # log2 of the constant beyond 800 at the middle of an interval: the sum of a
+    # rate's exponents might leave 64 bits
+    (lambda a, b, e: (1e-290, b, e), False),
+    (lambda a, b, e: (1e-60, -95.0, e), False),
+    # terms beyond 500
+    (lambda a, b, e: (a, b, 4e5), False)])
+def test_constants_outside_the_range_are_general(change, usable, tool, tmp_path):
+    """Rate constants that the fixed-point sums do not hold are left to the
+    general arithmetic; with all of them outside, the tables are not used."""
+    from create_rate_subs_gb300 import synth
+    from create_rate_subs_gb300.mechanism import Mechanism
+    text, therm = synth.make_mechanism(**synth.CONFIGS["small"])
+    lines = []
+    for line in text.split("\n"):
+        w = line.split()
+        if "=" in line:
+            line = "%-40s %13.6E %8.3f %10.1f" % ((w[0],) + change(*map(float, w[1:])))
+        lines.append(line)
+    mp, tp = tmp_path / "mech.inp", tmp_path / "therm.dat"
+    mp.write_text("\n".join(lines))
+    tp.write_text(therm)
+    assert tool(Mechanism.from_chemkin(str(mp), str(tp)))[0] == usable

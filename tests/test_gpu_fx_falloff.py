@@ -42,3 +42,41 @@ def test_small_centres(form, tmp_path):
     w = rs.wdot(*d, mode="fp64").cpu().numpy()
     assert wdot_errors(w, ref["wdot"], G)["scaled"] <= 1e-12
     assert rs.status() == (0, 0)
+
+
+def test_absent_reactants_and_colliders(tmp_path):
+    """Rates with up to four absent reactants, with very small constants, and
+    fall-off rates without their collider are zero, as in the general code."""
+    from create_rate_subs_gb300.mechanism import Mechanism
+    from create_rate_subs_gb300.rates import RateSubs
+    text, therm = synth.make_mechanism(**synth.CONFIGS["small"])
+    text = text[: text.rindex("END")] + """2H+2HO<=>2H2O 1.0E-200 -5.0 150000.0
+2H+2HO=>2H2O 1.0E+40 3.0 0.0
+H+HO(+H2O)<=>H2O(+H2O) 1.0E+13 0.0 0.0
+   LOW / 1.0E+18 -1.0 0.0 /
+   TROE / 0.5 100. 1000. /
+2HO(+O2)<=>H2O+O(+O2) 1.0E+13 0.0 0.0
+   HIGH / 1.0E+15 0.5 20.0 /
+   SRI / 0.5 300.0 900.0 1.2 0.3 /
+END
+"""
+    mp, tp = tmp_path / "mech.inp", tmp_path / "therm.dat"
+    mp.write_text(text)
+    tp.write_text(therm)
+    mech = Mechanism.from_chemkin(str(mp), str(tp))
+    N = mech.n_species
+    T, P, Y = synth.make_states(N, 515, seed=N, t_range=(250.0, 3000.0), p_atm=(1e-6, 1e3))
+    at = {k: list(mech.names).index(k) for k in ("H", "HO", "H2O", "O2")}
+    Y[at["H"], 0::3] = 0.0
+    Y[at["HO"], 0::6] = 0.0
+    Y[at["H2O"], 1::3] = 0.0
+    Y[at["H2O"], 0::6] = 0.0
+    Y[at["O2"], 2::6] = 0.0
+    ref = Oracle(mech.blob).eval(T, P, Y)
+    G = gross_scale(mech.tables, ref["fwd"], ref["rev"], ref["pm"])
+    rs = RateSubs(mech)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (T, P, Y[: N - 1])]
+    w = rs.wdot(*d, mode="fp64").cpu().numpy()
+    assert np.all(w[G == 0.0] == 0.0)
+    assert wdot_errors(w, ref["wdot"], G)["scaled"] <= 1e-12
+    assert rs.status() == (0, 0)
