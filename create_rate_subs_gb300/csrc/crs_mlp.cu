@@ -436,12 +436,13 @@ __device__ __forceinline__ float rows_of(const float *Ya, const float *Yb, int64
 // D as an input, see k_disagreement).  A state
 // goes back to the exact kernel as in k_output, or when g > stol (NaN
 // included).  gate[i] (optional) receives g, for calibrating stol.
-// Bound by memory: a warp reads its 32 states' rows whole (lane = column; 32
-// lanes reading 32 rows fetch each sector up to eight times) and keeps the
-// means in shared memory, column by state, for the sums over k that follow
-// with lane = state in the order of k, four k's table entries and
-// exponentials ahead of the sums.  2^20 states of 53 species: 488 us with a
-// row per thread, 374 with whole rows, 310 with both.
+// Bound by memory.  ROWS: a warp reads its 32 states' rows whole (lane =
+// column; 32 lanes reading 32 rows fetch each sector up to eight times) and
+// keeps the means in shared memory, column by state, for the sums over k that
+// follow with lane = state in the order of k, four k's table entries and
+// exponentials ahead of the sums; else a thread reads its state's row.  2^20
+// states of 53 species: 342 us without, 308 with.
+template <bool ROWS>
 __global__ void __launch_bounds__(256)
     k_output2(int64_t n, const float *Ya, const float *Yb, int64_t ldy, int nsp,
               const float *sm, const int *se, const float *cons, int nelem, float tol,
@@ -450,13 +451,16 @@ __global__ void __launch_bounds__(256)
               unsigned char *fallback, float *gate) {
   extern __shared__ float mean[];
   const int lane = threadIdx.x & 31;
-  float *col = mean + (size_t)(threadIdx.x >> 5) * nsp * 33;
+  float *col = mean + (ROWS ? (size_t)(threadIdx.x >> 5) * nsp * 33 : 0);
   const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; i0 < n;
        i0 += nwarp * 32) {
-    const int rows = n - i0 < 32 ? (int)(n - i0) : 32;
-    const float d = rows_of(Ya, Yb, ldy, i0, rows, nsp, lane, col);
-    __syncwarp();
+    float d = 0.0f;
+    if (ROWS) {
+      const int rows = n - i0 < 32 ? (int)(n - i0) : 32;
+      d = rows_of(Ya, Yb, ldy, i0, rows, nsp, lane, col);
+      __syncwarp();
+    }
     const int64_t i = i0 + lane;
     if (i < n) {
       float sum[MAX_ELEM], mag[MAX_ELEM];
@@ -464,7 +468,14 @@ __global__ void __launch_bounds__(256)
       for (int e = 0; e < MAX_ELEM; ++e) sum[e] = mag[e] = 0.0f;
 #pragma unroll 4
       for (int k = 0; k < nsp; ++k) {
-        const float y = col[k * 33 + lane];
+        float y;
+        if (ROWS) {
+          y = col[k * 33 + lane];
+        } else {
+          const float ya = Ya[i * ldy + k], yb = Yb[i * ldy + k];
+          d = fmaxf(d, fabsf(ya - yb));
+          y = 0.5f * (ya + yb);
+        }
         const float u = copysignf(expm1f(fabsf(y)), y);
         wdot[(int64_t)k * ld + i] = scale_to_double(u * sm[k], se[k]);
 #pragma unroll
@@ -491,16 +502,23 @@ __global__ void __launch_bounds__(256)
 
 // The members' disagreement D = max_k |y_k,a - y_k,b| as an input of the
 // error network: X[i][col] = bf16((log10(D + 1e-4) - mu) / sd).
-// A warp takes 32 states (see rows_of).
+// ROWS: a warp takes `per` states' rows whole (see rows_of), else (per = 32) a
+// thread a row.
+template <bool ROWS>
 __global__ void __launch_bounds__(256)
     k_disagreement(int64_t n, const float *Ya, const float *Yb, int64_t ldy, int nsp, float mu,
-                   float sd, __nv_bfloat16 *X, int64_t ldx, int col) {
+                   float sd, __nv_bfloat16 *X, int64_t ldx, int col, int per) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t i0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; i0 < n;
-       i0 += nwarp * 32) {
-    const int rows = n - i0 < 32 ? (int)(n - i0) : 32;
-    const float d = rows_of(Ya, Yb, ldy, i0, rows, nsp, lane, nullptr);
+  for (int64_t i0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; i0 < n;
+       i0 += nwarp * per) {
+    const int rows = n - i0 < per ? (int)(n - i0) : per;
+    float d = 0.0f;
+    if (ROWS)
+      d = rows_of(Ya, Yb, ldy, i0, rows, nsp, lane, nullptr);
+    else if (lane < rows)
+      for (int k = 0; k < nsp; ++k)
+        d = fmaxf(d, fabsf(Ya[(i0 + lane) * ldy + k] - Yb[(i0 + lane) * ldy + k]));
     if (lane < rows)
       X[(i0 + lane) * ldx + col] = __float2bfloat16_rn((log10f(d + 1.0e-4f) - mu) / sd);
   }
@@ -752,17 +770,33 @@ int crs_surrogate_output2(int64_t n, const float *Ya, const float *Yb, int64_t l
       (est && lde < 1))
     return bad(__func__);
   if (n == 0) return CRS_OK;
-  // as many warps per CTA (up to eight) as their columns of means allow
-  const size_t per_warp = (size_t)nsp * 33 * sizeof(float);
-  int nw = (int)(((size_t)200 << 10) / per_warp);
-  nw = nw > 8 ? 8 : nw;
-  if (nw < 1) return bad(__func__);
-  const cudaError_t e = mlp::raise_smem_limit(mlp::k_output2);
+  // Rows read whole pay from 32 species on (below, lanes idle: 10 species,
+  // 2^20 states 58 us with a row per thread, 101 so; 32: 304 and 176), in small
+  // batches from 48 (40 species, 500 states: 18.5 and 20.1), as long as the
+  // columns of means leave room for two CTAs of eight warps per SM (96 species,
+  // 2^20 states: 897 and 642; 112: 825 and 1,363), or all the states are on chip
+  // with one (300 species, 8,192 states: 137 and 114; 65,536: 198 and 340).
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return done(e, __func__);
-  mlp::k_output2<<<mlp::grid1(n, nw * 32), nw * 32, nw * per_warp,
-                   static_cast<cudaStream_t>(stream)>>>(
-      n, Ya, Yb, ldy, nsp, scale_m, scale_e, cons, nelem, tol, dweight, est, lde, stol,
-      out_of_box, wdot, ld, fallback, gate);
+  const size_t per_warp = (size_t)(nsp > 0 ? nsp : 1) * 33 * sizeof(float);
+  const size_t fit = ((size_t)200 << 10) / per_warp;
+  const int nw = fit < 8 ? (int)fit : 8;
+  const bool rows = (nsp >= 48 || (nsp >= 32 && n >= 32768)) &&
+                    (fit >= 16 || n <= (int64_t)sms * nw * 32);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (rows) {
+    e = mlp::raise_smem_limit(mlp::k_output2<true>);
+    if (e != cudaSuccess) return done(e, __func__);
+    mlp::k_output2<true><<<mlp::grid1(n, nw * 32), nw * 32, nw * per_warp, s>>>(
+        n, Ya, Yb, ldy, nsp, scale_m, scale_e, cons, nelem, tol, dweight, est, lde, stol,
+        out_of_box, wdot, ld, fallback, gate);
+  } else {
+    mlp::k_output2<false><<<mlp::grid1(n), 256, 0, s>>>(
+        n, Ya, Yb, ldy, nsp, scale_m, scale_e, cons, nelem, tol, dweight, est, lde, stol,
+        out_of_box, wdot, ld, fallback, gate);
+  }
   return done(cudaGetLastError(), __func__);
 }
 
@@ -772,8 +806,18 @@ int crs_surrogate_disagreement(int64_t n, const float *Ya, const float *Yb, int6
   if (n < 0 || !Ya || !Yb || !X || ldy < nsp || col < 0 || col >= ldx || !(sd > 0.0f))
     return bad(__func__);
   if (n == 0) return CRS_OK;
-  mlp::k_disagreement<<<mlp::grid1(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      n, Ya, Yb, ldy, nsp, mu, sd, static_cast<__nv_bfloat16 *>(X), ldx, col);
+  // rows read whole from 32 species on (2^20 states: 10 species 30 us with a row
+  // per thread, 68 so; 32: 232 and 72); eight rows per warp where that does not
+  // fill the chip
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (nsp >= 32) {
+    const int per = n < 32768 ? 8 : 32;
+    mlp::k_disagreement<true><<<mlp::grid1(n, 4 * per), 128, 0, s>>>(
+        n, Ya, Yb, ldy, nsp, mu, sd, static_cast<__nv_bfloat16 *>(X), ldx, col, per);
+  } else {
+    mlp::k_disagreement<false><<<mlp::grid1(n), 256, 0, s>>>(
+        n, Ya, Yb, ldy, nsp, mu, sd, static_cast<__nv_bfloat16 *>(X), ldx, col, 32);
+  }
   return done(cudaGetLastError(), __func__);
 }
 

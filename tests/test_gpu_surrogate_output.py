@@ -92,3 +92,15 @@ def test_threads_with_different_sizes():
     assert not errors
     for c in cases:
         c.check()
+
+
+# rows by threads and by warps, their lines at 32, 48 and 97 species and at one
+# CTA per SM; fewer than eight warps; species that no column of means holds; none
+@pytest.mark.parametrize("n,nsp", [(1, 1), (33, 0), (1000, 10), (77, 31), (77, 47), (77, 48),
+                                   (32767, 33), (32768, 33), (4099, 96), (4099, 101),
+                                   (4099, 194), (40000, 194), (65, 1551), (4099, 1551),
+                                   (300, 1552), (300, 2001)])
+def test_sizes(n, nsp):
+    c = Case(n, nsp, n + nsp)
+    c.run(torch.cuda.current_stream().cuda_stream)
+    c.check()
