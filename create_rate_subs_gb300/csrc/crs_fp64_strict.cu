@@ -217,7 +217,28 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// b.fwd / b.rev / b.pm are inputs.  Species by species over the species-major
+// b.fwd / b.rev / b.pm are inputs.  Reaction by reaction, as emitted: wdot
+// accumulates in place.  For batches that fill the chip with a state per
+// thread.
+__global__ void __launch_bounds__(128)
+    k_spec_rates_in_place(const unsigned char *__restrict__ img, ImgLayout L, Batch b) {
+  const Tab t = make_tab(img, L);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b.n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    Col W{b.wdot + i, b.ld};
+    for (int k = 0; k < t.N; ++k) W[k] = 0.0;
+    for (int r = 0; r < t.R; ++r) {
+      const int j = t.rev_idx[r], p = t.pm_idx[r];
+      const double f = b.fwd[(int64_t)r * b.ld + i];
+      const double net = (j >= 0) ? f - b.rev[(int64_t)j * b.ld + i] : f;
+      const double pm = (p >= 0) ? b.pm[(int64_t)p * b.ld + i] : 0.0;
+      for (int e = t.nu_ptr[r]; e < t.nu_ptr[r + 1]; ++e)
+        accumulate(t, e, net, pm, p >= 0, W);
+    }
+  }
+}
+
+// The same for smaller batches, species by species over the species-major
 // list, whose entries are in reaction order: the operations and the order of
 // eval_spec_rates' sums, in a register instead of in the output array.
 __global__ void __launch_bounds__(128)
@@ -309,6 +330,13 @@ cudaError_t launch_stage(int which, const unsigned char *img,
       break;
     }
     default: {
+      // six CTAs per SM fill it: 98,304 states of 53/325 1.79 ms in place, 1.64
+      // by species; 131,072: 2.09 and 2.15; 2^20: 15.7 and 17.2 (10/27 and
+      // 561/2539 cross between the same sizes)
+      if (b.n > (int64_t)sm_count * 6 * block) {
+        strict::k_spec_rates_in_place<<<grid, block, 0, s>>>(img, L, b);
+        break;
+      }
       const dim3 g = split(L.N, 1, per);
       strict::k_spec_rates<<<g, block, 0, s>>>(img, L, b, per);
       break;
