@@ -107,8 +107,8 @@ def fp64_slots(tables, precision, exp_slots):
     precision "fixed": what the state tiles of CRS_MODE_FP64 keep in FP64
         beside 64-bit fixed point: the two sums of the mass fractions, one
         FMA per third-body efficiency, two multiplies per three-body
-        reaction and one addition per nonzero net stoichiometric
-        coefficient.
+        reaction, one subtraction (forward - reverse) per reversible reaction
+        and one addition per nonzero net stoichiometric coefficient.
     precision "mixed": only what the mixed state tiles (and the mixed
         one-state-per-thread kernel) keep in FP64: one subtraction (forward - reverse) per reversible
         reaction, one multiply per reaction with a pres_mod term, one FMA
@@ -140,6 +140,7 @@ def fp64_slots(tables, precision, exp_slots):
         thd = sum(1 for k in t["pm_kind"][: int(t["dims"][3])] if int(k) == 0)
         parts = {"mass_fraction_sums": 2.0 * int(t["dims"][0]),
                  "third_body": float(len(t["pm_eff_val"])) + 2.0 * thd,
+                 "net_rate": float(NREV),
                  "accumulation": float(nnz)}
     elif precision in ("mixed", "operand", "mixed_tile", "rates"):
         single = all(int(t["kc_ptr"][j + 1]) - int(t["kc_ptr"][j]) <= 1 for j in range(NREV))
