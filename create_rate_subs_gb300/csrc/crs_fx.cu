@@ -37,8 +37,8 @@
 // states of 561/2539 4.87 -> 1.64 ms; FP64 pipe 53%, integer multiply pipe
 // 43% busy.
 //
-// States outside the scheme (T outside (200, 6000] K, a density beyond 2^+-60, a mean
-// 1/W out of range, |Y| >= 2, a subnormal Y) and reactions outside it (non-
+// States outside the scheme (T outside (200, 6000] K, a density beyond 2^+-60, a
+// mean 1/W out of range, |Y| >= 2, a subnormal Y) and reactions outside it (non-
 // integer coefficients, PLOG, Chebyshev, coefficients beyond the bounds)
 // are evaluated lane by lane by the general FP64 arithmetic (finish).
 #include <cuda_runtime.h>
@@ -77,8 +77,7 @@ struct Dot {
   int64_t hh, mid;
   __device__ __forceinline__ explicit Dot(int64_t c0) : hh(c0), mid(1LL << 31) {}
   __device__ __forceinline__ void add(Dg c, Dg f) {
-    // (long sums of products fuse from the C expression: 33 instructions for
-    // six functions against 48 with the instruction spelt out)
+    // (a long sum of products, left to the compiler to fuse)
     hh += (int64_t)c.hi * f.hi;
     mid += (int64_t)c.hi * f.lo;
     mid += (int64_t)c.lo * f.hi;
@@ -134,21 +133,27 @@ __device__ __forceinline__ int64_t falloff(const int2 *__restrict__ c, int flags
   return even(f);
 }
 
-// Concentrations of one state from its mass fractions (slow_net).
-struct YConc {
+// Concentrations of one state: on chip, where a state outside the scheme may have
+// them in place of its exponents, or from its mass fractions.
+struct StateConc {
+  const double *conc;  // the state's column, or NULL
   const double *Y;
   int64_t ld;
   double rho, yN;
   const double *inv_mw;
   int N;
   __device__ double operator[](int k) const {
+    if (conc) return conc[k * 32];
     return (k == N - 1 ? yN : Y[(int64_t)k * ld]) * (rho * inv_mw[k]);
   }
 };
 
-// Stands in a rate's place until the general FP64 arithmetic has formed it:
-// the loops that form the others then hold no call.
-constexpr uint64_t LATER = 0x7ff8c5a1d3b70e29ull;
+// Stands in a rate's place until the general FP64 arithmetic has formed it, as
+// any NaN does (net_of): the loops that form the others then hold no call.
+constexpr uint64_t LATER = 0x7ff8000000000000ull;
+__device__ __forceinline__ bool is_later(double v) {
+  return (bits_of(v) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull;
+}
 
 // The normalised functions of T of one state into column `lane` of the
 // block; returns the temperature interval.  irr: T outside the scheme.
@@ -334,11 +339,14 @@ __device__ __noinline__ void prepare(const FxTab &f, const Args &g, const double
   }
 }
 
-// The warp's rates left to the general FP64 arithmetic (all: every one), for
-// the lane's state i.
+// Rates left to the general FP64 arithmetic: one state's (i), of the warp's
+// records (all: every one, else those marked; conc: its concentrations on chip).
+// SPREAD: of records first, first + step, ...; else of all, or none if step is 0.
+template <bool SPREAD>
 __device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const Batch &b,
                                     int stride, Ring<DP> plain, Ring<DO> other, int64_t i,
-                                    bool all, double rho, double yN, unsigned char *q) {
+                                    bool all, const double *conc, double rho, double yN,
+                                    unsigned char *q, int first, int step) {
   const Tab t = make_tab(g.img, lay);
   fast::State s;
   s.T = b.T[i];
@@ -351,18 +359,57 @@ __device__ __noinline__ void finish(const Args &g, const ImgLayout &lay, const B
   kc.T = s.T;
   kc.logT = s.logT;
   kc.invT = s.invT;
-  const YConc C{b.Y + i, b.ld, rho, yN, t.inv_mw, t.N};
+  const StateConc C{conc, b.Y + i, b.ld, rho, yN, t.inv_mw, t.N};
+  const int n = SPREAD || step ? 2 * plain.n + other.n : 0;
 #pragma unroll 1
-  for (int p = 0; p < 2 * plain.n + other.n; ++p) {
+  for (int p = SPREAD ? first : 0; p < n; p += SPREAD ? step : 1) {
     const int o = p - 2 * plain.n;
     const int4 h = __ldg(reinterpret_cast<const int4 *>(
         o < 0 ? plain.src + (int64_t)p * stride : other.src + (int64_t)o * other.stride));
     double *v = reinterpret_cast<double *>(q + h.x);
     double fwd, rev, pm;
-    if (h.w >= 0 && (all || bits_of(*v) == LATER))
+    if (h.w >= 0 && (all || is_later(*v)))
       *v = fast::rxn_net(t, h.w, s, s.P * s.invT * fast::INV_RU, C, kc, fwd, rev, pm);
   }
 }
+
+// FP64 concentrations in place of the exponents, for a lane whose state i is
+// outside the scheme (o: its column of the block).
+__device__ __noinline__ void concentrations(const Batch &b, const double *inv_mw, int64_t i, int N,
+                                            int warp, int nw, const unsigned char *o,
+                                            unsigned char *yl) {
+  const double yN = *reinterpret_cast<const double *>(o + 7 * 256);
+  const double rho = *reinterpret_cast<const double *>(o + 8 * 256);
+#pragma unroll 1
+  for (int k = warp; k < N; k += nw)
+    *reinterpret_cast<double *>(yl + k * 256) =
+        (k == N - 1 ? yN : b.Y[(int64_t)k * b.ld + i]) * (rho * inv_mw[k]);
+}
+
+// A warp's lists, entry 0..6: its first plain record and the next warp's, its
+// first other record and the next warp's, its first species and the next warp's,
+// its first group of terms.  ON_CHIP: in shared memory, the registers being short.
+template <bool ON_CHIP>
+struct Lists {
+  int *chip;
+  int reg[7];
+  __device__ __forceinline__ Lists(const FxTab &f, const unsigned char *tab, int list, int gw,
+                                   int *chip_, int lane)
+      : chip(chip_) {
+    const int at[7] = {f.list_ptr[list][0], f.list_ptr[list][0], f.list_ptr[list][1],
+                       f.list_ptr[list][1], f.seg_ptr[list],     f.seg_ptr[list],
+                       f.term_ptr[list]};
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      if (!ON_CHIP)
+        reg[k] = reinterpret_cast<const int *>(tab + at[k])[gw + (k & 1)];
+      else if (lane == k)
+        chip[k] = reinterpret_cast<const int *>(tab + at[k])[gw + (k & 1)];
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ int operator[](int k) const { return ON_CHIP ? chip[k] : reg[k]; }
+};
 
 // Barrier of the CTAs that share a tile.
 template <int CL>
@@ -390,7 +437,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   const unsigned char *tab = g.tab;
   // shared memory: [N + 1][32] y, then the exponents of C (row N: zeros);
   // two blocks of per-state values; the small tables; each warp's ring of
-  // records; the net rates
+  // records; the warps' lists; the net rates
   unsigned char *yl = smem + lane * 8;
   unsigned char *next = smem + (N + 1) * 256;
   unsigned char *blk0 = next + lane * 8;
@@ -407,6 +454,17 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   const int rb = ring_bytes(f);
   unsigned char *ring = next + warp * rb;
   next += NW * rb;
+  // How rates are left to the general arithmetic.  SPREAD: the lanes may share
+  // them (see there), with the lists on chip to have the registers.  OUTS: whole
+  // tiles outside the scheme go there at once, and such states' concentrations are
+  // on chip.  Both cost the loops registers: with 24 warps none is missed (65,536
+  // states of 561/2539 3.68 ms either way; one state in 97 outside, 8,192 states:
+  // 2.85 -> 0.81 ms), with 8 OUTS takes 1% (2^18 states of 53/325 1.61 -> 1.63 ms;
+  // all outside: 10.1 -> 7.9) and SPREAD 4%, and with 16, for few tiles, where
+  // latency counts, both would take 4% (4,000 states 45.3 -> 47.2 us).
+  constexpr bool SPREAD = NW == 24, OUTS = NW != 16;
+  int *chip = reinterpret_cast<int *>(next) + warp * 8;
+  if (SPREAD) next += NW * 32;
   unsigned char *q = (QS && CL > 1 ? static_cast<unsigned char *>(__cluster_map_shared_rank(next, 0))
                       : QS ? next : reinterpret_cast<unsigned char *>(g.q) +
                                       (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256) + lane * 8;
@@ -417,21 +475,24 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     if (!QS || CL == 1) Q(f.R * 256) = 0.0;
     else reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
   }
-  Ring<DP> plain_ring;
-  Ring<DO> other_ring;
   const int gw = CL == 1 ? warp : (int)(blockIdx.x % CL) * NW + warp;  // the tile's warp
-  {
-    const int *lp = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][0]) + gw;
-    const int *lo = reinterpret_cast<const int *>(tab + f.list_ptr[LIST][1]) + gw;
-    plain_ring = Ring<DP>{tab + f.rec[LIST][0] + (int64_t)lp[0] * f.stride[0], smem_u32(ring),
-                          f.stride[0], lp[1] - lp[0], lane};
-    other_ring = Ring<DO>{tab + f.rec[LIST][1] + (int64_t)lo[0] * f.stride[1], smem_u32(ring),
-                          f.stride[1], lo[1] - lo[0], lane};
-  }
-  const int s0 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw];
-  const int s1 = reinterpret_cast<const int *>(tab + f.seg_ptr[LIST])[gw + 1];
-  const int4 *terms = reinterpret_cast<const int4 *>(tab + f.term[LIST]) +
-                      reinterpret_cast<const int *>(tab + f.term_ptr[LIST])[gw];
+  const Lists<SPREAD> lists(f, tab, LIST, gw, chip, lane);
+  auto plain_of = [&] {
+    return Ring<DP>{tab + f.rec[LIST][0] + (int64_t)lists[0] * f.stride[0], smem_u32(ring),
+                    f.stride[0], lists[1] - lists[0], lane};
+  };
+  auto other_of = [&] {
+    return Ring<DO>{tab + f.rec[LIST][1] + (int64_t)lists[2] * f.stride[1], smem_u32(ring),
+                    f.stride[1], lists[3] - lists[2], lane};
+  };
+  auto terms_of = [&] {
+    return reinterpret_cast<const int4 *>(tab + f.term[LIST]) + lists[6];
+  };
+  const Ring<DP> plain_kept = plain_of();
+  const Ring<DO> other_kept = other_of();
+  const int4 *terms_kept = terms_of();
+  auto plain_list = [&] { return SPREAD ? plain_of() : plain_kept; };
+  auto other_list = [&] { return SPREAD ? other_of() : other_kept; };
   const unsigned yrows = smem_u32(smem) + lane * 8;
   const double *inv_mw = reinterpret_cast<const double *>(g.img + lay.inv_mw);
   int bad = 0, bk = 0;
@@ -512,7 +573,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
       Yl(k * 256) = l;
     }
     if (odd) marks[32] = 1;
-    plain_ring.start();
+    plain_list().start();
     __syncthreads();
     // net rates
     {
@@ -522,8 +583,14 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
                 blk0 + (bk ^ 1) * ROWS * 256);
       }
       const int iv = marks[0] < 0 ? 0 : marks[0];
-      // states outside the scheme: every rate in FP64; later: single rates
-      bool later = false, all = marks[0] < 0 || marks[32];
+      // states outside the scheme: every rate in FP64, from concentrations in
+      // place of their exponents; later: single rates
+      const bool out = marks[0] < 0 || marks[32];
+      bool later = false;
+      if (OUTS && __any_sync(0xffffffffu, out)) {  // (the tile's marks: for all warps)
+        if (out) concentrations(b, inv_mw, ic, N, warp, NW, o, yl);
+        __syncthreads();
+      }
       Basis B;
       B.L = dg(*reinterpret_cast<const int2 *>(o));
       B.I = dg(*reinterpret_cast<const int2 *>(o + 256));
@@ -543,12 +610,14 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         }
         return Rec{at, at + co + COEF * idx};
       };
-      // two reactions at a time: independent chains side by side
       const int one = f.stride[0] / 2;
+      const bool skip = OUTS && __all_sync(0xffffffffu, out);  // a whole tile outside
+      // two reactions at a time: independent chains side by side
+      const Ring<DP> plain = plain_list();
       unsigned char *at = ring;
 #pragma unroll 1
-      for (int p = 0; p < plain_ring.n; ++p) {
-        plain_ring.next(p);
+      for (int p = skip ? plain.n : 0; p < plain.n; ++p) {
+        plain.next(p);
         int64_t yf[2], yr[2];
         int slot[2];
 #pragma unroll
@@ -570,15 +639,16 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         const double v1 = net_of<true>(yf[1], yr[1], et, far[1]);
         Q(slot[0]) = v0;
         Q(slot[1]) = v1;
-        all |= far[0] | far[1];
+        later |= far[0] | far[1];
         at = at == ring + 2 * f.stride[0] ? ring : at + f.stride[0];
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncwarp();
-      other_ring.start();
+      const Ring<DO> other = other_list();
+      other.start();
 #pragma unroll 1
-      for (int p = 0; p < other_ring.n; ++p) {
-        other_ring.next(p);
+      for (int p = skip ? other.n : 0; p < other.n; ++p) {
+        other.next(p);
         const Rec r = record(ring + (p % DO) * f.stride[1], HEAD + PMH + PMC * NI);
         const int4 h = r.word4(0), x = r.word4(16), ph = r.word4(HEAD);
         bool slow = h.y & RF_GEN;
@@ -610,10 +680,40 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
         Q(h.x) = slow ? of_bits(LATER) : v * thd;
         later |= slow;
       }
-      if (later || all)
-        finish(g, lay, b, one, plain_ring, other_ring, ic, all, rowd(8), rowd(7), q);
+      // What is left: lane = state or, for few states, lane = reaction, state by
+      // state, in as many turns as there are records for 32 lanes, each with the
+      // code of several kinds of reactions (2.5 times one's).
+      if (SPREAD) {
+        if (unsigned need = __ballot_sync(0xffffffffu, later || out)) {
+          const Ring<DP> plain = plain_list();
+          const Ring<DO> other = other_list();
+          const int n = 2 * plain.n + other.n;
+          const bool spread = 5 * __popc(need) * ((n + 31) / 32) < 2 * n;
+          if (!spread) need = 1u;
+          __syncwarp();  // the marks of the other lanes
+          do {
+            const int src = spread ? __ffs(need) - 1 : lane, off = (src - lane) * 8;
+            const bool all = __shfl_sync(0xffffffffu, (int)out, src);
+            const int64_t is = __shfl_sync(0xffffffffu, ic, src);
+            const double rho = __shfl_sync(0xffffffffu, rowd(8), src);
+            const double yN = __shfl_sync(0xffffffffu, rowd(7), src);
+            if (spread || later || out)
+              finish<true>(g, lay, b, one, plain, other, is, all,
+                           all ? reinterpret_cast<double *>(yl + off) : nullptr, rho, yN, q + off,
+                           spread ? lane : 0, spread ? 32 : 1);
+            __syncwarp();
+            need &= need - 1;
+          } while (need);
+        }
+      } else if (__any_sync(0xffffffffu, later || out)) {
+        finish<false>(g, lay, b, one, plain_kept, other_kept, ic, out,
+                      OUTS && out ? reinterpret_cast<double *>(yl) : nullptr, rowd(8), rowd(7), q,
+                      0, later || out);
+      }
     }
     // the first terms are on their way before the barrier
+    const int s0 = lists[4], s1 = lists[5];
+    const int4 *terms = SPREAD ? terms_of() : terms_kept;
     const int4 t0 = __ldg(terms), t1 = __ldg(terms + 1);
     const int4 sg0 = __ldg(reinterpret_cast<const int4 *>(tab + f.seg[LIST]) + s0);
     tile_barrier<CL>();
@@ -675,8 +775,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
 
 // Shared memory of a CTA of nw warps.
 size_t smem_of(const FxTab &f, int nw, bool qs, bool ts) {
-  return (size_t)(f.N + 1 + 2 * ROWS) * 256 + (ts ? TAB_BYTES : 0) + (size_t)nw * ring_bytes(f) +
-         (qs ? (size_t)(f.R + 1) * 256 : 0);
+  return (size_t)(f.N + 1 + 2 * ROWS) * 256 + (ts ? TAB_BYTES : 0) +
+         (size_t)nw * (ring_bytes(f) + 32) + (qs ? (size_t)(f.R + 1) * 256 : 0);
 }
 
 // How a launch over `tiles` tiles runs: warps per CTA, CTAs per SM and per

@@ -115,9 +115,7 @@ FX_FN Dg split(int64_t v) {
   return Dg{(int)(v >> 32) + (int)((unsigned)lo >> 31), lo};
 }
 
-// a b + c as one instruction; of the C expression the compiler makes a
-// product and a 64-bit sum where the sums are short (8 instructions a mul
-// against 12)
+// a b + c as one instruction, spelt out where the sums are short
 FX_FN int64_t mad(int a, int b, int64_t c) {
 #if defined(__CUDA_ARCH__)
   int64_t d;
@@ -323,7 +321,7 @@ FX_FN double value_of(int64_t y, const int64_t *tab) {
 
 // The value of one exponent as a normal double by integer operations; zero
 // far below the normal range.  far: overflow or gradual underflow, which
-// value_of has to form.
+// value_of has to form: NaN.
 FX_FN double normal_of(int64_t y, const int64_t *tab, bool &far) {
   uint64_t M;
   int E;
@@ -333,12 +331,12 @@ FX_FN double normal_of(int64_t y, const int64_t *tab, bool &far) {
   far = !in && E > NORMAL_MIN;
   const unsigned lo = (unsigned)(M >> 4);
   const unsigned hi = ((unsigned)(M >> 36) + (e << 20)) ^ ((unsigned)y << 31);
-  return of_bits((uint64_t)(in ? hi : 0u) << 32 | (in ? lo : 0u));
+  return of_bits((uint64_t)(in ? hi : far ? 0x7ff80000u : 0u) << 32 | (in ? lo : 0u));
 }
 
 // +-2^yf -+ 2^yr (bit 0 of each exponent: its sign).  REV false: the first
-// term alone.  special: a term lies outside the normal range and net_special
-// has to form the result; the code has no branch.
+// term alone.  special: a term lies outside the normal range, the result is NaN
+// and net_special has to form it; the code has no branch.
 template <bool REV>
 FX_FN double net_of(int64_t yf, int64_t yr, const int64_t *tab, bool &special) {
   const double f = normal_of(yf, tab, special);
