@@ -5,6 +5,9 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
+#include <queue>
+#include <utility>
 #include <vector>
 
 #include "../../include/crs_tables.h"
@@ -29,6 +32,7 @@ struct Form {
 // the coefficients use the half width that these integers realise.
 struct Norm {
   ld mT, hT, mL, hL, mI, hI;
+  ld pw[5][5];  // T^d = sum_k pw[d][k] t^k
   int64_t word[BASIS];
 };
 
@@ -50,6 +54,10 @@ Norm norm_of(double a, double b) {
   normalise(a, b, 49, &n.mT, &n.hT, n.word);
   normalise(std::log2((ld)a), std::log2((ld)b), 58, &n.mL, &n.hL, n.word + 3);
   normalise(1 / (ld)b, 1 / (ld)a, 68, &n.mI, &n.hI, n.word + 6);
+  static const int binom[5][5] = {{1}, {1, 1}, {1, 2, 1}, {1, 3, 3, 1}, {1, 4, 6, 4, 1}};
+  for (int d = 0; d <= 4; ++d)
+    for (int k = 0; k <= d; ++k)
+      n.pw[d][k] = binom[d][k] * std::pow(n.mT, (ld)(d - k)) * std::pow(n.hT, (ld)k);
   return n;
 }
 
@@ -83,12 +91,8 @@ Form form_of(const Norm &n, ld base, ld b, ld i, const ld *p) {
   f.c[1] = b * n.hL;
   f.c[2] = i * n.hI;
   if (p) {
-    static const int binom[5][5] = {{1}, {1, 1}, {1, 2, 1}, {1, 3, 3, 1}, {1, 4, 6, 4, 1}};
     for (int k = 0; k <= 4; ++k)
-      for (int d = k > 1 ? k : 1; d <= 4; ++d) {
-        const ld v = p[d - 1] * binom[d][k] * std::pow(n.mT, (ld)(d - k)) * std::pow(n.hT, (ld)k);
-        f.c[k == 0 ? 0 : 2 + k] += v;
-      }
+      for (int d = k > 1 ? k : 1; d <= 4; ++d) f.c[k == 0 ? 0 : 2 + k] += p[d - 1] * n.pw[d][k];
   }
   return f;
 }
@@ -118,12 +122,22 @@ int64_t number(int64_t v) {
 
 struct Buf {
   std::vector<unsigned char> b;
+  // a section: its offset; what is added until the next one belongs to it
+  int begin() {
+    b.resize((b.size() + 127) / 128 * 128);
+    return (int)b.size();
+  }
+  void add(const void *p, size_t n) {
+    const unsigned char *c = static_cast<const unsigned char *>(p);
+    b.insert(b.end(), c, c + n);
+  }
+  void end() { b.resize(b.size() + 16); }
   template <class T>
   int put(const std::vector<T> &v) {
-    const size_t off = (b.size() + 127) / 128 * 128;
-    b.resize(off + v.size() * sizeof(T) + 16);
-    if (!v.empty()) memcpy(b.data() + off, v.data(), v.size() * sizeof(T));
-    return (int)off;
+    const int off = begin();
+    add(v.data(), v.size() * sizeof(T));
+    end();
+    return off;
   }
 };
 
@@ -145,17 +159,29 @@ bool term(const Norm &n, ld a, ld x, bool inv, int64_t *w, int *flags, int bit) 
   return true;
 }
 
-// Lists of items for as many warps as `load` has entries (what they carry
-// already): longest first onto the least loaded.
-std::vector<std::vector<int>> deal(const std::vector<int> &w, std::vector<long long> load) {
+// Items by weight, the heaviest first.
+std::vector<int> by_weight(const std::vector<int> &w) {
   std::vector<int> order(w.size());
   for (size_t i = 0; i < w.size(); ++i) order[i] = (int)i;
   std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return w[a] > w[c]; });
+  return order;
+}
+
+// Lists of items for as many warps as `load` has entries (what they carry
+// already): in the order given, each onto the least loaded.
+std::vector<std::vector<int>> deal(const std::vector<int> &w, const std::vector<int> &order,
+                                   const std::vector<long long> &load) {
   std::vector<std::vector<int>> bins(load.size());
+  // the least loaded on top, the first of equal ones
+  typedef std::pair<long long, int> Load;
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+  for (size_t b = 0; b < load.size(); ++b) heap.push(Load(load[b], (int)b));
   for (int i : order) {
-    const int best = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-    bins[best].push_back(i);
-    load[best] += w[i];
+    Load l = heap.top();
+    heap.pop();
+    bins[l.second].push_back(i);
+    l.first += w[i];
+    heap.push(l);
   }
   return bins;
 }
@@ -279,17 +305,16 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
   Rec none = Rec();  // completes a pair: both rates zero, into the slot of zeros
   none.slot = R * 256;
   for (int q = 0; q < 6; ++q) none.fac[q] = (uint16_t)(N + 1);
+  const std::vector<int> order = by_weight(weight);
   for (int l = 0; l < NLIST; ++l) {
     const int nw = list_warps[l];
     std::vector<long long> load(nw, 0);
     load[0] = load[1] = 2 * N;  // the next tile's sums and functions of T
     load[2] = 20;
     std::vector<int32_t> ptr(1, 0), pairs;
-    std::vector<unsigned char> lr;
-    auto add = [&](const void *v, size_t n) {
-      lr.insert(lr.end(), (const unsigned char *)v, (const unsigned char *)v + n);
-    };
-    for (const auto &v : deal(weight, load)) {
+    f.mrec[l] = b.begin();
+    auto count = [&] { return (int32_t)((b.b.size() - f.mrec[l]) / MPAIR); };
+    for (const auto &v : deal(weight, order, load)) {
       for (int c = 0; c < 4; ++c) {
         std::vector<Rec> two;
         for (int r : v)
@@ -297,17 +322,17 @@ void build_mixed(const Tab &t, FxTab &f, Buf &b) {
         if (two.size() & 1) two.push_back(none);
         for (size_t q = 0; q < two.size(); q += 2)
           two[q].slot |= (c & 1 ? MF_MORE : 0) | (c < 2 ? MF_REV : 0);
-        if (!two.empty()) add(two.data(), two.size() * MREC);
+        b.add(two.data(), two.size() * MREC);
       }
-      pairs.push_back((int32_t)(lr.size() / MPAIR) - ptr.back());
+      pairs.push_back(count() - ptr.back());
       for (int c = 4; c < 8; ++c)
         for (int r : v)
-          if (kind[r] == c) add(&rec[r], MPAIR);
-      ptr.push_back((int32_t)(lr.size() / MPAIR));
+          if (kind[r] == c) b.add(&rec[r], MPAIR);
+      ptr.push_back(count());
     }
+    b.end();
     f.mlist_ptr[l] = b.put(ptr);
     f.mpairs[l] = b.put(pairs);
-    f.mrec[l] = b.put(lr);
   }
 }
 
@@ -329,6 +354,22 @@ int64_t bytes_bound(const Tab &t, int64_t one) {
   }
   return all;
 }
+
+// The tables that are the same for every mechanism, made once: 1,300
+// exponentials and logarithms in extended precision.
+struct Small {
+  std::vector<int64_t> small, hp;
+  Small() : small(EXP_WORDS + 2 * (LOGN + 1)), hp(2 * (LOGN + 1)) {
+    for (int k = 0; k <= EXPN; ++k)
+      small[k] = llroundl(std::ldexp(std::exp2((ld)k / EXPN), 56)) + 8;
+    for (int k = 0; k <= LOGN; ++k) {
+      const ld F = 1 + (ld)k / LOGN;
+      small[EXP_WORDS + 2 * k] = hp[2 * k] = llroundl(std::ldexp((ld)1, 62) / F);
+      small[EXP_WORDS + 2 * k + 1] = llroundl(std::ldexp(std::log2(F), YB));
+      hp[2 * k + 1] = llroundl(std::ldexp(std::log2(F), 62));
+    }
+  }
+};
 
 }  // namespace
 
@@ -545,18 +586,12 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
   f.usable = generic * 5 <= R;
   for (int k = 0; k < N; ++k) f.usable &= std::fabs(std::log2(t.inv_mw[k])) <= W_MAX;
   Buf b;
-  std::vector<int64_t> small(EXP_WORDS + 2 * (LOGN + 1)), hp(2 * (LOGN + 1)), lw(N);
-  for (int k = 0; k <= EXPN; ++k)
-    small[k] = llroundl(std::ldexp(std::exp2((ld)k / EXPN), 56)) + 8;
-  for (int k = 0; k <= LOGN; ++k) {
-    const ld F = 1 + (ld)k / LOGN;
-    small[EXP_WORDS + 2 * k] = hp[2 * k] = llroundl(std::ldexp((ld)1, 62) / F);
-    small[EXP_WORDS + 2 * k + 1] = llroundl(std::ldexp(std::log2(F), YB));
-    hp[2 * k + 1] = llroundl(std::ldexp(std::log2(F), 62));
-  }
+  b.b.reserve((size_t)bytes_bound(t, one));
+  static const Small constants;
+  std::vector<int64_t> lw(N);
   for (int k = 0; k < N; ++k) lw[k] = llroundl(std::ldexp(std::log2((ld)t.inv_mw[k]), YB));
-  f.small = b.put(small);
-  f.hp = b.put(hp);
+  f.small = b.put(constants.small);
+  f.hp = b.put(constants.hp);
   f.basis = b.put(basis);
   f.lw = b.put(lw);
   f.pm = b.put(pm);
@@ -605,6 +640,7 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
     }
   }
   // work lists
+  const std::vector<int> order = by_weight(weight), species_order = by_weight(sw);
   for (int l = 0; l < NLIST; ++l) {
     const int nw = list_warps[l];
     // warps 0 and 1 also form the next tile's sums (chains of N dependent
@@ -612,10 +648,10 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
     std::vector<long long> load(nw, 0);
     load[0] = load[1] = 2 * N;
     load[2] = 60;
-    std::vector<std::vector<int>> bins = deal(weight, load);
+    std::vector<std::vector<int>> bins = deal(weight, order, load);
     for (int c = 0; c < 2; ++c) {
       std::vector<int32_t> ptr(1, 0);
-      std::vector<unsigned char> lr;
+      f.rec[l][c] = b.begin();
       for (auto &v : bins) {
         std::sort(v.begin(), v.end(), [&](int x, int y) {
           return kind[x] != kind[y] ? kind[x] < kind[y] : x < y;
@@ -623,19 +659,19 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
         int n = 0;
         for (int r : v)
           if ((kind[r] != 0) == (c == 1)) {
-            lr.insert(lr.end(), rec[r].begin(), rec[r].end());
+            b.add(rec[r].data(), rec[r].size());
             ++n;
           }
         if (c == 0) {
-          if (n & 1) lr.insert(lr.end(), nothing.begin(), nothing.end());
+          if (n & 1) b.add(nothing.data(), nothing.size());
           n = (n + 1) / 2;
         }
         ptr.push_back(ptr.back() + n);
       }
+      b.end();
       f.list_ptr[l][c] = b.put(ptr);
-      f.rec[l][c] = b.put(lr);
     }
-    bins = deal(sw, std::vector<long long>(nw, 0));
+    bins = deal(sw, species_order, std::vector<long long>(nw, 0));
     std::vector<int32_t> ptr(1, 0), tptr(1, 0), seg, term;
     for (auto &v : bins) {
       std::stable_sort(v.begin(), v.end(), [&](int x, int y) {
