@@ -54,8 +54,8 @@ __device__ __forceinline__ double exp_t(double x, const double *tab) {
 // log1p by its degree-6 Taylor polynomial (truncation below 2^-58).  The
 // table holds 1/F and log F for j = 0..128 (tab[2j], tab[2j+1]); e ln2 is
 // split so that e times its head is exact.  Error about 1 ulp; 12 FP64
-// instructions against roughly 30 for CUDA's log.  Zero, negative,
-// subnormal, infinite and NaN arguments go to CUDA's log.
+// operations.  Zero, negative, subnormal, infinite and NaN arguments go to
+// CUDA's log.
 constexpr double LN2_HI = 0x1.62e42fefa3800p-1;  // ln 2 to 42 bits
 constexpr double LN2_LO = 0x1.ef35793c76730p-45; // ln 2 - LN2_HI
 constexpr int LOG_TAB_ENTRIES = 129;

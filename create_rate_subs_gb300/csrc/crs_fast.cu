@@ -9,7 +9,8 @@
 //  * evaluates exp with a table-driven method (Tang, ACM TOMS 15(2), 1989:
 //    x = (256 k + j) ln2/256 + r, exp(x) = 2^k 2^(j/256) p(r), |r| <=
 //    ln2/512, p the degree-4 Taylor polynomial; error below 1 ulp plus the
-//    table rounding) -- 9 FP64 instructions instead of ~19 for CUDA's exp;
+//    table rounding) -- 9 FP64 operations, at the rates that crs_probe
+//    measures in a run cheaper than CUDA's exp;
 //  * multiplies by 1/T (one division per state) instead of dividing;
 //  * forms the equilibrium constant from per-species Gibbs terms
 //    S_k = s_k/R - h_k/RT - ln T evaluated once per state (the reference

@@ -145,10 +145,11 @@ __global__ void k_conc(const unsigned char *__restrict__ img, ImgLayout L,
 
 // Exponentials and divisions by T of the two kernels of reactions, whose
 // bound they are: the table exponential (error below 1 ulp, 9 FP64
-// instructions), and a / T from T's correctly rounded reciprocal by two
-// fused multiply-adds (Markstein, IBM J. Res. Dev. 34 (1990): the correctly
-// rounded quotient), three instead of a division's ten.  Outside the range
-// where the latter holds the division stands.
+// operations), and a / T from T's correctly rounded reciprocal by a product and
+// two fused multiply-adds (Markstein, IBM J. Res. Dev. 34 (1990): the correctly
+// rounded quotient).  Outside the range where the latter holds the division
+// stands.  With both the four functions of 20,000 states of 53/325 took 1.75 ->
+// 1.38 ms.
 struct FastMath {
   const double *tab;
   double y;  // 1 / T
