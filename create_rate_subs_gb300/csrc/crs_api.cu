@@ -59,25 +59,27 @@ cudaError_t launch_spec_sum(const unsigned char *img, const ImgLayout &L, const 
 cudaError_t launch_pack_bf16(const double *q, int64_t ldq, int64_t n, int R, int Kh,
                              const int *escale, void *A, int64_t lda, unsigned *outflag,
                              int sm_count, cudaStream_t s);
-// FP64 state tiles in fixed point (crs_fx.cu): scratch bytes of a launch (0:
-// none, < 0: the mechanism does not fit) and the launch.
+// FP64 state tiles in fixed point (crs_fx.cu): whether a launch needs scratch (<
+// 0: the mechanism does not fit), the resources of those that do, the launch.
 cudaError_t fx_init(int smem_optin);
-long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+int fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+cudaError_t fx_slots(const fx::FxTab &f, int sm_count, int smem_optin, SlotUse &u);
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                            const unsigned char *tab, const Batch &b, int sm_count,
-                           int smem_optin, double *scratch, cudaStream_t s);
+                           int smem_optin, const TileScratch &scratch, cudaStream_t s);
 // Mixed precision by state tiles (crs_mixed_tile.cu), likewise.
 cudaError_t mixed_tile_init(int smem_optin);
-long long mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+int mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+cudaError_t mixed_tile_slots(const fx::FxTab &f, int sm_count, int smem_optin, SlotUse &u);
 cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                               const unsigned char *tab, const Batch &b, int sm_count,
-                              int smem_optin, double *scratch, cudaStream_t s);
+                              int smem_optin, const TileScratch &scratch, cudaStream_t s);
 // The contraction's operand by the same tiles.
-long long mixed_pack_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin);
+bool mixed_pack_fits(const fx::FxTab &f, int smem_optin);
 cudaError_t launch_mixed_pack(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                               const unsigned char *tab, const Batch &b, int sm_count,
-                              int smem_optin, double *scratch, void *A, int Kh, int *escale,
-                              cudaStream_t s);
+                              int smem_optin, const TileScratch &scratch, void *A, int Kh,
+                              int *escale, cudaStream_t s);
 // Tables the fast kernels derive from the blob's tables at load time.
 bool build_fast_tables(const std::vector<unsigned char> &img,
                        const ImgLayout &L, std::vector<Derived> &extra);
@@ -142,9 +144,10 @@ struct crs_mech {
   // producer): FP64 net rates of one chunk of states [R][q_rows]
   double *d_q = nullptr;
   int64_t q_rows = 0;
-  // state tiles: net rates of one tile per resident CTA
-  double *d_tile = nullptr;
-  size_t tile_bytes = 0;
+  // state tiles: net rates of one tile per CTA that can be resident (the slots'
+  // words at load, the blocks on first use)
+  std::mutex tile_mu;
+  crs::TileScratch tile;
   // recorded after the last kernel that used the workspaces, waited on by
   // the next call's stream: calls on several streams take turns on the GPU
   cudaEvent_t ws_done = nullptr;
@@ -676,78 +679,75 @@ cudaError_t make_pool(int device, cudaMemPool_t *pool) {
   return e;
 }
 
-// Scratch of the state tiles for the launches that follow on stream s (caller
-// holds ws_mu and ends with tile_scratch_end): the handle's buffer, whose users
-// take turns, of the most that any launch needs, so that it stays where it is
-// and in L2 (blocks of a pool, a new one for each call: 20,011 states of
-// 561/2539 1.28 -> 1.65 ms); while the stream is captured, a block of the pool
-// that becomes a node of the graph.  *q = NULL when there is no memory.
-int tile_scratch_begin(crs_mech *m, size_t bytes, cudaStream_t s, double **q, bool *node) {
-  *q = nullptr;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &cs);
-  if (e != cudaSuccess) return cuda_fail(e, "scratch");
-  *node = cs != cudaStreamCaptureStatusNone;
-  if (*node) {
-    e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(q), bytes, m->fx_pool, s);
-    if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return cuda_fail(e, "scratch");
-    if (e != cudaSuccess) cudaGetLastError();
-    return CRS_OK;
-  }
-  if (m->tile_bytes < bytes) {
-    if (m->d_tile) cudaFree(m->d_tile);
-    m->d_tile = nullptr;
-    m->tile_bytes = 0;
-    e = cudaMalloc(&m->d_tile, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      return CRS_OK;
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "scratch");
-    m->tile_bytes = bytes;
-  }
-  const int rc = ensure_q(m, 0, false, false);  // the event
-  if (rc != CRS_OK) return rc;
-  *q = m->d_tile;
-  return ws_begin(m, s);
+// As many slots as CTAs that hold one can be resident at a time, by any of the
+// SM's resources.
+cudaError_t make_slots(crs_mech *m) {
+  crs::SlotUse u;
+  int smem = 0, regs = 0, threads = 0, reserved = 0;
+  cudaError_t e = crs::fx_slots(m->fx, m->sm_count, m->smem_optin, u);
+  if (e == cudaSuccess) e = crs::mixed_tile_slots(m->fx, m->sm_count, m->smem_optin, u);
+  auto get = [&](int *v, cudaDeviceAttr a) {
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(v, a, m->device);
+  };
+  get(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor);
+  get(&reserved, cudaDevAttrReservedSharedMemoryPerBlock);
+  get(&regs, cudaDevAttrMaxRegistersPerMultiprocessor);
+  get(&threads, cudaDevAttrMaxThreadsPerMultiProcessor);
+  if (e != cudaSuccess || u.threads > threads) return e;  // (no launch needs one)
+  const long long per_sm = std::min<long long>(
+      {(long long)(smem / (u.smem + reserved)), regs / u.regs, threads / u.threads});
+  m->tile.slots = m->sm_count * (int)std::max<long long>(per_sm, 1);
+  e = cudaMalloc(&m->tile.busy, m->tile.slots * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(m->tile.busy, 0, m->tile.slots * sizeof(int));
+  return e;
 }
 
-int tile_scratch_end(crs_mech *m, double *q, bool node, cudaStream_t s) {
-  if (!node) return ws_end(m, s);
-  const cudaError_t e = cudaFreeAsync(q, s);
-  return e == cudaSuccess ? CRS_OK : cuda_fail(e, "scratch");
+// Allocations while this thread's or another's capture forbids them by default:
+// none of this thread's calls enters the capture meanwhile.
+struct Unchecked {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  Unchecked() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~Unchecked() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Scratch of the state tiles, made on first use and kept, for launches on any
+// streams at the same time, captured ones among them.  q = NULL when there is
+// no memory.
+int tile_scratch(crs_mech *m, crs::TileScratch &t) {
+  std::lock_guard<std::mutex> lk(m->tile_mu);
+  if (!m->tile.q && m->tile.slots > 0) {
+    const Unchecked unchecked;
+    const cudaError_t e =
+        cudaMalloc(&m->tile.q, (size_t)(m->tile.slots + 1) * (m->L.R + 1) * 32 * sizeof(double));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      m->tile.q = nullptr;
+    } else if (e != cudaSuccess) {
+      return cuda_fail(e, "scratch");
+    }
+  }
+  t = m->tile;
+  return CRS_OK;
 }
 
 // CRS_MODE_FP64 and CRS_MODE_MIXED by state tiles, when the mechanism fits
 // (and no intermediates are asked for); *taken = false otherwise.  Net rates
 // that do not fit on chip (at most one tile's per resident CTA) get scratch.
 int wdot_tiles(crs_mech *m, const crs::Batch &b, bool mixed, cudaStream_t s, bool *taken) {
-  auto scratch_of = [&](int64_t n) {
-    return mixed ? crs::mixed_tile_scratch(m->fx, n, m->sm_count, m->smem_optin)
-                 : crs::fx_scratch(m->fx, n, m->sm_count, m->smem_optin);
-  };
-  auto launch = [&](double *q) {
-    const cudaError_t e = (mixed ? crs::launch_mixed_tile : crs::launch_wdot_fx)(
-        m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, q, s);
-    return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
-  };
-  const long long scratch = scratch_of(b.n);
+  const int scratch = (mixed ? crs::mixed_tile_scratch : crs::fx_scratch)(
+      m->fx, b.n, m->sm_count, m->smem_optin);
   *taken = scratch >= 0 && !(b.conc || b.fwd || b.rev || b.pm);
   if (!*taken) return CRS_OK;
-  if (scratch == 0) return launch(nullptr);
-  std::lock_guard<std::mutex> lk(m->ws_mu);
-  double *q;
-  bool node;
-  const size_t most = (size_t)std::max(scratch, scratch_of((int64_t)1 << 40));
-  int rc = tile_scratch_begin(m, most, s, &q, &node);
-  if (rc != CRS_OK) return rc;
-  if (!q) {  // the kernels that need none
-    *taken = false;
-    return CRS_OK;
+  crs::TileScratch t;
+  if (scratch) {
+    const int rc = tile_scratch(m, t);
+    if (rc != CRS_OK) return rc;
+    *taken = t.q != nullptr;  // else the kernels that need none
+    if (!*taken) return CRS_OK;
   }
-  rc = launch(q);
-  const int rc2 = tile_scratch_end(m, q, node, s);
-  return rc != CRS_OK ? rc : rc2;
+  const cudaError_t e = (mixed ? crs::launch_mixed_tile : crs::launch_wdot_fx)(
+      m->d_img, m->L, m->fx, m->d_fx, b, m->sm_count, m->smem_optin, t, s);
+  return e == cudaSuccess ? CRS_OK : cuda_fail(e, "crs_wdot launch");
 }
 
 // CRS_MODE_GEMM: per chunk, the FP64 net rates (state tiles), their bf16
@@ -762,17 +762,11 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
   const int64_t K = 2 * (int64_t)m->Kh;
   const int64_t rows = q_chunk(m->L, b.n);
   // rates and packing in one kernel when the mechanism fits its tiles
-  const long long scratch = crs::mixed_pack_scratch(m->fx, rows, m->sm_count, m->smem_optin);
-  double *q = nullptr;
-  bool node = false;
-  if (scratch > 0) rc = tile_scratch_begin(m, (size_t)scratch, s, &q, &node);
-  if (rc != CRS_OK) return rc;
-  rc = ensure_q(m, rows, !q, true);
+  crs::TileScratch t;
+  if (crs::mixed_pack_fits(m->fx, m->smem_optin)) rc = tile_scratch(m, t);
+  if (rc == CRS_OK) rc = ensure_q(m, rows, !t.q, true);
   if (rc == CRS_OK) rc = ws_begin(m, s);
-  if (rc != CRS_OK) {
-    if (q) tile_scratch_end(m, q, node, s);
-    return rc;
-  }
+  if (rc != CRS_OK) return rc;
   for (int64_t c0 = 0; c0 < b.n && rc == CRS_OK; c0 += rows) {
     const int64_t cnt = std::min<int64_t>(rows, b.n - c0);
     crs::Batch bc = b;
@@ -782,9 +776,9 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
     bc.Y = b.Y + c0;
     bc.wdot = b.wdot + c0;
     cudaError_t e;
-    if (q) {
+    if (t.q) {
       e = crs::launch_mixed_pack(m->d_img, m->L, m->fx, m->d_fx, bc, m->sm_count, m->smem_optin,
-                                 q, m->d_ws, m->Kh, m->d_escale, s);
+                                 t, m->d_ws, m->Kh, m->d_escale, s);
     } else {
       e = crs::launch_rates_tile(m->d_img, m->L, bc, m->sm_count, m->smem_optin, s, m->d_q, rows,
                                  m->d_escale);
@@ -802,7 +796,6 @@ int wdot_gemm(crs_mech *m, const crs::Batch &b, cudaStream_t s) {
     if (e == cudaErrorNotSupported) rc = fail(CRS_ERR_UNSUPPORTED, "rates tile not available");
     else if (e != cudaSuccess) rc = cuda_fail(e, "gemm launch");
   }
-  if (q && node) cudaFreeAsync(q, s);
   const int rc2 = ws_end(m, s);
   return rc != CRS_OK ? rc : rc2;
 }
@@ -936,6 +929,7 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
     e = crs::fx_init(m->smem_optin);
     if (e == cudaSuccess) e = crs::mixed_tile_init(m->smem_optin);
     if (e == cudaSuccess) e = make_pool(m->device, &m->fx_pool);
+    if (e == cudaSuccess) e = make_slots(m);
     if (e != cudaSuccess) {
       int r = cuda_fail(e, "crs_mech_load");
       crs_mech_free(m);
@@ -1023,7 +1017,8 @@ int crs_mech_free(crs_mech *m) {
   if (m->d_escale) cudaFree(m->d_escale);
   if (m->d_outflag) cudaFree(m->d_outflag);
   if (m->d_q) cudaFree(m->d_q);
-  if (m->d_tile) cudaFree(m->d_tile);
+  if (m->tile.q) cudaFree(m->tile.q);
+  if (m->tile.busy) cudaFree(m->tile.busy);
   if (m->ws_done) cudaEventDestroy(m->ws_done);
   if (m->d_host) cudaFree(m->d_host);
   for (cudaStream_t st : m->hs)

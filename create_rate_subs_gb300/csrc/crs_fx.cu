@@ -186,7 +186,8 @@ __device__ __forceinline__ int basis_of(const FxTab &f, const unsigned char *tab
 struct Args {
   const unsigned char *tab;  // fixed-point tables
   const unsigned char *img;  // table image (general FP64 arithmetic)
-  double *q;                 // [gridDim.x / CL][R + 1][32] scratch when QS is false
+  double *q;                 // [slots][R + 1][32] scratch when QS is false
+  int *busy, slots;          // (tile::claim_slot)
   int list;                  // the work list for NW CL warps
 };
 
@@ -465,15 +466,16 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   constexpr bool SPREAD = NW == 24, OUTS = NW != 16;
   int *chip = reinterpret_cast<int *>(next) + warp * 8;
   if (SPREAD) next += NW * 32;
+  __shared__ int s_slot;
+  if (!QS && blockIdx.x % CL == 0 && threadIdx.x == 96)  // for the CTAs of the tile
+    s_slot = tile::claim_slot(g.busy, g.slots, blockIdx.x / CL, b.status);
   unsigned char *q = (QS && CL > 1 ? static_cast<unsigned char *>(__cluster_map_shared_rank(next, 0))
-                      : QS ? next : reinterpret_cast<unsigned char *>(g.q) +
-                                      (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256) + lane * 8;
+                                   : next) + lane * 8;  // (scratch: once there is a slot)
   auto Yl = [&](int off) -> int64_t & { return *reinterpret_cast<int64_t *>(yl + off); };
   auto Q = [&](int off) -> double & { return *reinterpret_cast<double *>(q + off); };
   if (warp == 0) {
     Yl(N * 256) = 0;
-    if (!QS || CL == 1) Q(f.R * 256) = 0.0;
-    else reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
+    if (QS) reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
   }
   const int gw = CL == 1 ? warp : (int)(blockIdx.x % CL) * NW + warp;  // the tile's warp
   const Lists<SPREAD> lists(f, tab, LIST, gw, chip, lane);
@@ -503,6 +505,13 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     const int64_t i = tile * 32 + lane < b.n ? tile * 32 + lane : tile * 32;
     load_y<NW>(b.Y + i, b.ld, N, warp, yrows);
     if (warp < 3) prepare(f, g, inv_mw, b, i, warp, lane, lt, blk0);
+  }
+  if (!QS) {  // (the claim ran beside the first tile's sums)
+    tile_barrier<CL>();
+    const int slot =
+        CL > 1 ? *static_cast<const int *>(__cluster_map_shared_rank(&s_slot, 0)) : s_slot;
+    q = reinterpret_cast<unsigned char *>(g.q) + (int64_t)slot * (f.R + 1) * 256 + lane * 8;
+    if (warp == 0) Q(f.R * 256) = 0.0;
   }
   for (; tile < ntiles; tile += step, bk ^= 1) {
     const int64_t i = tile * 32 + lane;
@@ -769,7 +778,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     }
     // rates are replaced only after the barrier at the loop's head
   }
-  if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here
+  if (!QS || CL > 1) tile_barrier<CL>();  // the tile's rates are read until here
+  if (!QS && blockIdx.x % CL == 0 && threadIdx.x == 0)
+    tile::release_slot(g.busy, g.slots, s_slot);
   if (bad && b.status) atomicAdd(&b.status[1], bad);
 }
 
@@ -859,29 +870,39 @@ static int64_t first_tiles(const fx::FxTab &f, int64_t tiles, int sm_count, int 
              : tiles - rest;
 }
 
-// Scratch bytes of a launch over n states (0: the net rates fit on chip);
+// Whether a launch over n states needs scratch (0: the net rates fit on chip);
 // < 0: the mechanism does not fit this kernel.
-long long fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
+int fx_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
   const int64_t tiles = (n + 31) / 32, first = first_tiles(f, tiles, sm_count, smem_optin);
-  long long most = 0;
+  int need = 0;
   for (int64_t part : {first, tiles - first}) {
     if (part == 0) continue;
     const fx::Plan p = fx::plan_of(f, part, sm_count, smem_optin);
     if (!p.ok) return -1;
-    if (p.qs) continue;
-    const long long need = (long long)std::min<int64_t>(part, (int64_t)sm_count * p.per_sm) *
-                           (f.R + 1) * 256;
-    most = std::max(most, need);
+    need |= !p.qs;
   }
-  return most;
+  return need;
+}
+
+// The resources of the launches that need scratch.
+cudaError_t fx_slots(const fx::FxTab &f, int sm_count, int smem_optin, SlotUse &u) {
+  cudaError_t e = cudaSuccess;
+  // every plan: few tiles, one per SM, more
+  for (int64_t tiles : {1, sm_count / 8 + 1, sm_count / 4 + 1, sm_count / 2 + 1, sm_count + 1}) {
+    const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
+    if (p.ok && !p.qs && e == cudaSuccess)
+      e = u.add(fx::kernel_of(p), p.nw * 32, fx::smem_of(f, p.nw, p.qs, p.ts));
+  }
+  return e;
 }
 
 static cudaError_t launch_tiles(const unsigned char *img, const ImgLayout &L,
                                 const fx::FxTab &f, const unsigned char *tab, const Batch &b,
-                                int sm_count, int smem_optin, double *scratch, cudaStream_t s) {
+                                int sm_count, int smem_optin, const TileScratch &scratch,
+                                cudaStream_t s) {
   const int64_t tiles = (b.n + 31) / 32;
   const fx::Plan p = fx::plan_of(f, tiles, sm_count, smem_optin);
-  if (!p.ok || (!p.qs && !scratch)) return cudaErrorInvalidValue;
+  if (!p.ok || (!p.qs && !scratch.q)) return cudaErrorInvalidValue;
   int list = 0;
   while (list < fx::NLIST - 1 && fx::list_warps[list] != p.nw * p.cl) ++list;
   const fx::Kernel k = fx::kernel_of(p);
@@ -898,12 +919,12 @@ static cudaError_t launch_tiles(const unsigned char *img, const ImgLayout &L,
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = p.cl > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k, L, f, fx::Args{tab, img, scratch, list}, b);
+  return cudaLaunchKernelEx(&cfg, k, L, f, fx::Args{tab, img, scratch.q, scratch.busy, scratch.slots, list}, b);
 }
 
 cudaError_t launch_wdot_fx(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                            const unsigned char *tab, const Batch &b, int sm_count,
-                           int smem_optin, double *scratch, cudaStream_t s) {
+                           int smem_optin, const TileScratch &scratch, cudaStream_t s) {
   const int64_t tiles = (b.n + 31) / 32, first = first_tiles(f, tiles, sm_count, smem_optin);
   Batch part = b;
   part.n = std::min<int64_t>(b.n, first * 32);

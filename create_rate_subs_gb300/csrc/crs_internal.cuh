@@ -35,6 +35,14 @@ struct Derived {
   std::vector<unsigned char> bytes;
 };
 
+// The state tiles' scratch of a handle: `slots` blocks of a tile's net rates and
+// a word for each that says whether a resident CTA has it (tile::claim_slot).
+struct TileScratch {
+  double *q = nullptr;
+  int *busy = nullptr;
+  int slots = 0;
+};
+
 // Arguments of one batched evaluation (device pointers, SoA with ld).
 struct Batch {
   int64_t n, ld;
@@ -245,6 +253,23 @@ template <class K>
 inline cudaError_t set_smem_limit(K k, size_t bytes) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
+
+// Per-SM resources of the CTAs that may hold a slot of the state tiles' scratch:
+// the least of each.
+struct SlotUse {
+  size_t smem = (size_t)1 << 30;
+  int regs = 1 << 30, threads = 1 << 30;
+  template <class K>
+  cudaError_t add(K k, int block, size_t dynamic) {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) return e;
+    smem = dynamic < smem ? dynamic : smem;
+    regs = a.numRegs * block < regs ? a.numRegs * block : regs;
+    threads = block < threads ? block : threads;
+    return cudaSuccess;
+  }
+};
 #endif
 
 }  // namespace crs

@@ -45,7 +45,8 @@ using namespace fx;
 struct Args {
   const unsigned char *tab;  // fixed-point tables (lists, records)
   const unsigned char *img;  // table image
-  double *q;                 // [gridDim.x / CL][R + 1][32] scratch when QS is false
+  double *q;                 // [slots][R + 1][32] scratch when QS is false
+  int *busy, slots;          // (tile::claim_slot)
   int list;                  // the work list for NW CL warps
   // contraction (PACK): bf16 rows [i][2 Kh] and the states' scale exponents
   __nv_bfloat16 *A;
@@ -477,17 +478,18 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   // (PACK) the warps' exponent sums, a bit per reaction with terms outside
   Scale *scales = reinterpret_cast<Scale *>(next) + threadIdx.x;
   unsigned *outside = reinterpret_cast<unsigned *>(next + NW * 32 * sizeof(Scale));
+  __shared__ int s_slot;
+  if (!QS && blockIdx.x % CL == 0 && threadIdx.x == 96)  // for the CTAs of the tile
+    s_slot = tile::claim_slot(g.busy, g.slots, blockIdx.x / CL, b.status);
   unsigned char *qt = QS && CL > 1 ? static_cast<unsigned char *>(__cluster_map_shared_rank(next, 0))
-                      : QS ? next : reinterpret_cast<unsigned char *>(g.q) +
-                                      (int64_t)(blockIdx.x / CL) * (f.R + 1) * 256;
+                                   : next;  // (scratch: once there is a slot)
   unsigned char *q = qt + lane * 8;
   auto Q = [&](int off) -> double & { return *reinterpret_cast<double *>(q + off); };
   if (warp == 0) {
     int2 *c = reinterpret_cast<int2 *>(smem) + N * 32 + lane;
     c[0] = make_int2(0x3f800000, 0);
     c[32] = make_int2(0, 0);
-    if (!QS || CL == 1) Q(f.R * 256) = 0.0;
-    else reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
+    if (QS) reinterpret_cast<double *>(next)[f.R * 32 + lane] = 0.0;  // before all CTAs run
   }
   const int gw = CL == 1 ? warp : (int)(blockIdx.x % CL) * NW + warp;  // the tile's warp
   const int *lp = reinterpret_cast<const int *>(tab + f.mlist_ptr[g.list]) + gw;
@@ -502,6 +504,14 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   const Tab t = make_tab(g.img, lay);
   if (tile < ntiles && warp < 3)
     prepare(t, b, tile * 32 + lane < b.n ? tile * 32 + lane : tile * 32, warp, lane, blk);
+  if (!QS) {  // (the claim ran beside the first tile's sums)
+    tile_barrier<CL>();
+    const int slot =
+        CL > 1 ? *static_cast<const int *>(__cluster_map_shared_rank(&s_slot, 0)) : s_slot;
+    qt = reinterpret_cast<unsigned char *>(g.q) + (int64_t)slot * (f.R + 1) * 256;
+    q = qt + lane * 8;
+    if (warp == 0) Q(f.R * 256) = 0.0;
+  }
   for (; tile < ntiles; tile += step, bk ^= 1) {
     const int64_t i = tile * 32 + lane;
     const bool valid = i < b.n;
@@ -716,7 +726,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     // rates are replaced only after the barrier at the loop's head
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  if (QS && CL > 1) tile_barrier<CL>();  // the first CTA's rates are read until here
+  if (!QS || CL > 1) tile_barrier<CL>();  // the tile's rates are read until here
+  if (!QS && blockIdx.x % CL == 0 && threadIdx.x == 0)
+    tile::release_slot(g.busy, g.slots, s_slot);
   if (bad && b.status) atomicAdd(&b.status[1], bad);
 }
 
@@ -786,6 +798,11 @@ cudaError_t mixed_tile_init(int smem_optin) {
   return e;
 }
 
+// Whether the contraction's producer takes the mechanism (it needs scratch).
+bool mixed_pack_fits(const fx::FxTab &f, int smem_optin) {
+  return f.mixed && mixt::smem_of(f, mixt::PACK_NW, false, true) <= (size_t)smem_optin;
+}
+
 static int64_t mixed_first(const fx::FxTab &f, int64_t tiles, int sm_count, int smem_optin) {
   const mixt::Plan p = mixt::plan_of(f, tiles, sm_count, smem_optin);
   const int64_t wave = (int64_t)sm_count * p.per_sm;
@@ -794,28 +811,38 @@ static int64_t mixed_first(const fx::FxTab &f, int64_t tiles, int sm_count, int 
                                                                                   : tiles - rest;
 }
 
-long long mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
+int mixed_tile_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
   const int64_t tiles = (n + 31) / 32, first = mixed_first(f, tiles, sm_count, smem_optin);
-  long long most = 0;
+  int need = 0;
   for (int64_t part : {first, tiles - first}) {
     if (part == 0) continue;
     const mixt::Plan p = mixt::plan_of(f, part, sm_count, smem_optin);
     if (!p.ok) return -1;
-    if (p.qs) continue;
-    const long long need = (long long)std::min<int64_t>(part, (int64_t)sm_count * p.per_sm) *
-                           (f.R + 1) * 256;
-    most = std::max(most, need);
+    need |= !p.qs;
   }
-  return most;
+  return need;
+}
+
+// The resources of the launches that need scratch.
+cudaError_t mixed_tile_slots(const fx::FxTab &f, int sm_count, int smem_optin, SlotUse &u) {
+  cudaError_t e = cudaSuccess;
+  for (int64_t tiles : {1, sm_count / 8 + 1, sm_count / 4 + 1, sm_count / 2 + 1, sm_count + 1}) {
+    const mixt::Plan p = mixt::plan_of(f, tiles, sm_count, smem_optin);
+    if (p.ok && !p.qs && e == cudaSuccess)
+      e = u.add(mixt::kernel_of(p), p.nw * 32, mixt::smem_of(f, p.nw, p.qs));
+  }
+  if (e == cudaSuccess && mixed_pack_fits(f, smem_optin))
+    e = u.add(mixt::k_pack, mixt::PACK_NW * 32, mixt::smem_of(f, mixt::PACK_NW, false, true));
+  return e;
 }
 
 static cudaError_t launch_mixed_part(const unsigned char *img, const ImgLayout &L,
                                      const fx::FxTab &f, const unsigned char *tab, const Batch &b,
-                                     int sm_count, int smem_optin, double *scratch,
+                                     int sm_count, int smem_optin, const TileScratch &scratch,
                                      cudaStream_t s) {
   const int64_t tiles = (b.n + 31) / 32;
   const mixt::Plan p = mixt::plan_of(f, tiles, sm_count, smem_optin);
-  if (!p.ok || (!p.qs && !scratch)) return cudaErrorInvalidValue;
+  if (!p.ok || (!p.qs && !scratch.q)) return cudaErrorInvalidValue;
   int list = 0;
   while (list < fx::NLIST - 1 && fx::list_warps[list] != p.nw * p.cl) ++list;
   const mixt::Kernel k = mixt::kernel_of(p);
@@ -832,12 +859,13 @@ static cudaError_t launch_mixed_part(const unsigned char *img, const ImgLayout &
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = p.cl > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k, L, f, mixt::Args{tab, img, scratch, list, nullptr, 0, nullptr}, b);
+  const mixt::Args args{tab, img, scratch.q, scratch.busy, scratch.slots, list, nullptr, 0, nullptr};
+  return cudaLaunchKernelEx(&cfg, k, L, f, args, b);
 }
 
 cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                               const unsigned char *tab, const Batch &b, int sm_count,
-                              int smem_optin, double *scratch, cudaStream_t s) {
+                              int smem_optin, const TileScratch &scratch, cudaStream_t s) {
   const int64_t tiles = (b.n + 31) / 32, first = mixed_first(f, tiles, sm_count, smem_optin);
   Batch part = b;
   part.n = std::min<int64_t>(b.n, first * 32);
@@ -852,25 +880,21 @@ cudaError_t launch_mixed_tile(const unsigned char *img, const ImgLayout &L, cons
   return launch_mixed_part(img, L, f, tab, part, sm_count, smem_optin, scratch, s);
 }
 
-// Scratch bytes of the contraction's producer over n states; < 0: the
-// mechanism does not fit.
-long long mixed_pack_scratch(const fx::FxTab &f, int64_t n, int sm_count, int smem_optin) {
-  if (!f.mixed || mixt::smem_of(f, mixt::PACK_NW, false, true) > (size_t)smem_optin) return -1;
-  return (long long)std::min<int64_t>((n + 31) / 32, sm_count) * (f.R + 1) * 256;
-}
-
 // A: rows of 2 Kh (a multiple of 64), 32-byte aligned.
 cudaError_t launch_mixed_pack(const unsigned char *img, const ImgLayout &L, const fx::FxTab &f,
                               const unsigned char *tab, const Batch &b, int sm_count,
-                              int smem_optin, double *scratch, void *A, int Kh, int *escale,
-                              cudaStream_t s) {
-  if (mixed_pack_scratch(f, b.n, sm_count, smem_optin) < 0 || Kh % 64 || Kh < f.R)
+                              int smem_optin, const TileScratch &scratch, void *A, int Kh,
+                              int *escale, cudaStream_t s) {
+  if (!mixed_pack_fits(f, smem_optin) || !scratch.q || Kh % 64 || Kh < f.R)
     return cudaErrorInvalidValue;
   int list = 0;
   while (list < fx::NLIST - 1 && fx::list_warps[list] != mixt::PACK_NW) ++list;
   mixt::k_pack<<<(unsigned)std::min<int64_t>((b.n + 31) / 32, sm_count), mixt::PACK_NW * 32,
                  mixt::smem_of(f, mixt::PACK_NW, false, true), s>>>(
-      L, f, mixt::Args{tab, img, scratch, list, static_cast<__nv_bfloat16 *>(A), Kh, escale}, b);
+      L, f,
+      mixt::Args{tab, img, scratch.q, scratch.busy, scratch.slots, list,
+                 static_cast<__nv_bfloat16 *>(A), Kh, escale},
+      b);
   return cudaGetLastError();
 }
 

@@ -62,6 +62,29 @@ __device__ __forceinline__ void tiles_done(unsigned long long *sched) {
   }
 }
 
+// A slot of the scratch that all launches on a handle share, for a resident
+// CTA (or cluster): `busy` has a word per slot, and as many slots as CTAs can be
+// resident on the device at a time, so that one is always free, whatever the
+// streams, graphs and copies of graphs that run.  A launch by itself finds slot
+// `first` at once.  One thread calls it.  None found (not expected): a spare
+// block, which other such CTAs may have too, and the status says so.
+__device__ __noinline__ inline int claim_slot(int *busy, int slots, int first, int32_t *status) {
+  for (int k = 0; k < 64 * slots; ++k) {
+    const int at = (first + k) % slots;
+    if (atomicCAS(busy + at, 0, 1) == 0) {
+      __threadfence();
+      return at;
+    }
+  }
+  if (status) atomicOr(&status[0], STATUS_STAGE_TIMEOUT);
+  return slots;
+}
+// (after the CTA's, or the cluster's, last access)
+__device__ __noinline__ inline void release_slot(int *busy, int slots, int slot) {
+  __threadfence();
+  if (slot < slots) atomicExch(busy + slot, 0);
+}
+
 // Scale exponent of state (lane) from the warps' partial exponent sums and
 // counts: the nearest integer to sum / count, by integer arithmetic.
 __device__ __forceinline__ int scale_exponent(int es, int ec) {

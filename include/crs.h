@@ -53,10 +53,10 @@ typedef struct crs_mech crs_mech;
 #define CRS_MODE_MIXED 2       /* FP32 bulk, float-float exponents, FP64 net rate/sum */
 /* CRS_MODE_FP64 and CRS_MODE_MIXED evaluate tiles of 32 states (the warps of
  * a CTA, or of a cluster when tiles are few, split the reactions).  Net rates
- * that do not fit on chip take scratch (one tile's per resident CTA: 38 MB at
- * 53/325, 99 MB at 561/2539), owned by the handle and allocated on first use:
- * calls that need it take turns on the GPU, whatever their streams.  A call
- * captured into a graph, be it the first, has its own as a node of the graph.
+ * that do not fit on chip take scratch (a tile's for each CTA that can be
+ * resident: 38 MB at 53/325, 99 MB at 561/2539), owned by the handle and
+ * allocated on first use.  A CTA takes a block while it runs, so that calls on
+ * any streams, from any threads and in any graphs run side by side.
  * Calls for intermediates and mechanisms outside the tiles' scheme take the
  * layouts below.
  *
