@@ -795,7 +795,7 @@ cudaError_t launch_wdot_fp64_tps(const unsigned char *img, const ImgLayout &L,
   if (kcm == 0) k = stages ? fast::k_wdot<true, 0> : fast::k_wdot<false, 0>;
   else if (kcm == 1) k = stages ? fast::k_wdot<true, 1> : fast::k_wdot<false, 1>;
   else k = stages ? fast::k_wdot<true, 2> : fast::k_wdot<false, 2>;
-  const cudaError_t e = set_smem_limit(k, bytes);
+  const cudaError_t e = raise_smem_limit(k);
   if (e != cudaSuccess) return e;
   k<<<grid_for(b.n, block, sm_count), block, bytes, s>>>(img, L, b);
   return cudaGetLastError();
@@ -809,7 +809,7 @@ cudaError_t launch_rates_tile64(const unsigned char *img, const ImgLayout &L, co
   const size_t bytes = (size_t)L.N * 32 * sizeof(double);
   if (bytes > (size_t)smem_optin || !b.sched) return cudaErrorNotSupported;
   auto k = L.kc_single ? fast::k_rates_tile64<true> : fast::k_rates_tile64<false>;
-  cudaError_t e = set_smem_limit(k, bytes);
+  cudaError_t e = raise_smem_limit(k);
   if (e != cudaSuccess) return e;
   int per_sm = 1;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, fast::FTW * 32, bytes);
@@ -840,7 +840,7 @@ cudaError_t launch_wdot_fp64(const unsigned char *img, const ImgLayout &L,
   const size_t bytes = (smem_tab ? tab : 0) + nw * pw;
   auto k = smem_tab ? (stages ? fast::k_wdot_warp<true, true> : fast::k_wdot_warp<false, true>)
                     : (stages ? fast::k_wdot_warp<true, false> : fast::k_wdot_warp<false, false>);
-  cudaError_t e = set_smem_limit(k, bytes);
+  cudaError_t e = raise_smem_limit(k);
   if (e != cudaSuccess) return e;
   int per_sm = 1;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nw * 32, bytes);

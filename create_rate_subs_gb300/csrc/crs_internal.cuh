@@ -247,11 +247,24 @@ struct KcPolyG {
 int report(int code, const char *msg);
 
 #ifdef __CUDACC__
-// Raise kernel k's dynamic shared-memory limit to `bytes`.  Every launcher
-// returns this error instead of launching when the limit was not applied.
+// Sets kernel k's dynamic shared-memory limit to `bytes`.  Every launcher
+// returns this error instead of launching when the limit was not applied.  All
+// threads share the limit: only for a size that is the same on every call.
 template <class K>
 inline cudaError_t set_smem_limit(K k, size_t bytes) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+// Raises it to what the device has beside the kernel's static part, so that no
+// call takes from another what that one has just set.
+template <class K>
+inline cudaError_t raise_smem_limit(K k) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k);
+  return e == cudaSuccess ? set_smem_limit(k, (size_t)most - a.sharedSizeBytes) : e;
 }
 
 // Per-SM resources of the CTAs that may hold a slot of the state tiles' scratch:

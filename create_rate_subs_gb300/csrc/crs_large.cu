@@ -248,7 +248,7 @@ cudaError_t launch_rates_tile(const unsigned char *img, const ImgLayout &L, cons
   const size_t bytes = large_rates_smem(L);
   if (bytes > (size_t)smem_optin || !b.sched) return cudaErrorNotSupported;
   auto k = L.kc_single ? large::k_rates_tile<true> : large::k_rates_tile<false>;
-  cudaError_t e = set_smem_limit(k, bytes);
+  cudaError_t e = raise_smem_limit(k);
   if (e != cudaSuccess) return e;
   int per_sm = 1;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, large::TW * 32, bytes);

@@ -343,7 +343,7 @@ cudaError_t launch_wdot_mixed_tps(const unsigned char *img, const ImgLayout &L,
   // the compact nu lists must be exact (else the warp kernel runs)
   if (block < 32 || !L.nu_hi_exact) return cudaErrorNotSupported;
   const size_t bytes = tab + per * block;
-  const cudaError_t e = set_smem_limit(k, bytes);
+  const cudaError_t e = raise_smem_limit(k);
   if (e != cudaSuccess) return e;
   k<<<grid_for(b.n, block, sm_count), block, bytes, s>>>(img, L, b);
   return cudaGetLastError();
@@ -375,7 +375,7 @@ cudaError_t launch_wdot_mixed_q(const unsigned char *img, const ImgLayout &L,
                                      : mixed::k_wdot_warp<false, true, false>)
                            : (stages ? mixed::k_wdot_warp<true, false, false>
                                      : mixed::k_wdot_warp<false, false, false>);
-  cudaError_t e = set_smem_limit(k, bytes);
+  cudaError_t e = raise_smem_limit(k);
   if (e != cudaSuccess) return e;
   int per_sm = 1;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nw * 32, bytes);

@@ -583,17 +583,6 @@ inline int grid1(int64_t n, int per = 256) {
   return (int)(g < 1 ? 1 : g);
 }
 
-// Kernel k's dynamic shared-memory limit, which all threads share: always the
-// device's, so that no call takes from another what that one has just set.
-template <class K>
-cudaError_t raise_smem_limit(K k) {
-  int dev = 0, most = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return e == cudaSuccess ? set_smem_limit(k, (size_t)most) : e;
-}
-
 template <class Epi>
 cudaError_t gemm_bn(const CUtensorMap &ta, const CUtensorMap &tb, int64_t M_pad, int64_t N_pad,
                     int64_t K, int bn, const Epi &epi, cudaStream_t s, int splits = 1) {
@@ -808,7 +797,7 @@ int crs_surrogate_output2(int64_t n, const float *Ya, const float *Yb, int64_t l
                     (fit >= 16 || n <= (int64_t)sms * nw * 32);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows) {
-    e = mlp::raise_smem_limit(mlp::k_output2<true>);
+    e = raise_smem_limit(mlp::k_output2<true>);
     if (e != cudaSuccess) return done(e, __func__);
     mlp::k_output2<true><<<mlp::grid1(n, nw * 32), nw * 32, nw * per_warp, s>>>(
         n, Ya, Yb, ldy, nsp, scale_m, scale_e, cons, nelem, tol, dweight, est, lde, stol,
