@@ -580,9 +580,10 @@ void build(const Tab &t, FxTab &f, std::vector<unsigned char> &out, int64_t limi
       add(v.data(), v.size() * sizeof(double));
     }
   }
-  // a reaction in FP64 costs this kernel about four times what it costs the
-  // kernels that evaluate every reaction so; beyond a fifth of such
-  // reactions those are faster
+  // General reactions gain nothing here.  131,072 states of 53/325 with PLOG in 5,
+  // 10, 15 and 19% of the reactions: 2.39, 3.68, 5.22 and 6.40 ms, by the kernels
+  // that evaluate every reaction in FP64 5.73, 7.17, 8.73 and 9.91; more was not
+  // measured and goes to those
   f.usable = generic * 5 <= R;
   for (int k = 0; k < N; ++k) f.usable &= std::fabs(std::log2(t.inv_mw[k])) <= W_MAX;
   Buf b;
