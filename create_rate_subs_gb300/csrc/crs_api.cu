@@ -1276,11 +1276,16 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
     if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host buffers");
     mm->host_chunk = most;
   }
-  // the first copy in and the last copy out stand alone (200,003 states:
+  // The first copy in and the last copy out stand alone (200,003 states:
   // chunks of 32,768 1.43 ms, of 65,536 1.52, of 16,384 2.16; 2^20: of 65,536
-  // 7.16 ms, of 32,768 7.22, of 131,072 7.42)
+  // 7.16 ms, of 32,768 7.22, of 131,072 7.42); but pageable arrays are copied by
+  // this thread, and the short kernels of small mechanisms hide none of it
+  // (CRS_MODE_MIXED, 10/27, 2^18 states: one chunk of 131,072 0.73 ms, of 32,768
+  // 0.89)
   int64_t chunk = std::max<int64_t>((n / 16 + 127) / 128 * 128, 32768);
-  if (chunk > most) chunk = most;
+  if (chunk > most || (m->L.R < 100 && !(mapped_view(T) && mapped_view(P) && mapped_view(Y) &&
+                                         mapped_view(wdot))))
+    chunk = most;
   for (int j = 0; j < 2 && e == cudaSuccess; ++j)
     if (!mm->hs[j]) e = cudaStreamCreateWithFlags(&mm->hs[j], cudaStreamNonBlocking);
   if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host streams");
