@@ -156,6 +156,7 @@ struct crs_mech {
   // states each (T, P, Y, wdot), allocated on first use
   std::mutex host_mu;
   cudaStream_t hs[2] = {nullptr, nullptr};
+  cudaEvent_t host_done = nullptr;  // after a chunk's kernels
   double *d_host = nullptr;
   int64_t host_chunk = 0;
 };
@@ -1023,6 +1024,7 @@ int crs_mech_free(crs_mech *m) {
   if (m->d_host) cudaFree(m->d_host);
   for (cudaStream_t st : m->hs)
     if (st) cudaStreamDestroy(st);
+  if (m->host_done) cudaEventDestroy(m->host_done);
   crs::host::free_aux(m->haux);
   delete m;
   return CRS_OK;
@@ -1229,13 +1231,13 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
   if (!mm->hs[0]) e = cudaStreamCreateWithFlags(&mm->hs[0], cudaStreamNonBlocking);
   if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host streams");
   const int64_t per = 2 + (N - 1) + N;  // doubles per state: T, P, Y, wdot
-  // The state tiles read mass fractions three times: from 2^17 states on
-  // chunked copies, each over the link once, are faster than reading in place
-  // (CRS_MODE_FP64, 53/325: 131,072 states 1.04 against 1.19 ms, 200,003 1.50
-  // against 2.22, 2^20 7.2 against 9.5; 561/2539, 131,072: 11.4 against 15.3;
-  // below, the copies' latency counts: 4,000 states of 53/325 0.10 against
-  // 0.07), but not the short rows of small mechanisms (10/27, 2^20: 1.09
-  // against 0.85)
+  // The state tiles read mass fractions three times: chunked copies, each over
+  // the link once, are faster than reading in place for all mechanisms from 2^17
+  // states on (in place and by copies, ms: 53/325 FP64 32,768 states 0.35 and
+  // 0.39, 65,536 0.64 and 0.61, 131,071 1.47 and 1.05; mixed 65,536 0.53 and 0.57,
+  // 98,304 0.75 and 0.77, 131,071 1.10 and 0.97; 561/2539 FP64 8,192 1.13 and
+  // 0.97, mixed 32,768 2.7 and 3.0, 65,536 5.4 and 4.7), but not the short rows of
+  // small mechanisms (10/27, 2^20: 0.85 and 1.27)
   const bool copies = n >= ((int64_t)1 << 17) && m->L.R >= 100 &&
                       ((mode == CRS_MODE_FP64 && m->fx.usable) ||
                        (mode == CRS_MODE_MIXED && m->fx.mixed));
@@ -1277,8 +1279,8 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
     mm->host_chunk = most;
   }
   // The first copy in and the last copy out stand alone (200,003 states:
-  // chunks of 32,768 1.43 ms, of 65,536 1.52, of 16,384 2.16; 2^20: of 65,536
-  // 7.16 ms, of 32,768 7.22, of 131,072 7.42); but pageable arrays are copied by
+  // chunks of 32,768 1.50 ms, of 65,536 1.52, of 16,384 2.16; 2^20: of 65,536
+  // 6.93 ms, of 32,768 7.22, of 131,072 7.42); but pageable arrays are copied by
   // this thread, and the short kernels of small mechanisms hide none of it
   // (CRS_MODE_MIXED, 10/27, 2^18 states: one chunk of 131,072 0.73 ms, of 32,768
   // 0.89)
@@ -1288,10 +1290,14 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
     chunk = most;
   for (int j = 0; j < 2 && e == cudaSuccess; ++j)
     if (!mm->hs[j]) e = cudaStreamCreateWithFlags(&mm->hs[j], cudaStreamNonBlocking);
+  if (e == cudaSuccess && !mm->host_done)
+    e = cudaEventCreateWithFlags(&mm->host_done, cudaEventDisableTiming);
   if (e != cudaSuccess) return cuda_fail(e, "crs_wdot_host streams");
   // chunk c on stream c % 2: its copies in overlap the other stream's
   // kernel, its copies out the next kernel; a buffer is reused only after
-  // the same stream has finished with it
+  // the same stream has finished with it.  The kernels take turns: side by side
+  // both end late, and the copies out with them (200,003 states of 53/325 2.16 ms,
+  // in turns 1.50)
   int result = CRS_OK;
   for (int64_t c0 = 0, c = 0; c0 < n && result == CRS_OK; c0 += chunk, ++c) {
     const int64_t cn = n - c0 < chunk ? n - c0 : chunk;
@@ -1310,8 +1316,16 @@ int crs_wdot_host(const crs_mech *m, int64_t n, const double *T, const double *P
     }
     crs::Batch b = make_batch(m, cn, cn);
     b.T = dT; b.P = dP; b.Y = dY; b.wdot = dW;
-    result = launch_mode(m, b, mode, s);
-    if (result != CRS_OK) break;
+    if (c > 0) e = cudaStreamWaitEvent(s, mm->host_done, 0);
+    if (e == cudaSuccess) {
+      result = launch_mode(m, b, mode, s);
+      if (result != CRS_OK) break;
+      e = cudaEventRecord(mm->host_done, s);
+    }
+    if (e != cudaSuccess) {
+      result = cuda_fail(e, "crs_wdot_host order");
+      break;
+    }
     e = cudaMemcpy2DAsync(wdot + c0, (size_t)ld * sizeof(double), dW, row, row, N,
                           cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) result = cuda_fail(e, "crs_wdot_host copy out");
