@@ -496,7 +496,6 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   const Ring<D> recs{tab + f.mrec[g.list] + (int64_t)lp[0] * MPAIR, smem_u32(ring), MPAIR,
                      lp[1] - lp[0], lane};
   const int npairs = reinterpret_cast<const int *>(tab + f.mpairs[g.list])[gw];
-  Sums sums(f, tab, g.list, gw);
   int bad = 0, bk = 0;
   int64_t tile = blockIdx.x / CL;
   const int64_t step = gridDim.x / CL;
@@ -506,12 +505,15 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
     prepare(t, b, tile * 32 + lane < b.n ? tile * 32 + lane : tile * 32, warp, lane, blk);
   if (!QS) {  // (the claim ran beside the first tile's sums)
     tile_barrier<CL>();
-    const int slot =
-        CL > 1 ? *static_cast<const int *>(__cluster_map_shared_rank(&s_slot, 0)) : s_slot;
+    int slot = CL > 1 ? *static_cast<const int *>(__cluster_map_shared_rank(&s_slot, 0)) : s_slot;
+    // the same for the whole warp, and known to be (see Sums::run: 2^18 states of
+    // 53/325 1.39 -> 1.35 ms)
+    if (!PACK) slot = __shfl_sync(0xffffffffu, slot, 0);
     qt = reinterpret_cast<unsigned char *>(g.q) + (int64_t)slot * (f.R + 1) * 256;
     q = qt + lane * 8;
     if (warp == 0) Q(f.R * 256) = 0.0;
   }
+  Sums sums(f, tab, g.list, gw);
   for (; tile < ntiles; tile += step, bk ^= 1) {
     const int64_t i = tile * 32 + lane;
     const bool valid = i < b.n;
