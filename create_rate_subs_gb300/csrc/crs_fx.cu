@@ -33,9 +33,9 @@
 // two warps beside the rates.
 //
 // Measured on GB300 (before: one state per thread, 561/2539 in two passes):
-// 2^20 states of 53/325 31.2 -> 6.41 ms, 97 states 716 -> 21.6 us, 20,011
-// states of 561/2539 4.87 -> 1.64 ms; FP64 pipe 53%, integer multiply pipe
-// 43% busy.
+// 2^20 states of 53/325 31.2 -> 6.43 ms, 97 states 716 -> 21.9 us, 20,011
+// states of 561/2539 4.87 -> 1.31 ms; FP64 pipe 58%, integer multiply pipe
+// 51% busy.
 //
 // States outside the scheme (T outside (200, 6000] K, a density beyond 2^+-60, a
 // mean 1/W out of range, |Y| >= 2, a subnormal Y) and reactions outside it (non-
@@ -458,10 +458,10 @@ __global__ void __launch_bounds__(NW * 32, PER_SM)
   // How rates are left to the general arithmetic.  SPREAD: the lanes may share
   // them (see there), with the lists on chip to have the registers.  OUTS: whole
   // tiles outside the scheme go there at once, and such states' concentrations are
-  // on chip.  Both cost the loops registers: with 24 warps none is missed (65,536
-  // states of 561/2539 3.68 ms either way; one state in 97 outside, 8,192 states:
-  // 2.85 -> 0.81 ms), with 8 OUTS takes 1% (2^18 states of 53/325 1.61 -> 1.63 ms;
-  // all outside: 10.1 -> 7.9) and SPREAD 4%, and with 16, for few tiles, where
+  // on chip.  Both cost the loops registers.  With 24 warps none is missed (8,192
+  // states of 561/2539, all outside: 2.84 -> 2.23 ms, one in 97: 2.85 -> 0.80);
+  // with 8 OUTS took 1% and SPREAD 4% (2^18 states of 53/325, all outside: 10.1 ->
+  // 7.86 ms with OUTS, one in 97: 4.9 -> 4.3); with 16, for few tiles, where
   // latency counts, both would take 4% (4,000 states 45.3 -> 47.2 us).
   constexpr bool SPREAD = NW == 24, OUTS = NW != 16;
   int *chip = reinterpret_cast<int *>(next) + warp * 8;
