@@ -937,6 +937,13 @@ int crs_mech_load(const void *blob, size_t nbytes, crs_mech **out) {
       return r;
     }
   }
+  // the counters are zero before any stream's launch, non-blocking ones included
+  e = cudaStreamSynchronize(nullptr);
+  if (e != cudaSuccess) {
+    int r = cuda_fail(e, "crs_mech_load");
+    crs_mech_free(m);
+    return r;
+  }
   *out = m;
   return CRS_OK;
 }

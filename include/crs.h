@@ -107,7 +107,8 @@ int crs_mech_dims(const crs_mech *mech, int64_t out[5]);
 const char *crs_last_error(void);
 /* Non-finite outputs and device-wait timeouts recorded since the last
  * crs_status_reset on this handle: out[0] = flag bits (1 = table staging
- * timed out, 2 = a tensor-core GEMM wait timed out), out[1] = count of
+ * timed out, or no block of scratch was free, 2 = a tensor-core GEMM wait
+ * timed out), out[1] = count of
  * non-finite wdot values.  Synchronises
  * `stream`. */
 int crs_status(const crs_mech *mech, void *stream, int32_t out[2]);
