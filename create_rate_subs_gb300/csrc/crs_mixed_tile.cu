@@ -19,11 +19,11 @@
 // concentrations are kept as mantissa and exponent, the reverse exponent has
 // its own coefficients, and the clamps of an exponential and of a double's
 // range are one test of its exponent, behind which the general code stands.
-// That took the warp instructions per state from 4,602 to 3,801 and the time
-// from 23.7 to 21.0 ms; the FP64 pipe is 65% busy, the schedulers 60%.
+// That took the warp instructions per state from 4,602 to 3,857 and the time
+// from 23.7 to 20.9 ms; the FP64 pipe is 65% busy, the schedulers 61%.
 //
 // Measured on GB300 (before: one state per thread, large mechanisms in two
-// passes): 2^22 states of 53/325 35.6 -> 21.0 ms, 65,536 of 561/2539 5.32 ->
+// passes): 2^22 states of 53/325 35.6 -> 20.9 ms, 65,536 of 561/2539 5.32 ->
 // 3.17 ms.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
